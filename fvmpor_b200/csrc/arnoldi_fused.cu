@@ -620,11 +620,11 @@ bool fused_prepare(fvm_ctx* c, int m) {
         P->op_self.upload(self, s);
         P->op_src.upload(opsrc, s);
         {
-            // the slice position of every Jacobian entry, for fd_gather
+            // the slice position of every Jacobian entry, for the set-up
             std::vector<int> opdst(P->nnz, 0);
             for (size_t e = 0; e < opsrc.size(); ++e)
                 if (opsrc[e] >= 0) opdst[opsrc[e]] = (int)e;
-            P->op_dst.upload(opdst, s);
+            fd_set_op_places(c, opdst);
         }
         P->halo_ptr.upload(halo_ptr, s);
         P->halo_node.upload(halo_node, s);
@@ -677,12 +677,11 @@ bool fused_prepare(fvm_ctx* c, int m) {
     }
     if (!P->fused_ok || !P->fused_var_ok[fused_variant(c)]) return false;
     if (P->op_setup_id != P->setup_id) {
-        // the values come from fd_gather once the layout exists; the first
-        // set-up after the layout was built copies them here
-        const long ne = P->op_vals_setup == P->setup_id ? 0 : (long)P->op_val.n;
-        const long nt = std::max(ne, (long)c->N);
-        fvm_launch(c, k_op_refresh, grid_for(nt, 256), 256, 0, s, ne, P->op_src.p, P->J.p, P->op_val.p, c->N,
-                   P->lu_row.p, P->ahhp.p, c->ntype.p, P->op_dg.p);
+        // the values come from the set-up's kernels once the layout exists;
+        // the first set-up after the layout was built copies them here
+        const long nt = std::max((long)P->op_val.n, (long)c->N);
+        fvm_launch(c, k_op_refresh, grid_for(nt, 256), 256, 0, s, (long)P->op_val.n, P->op_src.p, P->J.p, P->op_val.p,
+                   c->N, P->lu_row.p, P->ahhp.p, c->ntype.p, P->op_dg.p);
         P->op_setup_id = P->setup_id;
     }
     return true;

@@ -180,13 +180,6 @@ struct StageLayout {
     }
 };
 
-__device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                     tc05::smem_u32(dst)),
-                 "l"(src), "r"(bytes), "r"(tc05::smem_u32(bar))
-                 : "memory");
-}
-
 template <int NPE, bool VAR1, bool MZ>
 __device__ __forceinline__ void elem_issue(const ElemArgs& a, const StageLayout& L, unsigned char* st,
                                            int4* meta, uint64_t* bar, int c) {
@@ -199,19 +192,19 @@ __device__ __forceinline__ void elem_issue(const ElemArgs& a, const StageLayout&
                      (VAR1 ? (uint32_t)nep * 8 * (a.kiso ? 1 : 3) : 0) + (uint32_t)nep * NPE * 2 + (uint32_t)nnp * 2;
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(tc05::smem_u32(bar)), "r"(bytes)
                  : "memory");
-    if (MZ) bulk_g2s(st + L.h, a.ch_h + sg.x, nnp * 8, bar);
-    else bulk_g2s(st + L.h, a.ch_hk + 2 * (size_t)sg.x, nnp * 16, bar);
+    if (MZ) tc05::bulk_g2s(st + L.h, a.ch_h + sg.x, nnp * 8, bar);
+    else tc05::bulk_g2s(st + L.h, a.ch_hk + 2 * (size_t)sg.x, nnp * 16, bar);
     if (VAR1)
-        for (int d = 0; d < 3; ++d) bulk_g2s(st + L.xyz + (size_t)d * a.nnmax * 8, a.ch_xyz + d * a.P + sg.x, nnp * 8, bar);
-    bulk_g2s(st + L.eloc, a.elocal + e0, nep * 8, bar);
-    bulk_g2s(st + L.upw, a.upw + (size_t)8 * e0, nep * 8, bar);
+        for (int d = 0; d < 3; ++d) tc05::bulk_g2s(st + L.xyz + (size_t)d * a.nnmax * 8, a.ch_xyz + d * a.P + sg.x, nnp * 8, bar);
+    tc05::bulk_g2s(st + L.eloc, a.elocal + e0, nep * 8, bar);
+    tc05::bulk_g2s(st + L.upw, a.upw + (size_t)8 * e0, nep * 8, bar);
     if (VAR1) {
         const int nk = a.kiso ? 1 : 3;
         for (int d = 0; d < nk; ++d)
-            bulk_g2s(st + L.ek + (size_t)d * a.CE * 8, a.eK + (size_t)d * a.estride + e0, nep * 8, bar);
+            tc05::bulk_g2s(st + L.ek + (size_t)d * a.CE * 8, a.eK + (size_t)d * a.estride + e0, nep * 8, bar);
     }
-    bulk_g2s(st + L.lc, a.ch_lc + (size_t)e0 * NPE, nep * NPE * 2, bar);
-    bulk_g2s(st + L.lp, a.ch_lptr + sg.x, nnp * 2, bar);
+    tc05::bulk_g2s(st + L.lc, a.ch_lc + (size_t)e0 * NPE, nep * NPE * 2, bar);
+    tc05::bulk_g2s(st + L.lp, a.ch_lptr + sg.x, nnp * 2, bar);
 }
 
 template <int NPE, int NFE, int VAR, bool MZ, int EPT>

@@ -159,12 +159,31 @@ FVM_HD void tet_face_fluxes(const double* x0, const double* x1, const double* x2
 // 24 and grad N_k = cof_k / det (cof_1..3 = A, B, C, cof_0 = -(A + B + C)), so
 //   C[f][k] = -s_f P_f . (K o cof_k) / (24 |det|),
 //   G[f]    = -s_f sign(det) K_z P_fz / 24,
-// each column k the combinations of (A, B, C) . (K o cof_k), nine products of
-// the symmetric K-weighted Gram matrix of the cofactor rows (six distinct).
-// No square roots and no orientation tests; for kernels that need the
-// coefficients themselves (the finite-difference Jacobian).
-FVM_HD void tet_coefficients_fast(const double* x0, const double* x1, const double* x2, const double* x3,
-                                  double Kx, double Ky, double Kz, double Cf[6][4], double G[6]) {
+// each column k the face combinations of (A, B, C) . (K o cof_k): six distinct
+// products of the K-weighted Gram matrix of the cofactor rows give all 24
+// coefficients, formed a column at a time.  No square roots and no
+// orientation tests; for the finite-difference Jacobian, which needs the
+// coefficients themselves.
+struct TetGram {
+    double aa, ab, ac, bb, bc, cc;   // the Gram matrix over -24 |det|
+    double ga, gb, gc;               // -sign(det) K_z / 24 times the rows' z
+    // sum_k C[f][k] h_k + G[f] (every row of C sums to zero)
+    FVM_HD void fluxes(double h0, double h1, double h2, double h3, double q[6]) const {
+        const double d1 = h1 - h0, d2 = h2 - h0, d3 = h3 - h0;
+        tet_face_combine(aa * d1 + ab * d2 + ac * d3 + ga, ab * d1 + bb * d2 + bc * d3 + gb,
+                         ac * d1 + bc * d2 + cc * d3 + gc, q);
+    }
+    // C[.][k]
+    FVM_HD void column(int k, double c[6]) const {
+        if (k == 0) tet_face_combine(-(aa + ab + ac), -(ab + bb + bc), -(ac + bc + cc), c);
+        else if (k == 1) tet_face_combine(aa, ab, ac, c);
+        else if (k == 2) tet_face_combine(ab, bb, bc, c);
+        else tet_face_combine(ac, bc, cc, c);
+    }
+};
+
+FVM_HD TetGram tet_gram(const double* x0, const double* x1, const double* x2, const double* x3, double Kx, double Ky,
+                        double Kz) {
     double A[3], B[3], C[3], det;
     tet_cofactors(x0, x1, x2, x3, A, B, C, det);
     const double r24 = -1.0 / (24.0 * (det > 0.0 ? det : -det));
@@ -172,24 +191,17 @@ FVM_HD void tet_coefficients_fast(const double* x0, const double* x1, const doub
     const double kx = Kx * r24, ky = Ky * r24, kz = Kz * r24;
     const double KA[3] = {kx * A[0], ky * A[1], kz * A[2]};
     const double KB[3] = {kx * B[0], ky * B[1], kz * B[2]};
-    const double KC[3] = {kx * C[0], ky * C[1], kz * C[2]};
-    const double aa = KA[0] * A[0] + KA[1] * A[1] + KA[2] * A[2];
-    const double ab = KA[0] * B[0] + KA[1] * B[1] + KA[2] * B[2];
-    const double ac = KA[0] * C[0] + KA[1] * C[1] + KA[2] * C[2];
-    const double bb = KB[0] * B[0] + KB[1] * B[1] + KB[2] * B[2];
-    const double bc = KB[0] * C[0] + KB[1] * C[1] + KB[2] * C[2];
-    const double cc = KC[0] * C[0] + KC[1] * C[1] + KC[2] * C[2];
-    double c1[6], c2[6], c3[6];
-    tet_face_combine(aa, ab, ac, c1);
-    tet_face_combine(ab, bb, bc, c2);
-    tet_face_combine(ac, bc, cc, c3);
-    tet_face_combine(g24 * A[2], g24 * B[2], g24 * C[2], G);
-    for (int f = 0; f < 6; ++f) {
-        Cf[f][0] = -(c1[f] + c2[f] + c3[f]);
-        Cf[f][1] = c1[f];
-        Cf[f][2] = c2[f];
-        Cf[f][3] = c3[f];
-    }
+    TetGram g;
+    g.aa = KA[0] * A[0] + KA[1] * A[1] + KA[2] * A[2];
+    g.ab = KA[0] * B[0] + KA[1] * B[1] + KA[2] * B[2];
+    g.ac = KA[0] * C[0] + KA[1] * C[1] + KA[2] * C[2];
+    g.bb = KB[0] * B[0] + KB[1] * B[1] + KB[2] * B[2];
+    g.bc = KB[0] * C[0] + KB[1] * C[1] + KB[2] * C[2];
+    g.cc = kx * C[0] * C[0] + ky * C[1] * C[1] + kz * C[2] * C[2];
+    g.ga = g24 * A[2];
+    g.gb = g24 * B[2];
+    g.gc = g24 * C[2];
+    return g;
 }
 
 FVM_HD bool tri_coefficients(const double* x0, const double* x1, const double* x2, double Kx,

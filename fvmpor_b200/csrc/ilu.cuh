@@ -15,14 +15,20 @@ struct BlockILU {
     bool built = false;
     int nnz = 0, ncol = 0;
     std::vector<int> h_rowptr, h_col, h_colour;
-    DevBuf<int> rowof, col;
+    DevBuf<int> col;
     DevBuf<double> J;
-    DevBuf<double> shift;
-    // element-wise finite-difference Jacobian
-    DevBuf<int> fd_epos;      // [T*npe*npe] slot of (element, perturbed node, corner)
-    DevBuf<int> fd_jptr;      // [nnz+1] slots of each nonzero
-    DevBuf<double> fd_slots;  // [T*npe*npe]
-    DevBuf<double> krwb, krwp, dstor;
+    // element-wise finite-difference Jacobian: chunks of consecutive elements
+    // (the tables of FdTables, precond.cu)
+    DevBuf<int> fd_cnode_ptr, fd_cnode, fd_done_ptr, fd_share_ptr, fd_share, fd_sptr;
+    DevBuf<int2> fd_list_at;
+    DevBuf<int4> fd_done, fd_shared;
+    DevBuf<ushort4> fd_cloc;
+    DevBuf<unsigned short> fd_list;
+    DevBuf<double> fd_part;
+    int fd_nnmax = 0, fd_list_max = 0, fd_grp_max = 0;
+    DevBuf<int> lu_pos;       // [N] factor position of each node (inverse of lu_row)
+    DevBuf<double> fd_g, fd_dg, fd_gq;   // [nz][N] rho0 krw, its change over the shift, their quotient
+    DevBuf<double> fd_scale, fd_diag;    // [N] row scale, diagonal subtrahend
     // assembled-operator Krylov products (fvm_opts.krylov_operator = 1):
     // device row pointers of J, the storage coefficient ahh(h + d) behind
     // the cj term of J's diagonal, and the cj of the current set-up
@@ -38,8 +44,6 @@ struct BlockILU {
     bool op_built = false, fused_ok = false;
     long op_setup_id = -1;
     DevBuf<int> op_slptr, op_blksl, op_src;
-    DevBuf<int> op_dst;                        // [nnz] slice position of each Jacobian entry
-    long op_vals_setup = -1;                   // set-up whose values fd_gather wrote into op_val
     DevBuf<unsigned short> op_lcol, op_self;   // 16-bit columns into each block's node list
     DevBuf<int> halo_ptr, halo_node;           // each block's node list: its rows and halo
     DevBuf<int> nbr_ptr, nbr;                  // blocks whose rows a block's operator reads
@@ -50,8 +54,8 @@ struct BlockILU {
     int fused_threads = 0, fused_nrmax = 0, fused_nhmax = 0, fused_nqp = 0;
     int nb = 0, maxb = 0;
     DevBuf<int> bstart, lu_ptr, lu_src, lu_diag;
-    DevBuf<int> lu_dst;       // [nnz] factor position of each Jacobian entry, -1 off the blocks
-    DevBuf<double> Jw;        // the set-up's Jacobian in factor order (written by fd_gather)
+    DevBuf<double> Jw;        // the set-up's Jacobian in factor order, FP64 or (FP32 factor)
+                              // FP32 in the first half (written by the quotient kernels)
     DevBuf<int> lu_row;       // global row of each factor position (colour order inside the blocks)
     // ILU(0) elimination schedule of the shared-memory factorisation, one
     // contiguous segment per level (upd[seg_ptr[g] .. seg_ptr[g+1]) for the

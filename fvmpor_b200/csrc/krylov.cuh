@@ -79,6 +79,8 @@ void psolve_dev(fvm_ctx* c, const double* r, double* z, const int* skip = nullpt
 // set-up (the Krylov operator of fvm_opts.krylov_operator = 1)
 void jacobian_apply(fvm_ctx* c, double cj, const double* x, double* y, const int* skip = nullptr,
                     const double* dcj_dev = nullptr);
+// the operator layout's place of every Jacobian entry, for the set-ups to come
+void fd_set_op_places(fvm_ctx* c, const std::vector<int>& op_dst);
 double jacobian_cj_setup(fvm_ctx* c);   // cj of the last set-up
 int ilu_factored(fvm_ctx* c);           // precision of the current factor, -1 none
 bool schur_active(fvm_ctx* c);          // the Schur-coupled apply is on

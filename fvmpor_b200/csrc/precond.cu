@@ -39,15 +39,6 @@
 namespace fvmb {
 
 // ------------------------------------------------------------------ kernels
-__global__ void k_shift(int N, const double* __restrict__ y, const double* __restrict__ yp,
-                        const double* __restrict__ ewt, double h, double eps,
-                        double* __restrict__ shift) {
-    int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= N) return;
-    double a = fabs(y[j]), b = fabs(h * yp[j]), w = 1.0 / ewt[j];
-    shift[j] = eps * fmax(a, fmax(b, w));
-}
-
 // ---- finite-difference Jacobian, one element at a time
 // Column j of the reference's coloured difference quotient is
 // (F(y + d_j e_j, y' + cj d_j e_j) - F(y, y')) / d_j (preconditioner_dss.cpp:
@@ -56,25 +47,38 @@ __global__ void k_shift(int N, const double* __restrict__ y, const double* __res
 // single-column quotients.  With the upwind directions frozen, perturbing
 // node m changes only the elements that contain m, and only through h_m and
 // krw(h_m): each element forms the change of its corner partials for each of
-// its nodes in turn,
-//   dflux_f = rho0 (q_f (krw'_f - krw_f) + d_m C_fm krw'_f),
+// its nodes in turn, divided by d_m,
+//   dflux_f / d_m = q_f rho0 (krw'_f - krw_f) / d_m + C_fm rho0 krw'_f,
 // which is the same quotient written without the cancellation of two full
-// residuals.  The changes land in fixed slots (nonzero-major, ascending
-// element) and one pass per nonzero sums them, adds the storage term on the
-// diagonal and writes the Dirichlet rows: npe + 2 kernels per set-up instead
-// of one residual evaluation per colour.
+// residuals.  The elements are taken kFdChunk consecutive ones per block: the
+// changes stay in the block's shared memory, every non-zero (i, j) that the
+// chunk touches sums its own there in ascending element order, and only that
+// sum leaves the block -- the finished entry when no other chunk touches the
+// non-zero, else a partial that a second kernel adds in ascending chunk order.
 
-// per node: krw at h and h + d (every zone touching the node) and the change
-// of the storage term y' ahh(h) on the diagonal
-__global__ void k_fd_node(int N, const double* __restrict__ y, const double* __restrict__ yp, double cj,
-                          const double* __restrict__ shift, const ZoneDev* __restrict__ zones, int nz,
-                          const int* __restrict__ nz_ptr, const int* __restrict__ nz_zone,
-                          const double* __restrict__ nz_w, double rho0, double* __restrict__ krwb,
-                          double* __restrict__ krwp, double* __restrict__ dstor, double* __restrict__ ahhp_out) {
+// per node, in one pass: the shift d = eps max(|y|, |h y'|, 1 / w); for every
+// zone touching the node g = rho0 krw(h), its change dg = rho0 krw(h + d) - g
+// and the quotient dg / d; what the row's diagonal subtracts (the quotient of
+// the storage term y' ahh(h); on Dirichlet rows minus that of h_D - h), and the
+// storage term's cj coefficient, also in FP32 at the node's place in the
+// fused cycle's factor order (op_dg, once that layout exists)
+struct FdNode {
+    double *g, *dg, *q;        // [nz][N]
+    double* diag;              // [N]
+    double* ahhp;              // [N]
+    float* op_dg;
+    const int* lu_pos;
+};
+__global__ void k_fd_node(int N, const double* __restrict__ y, const double* __restrict__ yp,
+                          const double* __restrict__ ewt, double hstep, double eps, double cj,
+                          const ZoneDev* __restrict__ zones, int nz, const int* __restrict__ nz_ptr,
+                          const int* __restrict__ nz_zone, const double* __restrict__ nz_w, double rho0,
+                          const unsigned char* __restrict__ ntype, const double* __restrict__ hD, FdNode o) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= N) return;
-    const double h = y[i], d = shift[i];
-    const double hp = h + d;
+    const double h = y[i], ypi = yp[i];
+    const double d = eps * fmax(fabs(h), fmax(fabs(hstep * ypi), 1.0 / ewt[i]));
+    const double hp = h + d, rd = 1.0 / d;
     double phi = 0.0, dsw = 0.0, dswp = 0.0;
     const int p0 = nz == 1 ? i : nz_ptr[i], p1 = nz == 1 ? i + 1 : nz_ptr[i + 1];
     for (int p = p0; p < p1; ++p) {
@@ -83,15 +87,19 @@ __global__ void k_fd_node(int N, const double* __restrict__ y, const double* __r
         double Sw, ds, k, dsp, kp;
         van_genuchten(h, zones[z], Sw, ds, k);
         van_genuchten(hp, zones[z], Sw, dsp, kp);
-        krwb[(size_t)z * N + i] = k;
-        krwp[(size_t)z * N + i] = kp;
+        const double dg = rho0 * (kp - k);
+        o.g[(size_t)z * N + i] = rho0 * k;
+        o.dg[(size_t)z * N + i] = dg;
+        o.q[(size_t)z * N + i] = dg * rd;
         phi += zones[z].phi * w;
         dsw += ds * w;
         dswp += dsp * w;
     }
     const double ahh = (phi * dsw) * rho0, ahhp = (phi * dswp) * rho0;
-    dstor[i] = (yp[i] + cj * d) * ahhp - yp[i] * ahh;
-    ahhp_out[i] = ahhp;
+    const bool fixed = ntype[i] != 0;
+    o.diag[i] = fixed ? -(((hD[i] - hp) - (hD[i] - h)) / d) : ((ypi + cj * d) * ahhp - ypi * ahh) / d;
+    o.ahhp[i] = ahhp;
+    if (o.op_dg) o.op_dg[o.lu_pos[i]] = fixed ? 0.f : (float)ahhp;
 }
 
 // y = J x for the assembled difference-quotient Jacobian of the last
@@ -118,130 +126,293 @@ __global__ void k_jac_apply(int N, const int* __restrict__ rowptr, const int* __
     if (lane == 0) y[i] = ntype[i] ? acc : acc - dcj * ahhp[i] * x[i];
 }
 
-// per element: the npe x npe changes of its corner partials, one column
-// (perturbed node m) at a time, divided by d_m, into their slots
-// Slots are FP64, or FP32 when the factor is FP32 (the factor rounds every
-// entry to FP32 anyway; the slots then move half the bytes).
-template <int NPE, int NFE, bool RC, bool MZ, class S>
-// (two blocks per SM: 128 registers, no spills; the unbounded build took
-// 130 and ran one block of 8 warps per SM)
-__global__ void __launch_bounds__(256, 2) k_fd_elem(int T, int N, const int4* __restrict__ en,
-                                                 const double* __restrict__ coef, const double* __restrict__ xyz,
-                                                 const double* __restrict__ eK, int kiso, int estride,
-                                                 const int* __restrict__ ezone, const double* __restrict__ y,
-                                                 const double* __restrict__ shift, const double* __restrict__ krwb,
-                                                 const double* __restrict__ krwp,
-                                                 const unsigned char* __restrict__ upw, double rho0,
-                                                 const int* __restrict__ epos, S* __restrict__ slots) {
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= T) return;
-    const int4 nd = en[e];
-    const int g[4] = {nd.x, nd.y, nd.z, nd.w};
-    const size_t zo = MZ ? (size_t)ezone[e] * N : 0;
-    double hv[NPE], dl[NPE], kr[NPE], kp[NPE];
-#pragma unroll
-    for (int k = 0; k < NPE; ++k) {
-        hv[k] = y[g[k]];
-        dl[k] = shift[g[k]];
-        kr[k] = krwb[zo + g[k]];
-        kp[k] = krwp[zo + g[k]];
+// Jacobian entry q = (i, j) from its summed quotients: times 1/V_i (0 on
+// Dirichlet rows), minus the row's subtrahend on the diagonal.  Written to
+// the CSR values, to the place where the factorisation reads it (its block's
+// copy window, contiguous, in the factor's precision) and, once the fused
+// cycle's operator layout exists, to that layout.
+struct FdOut {
+    const double* scale;
+    const double* diag;
+    double* J;
+    void* Jw;
+    float* op_val;
+    // t: the entry's places in J, Jw (-1: another block's) and op_val
+    template <class S>
+    __device__ __forceinline__ void store(const int4& t, double s, double scale_i, bool on_diag, double diag_i) const {
+        double v = scale_i != 0.0 ? s * scale_i : 0.0;
+        if (on_diag) v = v - diag_i;
+        J[t.x] = v;
+        if (t.y >= 0) reinterpret_cast<S*>(Jw)[t.y] = (S)v;
+        if (op_val) op_val[t.z] = (float)v;
     }
-    double C[NFE][NPE], G[NFE];
-    if (RC) {
-        double X[4][3];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            X[k][0] = xyz[g[k]];
-            X[k][1] = xyz[(size_t)N + g[k]];
-            X[k][2] = xyz[(size_t)2 * N + g[k]];
+};
+
+struct FdArgs {
+    int T, N, kiso, estride, nnmax;
+    const int* cnode_ptr;          // [chunks + 1] nodes of each chunk
+    const int* cnode;              // global ids
+    const ushort4* cloc;           // [T] chunk-local corner ids
+    const int2* list_at;           // [chunks] the chunk's list: first 16-byte unit, groups of 32 non-zeros
+    const uint4* list;             // group offsets | places of the lanes' sums | entry-major slots
+    const int* done_ptr;           // [chunks + 1] non-zeros that no other chunk touches
+    const int4* done;              // place in J, Jw, op_val; 2 * chunk-local row + 1 on the diagonal
+    const int* share_ptr;          // [chunks + 1] the other ones
+    const int* share;              // place of the partial
+    int list_max, grp_max;         // largest chunk: list words, groups
+    double* part;
+    const double* coef;
+    const double* xyz;
+    const double* eK;
+    const int* ezone;
+    const double* y;
+    const double* g;               // [nz][N] rho0 krw, its change and quotient (k_fd_node)
+    const double* dg;
+    const double* gq;
+    const unsigned char* upw;
+    FdOut out;
+};
+
+constexpr int kFdThreads = 192;
+constexpr int kFdChunk = kFdThreads;   // elements per block, one per thread
+constexpr int kFdPre = 4;         // partials' places a thread fetches ahead
+
+// shared memory of k_fd_chunk: the quotients and a zero slot; the chunk's
+// nodes' h (and krw terms with one zone, coordinates when rebuilt), whose
+// place the non-zeros' sums take afterwards; their rows' scale and diagonal;
+// the list; its mbarrier
+struct FdSmem {
+    size_t nodes, rows, list, bar, bytes;
+    __host__ __device__ FdSmem(int npe, bool rc, bool mz, size_t sz, int nnmax, int list_max, int grp_max) {
+        const size_t nn = (size_t)nnmax * 8 * (1 + (mz ? 0 : 3) + (rc ? 3 : 0)), sums = (size_t)grp_max * 32 * 8;
+        nodes = round16(((size_t)npe * npe * kFdChunk + 1) * sz);
+        rows = nodes + round16(nn > sums ? nn : sums);
+        list = rows + 16 * (size_t)nnmax;
+        bar = list + (size_t)list_max * 2;
+        bytes = bar + 16;
+    }
+};
+// 16-bit words before the slots of a list of ng groups: ng + 1 group offsets
+// (in units of 32 slots), then 32 places per group
+__host__ __device__ inline int fd_list_offs(int ng) { return (ng + 8) & ~7; }
+
+// Quotient Jacobian of one chunk of elements.  Written one by one to their
+// slots in global memory, the npe^2 quotients of an element hit npe^2
+// scattered sectors, and a second kernel read them back: 129 + 63 us per set-up
+// on the 214k-node box (19.4 M FP32 quotients, one B200).  Here they stay in
+// shared memory (column-major over the chunk's elements, so a warp writes
+// consecutive words) and about two chunk sums per non-zero leave the block:
+// 85 us, and 24 us for the sums over chunks.  A block's phases (its nodes, its
+// quotients, its sums, its entries) each wait on memory or on FP64 chains, so
+// what counts is how many blocks share an SM: 192 elements, one per thread,
+// four blocks per SM at 85 registers; 512 elements over 256 threads at two per
+// SM took 108 us, 256 over 256 at three 91 us, 128 over 128 at six 92 us.
+// Everything a block reads after its quotients (the list of slots, by a bulk
+// copy; the sums' places) is on its way while they are formed.  The sums are
+// taken longest first, a non-zero per lane, so that a warp's lanes have like
+// lengths, and leave in ascending order of the non-zeros.
+// Quotients are FP64, or FP32 when the factor is FP32 (which rounds every
+// entry to FP32 anyway); all sums are FP64.
+template <int NPE, int NFE, bool RC, bool MZ, class S>
+__global__ void __launch_bounds__(kFdThreads, 4) k_fd_chunk(FdArgs a) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const FdSmem L(NPE, RC, MZ, sizeof(S), a.nnmax, a.list_max, a.grp_max);
+    S* slots = reinterpret_cast<S*>(smem_raw);
+    double* sh = reinterpret_cast<double*>(smem_raw + L.nodes);
+    double* sg = sh + a.nnmax;                  // one zone: g, dg, quotient
+    double* sx = sh + (MZ ? 1 : 4) * a.nnmax;   // rebuilt geometry
+    double* sums = sh;
+    double2* srow = reinterpret_cast<double2*>(smem_raw + L.rows);
+    uint64_t* bar = reinterpret_cast<uint64_t*>(smem_raw + L.bar);
+    const int2 la = a.list_at[blockIdx.x];
+    const int ng = la.y;
+    const unsigned short* goff = reinterpret_cast<const unsigned short*>(smem_raw + L.list);
+    const unsigned short* lrank = goff + fd_list_offs(ng);
+    const unsigned short* lslot = lrank + 32 * ng;
+    if (threadIdx.x == 0) {
+        tc05::mbar_init(bar, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        const uint32_t bytes = 16u * (uint32_t)(a.list_at[blockIdx.x + 1].x - la.x);
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(tc05::smem_u32(bar)), "r"(bytes)
+                     : "memory");
+        tc05::bulk_g2s(smem_raw + L.list, a.list + la.x, bytes, bar);
+    }
+    const int e0 = blockIdx.x * kFdChunk, ne = min(kFdChunk, a.T - e0);
+    const int el = threadIdx.x, e = e0 + el;
+    // the element's record
+    ushort4 lq = make_ushort4(0, 0, 0, 0);
+    uint2 uc = make_uint2(0u, 0u);
+    double K0 = 0.0, K1 = 0.0, K2 = 0.0;
+    if (el < ne) {
+        lq = a.cloc[e];
+        uc = *reinterpret_cast<const uint2*>(a.upw + (size_t)8 * e);
+        if (RC) {
+            K0 = K1 = K2 = a.eK[e];
+            if (!a.kiso) {
+                K1 = a.eK[(size_t)a.estride + e];
+                K2 = a.eK[(size_t)2 * a.estride + e];
+            }
         }
-        double Kx, Ky, Kz;
-        if (kiso) Kx = Ky = Kz = eK[e];
-        else { Kx = eK[e]; Ky = eK[(size_t)estride + e]; Kz = eK[(size_t)2 * estride + e]; }
-        double CC[6][4], GG[6];
-        tet_coefficients_fast(X[0], X[1], X[2], X[3], Kx, Ky, Kz, CC, GG);
+    }
+    const int n0 = a.cnode_ptr[blockIdx.x], nn = a.cnode_ptr[blockIdx.x + 1] - n0;
+    for (int k = threadIdx.x; k < nn; k += kFdThreads) {
+        const int g = a.cnode[n0 + k];
+        sh[k] = a.y[g];
+        srow[k] = make_double2(a.out.scale[g], a.out.diag[g]);
+        if (!MZ) {
+            sg[k] = a.g[g];
+            sg[a.nnmax + k] = a.dg[g];
+            sg[2 * a.nnmax + k] = a.gq[g];
+        }
+        if (RC) {
+            sx[k] = a.xyz[g];
+            sx[a.nnmax + k] = a.xyz[(size_t)a.N + g];
+            sx[2 * a.nnmax + k] = a.xyz[(size_t)2 * a.N + g];
+        }
+    }
+    if (threadIdx.x == 0) slots[NPE * NPE * kFdChunk] = (S)0;
+    __syncthreads();
+    if (el < ne) {
+        const int li[4] = {lq.x, lq.y, lq.z, lq.w};
+        double gk[NPE], dg[NPE], gq[NPE];
+        if (MZ) {
+            const size_t zo = (size_t)a.ezone[e] * a.N;
+#pragma unroll
+            for (int k = 0; k < NPE; ++k) {
+                const size_t g = zo + a.cnode[n0 + li[k]];
+                gk[k] = a.g[g];
+                dg[k] = a.dg[g];
+                gq[k] = a.gq[g];
+            }
+        } else {
+#pragma unroll
+            for (int k = 0; k < NPE; ++k) {
+                gk[k] = sg[li[k]];
+                dg[k] = sg[a.nnmax + li[k]];
+                gq[k] = sg[2 * a.nnmax + li[k]];
+            }
+        }
+        // C[f][m] of column m: with the rebuilt geometry the face
+        // combinations of one column of the cofactor rows' Gram matrix
+        double q[NFE];
+        TetGram G;
+        if constexpr (RC) {
+            double X[4][3];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                X[k][0] = sx[li[k]];
+                X[k][1] = sx[a.nnmax + li[k]];
+                X[k][2] = sx[2 * a.nnmax + li[k]];
+            }
+            G = tet_gram(X[0], X[1], X[2], X[3], K0, K1, K2);
+            G.fluxes(sh[li[0]], sh[li[1]], sh[li[2]], sh[li[3 % NPE]], q);
+        } else {
+#pragma unroll
+            for (int f = 0; f < NFE; ++f) {
+                const double* cf = a.coef + (size_t)(f * (NPE + 1)) * a.T + e;
+                double s = cf[0] * sh[li[0]];
+#pragma unroll
+                for (int k = 1; k < NPE; ++k) s += cf[(size_t)k * a.T] * sh[li[k]];
+                q[f] = s + cf[(size_t)NPE * a.T];
+            }
+        }
+        // upwind weights of each face's ends (1 and 0, or halves before the
+        // first step), the face's rho0 krw, and what its ends' own columns add
+        // to C rho0 krw: q times the quotient, C times the change
+        double gf[NFE], wa[NFE];
 #pragma unroll
         for (int f = 0; f < NFE; ++f) {
+            const int fa = NPE == 4 ? tet_edge_a(f) : tri_edge_a(f);
+            const int fb = NPE == 4 ? tet_edge_b(f) : tri_edge_b(f);
+            const unsigned u = (f < 4 ? uc.x >> (8 * f) : uc.y >> (8 * (f - 4))) & 0xffu;
+            wa[f] = u == 0 ? 1.0 : (u == 1 ? 0.0 : 0.5);
+            gf[f] = wa[f] * gk[fa] + (1.0 - wa[f]) * gk[fb];
+        }
 #pragma unroll
-            for (int k = 0; k < NPE; ++k) C[f][k] = CC[f][k];
-            G[f] = GG[f];
+        for (int m = 0; m < NPE; ++m) {
+            double C[NFE], dc[NPE];
+            if constexpr (RC) {
+                G.column(m, C);
+            } else {
+#pragma unroll
+                for (int f = 0; f < NFE; ++f) C[f] = a.coef[(size_t)(f * (NPE + 1) + m) * a.T + e];
+            }
+#pragma unroll
+            for (int k = 0; k < NPE; ++k) dc[k] = 0.0;
+#pragma unroll
+            for (int f = 0; f < NFE; ++f) {
+                const int fa = NPE == 4 ? tet_edge_a(f) : tri_edge_a(f);
+                const int fb = NPE == 4 ? tet_edge_b(f) : tri_edge_b(f);
+                double df = C[f] * gf[f];
+                if (fa == m || fb == m) df += (fa == m ? wa[f] : 1.0 - wa[f]) * (q[f] * gq[m] + C[f] * dg[m]);
+                dc[fa] -= df;
+                dc[fb] += df;
+            }
+#pragma unroll
+            for (int k = 0; k < NPE; ++k) slots[(m * NPE + k) * kFdChunk + el] = (S)dc[k];
+        }
+    }
+    const int d0 = a.done_ptr[blockIdx.x], nd = a.done_ptr[blockIdx.x + 1] - d0;
+    const int s0 = a.share_ptr[blockIdx.x], ns = a.share_ptr[blockIdx.x + 1] - s0;
+    // the sums' places, on their way while the sums are taken
+    int shr[kFdPre];
+#pragma unroll
+    for (int k = 0; k < kFdPre; ++k) {
+        const int p = threadIdx.x + k * kFdThreads;
+        shr[k] = p < ns ? a.share[s0 + p] : 0;
+    }
+    const int4 first = (int)threadIdx.x < nd ? a.done[d0 + threadIdx.x] : make_int4(0, -1, 0, 0);
+    // the list has landed; a block that gave up waiting for it would read
+    // unfilled shared memory, so it leaves its entries NaN (the solve fails)
+    const bool ok = tc05::mbar_wait(bar, 0) || tc05::mbar_wait(bar, 0);
+    const bool good = __syncthreads_and(ok ? 1 : 0) != 0;
+    // a warp's lanes each sum one non-zero; the lanes of a group are padded
+    // to its longest with the zero slot
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (good) {
+        for (int g = warp; g < ng; g += kFdThreads / 32) {
+            const int o1 = 32 * goff[g + 1];
+            double s = 0.0;
+#pragma unroll 4
+            for (int o = 32 * goff[g] + lane; o < o1; o += 32) s += (double)slots[lslot[o]];
+            sums[lrank[32 * g + lane]] = s;
         }
     } else {
-#pragma unroll
-        for (int f = 0; f < NFE; ++f) {
-#pragma unroll
-            for (int k = 0; k < NPE; ++k) C[f][k] = coef[(size_t)(f * (NPE + 1) + k) * T + e];
-            G[f] = coef[(size_t)(f * (NPE + 1) + NPE) * T + e];
-        }
+        for (int p = threadIdx.x; p < nd + ns; p += kFdThreads) sums[p] = nan("");
     }
-    const uint2 uw = *reinterpret_cast<const uint2*>(upw + (size_t)8 * e);
-    double q[NFE];
-    unsigned u[NFE];
+    __syncthreads();
 #pragma unroll
-    for (int f = 0; f < NFE; ++f) {
-        double s = C[f][0] * hv[0];
-#pragma unroll
-        for (int k = 1; k < NPE; ++k) s += C[f][k] * hv[k];
-        q[f] = s + G[f];
-        u[f] = (f < 4 ? uw.x >> (8 * f) : uw.y >> (8 * (f - 4))) & 0xffu;
+    for (int k = 0; k < kFdPre; ++k) {
+        const int p = threadIdx.x + k * kFdThreads;
+        if (p < ns) a.part[shr[k]] = sums[nd + p];
     }
-#pragma unroll
-    for (int m = 0; m < NPE; ++m) {
-        double dc[NPE];
-#pragma unroll
-        for (int k = 0; k < NPE; ++k) dc[k] = 0.0;
-#pragma unroll
-        for (int f = 0; f < NFE; ++f) {
-            const int a = NPE == 4 ? tet_edge_a(f) : tri_edge_a(f);
-            const int b = NPE == 4 ? tet_edge_b(f) : tri_edge_b(f);
-            const double kf = face_krw(u[f], kr[a], kr[b]);
-            const double kfp = face_krw(u[f], a == m ? kp[a] : kr[a], b == m ? kp[b] : kr[b]);
-            const double df = rho0 * (q[f] * (kfp - kf) + (dl[m] * C[f][m]) * kfp);
-            dc[a] -= df;
-            dc[b] += df;
-        }
-        const double inv = 1.0 / dl[m];
-#pragma unroll
-        for (int k = 0; k < NPE; ++k) slots[epos[(size_t)e * NPE * NPE + m * NPE + k]] = (S)(dc[k] * inv);
+    for (int p = threadIdx.x + kFdPre * kFdThreads; p < ns; p += kFdThreads) a.part[a.share[s0 + p]] = sums[nd + p];
+    for (int p = threadIdx.x; p < nd; p += kFdThreads) {
+        const int4 t = p < kFdThreads ? first : a.done[d0 + p];
+        const double2 r = srow[t.w >> 1];
+        a.out.store<S>(t, sums[p], r.x, t.w & 1, r.y);
     }
 }
 
-// per nonzero (i, j): J_ij = (1/V_i) sum of the slots - [i == j] dstor_i / d_i;
-// Dirichlet rows h_D - h differentiate to the quotient of that expression
+// the non-zeros touched by several chunks: their partials in ascending
+// chunk order.  at: place in J, Jw and op_val, and 2 * row + 1 on the diagonal
 template <class S>
-__global__ void k_fd_gather(int nnz, const int* __restrict__ rowof, const int* __restrict__ col,
-                            const int* __restrict__ jptr, const S* __restrict__ slots,
-                            const double* __restrict__ invV, const double* __restrict__ dstor,
-                            const unsigned char* __restrict__ ntype, const double* __restrict__ hD,
-                            const double* __restrict__ y, const double* __restrict__ shift,
-                            double* __restrict__ J, const int* __restrict__ lu_dst, double* __restrict__ Jw,
-                            const int* __restrict__ op_dst, float* __restrict__ op_val) {
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= nnz) return;
-    const int i = rowof[q], j = col[q];
-    double v;
-    if (ntype[i]) {
-        v = i == j ? ((hD[i] - (y[i] + shift[i])) - (hD[i] - y[i])) / shift[i] : 0.0;
-    } else {
-        double s = 0.0;
-        const int p1 = jptr[q + 1];
-        for (int p = jptr[q]; p < p1; ++p) s += (double)slots[p];
-        v = s * invV[i];
-        if (i == j) v = v - dstor[i] / shift[i];
-    }
-    J[q] = v;
-    // the same value where the factorisation reads it (its block's copy
-    // window, so that it loads its block contiguously) and, once the fused
-    // cycle's operator layout exists, in that layout
-    const int pw = lu_dst[q];
-    if (pw >= 0) Jw[pw] = v;
-    if (op_val) op_val[op_dst[q]] = (float)v;
+__global__ void k_fd_shared(int n, const int4* __restrict__ at, const int* __restrict__ sptr,
+                            const double* __restrict__ part, FdOut out) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= n) return;
+    const int4 w = at[t];
+    const int p0 = sptr[t], p1 = sptr[t + 1];
+    const double scale = out.scale[w.w >> 1], diag = w.w & 1 ? out.diag[w.w >> 1] : 0.0;
+    double s = 0.0;
+    for (int p = p0; p < p1; ++p) s += part[p];
+    out.store<S>(w, s, scale, w.w & 1, diag);
 }
 
 template <class T>
 __global__ void __launch_bounds__(128) k_ilu_factor(const int* __restrict__ bstart,
                                                     const int* __restrict__ lu_ptr,
-                                                    const double* __restrict__ Jw,
+                                                    const T* __restrict__ Jw,
                                                     const int* __restrict__ lu_diag,
                                                     const unsigned short* __restrict__ lu_col,
                                                     const int* __restrict__ lvl_ptr,
@@ -250,7 +421,7 @@ __global__ void __launch_bounds__(128) k_ilu_factor(const int* __restrict__ bsta
                                                     int* status) {
     int b = blockIdx.x;
     int r0 = bstart[b], r1 = bstart[b + 1];
-    for (int p = lu_ptr[r0] + threadIdx.x; p < lu_ptr[r1]; p += blockDim.x) lu[p] = (T)Jw[p];
+    for (int p = lu_ptr[r0] + threadIdx.x; p < lu_ptr[r1]; p += blockDim.x) lu[p] = Jw[p];
     __syncthreads();
     for (int l = blk_lvl[b]; l < blk_lvl[b + 1]; ++l) {
         for (int q = lvl_ptr[l] + threadIdx.x; q < lvl_ptr[l + 1]; q += blockDim.x) {
@@ -574,7 +745,7 @@ constexpr int kIluFactorPre = 8;
 template <class T>
 __global__ void __launch_bounds__(kIluFactorThreads, 1) k_ilu_factor_smem(const int* __restrict__ bstart,
                                                          const int* __restrict__ lu_ptr,
-                                                         const double* __restrict__ Jw,
+                                                         const T* __restrict__ Jw,
                                                          const int* __restrict__ lu_diag,
                                                          const unsigned short* __restrict__ lu_col,
                                                          const int* __restrict__ lvl_ptr,
@@ -599,7 +770,7 @@ __global__ void __launch_bounds__(kIluFactorThreads, 1) k_ilu_factor_smem(const 
     const int lq0 = lvl_ptr[la];
 #pragma unroll 4
     for (int p = e0 + threadIdx.x; p < e1; p += blockDim.x) {
-        val[p - w.base] = (T)Jw[p];
+        val[p - w.base] = Jw[p];
         col[p - w.base] = lu_col[p];
     }
     for (int i = threadIdx.x; i <= nr; i += blockDim.x) rp[i] = (unsigned short)(lu_ptr[r0 + i] - w.base);
@@ -724,6 +895,133 @@ static std::vector<int> block_colour_order(const std::vector<int>& rp, const std
     return ord;
 }
 
+// Tables of the quotient Jacobian's chunks (k_fd_chunk): the distinct nodes of
+// every chunk with the elements' local corner ids; the non-zeros it touches,
+// first those no other chunk touches, then the others with the places of
+// their partials, each ascending; and the list of all of them longest first
+// in groups of 32, with their slots in ascending element order.  The places
+// in the operator layout (done, shared: .z) follow once that layout exists.
+struct FdTables {
+    std::vector<int> cnode_ptr, cnode, done_ptr, share_ptr, share, sptr;
+    std::vector<int2> list_at;
+    std::vector<int4> done, shared;
+    std::vector<ushort4> cloc;
+    std::vector<unsigned short> list;
+    int nnmax = 0, list_max = 0, grp_max = 0;
+};
+
+static void build_fd_tables(const fvm_ctx* c, const BlockILU* P, const std::vector<int>& rowof,
+                            const std::vector<int>& lu_dst, FdTables& fd) {
+    const int N = c->N, T = c->T, npe = c->npe, npe2 = npe * npe;
+    const std::vector<int>&rp = P->h_rowptr, &cl = P->h_col;
+    const int nch = (T + kFdChunk - 1) / kFdChunk;
+    // chunks touching each non-zero, then the places of the shared ones'
+    // partials (non-zero-major, ascending chunk)
+    std::vector<int> fq((size_t)T * npe2), seen(P->nnz, -1), nchunk(P->nnz, 0);
+    for (int e = 0; e < T; ++e) {
+        const int* v = &c->h_elem_nodes[(size_t)e * npe];
+        for (int m = 0; m < npe; ++m)
+            for (int k = 0; k < npe; ++k) {
+                const int i = v[k], j = v[m];
+                const int q = (int)(std::lower_bound(&cl[rp[i]], &cl[0] + rp[i + 1], j) - &cl[0]);
+                fq[(size_t)e * npe2 + m * npe + k] = q;
+                if (seen[q] != e / kFdChunk) { seen[q] = e / kFdChunk; nchunk[q]++; }
+            }
+    }
+    std::vector<int> place(P->nnz, -1);
+    fd.sptr.assign(1, 0);
+    for (int q = 0; q < P->nnz; ++q)
+        if (nchunk[q] > 1) {
+            place[q] = fd.sptr.back();
+            fd.shared.push_back(make_int4(q, lu_dst[q], 0, 2 * rowof[q] + (cl[q] == rowof[q] ? 1 : 0)));
+            fd.sptr.push_back(fd.sptr.back() + nchunk[q]);
+        }
+    fd.cnode_ptr.assign(1, 0);
+    fd.done_ptr.assign(1, 0);
+    fd.share_ptr.assign(1, 0);
+    fd.cloc.assign(T, make_ushort4(0, 0, 0, 0));
+    std::fill(seen.begin(), seen.end(), -1);
+    std::vector<int> stamp(N, -1), lid(N, 0), local(P->nnz, 0), nodes, qs, cnt, pos, order, hist, asc, rank;
+    std::vector<unsigned short> sl;
+    for (int ch = 0; ch < nch; ++ch) {
+        const int e0 = ch * kFdChunk, e1 = std::min(T, e0 + kFdChunk);
+        nodes.clear();
+        qs.clear();
+        cnt.clear();
+        for (int e = e0; e < e1; ++e) {
+            for (int k = 0; k < npe; ++k) {
+                const int g = c->h_elem_nodes[(size_t)e * npe + k];
+                if (stamp[g] != ch) { stamp[g] = ch; nodes.push_back(g); }
+            }
+            for (int t = 0; t < npe2; ++t) {
+                const int q = fq[(size_t)e * npe2 + t];
+                if (seen[q] != ch) { seen[q] = ch; local[q] = (int)qs.size(); qs.push_back(q); cnt.push_back(0); }
+                cnt[local[q]]++;
+            }
+        }
+        std::sort(nodes.begin(), nodes.end());
+        for (size_t k = 0; k < nodes.size(); ++k) lid[nodes[k]] = (int)k;
+        for (int e = e0; e < e1; ++e) {
+            unsigned short l[4] = {0, 0, 0, 0};
+            for (int k = 0; k < npe; ++k) l[k] = (unsigned short)lid[c->h_elem_nodes[(size_t)e * npe + k]];
+            fd.cloc[e] = make_ushort4(l[0], l[1], l[2], l[3]);
+        }
+        fd.nnmax = std::max(fd.nnmax, (int)nodes.size());
+        fd.cnode.insert(fd.cnode.end(), nodes.begin(), nodes.end());
+        fd.cnode_ptr.push_back((int)fd.cnode.size());
+        // the sums' places: finished non-zeros, then shared ones, ascending
+        const int np = (int)qs.size();
+        asc.resize(np);
+        for (int p = 0; p < np; ++p) asc[p] = p;
+        std::sort(asc.begin(), asc.end(), [&](int x, int y) {
+            const bool sx = place[qs[x]] >= 0, sy = place[qs[y]] >= 0;
+            return sx != sy ? sy : qs[x] < qs[y];
+        });
+        rank.resize(np);
+        for (int r = 0; r < np; ++r) {
+            const int q = qs[asc[r]];
+            rank[asc[r]] = r;
+            if (place[q] >= 0) fd.share.push_back(place[q]++);
+            else fd.done.push_back(make_int4(q, lu_dst[q], 0, 2 * lid[rowof[q]] + (cl[q] == rowof[q] ? 1 : 0)));
+        }
+        fd.done_ptr.push_back((int)fd.done.size());
+        fd.share_ptr.push_back((int)fd.share.size());
+        // the non-zeros by falling number of slots (a counting sort)
+        const int most = *std::max_element(cnt.begin(), cnt.end());
+        hist.assign(most + 2, 0);
+        for (int p = 0; p < np; ++p) hist[most - cnt[p] + 1]++;
+        for (int k = 0; k <= most; ++k) hist[k + 1] += hist[k];
+        order.resize(np);
+        for (int p = 0; p < np; ++p) order[hist[most - cnt[p]]++] = p;
+        pos.assign(np + 1, 0);
+        for (int p = 0; p < np; ++p) pos[p + 1] = pos[p] + cnt[p];
+        sl.resize((size_t)(e1 - e0) * npe2);
+        for (int e = e0; e < e1; ++e)
+            for (int t = 0; t < npe2; ++t)
+                sl[pos[local[fq[(size_t)e * npe2 + t]]]++] = (unsigned short)(t * kFdChunk + (e - e0));
+        // pos[p] is now the end of non-zero p's slots
+        const int ng = (np + 31) / 32;
+        const size_t l0 = fd.list.size();
+        fd.list_at.push_back(make_int2((int)(l0 / 8), ng));
+        fd.list.resize(l0 + fd_list_offs(ng), 0);
+        for (int g = 0; g < ng; ++g) fd.list[l0 + g + 1] = (unsigned short)(fd.list[l0 + g] + cnt[order[32 * g]]);
+        // lanes past the last non-zero leave their zero past the sums
+        for (int r = 0; r < 32 * ng; ++r) fd.list.push_back((unsigned short)(r < np ? rank[order[r]] : r));
+        for (int g = 0; g < ng; ++g) {
+            const size_t base = fd.list.size();
+            fd.list.resize(base + 32 * (size_t)cnt[order[32 * g]], (unsigned short)(npe2 * kFdChunk));
+            for (int l = 0; l < 32 && 32 * g + l < np; ++l) {
+                const int p = order[32 * g + l];
+                for (int k = 0; k < cnt[p]; ++k) fd.list[base + 32 * (size_t)k + l] = sl[pos[p] - cnt[p] + k];
+            }
+        }
+        fd.list_max = std::max(fd.list_max, (int)(fd.list.size() - l0));
+        fd.grp_max = std::max(fd.grp_max, ng);
+    }
+    if (fd.list.size() / 8 >= (size_t)INT32_MAX) throw Error("difference quotients: mesh too large");
+    fd.list_at.push_back(make_int2((int)(fd.list.size() / 8), 0));
+}
+
 static void build_pattern(fvm_ctx* c, BlockILU* P) {
     const int N = c->N, npe = c->npe, T = c->T;
     // node -> elements (host copy of the incidence lists)
@@ -776,28 +1074,6 @@ static void build_pattern(fvm_ctx* c, BlockILU* P) {
     std::vector<int> rowof(P->nnz);
     for (int i = 0; i < N; ++i)
         for (int p = rp[i]; p < rp[i + 1]; ++p) rowof[p] = i;
-    // element-wise difference quotients: slot of (element e, perturbed node
-    // m, corner k) -> nonzero (node of k, node of m); slots of one nonzero
-    // are contiguous and in ascending element order
-    const int npe2 = npe * npe;
-    std::vector<int> fd_q((size_t)T * npe2), fd_jptr(P->nnz + 1, 0), fd_epos((size_t)T * npe2);
-    for (int e = 0; e < T; ++e) {
-        const int* v = &c->h_elem_nodes[(size_t)e * npe];
-        for (int m = 0; m < npe; ++m)
-            for (int k = 0; k < npe; ++k) {
-                const int i = v[k], j = v[m];
-                const int* b = &cl[rp[i]];
-                const int* f = std::lower_bound(b, &cl[0] + rp[i + 1], j);
-                const int q = (int)(f - &cl[0]);
-                fd_q[(size_t)e * npe2 + m * npe + k] = q;
-                fd_jptr[q + 1]++;
-            }
-    }
-    for (int q = 0; q < P->nnz; ++q) fd_jptr[q + 1] += fd_jptr[q];
-    {
-        std::vector<int> fill(fd_jptr.begin(), fd_jptr.end() - 1);
-        for (size_t t = 0; t < fd_q.size(); ++t) fd_epos[t] = fill[fd_q[t]]++;
-    }
     // blocks of contiguous nodes; on a large mesh a multiple of the SM count
     // (c->ilu_per_sm blocks per SM: fewer, larger blocks precondition better,
     // more, smaller ones have shorter level chains and share an SM)
@@ -1054,15 +1330,26 @@ static void build_pattern(fvm_ctx* c, BlockILU* P) {
         *P->h_serr = 0;
     }
     P->col.upload(P->h_col, s);
-    P->rowof.upload(rowof, s);
     P->J.alloc(P->nnz);
-    P->shift.alloc(N);
-    P->fd_epos.upload(fd_epos, s);
-    P->fd_jptr.upload(fd_jptr, s);
-    P->fd_slots.alloc(fd_epos.size());
-    P->krwb.alloc((size_t)c->nz * N);
-    P->krwp.alloc((size_t)c->nz * N);
-    P->dstor.alloc(N);
+    {
+        std::vector<int> lu_pos(N);
+        for (int q = 0; q < N; ++q) lu_pos[lu_row[q]] = q;
+        P->lu_pos.upload(lu_pos, s);
+    }
+    P->fd_g.alloc((size_t)c->nz * N);
+    P->fd_dg.alloc((size_t)c->nz * N);
+    P->fd_gq.alloc((size_t)c->nz * N);
+    P->fd_diag.alloc(N);
+    {
+        // 1/V of free rows, 0 on Dirichlet rows
+        std::vector<double> sc(N);
+        FVM_CUDA(cudaMemcpyAsync(sc.data(), c->invV.p, sizeof(double) * N, cudaMemcpyDeviceToHost, s));
+        FVM_CUDA(cudaStreamSynchronize(s));
+        for (int i = 0; i < N; ++i)
+            if (c->h_node_type[i]) sc[i] = 0.0;
+        P->fd_scale.upload(sc, s);
+        FVM_CUDA(cudaStreamSynchronize(s));
+    }
     P->ahhp.alloc(N);
     P->rowptr.upload(P->h_rowptr, s);
     P->bstart.upload(bstart, s);
@@ -1071,10 +1358,28 @@ static void build_pattern(fvm_ctx* c, BlockILU* P) {
     P->lu_ptr.upload(lu_ptr, s);
     // 8 padding entries so every block's widened copy window stays inside
     {
-        // where fd_gather puts each Jacobian entry for the factorisation
+        // where the quotient kernels put each Jacobian entry for the factorisation
         std::vector<int> lu_dst(P->nnz, -1);
         for (size_t p = 0; p < lu_src.size(); ++p) lu_dst[lu_src[p]] = (int)p;
-        P->lu_dst.upload(lu_dst, s);
+        FdTables fd;
+        build_fd_tables(c, P, rowof, lu_dst, fd);
+        P->fd_cnode_ptr.upload(fd.cnode_ptr, s);
+        P->fd_cnode.upload(fd.cnode, s);
+        P->fd_cloc.upload(fd.cloc, s);
+        P->fd_list_at.upload(fd.list_at, s);
+        P->fd_list.upload(fd.list, s);
+        P->fd_done_ptr.upload(fd.done_ptr, s);
+        P->fd_done.upload(fd.done, s);
+        P->fd_share_ptr.upload(fd.share_ptr, s);
+        P->fd_share.upload(fd.share, s);
+        P->fd_shared.upload(fd.shared, s);
+        P->fd_sptr.upload(fd.sptr, s);
+        P->fd_part.alloc(fd.sptr.back());
+        P->fd_nnmax = fd.nnmax;
+        P->fd_list_max = fd.list_max;
+        P->fd_grp_max = fd.grp_max;
+        // the tables' host memory is read by copies still in flight
+        FVM_CUDA(cudaStreamSynchronize(s));
     }
     lu_src.resize(lu_src.size() + 8, 0);
     lu_col.resize(lu_col.size() + 8, 0);
@@ -1102,6 +1407,20 @@ static void build_pattern(fvm_ctx* c, BlockILU* P) {
     P->built = true;
 }
 
+// fills in the operator layout's places of the quotient kernels' outputs
+__global__ void k_fd_op_places(int n, int4* __restrict__ at, const int* __restrict__ op_dst) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t < n) at[t].z = op_dst[at[t].x];
+}
+void fd_set_op_places(fvm_ctx* c, const std::vector<int>& op_dst) {
+    BlockILU* P = c->ilu;
+    DevBuf<int> d;
+    d.upload(op_dst, c->stream);
+    for (DevBuf<int4>* b : {&P->fd_done, &P->fd_shared})
+        if (b->n) fvm_launch(c, k_fd_op_places, grid_for((long)b->n, 256), 256, 0, c->stream, (int)b->n, b->p, d.p);
+    FVM_CUDA(cudaStreamSynchronize(c->stream));
+}
+
 void psetup_dev(fvm_ctx* c, double cj, double h, const double* y, const double* yp,
                 const double* F0, const double* ewt, int precision) {
     if (!c->ilu) c->ilu = new BlockILU();
@@ -1111,37 +1430,45 @@ void psetup_dev(fvm_ctx* c, double cj, double h, const double* y, const double* 
     const int N = c->N;
     c->tm.begin(TM_FD_JAC, s);
     (void)F0;   // the element-wise quotients difference each element's own partials
-    fvm_launch(c, k_shift, grid_for(N, 256), 256, 0, s, N, y, yp, ewt, h, std::sqrt(DBL_EPSILON), P->shift.p);
-    fvm_launch(c, k_fd_node, grid_for(N, 256), 256, 0, s, N, y, yp, cj, P->shift.p, c->zones.p, c->nz, c->nz_ptr.p,
-               c->nz_zone.p, c->nz_w.p, c->rho0, P->krwb.p, P->krwp.p, P->dstor.p, P->ahhp.p);
+    // the fused cycle's operator values too, once its layout exists
+    const bool op = P->op_built && P->fused_ok;
+    fvm_launch(c, k_fd_node, grid_for(N, 256), 256, 0, s, N, y, yp, ewt, h, std::sqrt(DBL_EPSILON), cj, c->zones.p,
+               c->nz, c->nz_ptr.p, c->nz_zone.p, c->nz_w.p, c->rho0, c->ntype.p, c->hD.p,
+               FdNode{P->fd_g.p, P->fd_dg.p, P->fd_gq.p, P->fd_diag.p, P->ahhp.p, op ? P->op_dg.p : nullptr,
+                      P->lu_pos.p});
     P->cj_setup = cj;
     P->setup_id++;
+    P->op_setup_id = op ? P->setup_id : -1;
     {
-        const int gb = grid_for(c->T, 256);
-        const bool mz = c->nz > 1;
-        auto run = [&](auto* slots) {
-            using S = std::remove_pointer_t<decltype(slots)>;
-            auto go = [&](auto kern) {
-                fvm_launch(c, kern, gb, 256, 0, s, c->T, N, c->enodes.p, c->coef.p, c->xyz.p, c->eK.p,
-                           c->kiso ? 1 : 0, c->estride, c->ezone.p, y, P->shift.p, P->krwb.p, P->krwp.p, c->upw.p,
-                           c->rho0, P->fd_epos.p, slots);
+        FdArgs a;
+        a.T = c->T; a.N = N; a.kiso = c->kiso ? 1 : 0; a.estride = c->estride; a.nnmax = P->fd_nnmax;
+        a.cnode_ptr = P->fd_cnode_ptr.p; a.cnode = P->fd_cnode.p; a.cloc = P->fd_cloc.p;
+        a.list_at = P->fd_list_at.p; a.list = reinterpret_cast<const uint4*>(P->fd_list.p);
+        a.done_ptr = P->fd_done_ptr.p; a.done = P->fd_done.p; a.share_ptr = P->fd_share_ptr.p; a.share = P->fd_share.p;
+        a.list_max = P->fd_list_max; a.grp_max = P->fd_grp_max; a.part = P->fd_part.p;
+        a.coef = c->coef.p; a.xyz = c->xyz.p; a.eK = c->eK.p; a.ezone = c->ezone.p;
+        a.y = y; a.g = P->fd_g.p; a.dg = P->fd_dg.p; a.gq = P->fd_gq.p; a.upw = c->upw.p;
+        a.out = FdOut{P->fd_scale.p, P->fd_diag.p, P->J.p, P->Jw.p, op ? P->op_val.p : nullptr};
+        auto run = [&](auto one) {
+            using S = decltype(one);
+            auto go = [&](auto kern, size_t sm) {
+                if (sm > 48 * 1024) raise_smem_limit(kern, sm);
+                fvm_launch(c, kern, (c->T + kFdChunk - 1) / kFdChunk, kFdThreads, sm, s, a);
             };
-            if (c->dim == 3) {
-                if (c->recompute) mz ? go(k_fd_elem<4, 6, true, true, S>) : go(k_fd_elem<4, 6, true, false, S>);
-                else mz ? go(k_fd_elem<4, 6, false, true, S>) : go(k_fd_elem<4, 6, false, false, S>);
-            } else {
-                mz ? go(k_fd_elem<3, 3, false, true, S>) : go(k_fd_elem<3, 3, false, false, S>);
-            }
-            // the fused cycle's operator values too, once its layout exists
-            float* opv = P->op_built && P->fused_ok ? P->op_val.p : nullptr;
-            fvm_launch(c, k_fd_gather<S>, grid_for(P->nnz, 256), 256, 0, s, P->nnz, P->rowof.p, P->col.p,
-                       P->fd_jptr.p, slots, c->invV.p, P->dstor.p, c->ntype.p, c->hD.p, y, P->shift.p, P->J.p,
-                       P->lu_dst.p, P->Jw.p, opv ? P->op_dst.p : nullptr, opv);
-            P->op_vals_setup = opv ? P->setup_id : -1;
+#define FVM_FD(NPE, NFE, RC, MZ) \
+    go(k_fd_chunk<NPE, NFE, RC, MZ, S>, FdSmem(NPE, RC, MZ, sizeof(S), a.nnmax, a.list_max, a.grp_max).bytes)
+            const bool mz = c->nz > 1;
+            if (c->dim == 2) mz ? FVM_FD(3, 3, false, true) : FVM_FD(3, 3, false, false);
+            else if (c->recompute) mz ? FVM_FD(4, 6, true, true) : FVM_FD(4, 6, true, false);
+            else mz ? FVM_FD(4, 6, false, true) : FVM_FD(4, 6, false, false);
+#undef FVM_FD
+            const int ns = (int)P->fd_shared.n;
+            if (ns)
+                fvm_launch(c, k_fd_shared<S>, grid_for(ns, 256), 256, 0, s, ns, P->fd_shared.p, P->fd_sptr.p,
+                           P->fd_part.p, a.out);
         };
-        // the FP64 slot buffer holds the FP32 slots in its first half
-        if (precision) run(reinterpret_cast<float*>(P->fd_slots.p));
-        else run(P->fd_slots.p);
+        if (precision) run(0.f);
+        else run(0.0);
     }
     c->tm.end(TM_FD_JAC, s);
     FVM_CUDA(cudaMemsetAsync(P->status.p, 0, sizeof(int), s));
@@ -1153,9 +1480,9 @@ void psetup_dev(fvm_ctx* c, double cj, double h, const double* y, const double* 
         size_t sm = (size_t)so + 8 * (size_t)sw;
         if (precision) {
             P->lu32.alloc(nlu);
-            fvm_launch(c, k_ilu_factor_smem<float>, P->nb, kIluFactorThreads, sm, s, P->bstart.p, P->lu_ptr.p, P->Jw.p,
-                       P->lu_diag.p, P->lu_col.p, P->lvl_ptr.p, P->lvl_rows.p, P->blk_lvl.p, P->seg_ptr.p, P->upd.p,
-                       so, sw, P->lu32.p, P->status.p);
+            fvm_launch(c, k_ilu_factor_smem<float>, P->nb, kIluFactorThreads, sm, s, P->bstart.p, P->lu_ptr.p,
+                       reinterpret_cast<const float*>(P->Jw.p), P->lu_diag.p, P->lu_col.p, P->lvl_ptr.p, P->lvl_rows.p,
+                       P->blk_lvl.p, P->seg_ptr.p, P->upd.p, so, sw, P->lu32.p, P->status.p);
         } else {
             P->lu64.alloc(nlu);
             fvm_launch(c, k_ilu_factor_smem<double>, P->nb, kIluFactorThreads, sm, s, P->bstart.p, P->lu_ptr.p, P->Jw.p,
@@ -1164,7 +1491,8 @@ void psetup_dev(fvm_ctx* c, double cj, double h, const double* y, const double* 
         }
     } else if (precision) {
         P->lu32.alloc(nlu);
-        fvm_launch(c, k_ilu_factor<float>, P->nb, 128, 0, s, P->bstart.p, P->lu_ptr.p, P->Jw.p, P->lu_diag.p, P->lu_col.p,
+        fvm_launch(c, k_ilu_factor<float>, P->nb, 128, 0, s, P->bstart.p, P->lu_ptr.p,
+                   reinterpret_cast<const float*>(P->Jw.p), P->lu_diag.p, P->lu_col.p,
                                                   P->lvl_ptr.p, P->lvl_rows.p, P->blk_lvl.p, P->lu32.p,
                                                   P->status.p);
     } else {

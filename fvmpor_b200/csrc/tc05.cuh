@@ -76,6 +76,15 @@ __device__ __forceinline__ void mma_commit(uint64_t* bar) {
         smem_u32(bar)));
 }
 
+// 1D bulk copy into shared memory, completion counted on the mbarrier (both
+// addresses and the size multiples of 16 bytes)
+__device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                     smem_u32(dst)),
+                 "l"(src), "r"(bytes), "r"(smem_u32(bar))
+                 : "memory");
+}
+
 // bounded wait for the given phase parity; false on timeout
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32_t max_iter = (1u << 26)) {
     uint32_t addr = smem_u32(bar);
