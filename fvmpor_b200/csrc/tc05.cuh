@@ -107,19 +107,27 @@ __device__ __forceinline__ void fence_after_sync() { asm volatile("tcgen05.fence
 // make generic-proxy shared-memory writes visible to the tensor core (async proxy)
 __device__ __forceinline__ void fence_smem_async() { asm volatile("fence.proxy.async.shared::cta;"); }
 
-// 16 consecutive FP32 columns of this thread's TMEM lane (warp w may only
-// address lanes 32w .. 32w+31)
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
-    uint32_t r[16];
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
-        "%14, %15}, [%16];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-        : "r"(taddr));
-    asm volatile("tcgen05.wait::ld.sync.aligned;");
+// NC consecutive FP32 columns of this thread's TMEM lane (warp w may only
+// address lanes 32 (w % 4) .. 32 (w % 4) + 31)
+template <int NC> __device__ __forceinline__ void tmem_ld(uint32_t taddr, float (&v)[NC]) {
+    static_assert(NC % 16 == 0, "read 16 columns at a time");
+    uint32_t r[NC];
 #pragma unroll
-    for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
+    for (int c = 0; c < NC; c += 16)
+        asm volatile(
+            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
+            "%14, %15}, [%16];"
+            : "=r"(r[c]), "=r"(r[c + 1]), "=r"(r[c + 2]), "=r"(r[c + 3]), "=r"(r[c + 4]), "=r"(r[c + 5]),
+              "=r"(r[c + 6]), "=r"(r[c + 7]), "=r"(r[c + 8]), "=r"(r[c + 9]), "=r"(r[c + 10]), "=r"(r[c + 11]),
+              "=r"(r[c + 12]), "=r"(r[c + 13]), "=r"(r[c + 14]), "=r"(r[c + 15])
+            : "r"(taddr + c));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int i = 0; i < NC; ++i) {
+        // the registers are defined only after the wait
+        asm volatile("" : "+r"(r[i]));
+        v[i] = __uint_as_float(r[i]);
+    }
 }
 
 // byte offset of element (r, k) in an interleaved tile with K columns
