@@ -12,8 +12,8 @@
 // dot products.  So one CTA owns one ILU block for the whole cycle:
 //   - its factor window and metadata are brought into shared memory ONCE per
 //     cycle by bulk copies (the staged apply reloads them on every apply);
-//   - per step it gathers the direction at its own and its halo nodes into
-//     shared memory, forms its rows of J t from there (rows in factor order,
+//   - per step it has the direction at its own nodes from its last basis pass,
+//     gathers it at its halo nodes into shared memory, forms its rows of J t from there (rows in factor order,
 //     one warp per 32 rows, entry-major slices with 16-bit local columns)
 //     straight into the shared-memory vector the triangular sweeps work on,
 //     runs both sweeps there, scales by ewt, and
@@ -42,7 +42,7 @@
 namespace fvmb {
 
 struct FusedArgs {
-    int N, m, nr_max, nh_max;
+    int N, m, nr_max, nh_max, halo_max;
     int nqp;                   // quads per block row array in shared memory (quad-transposed, quad_pos)
     size_t stage_max;          // shared bytes of the largest block's staged factor
     ArnState* st;
@@ -54,7 +54,6 @@ struct FusedArgs {
     const int* slptr;          // [slices + 1] first entry of each slice
     const int* blksl;          // [nb + 1] first slice of each block
     const unsigned short* op_lcol;   // entry -> index in the block's node list
-    const unsigned short* op_self;   // [N], factor order: the row's own index there
     const int* halo_ptr;       // [nb + 1] the block's node list: its rows and halo
     const int* halo_node;
     const int* nbr_ptr;        // [nb + 1] blocks whose flags a block waits for
@@ -65,12 +64,9 @@ struct FusedArgs {
     const float* op_dg;        // [N], factor order: ahh(h + d) on free rows, else 0
     float dcj;                 // cj - cj of the set-up
     const int* bstart;
-    const int* lu_ptr;
+    const IluBlk* blk;
     const unsigned short* lu_col;
     const unsigned short* meta;
-    const int* meta_off;
-    const int* blk_lvl;
-    const int* blk_ulvl;
     const float* lu;
     const int* lu_row;
     const double* beta2;       // ||D P^-1 r||^2 of the cycle's start
@@ -132,16 +128,81 @@ __device__ __forceinline__ bool fused_sync(unsigned* sync, int* err, int* s_ok) 
     return *s_ok != 0;
 }
 
+// the unrotated Hessenberg matrix by columns, c + 2 entries in column c: where
+// column c starts
+__host__ __device__ __forceinline__ int hess_words(int c) { return c * (c + 3) / 2; }
+
 // barrier among `count` threads (whole warps) of the block on barrier `id`
 __device__ __forceinline__ void named_barrier(int id, int count) {
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory");
+}
+
+// One lane's row of an operator slice, up to 16 entries of it (longer rows read
+// the rest in place).  Entries are stored four to a lane, so a slice is a few
+// 16-byte loads of values and 8-byte loads of columns per lane: with single
+// entries (24 loads of 4 and 2 bytes) the loads in flight took more registers
+// and the operator 6.1 us per step on the 214k-node box instead of 4.9 (4.0
+// with the directions in factor order, fused_prepare).
+struct OpSlice {
+    float4 v[4];
+    uint2 c[4];
+    float dg;
+    int w;
+};
+constexpr int kOpGroup = 128;   // entries per group: four per lane
+__device__ __forceinline__ void op_four(float& acc, const float* tl, const float4& v, const uint2& c) {
+    acc = fmaf(v.x, tl[c.x & 0xffffu], acc);
+    acc = fmaf(v.y, tl[c.x >> 16], acc);
+    acc = fmaf(v.z, tl[c.y & 0xffffu], acc);
+    acc = fmaf(v.w, tl[c.y >> 16], acc);
+}
+
+// the loads of slice sl (rows.x slices, rows.y the block's first row, rows.z
+// rows; starts Sl): streamed once per step through L2 only, so that L1 keeps
+// the block's basis rows between the passes.  All set before the conditional
+// loads: see ilu_sweep
+__device__ __forceinline__ void op_load(const FusedArgs& a, OpSlice& R, const int* Sl, const int3& rows, int sl,
+                                        int lane) {
+    R.w = 0;
+    R.dg = 0.f;
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {
+        R.v[g] = make_float4(0.f, 0.f, 0.f, 0.f);
+        R.c[g] = make_uint2(0u, 0u);
+    }
+    if (sl >= rows.x) return;
+    const int base = Sl[sl];
+    R.w = (Sl[sl + 1] - base) / kOpGroup;
+    const float4* pv = reinterpret_cast<const float4*>(a.op_val + base) + lane;
+    const uint2* pc = reinterpret_cast<const uint2*>(a.op_lcol + base) + lane;
+#pragma unroll
+    for (int g = 0; g < 4; ++g)
+        if (g < R.w) {
+            R.v[g] = __ldcg(pv + 32 * g);
+            R.c[g] = __ldcg(pc + 32 * g);
+        }
+    R.dg = __ldcg(a.op_dg + rows.y + min(32 * sl + lane, rows.z - 1));
+}
+__device__ __forceinline__ void op_apply(const FusedArgs& a, const OpSlice& R, float* x, const float* tl,
+                                         const int* Sl, const int3& rows, int sl, int lane) {
+    if (sl >= rows.x) return;
+    float acc = 0.f;
+#pragma unroll
+    for (int g = 0; g < 4; ++g)
+        if (g < R.w) op_four(acc, tl, R.v[g], R.c[g]);
+#pragma unroll 1
+    for (int g = 4; g < R.w; ++g)
+        op_four(acc, tl, __ldcg(reinterpret_cast<const float4*>(a.op_val + Sl[sl]) + lane + 32 * g),
+                __ldcg(reinterpret_cast<const uint2*>(a.op_lcol + Sl[sl]) + lane + 32 * g));
+    const int q = 32 * sl + lane;
+    if (q < rows.z) x[q] = fmaf(-a.dcj * R.dg, tl[q], acc);
 }
 
 // at most 384 threads (one per row quad of a 1,536-row block; larger blocks
 // loop), so a thread may hold up to 170 registers
 constexpr int kFusedThreads = 384;
 
-template <int KM, bool DEL>
+template <bool DEL>
 __global__ void __launch_bounds__(kFusedThreads, 1) k_arnoldi_fused(FusedArgs a) {
     // ca holds up to 2 (m + 1) + 2 reduced numbers on the delayed variant
     __shared__ double ca[DEL ? 132 : 64], cb[64], coef[64], sc[64], rc[64], rs[64], gs[64];
@@ -152,47 +213,48 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_arnoldi_fused(FusedArgs a)
     // warp partials of the delayed variant's dot pass (two alternating groups)
     __shared__ double red[DEL ? 2 * (kFusedThreads / 32) * 2 * kCgsGroup : 1];
     __shared__ int s_done, s_ok;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
+    // the factor's place, read again for each sweep: held in registers through
+    // the basis passes, which need them all, it would be spilled
+    __shared__ IluShared<float> s_view;
+    __shared__ int3 s_rows;   // operator slices, first row, rows
+    unsigned char* const smem_raw = ilu_smem();
     const int b = blockIdx.x, nblk = gridDim.x;
     const int r0 = a.bstart[b], r1 = a.bstart[b + 1], nr = r1 - r0;
-    const IluWindow w = ilu_window(a.lu_ptr[r0], a.lu_ptr[r1]);
-    const int la = a.blk_lvl[b], nl = a.blk_lvl[b + 1] - la;
-    const int ua = a.blk_ulvl[b], nu = a.blk_ulvl[b + 1] - ua;
+    const IluBlk B = a.blk[b];
     // staged factor (the layout of k_ilu_apply_smem), then the inverse of
     // the block's row order and its rows of W
-    float* x = reinterpret_cast<float*>(smem_raw);
-    float* val = reinterpret_cast<float*>(smem_raw + round16(sizeof(float) * nr));
-    unsigned short* col = reinterpret_cast<unsigned short*>(val + w.wn);
-    unsigned short* rp = col + w.wn;
-    unsigned short* dg = rp + nr + 1;
-    unsigned short* lrow = dg + nr;
-    unsigned short* urow = lrow + nr;
-    unsigned short* lptr = urow + nr;
-    unsigned short* uptr = lptr + nl + 1;
-    uint64_t* mbar = reinterpret_cast<uint64_t*>(smem_raw + ilu_stage_bytes(nr, w.wn, nl + nu + 2, sizeof(float)) - 16);
+    const IluStage<float> S(B, nr);
+    float* x = S.x;
+    uint64_t* mbar = S.bar;
     unsigned short* inv = reinterpret_cast<unsigned short*>(smem_raw + a.stage_max);
     // the block's rows of W (and of the pending vector), quad-transposed
     const int nqp = a.nqp;
     double* Ws = reinterpret_cast<double*>(smem_raw + a.stage_max + round16(2 * (size_t)a.nr_max));
     float* tl = reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(Ws) + 32 * (size_t)nqp);
     // delayed variant: the block's rows of the pending vector v_k, then the
-    // unrotated Hessenberg matrix (column c at Hs[64 c ..])
+    // unrotated Hessenberg matrix (column c at Hs[hess_words(c) ..])
     double* Vs = reinterpret_cast<double*>(reinterpret_cast<unsigned char*>(tl) + round16(4 * (size_t)a.nh_max));
     double* Hs = Vs + 4 * (size_t)nqp;
     // delayed variant: the block's rows of ewt (quad-transposed, 1 in the
     // edge quads' padding), read by every step's scaling of W and of the
     // next direction instead of going to L2 for them
-    double* Es = Hs + 64 * 64;
-    // delayed variant: the block's node list (its rows, then its halo), for
-    // the gather of every step's direction
+    double* Es = Hs + hess_words(a.m);
+    // delayed variant: the halo's nodes, for the gather of every step's
+    // direction there
     int* Hn = reinterpret_cast<int*>(Es + 4 * (size_t)nqp);
+    // first entry of each of the block's operator slices
+    int* Sl = DEL ? Hn + a.halo_max : reinterpret_cast<int*>(Vs);
     if (threadIdx.x == 0) {
         tc05::mbar_init(mbar, 1);
         asm volatile("fence.mbarrier_init.release.cluster;");
     }
     __syncthreads();
-    const int mo = a.meta_off[b];
-    ilu_stage_bulk(val, col, a.lu, a.lu_col, w, mbar, rp, a.meta + mo, a.meta_off[b + 1] - mo);
+    ilu_stage_bulk(S, B, nr, a.lu, a.lu_col, a.meta);
+    if (threadIdx.x == 0) {
+        x[nr] = 0.f;
+        s_view = S.view(B);
+        s_rows = make_int3(a.blksl[b + 1] - a.blksl[b], r0, nr);
+    }
     for (int q = threadIdx.x; q < nr; q += blockDim.x) inv[a.lu_row[r0 + q] - r0] = (unsigned short)q;
     const int m = a.m;
     const double tol = a.st->tol, sqrtN = a.st->sqrtN;
@@ -231,11 +293,12 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_arnoldi_fused(FusedArgs a)
     const int q0 = r0 & ~3;
     const int h0 = a.halo_ptr[b], nh = a.halo_ptr[b + 1] - h0;
     const int nb0 = a.nbr_ptr[b], nb1 = a.nbr_ptr[b + 1];
+    for (int k = threadIdx.x; k <= nsl; k += blockDim.x) Sl[k] = a.slptr[sl0 + k];
     // step 0's direction s_0 U_0 / ewt at the block's own and halo nodes
     // (U_0 was written before the launch)
     for (int k = threadIdx.x; k < nh; k += blockDim.x) {
         const int node = a.halo_node[h0 + k];
-        if constexpr (DEL) Hn[k] = node;
+        if (DEL && k >= nr) Hn[k - nr] = node;
         tl[k] = (float)(s0 * (double)__ldcg(a.U + node) / a.ewt[node]);
     }
     // the padding rows of the edge quads stay zero
@@ -250,40 +313,28 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_arnoldi_fused(FusedArgs a)
     __syncthreads();
     for (int j = 0;; ++j) {
         const int nv = j + 1;
-        // operator: x = J(cj) t for the block's rows, in factor order; a
-        // warp takes two slices at a time, eight entries of each in flight
-        for (int sl = warp; sl < nsl; sl += 2 * nw) {
-            const int slb = sl + nw < nsl ? sl + nw : sl;
-            const int ea = a.slptr[sl0 + sl] + lane, ea1 = a.slptr[sl0 + sl + 1];
-            const int eb = a.slptr[sl0 + slb] + lane, eb1 = slb != sl ? a.slptr[sl0 + slb + 1] : eb;
-            float acc_a = 0.f, acc_b = 0.f;
-            for (int k = 0; ea + 32 * k < ea1 || eb + 32 * k < eb1; k += 8) {
-                float va[8], vb[8];
-                unsigned short ca_[8], cb_[8];
-#pragma unroll
-                for (int t = 0; t < 8; ++t) {
-                    const int e = ea + 32 * (k + t), f = eb + 32 * (k + t);
-                    // streamed once per step through L2 only, so that L1
-                    // keeps the block's basis rows between the passes
-                    va[t] = e < ea1 ? __ldcg(a.op_val + e) : 0.f;
-                    ca_[t] = e < ea1 ? __ldcg(a.op_lcol + e) : (unsigned short)0;
-                    vb[t] = f < eb1 ? __ldcg(a.op_val + f) : 0.f;
-                    cb_[t] = f < eb1 ? __ldcg(a.op_lcol + f) : (unsigned short)0;
-                }
-#pragma unroll
-                for (int t = 0; t < 8; ++t) {
-                    acc_a = fmaf(va[t], tl[ca_[t]], acc_a);
-                    acc_b = fmaf(vb[t], tl[cb_[t]], acc_b);
-                }
+        // operator: x = J(cj) t for the block's rows, in factor order; a warp
+        // keeps two slices in flight
+        {
+            const int lane = tid_here() & 31, first = tid_here() >> 5;
+            OpSlice A, B;
+            op_load(a, A, Sl, s_rows, first, lane);
+            op_load(a, B, Sl, s_rows, first + nw, lane);
+#pragma unroll 1
+            for (int sl = first; sl < s_rows.x; sl += 2 * nw) {
+                op_apply(a, A, x, tl, Sl, s_rows, sl, lane);
+                op_load(a, A, Sl, s_rows, sl + 2 * nw, lane);
+                op_apply(a, B, x, tl, Sl, s_rows, sl + nw, lane);
+                op_load(a, B, Sl, s_rows, sl + 3 * nw, lane);
             }
-            const int qa = 32 * sl + lane, qb = 32 * slb + lane;
-            if (qa < nr) x[qa] = fmaf(-a.dcj * a.op_dg[r0 + qa], tl[a.op_self[r0 + qa]], acc_a);
-            if (slb != sl && qb < nr) x[qb] = fmaf(-a.dcj * a.op_dg[r0 + qb], tl[a.op_self[r0 + qb]], acc_b);
         }
         __syncthreads();
         // preconditioner: both triangular sweeps in shared memory
-        ilu_sweep<float, KM, false>(x, val, col, rp, dg, lrow, lptr, 1, nl);
-        ilu_sweep<float, KM, true>(x, val, col, rp, dg, urow, uptr, 0, nu);
+        {
+            const IluShared<float> V = s_view;
+            ilu_sweep<float, false>(V, 1, V.nl);
+            ilu_sweep<float, true>(V, 0, V.nu);
+        }
         for (int k = threadIdx.x; k < nr; k += blockDim.x) {
             const int qp = quad_pos(r0, nqp, r0 + k);
             Ws[qp] = (DEL ? Es[qp] : a.ewt[r0 + k]) * (double)x[inv[k]];
@@ -336,7 +387,9 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_arnoldi_fused(FusedArgs a)
                 if (k >= r0 && k < r1) {
                     const float u = (float)(Ws[quad_pos(r0, nqp, k)] - acc[e]);
                     Un[k] = u;
-                    a.tdir[k] = (float)(snv * (double)u / a.ewt[k]);
+                    const float t = (float)(snv * (double)u / a.ewt[k]);
+                    a.tdir[k] = t;
+                    tl[inv[k - r0]] = t;
                 }
             }
         }
@@ -360,8 +413,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_arnoldi_fused(FusedArgs a)
         // four and two; the column of step k is final one step later.
         const int k = j;
         const int nbv = k == 0 ? 1 : k;   // basis vectors this step reads
-        float4 kept[kCgsGroup];
-        block_dots2_by_quad(a.U, a.ld, Vs, Ws, nqp, r0, r1, nbv, red, ca, kept);
+        block_dots2_by_quad(a.U, a.ld, Vs, Ws, nqp, r0, r1, nbv, red, ca);
         const int nred = 2 * nbv + 2;
         for (int i = threadIdx.x; i < nred; i += blockDim.x) pa[(size_t)i * nblk + b] = ca[i];
         if (!fused_sync(a.sync, a.err, &s_ok)) return;
@@ -377,29 +429,43 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_arnoldi_fused(FusedArgs a)
             }
             hcol = -1;
         } else {
-            double tt = 0.0;
-            for (int i = 0; i < k; ++i) {
-                const double t = sc[i] * ca[i];
-                tt += t * t;
-            }
-            const double b2 = ca[2 * k] - tt;
+            // four partial sums each: one chain of k dependent FP64
+            // operations is a microsecond at the end of a cycle
+            double t4[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll 1
+            for (int i = 0; i < k; i += 4)
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const double t = i + u < k ? sc[i + u] * ca[i + u] : 0.0;
+                    t4[u] += t * t;
+                }
+            const double b2 = ca[2 * k] - ((t4[0] + t4[1]) + (t4[2] + t4[3]));
             beta = b2 > 0.0 ? sqrt(b2) : 0.0;
             for (int i = threadIdx.x; i <= k; i += blockDim.x) {
                 const double t = i < k ? sc[i] * ca[i] : 0.0;
                 tv[i] = t;
                 pv[i] = i < k ? sc[i] * ca[k + i] : 0.0;
-                Hs[(size_t)(k - 1) * 64 + i] = i < k ? hp[i] + t : beta;
+                Hs[hess_words(k - 1) + i] = i < k ? hp[i] + t : beta;
             }
             __syncthreads();
             // Ht = H[0..k][0..k-1] t (H[i][c] is zero below c + 1)
             for (int i = threadIdx.x; i <= k; i += blockDim.x) {
-                double acc = 0.0;
-                for (int c = i > 0 ? i - 1 : 0; c < k; ++c) acc += Hs[(size_t)c * 64 + i] * tv[c];
-                htv[i] = acc;
+                double h4[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll 1
+                for (int c = i > 0 ? i - 1 : 0; c < k; c += 4)
+#pragma unroll
+                    for (int u = 0; u < 4; ++u)
+                        if (c + u < k) h4[u] += Hs[hess_words(c + u) + i] * tv[c + u];
+                htv[i] = (h4[0] + h4[1]) + (h4[2] + h4[3]);
             }
+            double p4[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll 1
+            for (int i = 0; i < k; i += 4)
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                    if (i + u < k) p4[u] += tv[i + u] * pv[i + u];
+            const double tp = (p4[0] + p4[1]) + (p4[2] + p4[3]);
             __syncthreads();
-            double tp = 0.0;
-            for (int i = 0; i < k; ++i) tp += tv[i] * pv[i];
             const double rb = beta > 0.0 ? 1.0 / beta : 0.0;
             const double sk = (ca[2 * k + 1] - tp - beta * htv[k]) * rb * rb;
             ck = htv[k] * rb + sk;
@@ -426,8 +492,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_arnoldi_fused(FusedArgs a)
             const double vcoef = k == 0 ? 0.0 : ck * rb;
             for (int r = q0 + 4 * threadIdx.x; r < r1; r += 4 * blockDim.x) {
                 double acc1[4], acc2[4];
-                if (r == q0 + 4 * (int)threadIdx.x) quad_combine2_kept(UR, c1, c2, nbv, r, kept, acc1, acc2);
-                else quad_combine2(UR, c1, c2, nbv, r, acc1, acc2);
+                quad_combine2(UR, c1, c2, nbv, r, acc1, acc2);
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
                     const int q = r + e;
@@ -437,7 +502,9 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_arnoldi_fused(FusedArgs a)
                         if (k >= 1) Uk[q] = (float)(vq - acc1[e]);
                         const double vn = Ws[qp] * rb - vcoef * vq - acc2[e];
                         Vs[qp] = vn;
-                        a.tdir[q] = (float)(vn / Es[qp]);
+                        const float t = (float)(vn / Es[qp]);
+                        a.tdir[q] = t;
+                        tl[inv[q - r0]] = t;
                     }
                 }
             }
@@ -462,14 +529,14 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_arnoldi_fused(FusedArgs a)
                 }
             }
             named_barrier(1, blockDim.x - 32);
-            for (int kk = threadIdx.x - 32; kk < nh; kk += blockDim.x - 32)
-                tl[kk] = __ldcg(a.tdir + (DEL ? Hn[kk] : a.halo_node[h0 + kk]));
+            for (int kk = nr + threadIdx.x - 32; kk < nh; kk += blockDim.x - 32)
+                tl[kk] = __ldcg(a.tdir + (DEL ? Hn[kk - nr] : a.halo_node[h0 + kk]));
         } else if (threadIdx.x == 0) {
             int done = 0;
             if (hcol >= 0) {
                 double* hc = ca;
                 if constexpr (DEL) {
-                    for (int i = 0; i <= hcol; ++i) hc[i] = Hs[(size_t)hcol * 64 + i];
+                    for (int i = 0; i <= hcol; ++i) hc[i] = Hs[hess_words(hcol) + i];
                 }
                 hc[hcol + 1] = hn;
                 if (!isfinite(hn) || !isfinite(hc[hcol])) {
@@ -518,14 +585,20 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_arnoldi_fused(FusedArgs a)
 
 static int fused_sync_slot(int nb) { return ((nb + 31) & ~31) + 32; }
 
-static const void* fused_kernel(int lanes, int variant) {
-    if (lanes == 8) return variant ? (const void*)k_arnoldi_fused<8, true> : (const void*)k_arnoldi_fused<8, false>;
-    return variant ? (const void*)k_arnoldi_fused<4, true> : (const void*)k_arnoldi_fused<4, false>;
+static const void* fused_kernel(int variant) {
+    return variant ? (const void*)k_arnoldi_fused<true> : (const void*)k_arnoldi_fused<false>;
 }
+
+constexpr int kFusedMaxDim = 62;   // the reduced numbers' arrays
 
 // Gram-Schmidt of the fused cycle on this context: 0 CGS2 (two projections,
 // two grid barriers per step), 1 delayed reorthogonalisation (DCGS2)
 static int fused_variant(const fvm_ctx* c) { return c->krylov_variant ? 1 : 0; }
+
+// dynamic shared bytes of a cycle of up to m steps
+static size_t fused_bytes(const BlockILU* P, int variant, int m) {
+    return variant ? P->fused_smem_d + 8 * (size_t)hess_words(m) : P->fused_smem;
+}
 
 // values of the operator's slices from the set-up's Jacobian (FP64 CSR) and
 // the cj coefficient of its diagonal, in factor order
@@ -551,7 +624,7 @@ bool fused_prepare(fvm_ctx* c, int m) {
     BlockILU* P = c->ilu;
     // the cycle inlines the block-Jacobi apply; the Schur-coupled apply
     // runs as its own cooperative launch between the separate kernels
-    if (!P || !P->built || P->factored != 1 || m + 2 > 64 || P->schur_iters >= 0) return false;
+    if (!P || !P->built || P->factored != 1 || m > kFusedMaxDim || P->schur_iters >= 0) return false;
     cudaStream_t s = c->stream;
     if (!P->op_built) {
         P->op_built = true;
@@ -560,9 +633,9 @@ bool fused_prepare(fvm_ctx* c, int m) {
         if (!P->smem_stage[1]) return false;
         std::vector<int> slptr(1, 0), blksl(1, 0), opcol, opsrc;
         std::vector<int> halo_ptr(1, 0), halo_node, nbr_ptr(1, 0), nbr;
-        std::vector<unsigned short> lcol, self(c->N);
+        std::vector<unsigned short> lcol;
         std::vector<int> where(c->N, -1);
-        int nr_max = 0, nh_max = 0;
+        int nr_max = 0, nh_max = 0, halo_max = 0;
         for (int b = 0; b < nb; ++b) {
             const int r0 = P->h_bstart[b], r1 = P->h_bstart[b + 1];
             nr_max = std::max(nr_max, r1 - r0);
@@ -574,6 +647,7 @@ bool fused_prepare(fvm_ctx* c, int m) {
                     const int row = P->h_lu_row[q0 + l];
                     width = std::max(width, P->h_rowptr[row + 1] - P->h_rowptr[row]);
                 }
+                width = (width + 3) & ~3;
                 const size_t base = opcol.size();
                 opcol.resize(base + 32 * (size_t)width);
                 opsrc.resize(base + 32 * (size_t)width);
@@ -581,28 +655,37 @@ bool fused_prepare(fvm_ctx* c, int m) {
                     const int row = l < n ? P->h_lu_row[q0 + l] : P->h_lu_row[q0];
                     const int p0 = P->h_rowptr[row], len = l < n ? P->h_rowptr[row + 1] - p0 : 0;
                     for (int k = 0; k < width; ++k) {
-                        opcol[base + 32 * (size_t)k + l] = k < len ? P->h_col[p0 + k] : row;
-                        opsrc[base + 32 * (size_t)k + l] = k < len ? p0 + k : -1;
+                        const size_t e = base + (size_t)kOpGroup * (k / 4) + 4 * l + k % 4;
+                        opcol[e] = k < len ? P->h_col[p0 + k] : row;
+                        opsrc[e] = k < len ? p0 + k : -1;
                     }
                 }
                 if (opcol.size() >= (size_t)INT32_MAX) return false;
                 slptr.push_back((int)opcol.size());
             }
             blksl.push_back((int)slptr.size() - 1);
-            // the block's node list (its operator columns, sorted), local
-            // column indices, and the blocks owning those nodes
-            std::vector<int> nodes(opcol.begin() + ebase, opcol.end());
-            std::sort(nodes.begin(), nodes.end());
-            nodes.erase(std::unique(nodes.begin(), nodes.end()), nodes.end());
+            // the block's node list (its rows in factor order, then the other
+            // operator columns, sorted), local column indices, and the blocks
+            // owning those nodes.  A slice's rows have one colour and are
+            // consecutive in factor order, and so are, mostly, their
+            // neighbours of another colour: a warp's reads of the direction
+            // hit few banks twice (in node order, eight lanes to a bank)
+            std::vector<int> halo;
+            for (size_t e = ebase; e < opcol.size(); ++e)
+                if (opcol[e] < r0 || opcol[e] >= r1) halo.push_back(opcol[e]);
+            std::sort(halo.begin(), halo.end());
+            halo.erase(std::unique(halo.begin(), halo.end()), halo.end());
+            std::vector<int> nodes(P->h_lu_row.begin() + r0, P->h_lu_row.begin() + r1);
+            nodes.insert(nodes.end(), halo.begin(), halo.end());
             if (nodes.size() >= 65535) return false;
             nh_max = std::max(nh_max, (int)nodes.size());
+            halo_max = std::max(halo_max, (int)halo.size());
             for (size_t k = 0; k < nodes.size(); ++k) where[nodes[k]] = (int)k;
             for (size_t e = ebase; e < opcol.size(); ++e) lcol.push_back((unsigned short)where[opcol[e]]);
-            for (int q = r0; q < r1; ++q) self[q] = (unsigned short)where[P->h_lu_row[q]];
             std::vector<int> nbs;
             if (b > 0) nbs.push_back(b - 1);
             if (b + 1 < nb) nbs.push_back(b + 1);
-            for (int v : nodes) {
+            for (int v : halo) {
                 const int ob = (int)(std::upper_bound(P->h_bstart.begin(), P->h_bstart.end(), v) - P->h_bstart.begin()) - 1;
                 if (ob != b) nbs.push_back(ob);
             }
@@ -617,7 +700,6 @@ bool fused_prepare(fvm_ctx* c, int m) {
         P->op_slptr.upload(slptr, s);
         P->op_blksl.upload(blksl, s);
         P->op_lcol.upload(lcol, s);
-        P->op_self.upload(self, s);
         P->op_src.upload(opsrc, s);
         {
             // the slice position of every Jacobian entry, for the set-up
@@ -637,18 +719,21 @@ bool fused_prepare(fvm_ctx* c, int m) {
         P->op_dg.alloc(c->N);
         P->fused_nrmax = nr_max;
         P->fused_nhmax = nh_max;
+        P->fused_hmax = halo_max;
         P->fused_stage = round16(P->smem_stage[1]);
         // CGS2: staged factor | row order | rows of W | direction at the
         // block's nodes; the delayed variant adds the pending vector's rows
-        // and the unrotated Hessenberg matrix (64 x 64), then the block's
-        // rows of ewt and its node list
+        // and (by the cycle's length, fused_smem) the unrotated Hessenberg
+        // matrix, then the block's rows of ewt and its node list; both the
+        // slices' starts
         // block row arrays quad-transposed: nqp quads cover any block's rows
         // from its first quad boundary
         P->fused_nqp = nr_max / 4 + 2;
         const size_t rows = 32 * (size_t)P->fused_nqp;
         const size_t base = P->fused_stage + round16(2 * (size_t)nr_max) + rows;
-        P->fused_smem = base + 4 * (size_t)nh_max;
-        P->fused_smem_d = base + round16(4 * (size_t)nh_max) + rows + 8 * 64 * 64 + rows + round16(4 * (size_t)nh_max);
+        const size_t slices = 4 * ((size_t)(nr_max + 31) / 32 + 1);
+        P->fused_smem = base + round16(4 * (size_t)nh_max) + slices;
+        P->fused_smem_d = base + round16(4 * (size_t)nh_max) + rows + rows + 4 * (size_t)halo_max + slices;
         // one thread per row quad of the largest block, whole warps
         P->fused_threads = std::min(kFusedThreads, std::max(128, ((nr_max + 3) / 4 + 1 + 31) / 32 * 32));
         int dev = 0, coop = 0, nsm = 0;
@@ -656,16 +741,18 @@ bool fused_prepare(fvm_ctx* c, int m) {
         FVM_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
         FVM_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
         for (int v = 0; v < 2; ++v) {
-            const size_t smem = v ? P->fused_smem_d : P->fused_smem;
+            const void* kfn = fused_kernel(v);
+            cudaFuncAttributes fa;
+            FVM_CUDA(cudaFuncGetAttributes(&fa, kfn));
+            P->fused_room[v] = kMaxDynSmem - fa.sharedSizeBytes;
             P->fused_var_ok[v] = false;
-            if (smem > kMaxDynSmem) continue;
-            const void* kfn = fused_kernel(P->lanes, v);
+            if (fused_bytes(P, v, 1) > P->fused_room[v]) continue;
+            // enough for the longest cycle, or what there is
+            const size_t smem = std::min(P->fused_room[v], fused_bytes(P, v, kFusedMaxDim));
             raise_smem_limit(kfn, smem);
             // the smallest shared-memory carveout that holds the block's
             // shared data (dynamic + static, about 1 KB reserved), so that
             // the rest of the SM's 256 KB stays L1 for the block's basis rows
-            cudaFuncAttributes fa;
-            FVM_CUDA(cudaFuncGetAttributes(&fa, kfn));
             const double need = (double)(smem + fa.sharedSizeBytes + 1024);
             const int pct = std::min(100, (int)std::ceil(100.0 * need / (228.0 * 1024.0)));
             FVM_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributePreferredSharedMemoryCarveout, pct));
@@ -675,7 +762,8 @@ bool fused_prepare(fvm_ctx* c, int m) {
         }
         P->fused_ok = P->fused_var_ok[0] || P->fused_var_ok[1];
     }
-    if (!P->fused_ok || !P->fused_var_ok[fused_variant(c)]) return false;
+    const int var = fused_variant(c);
+    if (!P->fused_ok || !P->fused_var_ok[var] || fused_bytes(P, var, m) > P->fused_room[var]) return false;
     if (P->op_setup_id != P->setup_id) {
         // the values come from the set-up's kernels once the layout exists;
         // the first set-up after the layout was built copies them here
@@ -701,6 +789,7 @@ void fused_cycle(fvm_ctx* c, Krylov* K, double cj, const double* ewt, double* H_
     a.nr_max = P->fused_nrmax;
     a.nqp = P->fused_nqp;
     a.nh_max = P->fused_nhmax;
+    a.halo_max = P->fused_hmax;
     a.stage_max = P->fused_stage;
     a.st = K->st.p;
     a.U = U;
@@ -711,7 +800,6 @@ void fused_cycle(fvm_ctx* c, Krylov* K, double cj, const double* ewt, double* H_
     a.slptr = P->op_slptr.p;
     a.blksl = P->op_blksl.p;
     a.op_lcol = P->op_lcol.p;
-    a.op_self = P->op_self.p;
     a.halo_ptr = P->halo_ptr.p;
     a.halo_node = P->halo_node.p;
     a.nbr_ptr = P->nbr_ptr.p;
@@ -722,12 +810,9 @@ void fused_cycle(fvm_ctx* c, Krylov* K, double cj, const double* ewt, double* H_
     a.op_dg = P->op_dg.p;
     a.dcj = (float)(cj - P->cj_setup);
     a.bstart = P->bstart.p;
-    a.lu_ptr = P->lu_ptr.p;
+    a.blk = P->blk.p;
     a.lu_col = P->lu_col.p;
     a.meta = P->meta.p;
-    a.meta_off = P->meta_off.p;
-    a.blk_lvl = P->blk_lvl.p;
-    a.blk_ulvl = P->blk_ulvl.p;
     a.lu = P->lu32.p;
     a.lu_row = P->lu_row.p;
     a.beta2 = K->res.p;
@@ -741,7 +826,7 @@ void fused_cycle(fvm_ctx* c, Krylov* K, double cj, const double* ewt, double* H_
     cfg.gridDim = dim3(P->nb);
     cfg.blockDim = dim3(P->fused_threads);
     const int var = fused_variant(c);
-    cfg.dynamicSmemBytes = var ? P->fused_smem_d : P->fused_smem;
+    cfg.dynamicSmemBytes = fused_bytes(P, var, K->m);
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeCooperative;
@@ -750,13 +835,8 @@ void fused_cycle(fvm_ctx* c, Krylov* K, double cj, const double* ewt, double* H_
     cfg.numAttrs = 1;
     P->flags.zero(s);
     c->tm.begin(TM_CGS, s);
-    if (P->lanes == 8) {
-        if (var) FVM_CUDA(cudaLaunchKernelEx(&cfg, k_arnoldi_fused<8, true>, a));
-        else FVM_CUDA(cudaLaunchKernelEx(&cfg, k_arnoldi_fused<8, false>, a));
-    } else {
-        if (var) FVM_CUDA(cudaLaunchKernelEx(&cfg, k_arnoldi_fused<4, true>, a));
-        else FVM_CUDA(cudaLaunchKernelEx(&cfg, k_arnoldi_fused<4, false>, a));
-    }
+    if (var) FVM_CUDA(cudaLaunchKernelEx(&cfg, k_arnoldi_fused<true>, a));
+    else FVM_CUDA(cudaLaunchKernelEx(&cfg, k_arnoldi_fused<false>, a));
     c->tm.end(TM_CGS, s);
     c->launches++;
 }

@@ -350,56 +350,46 @@ __device__ __forceinline__ void block_dots2_by_warp(const float* __restrict__ U,
 // (index b1 + 2 b2 + 4 b3 + 8 b4 of its lane bits) summed over 16 lanes, and
 // offset 1 completes it; 16 exchanges instead of 5 per value.  The warps'
 // sums are then added in warp order.  red holds 2 x (warps x 2 kCgsGroup)
-// doubles (alternating groups, so one barrier per group).  keep receives
-// the thread's first quad of the last group's vectors (from kept_first(nb)
-// on, zeros past nb - 1), for a later pass over the same rows.
-__host__ __device__ inline int kept_first(int nb) { return nb & ~(kCgsGroup - 1); }
+// doubles (alternating groups, so one barrier per group).
 __device__ __forceinline__ void block_dots2_by_quad(const float* __restrict__ U, size_t ld,
                                                     const double* __restrict__ A, const double* __restrict__ Bv,
-                                                    int nqp, int k0, int k1, int nb, double* red, double* out,
-                                                    float4 (&keep)[kCgsGroup]) {
+                                                    int nqp, int k0, int k1, int nb, double* red, double* out) {
     constexpr int G = kCgsGroup, NV = 2 * kCgsGroup;
     static_assert(NV == 16, "the butterfly below reduces 16 values per lane");
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
     const int a0 = k0 & ~3;
     const int nq = (k1 - a0 + 3) >> 2;
     const int idx = ((lane >> 1) & 1) | (((lane >> 2) & 1) << 1) | (((lane >> 3) & 1) << 2) | (((lane >> 4) & 1) << 3);
-    int buf = 0;
-    for (int i0 = 0; i0 <= nb; i0 += G, buf ^= 1) {
-        double v[NV];
+    // one group: the quads' products, then the reduction into out
+    auto quad = [&](int i0, int q, double (&v)[NV]) {
+        float4 u[G];
 #pragma unroll
-        for (int j = 0; j < NV; ++j) v[j] = 0.0;
-        for (int q = threadIdx.x; q < nq; q += blockDim.x) {
-            float4 u[G];
+        for (int g = 0; g < G; ++g) {
+            const int i = i0 + g;
+            u[g] = i < nb ? __ldg(reinterpret_cast<const float4*>(U + ld * i + a0 + 4 * q))
+                          : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        double x[4], y[4];
 #pragma unroll
-            for (int g = 0; g < G; ++g) {
-                const int i = i0 + g;
-                u[g] = i < nb ? __ldg(reinterpret_cast<const float4*>(U + ld * i + a0 + 4 * q))
-                              : make_float4(0.f, 0.f, 0.f, 0.f);
-            }
-            if (i0 + G > nb && q == (int)threadIdx.x) {
+        for (int e = 0; e < 4; ++e) {
+            x[e] = A[e * nqp + q];
+            y[e] = Bv[e * nqp + q];
+        }
 #pragma unroll
-                for (int g = 0; g < G; ++g) keep[g] = u[g];
-            }
-            double x[4], y[4];
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                x[e] = A[e * nqp + q];
-                y[e] = Bv[e * nqp + q];
-            }
-#pragma unroll
-            for (int g = 0; g < G; ++g) {
-                const int i = i0 + g;
-                if (i < nb) {
-                    const double u0 = u[g].x, u1 = u[g].y, u2 = u[g].z, u3 = u[g].w;
-                    v[2 * g] += u0 * x[0] + u1 * x[1] + u2 * x[2] + u3 * x[3];
-                    v[2 * g + 1] += u0 * y[0] + u1 * y[1] + u2 * y[2] + u3 * y[3];
-                } else if (i == nb) {
-                    v[2 * g] += x[0] * x[0] + x[1] * x[1] + x[2] * x[2] + x[3] * x[3];
-                    v[2 * g + 1] += x[0] * y[0] + x[1] * y[1] + x[2] * y[2] + x[3] * y[3];
-                }
+        for (int g = 0; g < G; ++g) {
+            const int i = i0 + g;
+            if (i < nb) {
+                const double u0 = u[g].x, u1 = u[g].y, u2 = u[g].z, u3 = u[g].w;
+                v[2 * g] += u0 * x[0] + u1 * x[1] + u2 * x[2] + u3 * x[3];
+                v[2 * g + 1] += u0 * y[0] + u1 * y[1] + u2 * y[2] + u3 * y[3];
+            } else if (i == nb) {
+                v[2 * g] += x[0] * x[0] + x[1] * x[1] + x[2] * x[2] + x[3] * x[3];
+                v[2 * g + 1] += x[0] * y[0] + x[1] * y[1] + x[2] * y[2] + x[3] * y[3];
             }
         }
+    };
+    int buf = 0;
+    auto reduce = [&](int i0, double (&v)[NV]) {
 #pragma unroll
         for (int s = 0; s < 4; ++s) {
             const int o = 16 >> s, c = NV >> (s + 1);
@@ -413,6 +403,7 @@ __device__ __forceinline__ void block_dots2_by_quad(const float* __restrict__ U,
         }
         v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
         double* rb = red + buf * nw * NV;
+        buf ^= 1;
         if (!(lane & 1)) rb[warp * NV + idx] = v[0];
         __syncthreads();
         if (threadIdx.x < NV) {
@@ -424,47 +415,17 @@ __device__ __forceinline__ void block_dots2_by_quad(const float* __restrict__ U,
                 else out[2 * nb + (threadIdx.x & 1)] = t;
             }
         }
+    };
+#pragma unroll 1
+    for (int i0 = 0; i0 <= nb; i0 += G) {
+        double v[NV];
+#pragma unroll
+        for (int j = 0; j < NV; ++j) v[j] = 0.0;
+#pragma unroll 1
+        for (int q = threadIdx.x; q < nq; q += blockDim.x) quad(i0, q, v);
+        reduce(i0, v);
     }
     __syncthreads();
-}
-
-// quad_combine2 for a row quad whose vectors from kept_first(nv) on are
-// already in registers (keep, from block_dots2_by_quad): those first, then
-// the others loaded kCgsGroup at a time
-template <class B, bool CG>
-__device__ __forceinline__ void quad_combine2_kept(const BasisRows<B, CG>& U, const double* c1, const double* c2,
-                                                   int nv, int r, const float4 (&keep)[kCgsGroup], double acc1[4],
-                                                   double acc2[4]) {
-    const int i1 = kept_first(nv);
-#pragma unroll
-    for (int e = 0; e < 4; ++e) acc1[e] = acc2[e] = 0.0;
-#pragma unroll
-    for (int q = 0; q < kCgsGroup; ++q) {
-        const int i = i1 + q;
-        if (i < nv) {
-            const double u[4] = {keep[q].x, keep[q].y, keep[q].z, keep[q].w};
-            const double a = c1[i], b = c2[i];
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                acc1[e] += a * u[e];
-                acc2[e] += b * u[e];
-            }
-        }
-    }
-    for (int i0 = 0; i0 < i1; i0 += kCgsGroup) {
-#pragma unroll
-        for (int q = 0; q < kCgsGroup; ++q) {
-            const int i = i0 + q;
-            double u[4];
-            U.quad(i, r, u);
-            const double a = c1[i], b = c2[i];
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                acc1[e] += a * u[e];
-                acc2[e] += b * u[e];
-            }
-        }
-    }
 }
 
 // acc1[e] = sum_i c1[i] U_i[r + e], acc2[e] = sum_i c2[i] U_i[r + e] (e < 4)

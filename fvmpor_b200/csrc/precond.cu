@@ -215,7 +215,7 @@ __host__ __device__ inline int fd_list_offs(int ng) { return (ng + 8) & ~7; }
 // entry to FP32 anyway); all sums are FP64.
 template <int NPE, int NFE, bool RC, bool MZ, class S>
 __global__ void __launch_bounds__(kFdThreads, 4) k_fd_chunk(FdArgs a) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
+    unsigned char* const smem_raw = ilu_smem();
     const FdSmem L(NPE, RC, MZ, sizeof(S), a.nnmax, a.list_max, a.grp_max);
     S* slots = reinterpret_cast<S*>(smem_raw);
     double* sh = reinterpret_cast<double*>(smem_raw + L.nodes);
@@ -409,143 +409,124 @@ __global__ void k_fd_shared(int n, const int4* __restrict__ at, const int* __res
     out.store<S>(w, s, scale, w.w & 1, diag);
 }
 
+// Factorisation and sweeps of a block whose window does not fit into shared
+// memory, in place in global memory.  Row i's entries in column order: its
+// lower ones, the pivot, its upper ones (up[] gives an upper lane's place).
 template <class T>
-__global__ void __launch_bounds__(128) k_ilu_factor(const int* __restrict__ bstart,
-                                                    const int* __restrict__ lu_ptr,
+__global__ void __launch_bounds__(128) k_ilu_factor(const int* __restrict__ bstart, const IluBlk* __restrict__ blk,
+                                                    const unsigned short* __restrict__ meta, const int* __restrict__ up,
                                                     const T* __restrict__ Jw,
-                                                    const int* __restrict__ lu_diag,
-                                                    const unsigned short* __restrict__ lu_col,
-                                                    const int* __restrict__ lvl_ptr,
-                                                    const int* __restrict__ lvl_rows,
-                                                    const int* __restrict__ blk_lvl, T* lu,
-                                                    int* status) {
-    int b = blockIdx.x;
-    int r0 = bstart[b], r1 = bstart[b + 1];
-    for (int p = lu_ptr[r0] + threadIdx.x; p < lu_ptr[r1]; p += blockDim.x) lu[p] = Jw[p];
+                                                    const unsigned short* __restrict__ lu_col, T* lu, int* status) {
+    const IluBlk B = blk[blockIdx.x];
+    const int r0 = bstart[blockIdx.x], nr = bstart[blockIdx.x + 1] - r0;
+    const long wn = (long)ilu_window(nr, B.dp);
+    T* val = lu + B.v0;
+    for (long p = threadIdx.x; p < wn; p += blockDim.x) val[p] = Jw[B.v0 + p];
     __syncthreads();
-    for (int l = blk_lvl[b]; l < blk_lvl[b + 1]; ++l) {
-        for (int q = lvl_ptr[l] + threadIdx.x; q < lvl_ptr[l + 1]; q += blockDim.x) {
-            int i = lvl_rows[q];
-            int s = lu_ptr[i], e = lu_ptr[i + 1], di = lu_diag[i];
-            for (int kk = s; kk < di; ++kk) {
-                int k = r0 + lu_col[kk];
-                T lik = lu[kk] * lu[lu_diag[k]];
-                lu[kk] = lik;
-                int kpos = lu_diag[k] + 1, kend = lu_ptr[k + 1];
-                for (int jj = kk + 1; jj < e && kpos < kend; ++jj) {
-                    int j = lu_col[jj];
-                    while (kpos < kend && lu_col[kpos] < j) ++kpos;
-                    if (kpos < kend && lu_col[kpos] == j) lu[jj] = lu[jj] - lik * lu[kpos];
+    const auto V = ilu_view<IluGlobal<T>>(B, val, lu_col + B.c0, meta + B.mo);
+    const int D = 32 * B.dp;
+    for (int l = 0; l < B.nl; ++l) {
+        for (int q = 32 * ilu_level(V, false, l) + threadIdx.x; q < 32 * ilu_level(V, false, l + 1); q += blockDim.x) {
+            const int i = ilu_row(V, false, q);
+            if (i == kIluNoRow) continue;
+            const int w = ilu_start(V, false, (q >> 5) + 1) - ilu_start(V, false, q >> 5);
+            const int lo = 32 * ilu_start(V, false, q >> 5) + (q & 31);
+            const int ui = up[r0 + i], ai = ilu_start(V, true, ui >> 5);
+            const int uwi = ilu_start(V, true, (ui >> 5) + 1) - ai, hi = 32 * ai + (ui & 31);
+            for (int kk = 0; kk < w; ++kk) {
+                const int k = (int)V.col(lo + 32 * kk);
+                if (k == nr) break;
+                const T lik = val[lo + 32 * kk] * val[D + k];
+                val[lo + 32 * kk] = lik;
+                // U(k) against the rest of row i
+                const int uk = up[r0 + k], ak = ilu_start(V, true, uk >> 5);
+                const int uwk = ilu_start(V, true, (uk >> 5) + 1) - ak, hk = 32 * ak + (uk & 31);
+                int a = kk + 1, c = 0;
+                for (int u = 0; u < uwk; ++u) {
+                    const int j = (int)V.col(hk + 32 * u);
+                    if (j == nr) break;
+                    int at = -1;
+                    if (j < i) {
+                        while (a < w && (int)V.col(lo + 32 * a) < j) ++a;
+                        if (a < w && (int)V.col(lo + 32 * a) == j) at = lo + 32 * a;
+                    } else if (j == i) {
+                        at = D + i;
+                    } else {
+                        while (c < uwi && (int)V.col(hi + 32 * c) < j) ++c;
+                        if (c < uwi && (int)V.col(hi + 32 * c) == j) at = hi + 32 * c;
+                    }
+                    if (at >= 0) val[at] = val[at] - lik * val[hk + 32 * u];
                 }
             }
-            T d = lu[di];
+            T d = val[D + i];
             if (d == (T)0 || !isfinite((double)d)) {
                 atomicExch(status, 1);
                 d = (T)1;
             }
-            lu[di] = (T)1 / d;
+            val[D + i] = (T)1 / d;
         }
         __syncthreads();
     }
 }
 
 template <class T>
-__global__ void __launch_bounds__(128) k_ilu_apply(const int* __restrict__ bstart,
-                                                   const int* __restrict__ lu_ptr,
-                                                   const int* __restrict__ lu_diag,
+__global__ void __launch_bounds__(128) k_ilu_apply(const int* __restrict__ bstart, const IluBlk* __restrict__ blk,
                                                    const unsigned short* __restrict__ lu_col,
-                                                   const int* __restrict__ lvl_ptr,
-                                                   const int* __restrict__ lvl_rows,
-                                                   const int* __restrict__ blk_lvl,
-                                                   const int* __restrict__ ulvl_ptr,
-                                                   const int* __restrict__ ulvl_rows,
-                                                   const int* __restrict__ blk_ulvl,
-                                                   const T* __restrict__ lu, const int* __restrict__ lu_row,
-                                                   const double* __restrict__ r,
+                                                   const unsigned short* __restrict__ meta, const T* __restrict__ lu,
+                                                   const int* __restrict__ lu_row, const double* __restrict__ r,
                                                    double* __restrict__ z, const int* __restrict__ skip) {
-    extern __shared__ unsigned char smem_raw[];
+    unsigned char* const smem_raw = ilu_smem();
     pdl_wait_and_trigger();
     if (skip && *skip) return;
     T* x = reinterpret_cast<T*>(smem_raw);
-    int b = blockIdx.x;
-    int r0 = bstart[b], r1 = bstart[b + 1];
-    for (int i = r0 + threadIdx.x; i < r1; i += blockDim.x) x[i - r0] = (T)r[lu_row[i]];
+    const IluBlk B = blk[blockIdx.x];
+    const int r0 = bstart[blockIdx.x], nr = bstart[blockIdx.x + 1] - r0;
+    for (int i = threadIdx.x; i < nr; i += blockDim.x) x[i] = (T)r[lu_row[r0 + i]];
+    if (threadIdx.x == 0) x[nr] = (T)0;
     __syncthreads();
-    // forward: unit lower triangle
-    for (int l = blk_lvl[b] + 1; l < blk_lvl[b + 1]; ++l) {
-        for (int q = lvl_ptr[l] + threadIdx.x; q < lvl_ptr[l + 1]; q += blockDim.x) {
-            int i = lvl_rows[q];
-            T acc = x[i - r0];
-            for (int p = lu_ptr[i]; p < lu_diag[i]; ++p) acc -= lu[p] * x[lu_col[p]];
-            x[i - r0] = acc;
-        }
-        __syncthreads();
-    }
-    // backward: upper triangle with inverted pivots
-    for (int l = blk_ulvl[b]; l < blk_ulvl[b + 1]; ++l) {
-        for (int q = ulvl_ptr[l] + threadIdx.x; q < ulvl_ptr[l + 1]; q += blockDim.x) {
-            int i = ulvl_rows[q];
-            int di = lu_diag[i];
-            T acc = x[i - r0];
-            for (int p = di + 1; p < lu_ptr[i + 1]; ++p) acc -= lu[p] * x[lu_col[p]];
-            x[i - r0] = acc * lu[di];
-        }
-        __syncthreads();
-    }
-    for (int i = r0 + threadIdx.x; i < r1; i += blockDim.x) z[lu_row[i]] = (double)x[i - r0];
+    const auto V = ilu_view<IluGlobal<T>>(B, lu + B.v0, lu_col + B.c0, meta + B.mo);
+    // level 0 of the lower sweep has no off-diagonal entries
+    ilu_sweep<T, false>(V, 1, V.nl);
+    ilu_sweep<T, true>(V, 0, V.nu);
+    for (int i = threadIdx.x; i < nr; i += blockDim.x) z[lu_row[r0 + i]] = (double)x[i];
 }
 
-template <class T, int KM>
-__global__ void __launch_bounds__(kIluThreads) k_ilu_apply_smem(const int* __restrict__ bstart,
-                                                        const int* __restrict__ lu_ptr,
+template <class T>
+__global__ void __launch_bounds__(kIluThreads, 1) k_ilu_apply_smem(const int* __restrict__ bstart,
+                                                        const IluBlk* __restrict__ blk,
                                                         const unsigned short* __restrict__ lu_col,
                                                         const unsigned short* __restrict__ meta,
-                                                        const int* __restrict__ meta_off,
-                                                        const int* __restrict__ blk_lvl,
-                                                        const int* __restrict__ blk_ulvl,
                                                         const T* __restrict__ lu,
                                                         const int* __restrict__ lu_row,
                                                         const double* __restrict__ r,
                                                         double* __restrict__ z, int* __restrict__ err,
                                                         const int* __restrict__ skip) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int b = blockIdx.x;
-    const int r0 = bstart[b], r1 = bstart[b + 1], nr = r1 - r0;
-    const IluWindow w = ilu_window(lu_ptr[r0], lu_ptr[r1]);
-    const int la = blk_lvl[b], nl = blk_lvl[b + 1] - la;
-    const int ua = blk_ulvl[b], nu = blk_ulvl[b + 1] - ua;
-    T* x = reinterpret_cast<T*>(smem_raw);
-    T* val = reinterpret_cast<T*>(smem_raw + round16(sizeof(T) * nr));
-    unsigned short* col = reinterpret_cast<unsigned short*>(val + w.wn);
-    unsigned short* rp = col + w.wn;
-    unsigned short* dg = rp + nr + 1;
-    unsigned short* lrow = dg + nr;
-    unsigned short* urow = lrow + nr;
-    unsigned short* lptr = urow + nr;
-    unsigned short* uptr = lptr + nl + 1;
-    uint64_t* bar = reinterpret_cast<uint64_t*>(smem_raw + ilu_stage_bytes(nr, w.wn, nl + nu + 2, sizeof(T)) - 16);
+    unsigned char* const smem_raw = ilu_smem();
+    const IluBlk B = blk[blockIdx.x];
+    const int r0 = bstart[blockIdx.x], nr = bstart[blockIdx.x + 1] - r0;
+    const IluStage<T> S(B, nr);
+    T* x = S.x;
     if (threadIdx.x == 0) {
-        tc05::mbar_init(bar, 1);
+        tc05::mbar_init(S.bar, 1);
         asm volatile("fence.mbarrier_init.release.cluster;");
     }
     __syncthreads();
-    // factor window and the block's metadata record (row pointers, pivot
-    // positions, level lists) by three bulk copies; the right-hand side by
-    // the threads meanwhile.  The copies read only set-up data, so they are
-    // issued before the wait for the previous kernel (the factorisation has
-    // completed before any kernel that lets this launch start early); the
-    // right-hand side and the skip flag are read after it.
-    const int mo = meta_off[b];
-    ilu_stage_bulk(val, col, lu, lu_col, w, bar, rp, meta + mo, meta_off[b + 1] - mo);
+    // factor window, columns and the block's record by three bulk copies; the
+    // right-hand side by the threads meanwhile.  The copies read only set-up
+    // data, so they are issued before the wait for the previous kernel (the
+    // factorisation has completed before any kernel that lets this launch
+    // start early); the right-hand side and the skip flag are read after it.
+    ilu_stage_bulk(S, B, nr, lu, lu_col, meta);
     pdl_wait_and_trigger();
     if (skip && *skip) {
         // a step queued after the stop: let the copies land (bounded), leave
-        tc05::mbar_wait(bar, 0);
+        tc05::mbar_wait(S.bar, 0);
         return;
     }
     for (int i = threadIdx.x; i < nr; i += blockDim.x) x[i] = (T)r[lu_row[r0 + i]];
-    bool ok = tc05::mbar_wait(bar, 0);
-    if (!ok) ok = tc05::mbar_wait(bar, 0);   // copies in flight get a second bounded chance
+    if (threadIdx.x == 0) x[nr] = (T)0;
+    bool ok = tc05::mbar_wait(S.bar, 0);
+    if (!ok) ok = tc05::mbar_wait(S.bar, 0);   // copies in flight get a second bounded chance
     if (!__syncthreads_and(ok ? 1 : 0)) {
         // the factor never arrived: report it and pass the vector through
         // unpreconditioned instead of reading unfilled shared memory
@@ -553,9 +534,10 @@ __global__ void __launch_bounds__(kIluThreads) k_ilu_apply_smem(const int* __res
         for (int i = threadIdx.x; i < nr; i += blockDim.x) z[lu_row[r0 + i]] = (double)x[i];
         return;
     }
+    const IluShared<T> V = S.view(B);
     // level 0 of the lower sweep has no off-diagonal entries
-    ilu_sweep<T, KM, false>(x, val, col, rp, dg, lrow, lptr, 1, nl);
-    ilu_sweep<T, KM, true>(x, val, col, rp, dg, urow, uptr, 0, nu);
+    ilu_sweep<T, false>(V, 1, V.nl);
+    ilu_sweep<T, true>(V, 0, V.nu);
     for (int i = threadIdx.x; i < nr; i += blockDim.x) z[lu_row[r0 + i]] = (double)x[i];
 }
 
@@ -583,12 +565,9 @@ template <class T> struct SchurArgs {
     int N, iters;
     size_t stage_max;          // offset of the forward result in shared memory
     const int* bstart;
-    const int* lu_ptr;
+    const IluBlk* blk;
     const unsigned short* lu_col;
     const unsigned short* meta;
-    const int* meta_off;
-    const int* blk_lvl;
-    const int* blk_ulvl;
     const T* lu;
     const int* lu_row;
     const int* sch_lv;
@@ -606,32 +585,22 @@ template <class T> struct SchurArgs {
     const int* skip;
 };
 
-template <class T, int KM>
-__global__ void __launch_bounds__(kIluThreads) k_ilu_apply_schur(SchurArgs<T> a) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
+template <class T>
+__global__ void __launch_bounds__(kIluThreads, 1) k_ilu_apply_schur(SchurArgs<T> a) {
+    unsigned char* const smem_raw = ilu_smem();
     const int b = blockIdx.x;
-    const int r0 = a.bstart[b], r1 = a.bstart[b + 1], nr = r1 - r0;
-    const IluWindow w = ilu_window(a.lu_ptr[r0], a.lu_ptr[r1]);
-    const int la = a.blk_lvl[b], nl = a.blk_lvl[b + 1] - la;
-    const int ua = a.blk_ulvl[b], nu = a.blk_ulvl[b + 1] - ua;
-    T* x = reinterpret_cast<T*>(smem_raw);
-    T* val = reinterpret_cast<T*>(smem_raw + round16(sizeof(T) * nr));
-    unsigned short* col = reinterpret_cast<unsigned short*>(val + w.wn);
-    unsigned short* rp = col + w.wn;
-    unsigned short* dg = rp + nr + 1;
-    unsigned short* lrow = dg + nr;
-    unsigned short* urow = lrow + nr;
-    unsigned short* lptr = urow + nr;
-    unsigned short* uptr = lptr + nl + 1;
-    uint64_t* mbar = reinterpret_cast<uint64_t*>(smem_raw + ilu_stage_bytes(nr, w.wn, nl + nu + 2, sizeof(T)) - 16);
+    const IluBlk B = a.blk[b];
+    const int r0 = a.bstart[b], nr = a.bstart[b + 1] - r0;
+    const IluStage<T> S(B, nr);
+    T* x = S.x;
+    uint64_t* mbar = S.bar;
     T* zs = reinterpret_cast<T*>(smem_raw + a.stage_max);
     if (threadIdx.x == 0) {
         tc05::mbar_init(mbar, 1);
         asm volatile("fence.mbarrier_init.release.cluster;");
     }
     __syncthreads();
-    const int mo = a.meta_off[b];
-    ilu_stage_bulk(val, col, a.lu, a.lu_col, w, mbar, rp, a.meta + mo, a.meta_off[b + 1] - mo);
+    ilu_stage_bulk(S, B, nr, a.lu, a.lu_col, a.meta);
     pdl_wait_and_trigger();
     if (a.skip && *a.skip) {
         // a step queued after the stop: every block leaves before any barrier
@@ -639,16 +608,18 @@ __global__ void __launch_bounds__(kIluThreads) k_ilu_apply_schur(SchurArgs<T> a)
         return;
     }
     for (int i = threadIdx.x; i < nr; i += blockDim.x) x[i] = (T)a.r[a.lu_row[r0 + i]];
+    if (threadIdx.x == 0) x[nr] = (T)0;
     bool ok = tc05::mbar_wait(mbar, 0);
     if (!ok) ok = tc05::mbar_wait(mbar, 0);
     const bool good = __syncthreads_and(ok ? 1 : 0) != 0;
     if (!good && threadIdx.x == 0) atomicExch(a.err, 2);
     const int lvB = a.sch_lv[2 * b], uvS = a.sch_lv[2 * b + 1], nin = a.sch_nin[b];
+    const IluShared<T> V = S.view(B);
     if (good) {
-        ilu_sweep<T, KM, false>(x, val, col, rp, dg, lrow, lptr, 1, nl);
+        ilu_sweep<T, false>(V, 1, V.nl);
         for (int i = threadIdx.x; i < nr; i += blockDim.x) zs[i] = x[i];
         __syncthreads();
-        ilu_sweep<T, KM, true>(x, val, col, rp, dg, urow, uptr, 0, uvS);
+        ilu_sweep<T, true>(V, 0, uvS);
     }
     for (int it = 0; it < a.iters; ++it) {
         double* xo = a.xg + (size_t)(it & 1) * a.N;
@@ -665,10 +636,10 @@ __global__ void __launch_bounds__(kIluThreads) k_ilu_apply_schur(SchurArgs<T> a)
             x[q] = acc;
         }
         __syncthreads();
-        ilu_sweep<T, KM, false>(x, val, col, rp, dg, lrow, lptr, lvB, nl);
+        ilu_sweep<T, false>(V, lvB, V.nl);
         for (int q = nin + threadIdx.x; q < nr; q += blockDim.x) x[q] = zs[q] - x[q];
         __syncthreads();
-        ilu_sweep<T, KM, true>(x, val, col, rp, dg, urow, uptr, 0, uvS);
+        ilu_sweep<T, true>(V, 0, uvS);
     }
     if (!good) {
         for (int i = threadIdx.x; i < nr; i += blockDim.x) a.z[a.lu_row[r0 + i]] = (double)x[i];
@@ -678,13 +649,12 @@ __global__ void __launch_bounds__(kIluThreads) k_ilu_apply_schur(SchurArgs<T> a)
         for (int q = threadIdx.x; q < nin; q += blockDim.x) x[q] = zs[q];
         __syncthreads();
     }
-    ilu_sweep<T, KM, true>(x, val, col, rp, dg, urow, uptr, uvS, nu);
+    ilu_sweep<T, true>(V, uvS, V.nu);
     for (int i = threadIdx.x; i < nr; i += blockDim.x) a.z[a.lu_row[r0 + i]] = (double)x[i];
 }
 
-static const void* schur_kernel(int precision, int lanes) {
-    if (precision) return lanes == 8 ? (const void*)k_ilu_apply_schur<float, 8> : (const void*)k_ilu_apply_schur<float, 4>;
-    return lanes == 8 ? (const void*)k_ilu_apply_schur<double, 8> : (const void*)k_ilu_apply_schur<double, 4>;
+static const void* schur_kernel(int precision) {
+    return precision ? (const void*)k_ilu_apply_schur<float> : (const void*)k_ilu_apply_schur<double>;
 }
 
 template <class T>
@@ -694,12 +664,9 @@ static void launch_schur_apply(fvm_ctx* c, BlockILU* P, const T* lu, const doubl
     a.iters = P->schur_iters;
     a.stage_max = round16(P->smem_stage[P->factored]);
     a.bstart = P->bstart.p;
-    a.lu_ptr = P->lu_ptr.p;
+    a.blk = P->blk.p;
     a.lu_col = P->lu_col.p;
     a.meta = P->meta.p;
-    a.meta_off = P->meta_off.p;
-    a.blk_lvl = P->blk_lvl.p;
-    a.blk_ulvl = P->blk_ulvl.p;
     a.lu = lu;
     a.lu_row = P->lu_row.p;
     a.sch_lv = P->sch_lv.p;
@@ -727,59 +694,45 @@ static void launch_schur_apply(fvm_ctx* c, BlockILU* P, const T* lu, const doubl
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 2;
-    if (P->lanes == 8) FVM_CUDA(cudaLaunchKernelEx(&cfg, k_ilu_apply_schur<T, 8>, a));
-    else FVM_CUDA(cudaLaunchKernelEx(&cfg, k_ilu_apply_schur<T, 4>, a));
+    FVM_CUDA(cudaLaunchKernelEx(&cfg, k_ilu_apply_schur<T>, a));
     c->launches++;
 }
 
-// Shared-memory factorisation: gather the block's Jacobian entries into the
+// Shared-memory factorisation: bring the block's Jacobian entries into the
 // same copy window the apply uses, eliminate level by level in shared
 // memory (IKJ, pivots inverted after their row), write the block back.
-// 1024 threads: one block per SM, so the copies in and out and the
-// schedule prefetch keep many loads in flight, while a level's rows (one
-// thread each, a few hundred) run on the first warps.  Schedule words of
-// the next level each thread holds:
+// 1024 threads: one block per SM, so the schedule prefetch and the copy out
+// keep many loads in flight.  A row's updates by one L entry touch different
+// entries, so four lanes share a row: the row's chain per L entry is one or
+// two updates instead of up to eight, and a level's rows (a few hundred) keep
+// all the warps busy.  Schedule words of the next level each thread holds:
 constexpr int kIluFactorThreads = 1024;
 constexpr int kIluFactorPre = 8;
+constexpr int kIluFactorLanes = 4;
 
 template <class T>
 __global__ void __launch_bounds__(kIluFactorThreads, 1) k_ilu_factor_smem(const int* __restrict__ bstart,
-                                                         const int* __restrict__ lu_ptr,
+                                                         const IluBlk* __restrict__ blk,
+                                                         const unsigned short* __restrict__ meta,
                                                          const T* __restrict__ Jw,
-                                                         const int* __restrict__ lu_diag,
                                                          const unsigned short* __restrict__ lu_col,
-                                                         const int* __restrict__ lvl_ptr,
-                                                         const int* __restrict__ lvl_rows,
-                                                         const int* __restrict__ blk_lvl,
                                                          const int* __restrict__ seg_ptr,
                                                          const unsigned* __restrict__ upd, int scr_off,
                                                          int scr_words, T* __restrict__ lu,
                                                          int* status) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
+    unsigned char* const smem_raw = ilu_smem();
     const int b = blockIdx.x;
-    const int r0 = bstart[b], r1 = bstart[b + 1], nr = r1 - r0;
-    const int e0 = lu_ptr[r0], e1 = lu_ptr[r1];
-    const IluWindow w = ilu_window(e0, e1);
-    T* val = reinterpret_cast<T*>(smem_raw + round16(sizeof(T) * nr));
-    unsigned short* col = reinterpret_cast<unsigned short*>(val + w.wn);
-    unsigned short* rp = col + w.wn;
-    unsigned short* dg = rp + nr + 1;
-    unsigned short* lrow = dg + nr;
-    unsigned short* lptr = lrow + 2 * nr;
-    const int la = blk_lvl[b], nl = blk_lvl[b + 1] - la;
-    const int lq0 = lvl_ptr[la];
-#pragma unroll 4
-    for (int p = e0 + threadIdx.x; p < e1; p += blockDim.x) {
-        val[p - w.base] = Jw[p];
-        col[p - w.base] = lu_col[p];
+    const IluBlk B = blk[b];
+    const int r0 = bstart[b], nr = bstart[b + 1] - r0;
+    const IluStage<T> S(B, nr);
+    T* const val = S.val;
+    if (threadIdx.x == 0) {
+        tc05::mbar_init(S.bar, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;");
     }
-    for (int i = threadIdx.x; i <= nr; i += blockDim.x) rp[i] = (unsigned short)(lu_ptr[r0 + i] - w.base);
-    for (int i = threadIdx.x; i < nr; i += blockDim.x) {
-        dg[i] = (unsigned short)(lu_diag[r0 + i] - w.base);
-        lrow[i] = (unsigned short)(lvl_rows[lq0 + i] - r0);
-    }
-    for (int l = threadIdx.x; l <= nl; l += blockDim.x) lptr[l] = (unsigned short)(lvl_ptr[la + l] - lq0);
     __syncthreads();
+    ilu_stage_bulk(S, B, nr, Jw, lu_col, meta);
+    const int la = B.seg, nl = B.nl;
     // Each level's schedule segment is in shared memory when its rows run
     // (read in place from global when it is larger than a buffer), so a
     // row's update chain never waits on global loads: two buffers; while a
@@ -793,7 +746,17 @@ __global__ void __launch_bounds__(kIluFactorThreads, 1) k_ilu_factor_smem(const 
 #pragma unroll 4
         for (int t = threadIdx.x; t < lenc; t += blockDim.x) buf0[t] = upd[sgc + t];
     }
-    __syncthreads();
+    bool ok = tc05::mbar_wait(S.bar, 0);
+    if (!ok) ok = tc05::mbar_wait(S.bar, 0);   // copies in flight get a second bounded chance
+    if (!__syncthreads_and(ok ? 1 : 0)) {
+        // the block never arrived: report it as a failed factorisation
+        if (threadIdx.x == 0) atomicExch(status, 2);
+        return;
+    }
+    const IluShared<T> V = S.view(B);
+    const int D = 32 * B.dp;
+    constexpr int G = kIluFactorLanes, R = 32 / G;   // lanes per row, rows per warp
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
     for (int l = 0; l < nl; ++l) {
         int sgn = 0, lenn = 0;
         bool nxt_smem = false;
@@ -811,30 +774,43 @@ __global__ void __launch_bounds__(kIluFactorThreads, 1) k_ilu_factor_smem(const 
             }
         }
         const unsigned* L = cur_smem ? ((l & 1) ? buf1 : buf0) : upd + sgc;
-        const int q0 = lptr[l], nq = lptr[l + 1] - q0;
-        for (int qq = threadIdx.x; qq < nq; qq += blockDim.x) {
-            int li = lrow[q0 + qq];
-            int s0 = rp[li], di = dg[li];
-            // IKJ with the precomputed schedule: the updates of the L entry
-            // kk, in the order a merge of row li with U(k) would find them
-            int t = (int)L[qq];
-            for (int kk = s0; kk < di; ++kk) {
-                const int cnt = (int)L[t++];
-                const int k = col[kk];
-                T lik = val[kk] * val[dg[k]];
-                val[kk] = lik;
-                for (int u = 0; u < cnt; ++u) {
-                    const unsigned pr = L[t++];
-                    const int jj = (int)(pr & 0xffffu), kp = (int)(pr >> 16);
-                    val[jj] = val[jj] - lik * val[kp];
+        const int s0 = ilu_level(V, false, l), s1 = ilu_level(V, false, l + 1);
+        // a warp takes R consecutive lanes' rows of a slice
+        for (int it = warp; it < (s1 - s0) * G; it += nw) {
+            const int s = s0 + it / G, q = (it % G) * R + lane / G, g = lane % G;
+            const int ps = ilu_start(V, false, s), w = ilu_start(V, false, s + 1) - ps, p0 = 32 * ps + q;
+            const int i = ilu_row(V, false, 32 * s + q);
+            const bool row = i != kIluNoRow;
+            // IKJ with the precomputed schedule: the updates of each L entry,
+            // in the order a merge of the row with U(k) would find them
+            int t = row ? (int)L[32 * (s - s0) + q] : 0;
+            for (int kk = 0; kk < w; ++kk) {
+                const int p = p0 + 32 * kk;
+                const int k = (int)V.col(p);
+                const bool act = row && k != nr;
+                T lik = (T)0;
+                if (act) {
+                    const int cnt = (int)L[t];
+                    lik = val[p] * val[D + k];
+                    for (int u = g; u < cnt; u += G) {
+                        const unsigned pr = L[t + 1 + u];
+                        const int jj = (int)(pr & 0xffffu), kp = (int)(pr >> 16);
+                        val[jj] = val[jj] - lik * val[kp];
+                    }
+                    t += 1 + cnt;
                 }
+                __syncwarp();
+                // the entry itself was read by the row's other lanes above
+                if (act && g == 0) val[p] = lik;
             }
-            T d = val[di];
-            if (d == (T)0 || !isfinite((double)d)) {
-                atomicExch(status, 1);
-                d = (T)1;
+            if (row && g == 0) {
+                T d = val[D + i];
+                if (d == (T)0 || !isfinite((double)d)) {
+                    atomicExch(status, 1);
+                    d = (T)1;
+                }
+                val[D + i] = (T)1 / d;
             }
-            val[di] = (T)1 / d;
         }
         if (nxt_smem) {
             unsigned* nb = (l & 1) ? buf0 : buf1;   // the buffer of level l - 1, finished
@@ -849,7 +825,8 @@ __global__ void __launch_bounds__(kIluFactorThreads, 1) k_ilu_factor_smem(const 
         lenc = lenn;
         cur_smem = nxt_smem;
     }
-    for (int p = e0 + threadIdx.x; p < e1; p += blockDim.x) lu[p] = val[p - w.base];
+    const int wn = (int)ilu_window(nr, B.dp);
+    for (int p = threadIdx.x; p < wn; p += blockDim.x) lu[B.v0 + p] = val[p];
 }
 
 // ------------------------------------------------------------------ host set-up
@@ -1178,20 +1155,81 @@ static void build_pattern(fvm_ctx* c, BlockILU* P) {
         }
         blk_ulvl.push_back((int)ulvl_ptr.size() - 1);
     }
-    // elimination schedule in level order (window positions relative to
-    // each block's 8-aligned window base, as the factorisation indexes); the
-    // same update set and order as merging row i with U(k) for each L entry
+    P->nb = nb;
+    P->maxb = maxb;
+    P->nlevels_max = nlmax;
+    // the sliced layout of every block (IluBlk) and its record: a level's rows
+    // longest first, stable
+    std::vector<IluBlk> blk(nb);
+    std::vector<unsigned short> meta, scol;
+    std::vector<int> spos(lu_src.size()), up(N);
+    size_t nlu = 0;
+    for (int b = 0; b < nb; ++b) {
+        const int r0 = bstart[b], r1 = bstart[b + 1], nr = r1 - r0;
+        IluBlk& B = blk[b];
+        B = IluBlk{};
+        B.nl = blk_lvl[b + 1] - blk_lvl[b];
+        B.nu = blk_ulvl[b + 1] - blk_ulvl[b];
+        B.seg = blk_lvl[b];
+        std::vector<int> first[2], start(1, 0), rows[2];
+        for (int upper = 0; upper < 2; ++upper) {
+            const std::vector<int>& ptr = upper ? ulvl_ptr : lvl_ptr;
+            std::vector<int>& ord = upper ? ulvl_rows : lvl_rows;
+            auto begin = [&](int i) { return upper ? lu_diag[i] + 1 : lu_ptr[i]; };
+            auto length = [&](int i) { return upper ? lu_ptr[i + 1] - lu_diag[i] - 1 : lu_diag[i] - lu_ptr[i]; };
+            first[upper].push_back(0);
+            for (int g = upper ? blk_ulvl[b] : blk_lvl[b]; g < (upper ? blk_ulvl[b + 1] : blk_lvl[b + 1]); ++g) {
+                std::stable_sort(ord.begin() + ptr[g], ord.begin() + ptr[g + 1],
+                                 [&](int x, int y) { return length(x) > length(y); });
+                for (int q = ptr[g]; q < ptr[g + 1]; q += 32) {
+                    const int w = length(ord[q]), at = 32 * start.back();
+                    for (int l = 0; l < 32; ++l) {
+                        const int i = q + l < ptr[g + 1] ? ord[q + l] : -1;
+                        if (i >= 0 && upper) up[i] = (int)rows[1].size();
+                        rows[upper].push_back(i < 0 ? (int)kIluNoRow : i - r0);
+                        for (int k = 0; i >= 0 && k < length(i); ++k)
+                            spos[begin(i) + k] = (int)nlu + at + 32 * k + l;
+                    }
+                    start.push_back(start.back() + w);
+                }
+                first[upper].push_back((int)rows[upper].size() / 32);
+            }
+        }
+        B.v0 = (int)nlu;
+        B.dp = start.back();
+        B.nsl = (int)rows[0].size() / 32;
+        B.nsu = (int)rows[1].size() / 32;
+        for (int i = r0; i < r1; ++i) spos[lu_diag[i]] = (int)nlu + 32 * B.dp + i - r0;
+        nlu += ilu_window(nr, B.dp);
+        if (nlu >= (size_t)INT32_MAX || B.dp > 65535) throw Error("block-ILU: block too large");
+        B.c0 = (int)scol.size();
+        scol.resize(scol.size() + 32 * (size_t)B.dp, (unsigned short)nr);
+        for (int i = r0; i < r1; ++i)
+            for (int p = lu_ptr[i]; p < lu_ptr[i + 1]; ++p)
+                if (p != lu_diag[i]) scol[B.c0 + spos[p] - B.v0] = lu_col[p];
+        scol.resize(scol.size() + kIluSlack, 0);
+        if (scol.size() >= (size_t)INT32_MAX) throw Error("block-ILU: block too large");
+        B.mo = (int)meta.size();
+        B.mw = (int)ilu_meta_words(B.nl, B.nu, B.nsl, B.nsu);
+        for (const std::vector<int>* v : {&first[0], &first[1], &start, &rows[0], &rows[1]})
+            meta.insert(meta.end(), v->begin(), v->end());
+        meta.resize((size_t)B.mo + B.mw, 0);
+        if (meta.size() >= (size_t)INT32_MAX) throw Error("block-ILU: records too large");
+    }
+    P->nlu = nlu;
+    // elimination schedule in level order (window positions relative to each
+    // block's first entry, as the factorisation indexes); the same update set
+    // and order as merging row i with U(k) for each L entry
     std::vector<int> seg_ptr(lvl_ptr.size(), 0);
     std::vector<unsigned> upd;
     size_t seg_max = 0;
     for (int b = 0; b < nb; ++b) {
-        const int r0 = bstart[b];
-        const int base = lu_ptr[r0] & ~7;
+        const int r0 = bstart[b], base = blk[b].v0;
         for (int g = blk_lvl[b]; g < blk_lvl[b + 1]; ++g) {
             seg_ptr[g] = (int)upd.size();
             const int q0 = lvl_ptr[g], q1 = lvl_ptr[g + 1];
             const size_t head = upd.size();
-            upd.resize(head + (q1 - q0), 0u);
+            upd.resize(head + (q1 - q0 + 31) / 32 * 32, 0u);
             for (int q = q0; q < q1; ++q) {
                 const int i = lvl_rows[q];
                 upd[head + (q - q0)] = (unsigned)(upd.size() - head);
@@ -1205,7 +1243,7 @@ static void build_pattern(fvm_ctx* c, BlockILU* P) {
                         const int j = lu_col[jj];
                         while (kpos < kend && lu_col[kpos] < j) ++kpos;
                         if (kpos < kend && lu_col[kpos] == j)
-                            upd.push_back((unsigned)(jj - base) | ((unsigned)(kpos - base) << 16));
+                            upd.push_back((unsigned)(spos[jj] - base) | ((unsigned)(spos[kpos] - base) << 16));
                     }
                     upd[cw] = (unsigned)(upd.size() - cw - 1);
                 }
@@ -1215,39 +1253,15 @@ static void build_pattern(fvm_ctx* c, BlockILU* P) {
         seg_ptr[blk_lvl[b + 1]] = (int)upd.size();
     }
     if (upd.size() >= (size_t)INT32_MAX) throw Error("block-ILU: elimination schedule too large");
-    P->nb = nb;
-    P->maxb = maxb;
-    P->nlevels_max = nlmax;
-    // per-block metadata records of the staged apply (layout of
-    // ilu_meta_words), 16-byte aligned
-    std::vector<unsigned short> meta;
-    std::vector<int> meta_off(1, 0);
-    for (int b = 0; b < nb; ++b) {
-        const int r0 = bstart[b], r1 = bstart[b + 1], nr = r1 - r0;
-        const int base = lu_ptr[r0] & ~7;
-        const int la = blk_lvl[b], nl = blk_lvl[b + 1] - la;
-        const int ua = blk_ulvl[b], nu = blk_ulvl[b + 1] - ua;
-        const size_t start = meta.size();
-        for (int i = 0; i <= nr; ++i) meta.push_back((unsigned short)(lu_ptr[r0 + i] - base));
-        for (int i = 0; i < nr; ++i) meta.push_back((unsigned short)(lu_diag[r0 + i] - base));
-        for (int i = 0; i < nr; ++i) meta.push_back((unsigned short)(lvl_rows[r0 + i] - r0));
-        for (int i = 0; i < nr; ++i) meta.push_back((unsigned short)(ulvl_rows[r0 + i] - r0));
-        for (int l = 0; l <= nl; ++l) meta.push_back((unsigned short)(lvl_ptr[la + l] - r0));
-        for (int l = 0; l <= nu; ++l) meta.push_back((unsigned short)(ulvl_ptr[ua + l] - r0));
-        meta.resize(start + ilu_meta_words(nr, (size_t)nl + nu + 2), 0);
-        meta_off.push_back((int)meta.size());
-    }
     {
         size_t need64 = 0, need32 = 0;
         bool fits16 = true;
         for (int b = 0; b < nb; ++b) {
-            size_t nr = bstart[b + 1] - bstart[b];
-            // the 16-byte aligned copy window of ilu_window()
-            size_t wn = (size_t)(((lu_ptr[bstart[b + 1]] + 7) & ~7) - (lu_ptr[bstart[b]] & ~7));
-            if (wn >= 65535 || nr + 1 >= 65535) fits16 = false;
-            size_t nlev = (size_t)(blk_lvl[b + 1] - blk_lvl[b]) + (size_t)(blk_ulvl[b + 1] - blk_ulvl[b]) + 2;
+            const size_t nr = bstart[b + 1] - bstart[b], dp = blk[b].dp;
+            // the schedule's window positions and the columns are 16-bit words
+            if (ilu_window(nr, dp) >= 65536 || nr + 1 >= 65535) fits16 = false;
             for (size_t sz : {(size_t)8, (size_t)4}) {
-                size_t need = ilu_stage_bytes(nr, wn, nlev, sz);
+                const size_t need = ilu_stage_bytes(nr, dp, blk[b].mw, sz);
                 if (sz == 8) need64 = std::max(need64, need);
                 else need32 = std::max(need32, need);
             }
@@ -1261,9 +1275,6 @@ static void build_pattern(fvm_ctx* c, BlockILU* P) {
             const size_t room = P->smem_stage[pr] && st < kMaxDynSmem ? (kMaxDynSmem - st) / 8 : 0;
             P->scr_words[pr] = (int)std::min<size_t>(std::min<size_t>(seg_max, room), (size_t)kIluFactorThreads * kIluFactorPre);
         }
-        // entries per row held in registers by the staged triangular sweeps:
-        // 8 covers the lower or upper part of a 3D row, 4 of a 2D row
-        P->lanes = (double)lu_ptr[N] / N > 9.0 ? 8 : 4;
         // one thread per row of the widest level, in whole warps of 128 or 256
         int widest = 0;
         for (size_t g = 0; g + 1 < lvl_ptr.size(); ++g) widest = std::max(widest, lvl_ptr[g + 1] - lvl_ptr[g]);
@@ -1271,23 +1282,21 @@ static void build_pattern(fvm_ctx* c, BlockILU* P) {
         P->apply_threads = widest > 128 ? 256 : 128;
         // the global-memory apply keeps the block's vector in shared memory
         if (!P->smem_stage[0]) {
-            if (sizeof(double) * (size_t)maxb > kMaxDynSmem)
+            if (sizeof(double) * ((size_t)maxb + 1) > kMaxDynSmem)
                 throw Error("block-ILU: blocks too large for the FP64 apply (set more blocks per SM)");
-            raise_smem_limit(k_ilu_apply<double>, sizeof(double) * (size_t)maxb);
+            raise_smem_limit(k_ilu_apply<double>, sizeof(double) * ((size_t)maxb + 1));
         }
         if (!P->smem_stage[1]) {
-            if (sizeof(float) * (size_t)maxb > kMaxDynSmem)
+            if (sizeof(float) * ((size_t)maxb + 1) > kMaxDynSmem)
                 throw Error("block-ILU: blocks too large for the FP32 apply (set more blocks per SM)");
-            raise_smem_limit(k_ilu_apply<float>, sizeof(float) * (size_t)maxb);
+            raise_smem_limit(k_ilu_apply<float>, sizeof(float) * ((size_t)maxb + 1));
         }
         if (P->smem_stage[0]) {
-            raise_smem_limit(k_ilu_apply_smem<double, 4>, (size_t)P->smem_stage[0]);
-            raise_smem_limit(k_ilu_apply_smem<double, 8>, (size_t)P->smem_stage[0]);
+            raise_smem_limit(k_ilu_apply_smem<double>, (size_t)P->smem_stage[0]);
             raise_smem_limit(k_ilu_factor_smem<double>, (size_t)(round16(P->smem_stage[0]) + 8 * (size_t)P->scr_words[0]));
         }
         if (P->smem_stage[1]) {
-            raise_smem_limit(k_ilu_apply_smem<float, 4>, (size_t)P->smem_stage[1]);
-            raise_smem_limit(k_ilu_apply_smem<float, 8>, (size_t)P->smem_stage[1]);
+            raise_smem_limit(k_ilu_apply_smem<float>, (size_t)P->smem_stage[1]);
             raise_smem_limit(k_ilu_factor_smem<float>, (size_t)(round16(P->smem_stage[1]) + 8 * (size_t)P->scr_words[1]));
         }
     }
@@ -1304,7 +1313,7 @@ static void build_pattern(fvm_ctx* c, BlockILU* P) {
             const size_t sz = pr ? sizeof(float) : sizeof(double);
             const size_t need = round16(P->smem_stage[pr]) + round16(sz * (size_t)maxb);
             if (need > kMaxDynSmem) continue;
-            const void* kfn = schur_kernel(pr, P->lanes);
+            const void* kfn = schur_kernel(pr);
             raise_smem_limit(kfn, need);
             int per_sm = 0;
             FVM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kfn, P->apply_threads, need));
@@ -1355,12 +1364,10 @@ static void build_pattern(fvm_ctx* c, BlockILU* P) {
     P->bstart.upload(bstart, s);
     P->h_bstart = bstart;
     P->h_lu_row = lu_row;
-    P->lu_ptr.upload(lu_ptr, s);
-    // 8 padding entries so every block's widened copy window stays inside
     {
         // where the quotient kernels put each Jacobian entry for the factorisation
         std::vector<int> lu_dst(P->nnz, -1);
-        for (size_t p = 0; p < lu_src.size(); ++p) lu_dst[lu_src[p]] = (int)p;
+        for (size_t p = 0; p < lu_src.size(); ++p) lu_dst[lu_src[p]] = spos[p];
         FdTables fd;
         build_fd_tables(c, P, rowof, lu_dst, fd);
         P->fd_cnode_ptr.upload(fd.cnode_ptr, s);
@@ -1381,25 +1388,14 @@ static void build_pattern(fvm_ctx* c, BlockILU* P) {
         // the tables' host memory is read by copies still in flight
         FVM_CUDA(cudaStreamSynchronize(s));
     }
-    lu_src.resize(lu_src.size() + 8, 0);
-    lu_col.resize(lu_col.size() + 8, 0);
-    P->lu_src.upload(lu_src, s);
-    P->Jw.alloc(lu_src.size());
-    P->Jw.zero(s);
-    P->lu_diag.upload(lu_diag, s);
+    P->blk.upload(blk, s);
+    if (!P->smem_stage[0] || !P->smem_stage[1]) P->lu_up.upload(up, s);
     P->lu_row.upload(lu_row, s);
-    P->lu_col.upload(lu_col, s);
+    P->lu_col.upload(scol, s);
     if (upd.empty()) upd.push_back(0u);
     P->seg_ptr.upload(seg_ptr, s);
     P->upd.upload(upd, s);
     P->meta.upload(meta, s);
-    P->meta_off.upload(meta_off, s);
-    P->lvl_ptr.upload(lvl_ptr, s);
-    P->lvl_rows.upload(lvl_rows, s);
-    P->blk_lvl.upload(blk_lvl, s);
-    P->ulvl_ptr.upload(ulvl_ptr, s);
-    P->ulvl_rows.upload(ulvl_rows, s);
-    P->blk_ulvl.upload(blk_ulvl, s);
     P->status.alloc(1);
     P->status.zero(s);
     FVM_CUDA(cudaMallocHost(&P->h_status, sizeof(int)));
@@ -1448,7 +1444,16 @@ void psetup_dev(fvm_ctx* c, double cj, double h, const double* y, const double* 
         a.list_max = P->fd_list_max; a.grp_max = P->fd_grp_max; a.part = P->fd_part.p;
         a.coef = c->coef.p; a.xyz = c->xyz.p; a.eK = c->eK.p; a.ezone = c->ezone.p;
         a.y = y; a.g = P->fd_g.p; a.dg = P->fd_dg.p; a.gq = P->fd_gq.p; a.upw = c->upw.p;
-        a.out = FdOut{P->fd_scale.p, P->fd_diag.p, P->J.p, P->Jw.p, op ? P->op_val.p : nullptr};
+        // one buffer per precision: the slices' padding stays zero in each
+        auto window = [&](auto& w) -> void* {
+            if (!w.n) {
+                w.alloc(P->nlu);
+                w.zero(s);
+            }
+            return w.p;
+        };
+        a.out = FdOut{P->fd_scale.p, P->fd_diag.p, P->J.p, precision ? window(P->Jw32) : window(P->Jw),
+                      op ? P->op_val.p : nullptr};
         auto run = [&](auto one) {
             using S = decltype(one);
             auto go = [&](auto kern, size_t sm) {
@@ -1472,35 +1477,23 @@ void psetup_dev(fvm_ctx* c, double cj, double h, const double* y, const double* 
     }
     c->tm.end(TM_FD_JAC, s);
     FVM_CUDA(cudaMemsetAsync(P->status.p, 0, sizeof(int), s));
-    size_t nlu = P->lu_src.n;
     c->tm.begin(TM_ILU_FACTOR, s);
-    if (P->smem_stage[precision]) {
-        const int so = (int)round16(P->smem_stage[precision]);
-        const int sw = P->scr_words[precision];
-        size_t sm = (size_t)so + 8 * (size_t)sw;
-        if (precision) {
-            P->lu32.alloc(nlu);
-            fvm_launch(c, k_ilu_factor_smem<float>, P->nb, kIluFactorThreads, sm, s, P->bstart.p, P->lu_ptr.p,
-                       reinterpret_cast<const float*>(P->Jw.p), P->lu_diag.p, P->lu_col.p, P->lvl_ptr.p, P->lvl_rows.p,
-                       P->blk_lvl.p, P->seg_ptr.p, P->upd.p, so, sw, P->lu32.p, P->status.p);
+    auto factor = [&](auto& lu, auto* Jw) {
+        using T = std::remove_pointer_t<decltype(Jw)>;
+        lu.alloc(P->nlu + kIluSlack);   // a sweep in place may read past the last block's
+        if (P->smem_stage[precision]) {
+            const int so = (int)round16(P->smem_stage[precision]);
+            const int sw = P->scr_words[precision];
+            fvm_launch(c, k_ilu_factor_smem<T>, P->nb, kIluFactorThreads, (size_t)so + 8 * (size_t)sw, s, P->bstart.p,
+                       P->blk.p, P->meta.p, (const T*)Jw, P->lu_col.p, P->seg_ptr.p, P->upd.p, so, sw, lu.p,
+                       P->status.p);
         } else {
-            P->lu64.alloc(nlu);
-            fvm_launch(c, k_ilu_factor_smem<double>, P->nb, kIluFactorThreads, sm, s, P->bstart.p, P->lu_ptr.p, P->Jw.p,
-                       P->lu_diag.p, P->lu_col.p, P->lvl_ptr.p, P->lvl_rows.p, P->blk_lvl.p, P->seg_ptr.p, P->upd.p,
-                       so, sw, P->lu64.p, P->status.p);
+            fvm_launch(c, k_ilu_factor<T>, P->nb, 128, 0, s, P->bstart.p, P->blk.p, P->meta.p, P->lu_up.p,
+                       (const T*)Jw, P->lu_col.p, lu.p, P->status.p);
         }
-    } else if (precision) {
-        P->lu32.alloc(nlu);
-        fvm_launch(c, k_ilu_factor<float>, P->nb, 128, 0, s, P->bstart.p, P->lu_ptr.p,
-                   reinterpret_cast<const float*>(P->Jw.p), P->lu_diag.p, P->lu_col.p,
-                                                  P->lvl_ptr.p, P->lvl_rows.p, P->blk_lvl.p, P->lu32.p,
-                                                  P->status.p);
-    } else {
-        P->lu64.alloc(nlu);
-        fvm_launch(c, k_ilu_factor<double>, P->nb, 128, 0, s, P->bstart.p, P->lu_ptr.p, P->Jw.p, P->lu_diag.p, P->lu_col.p,
-                                                   P->lvl_ptr.p, P->lvl_rows.p, P->blk_lvl.p, P->lu64.p,
-                                                   P->status.p);
-    }
+    };
+    if (precision) factor(P->lu32, P->Jw32.p);
+    else factor(P->lu64, P->Jw.p);
     c->tm.end(TM_ILU_FACTOR, s);
     FVM_CUDA(cudaMemcpyAsync(P->h_status, P->status.p, sizeof(int), cudaMemcpyDeviceToHost, s));
     P->factored = precision;
@@ -1554,30 +1547,17 @@ void psolve_dev(fvm_ctx* c, const double* r, double* z, const int* skip) {
         else launch_schur_apply(c, P, P->lu64.p, r, z, skip);
         return;
     }
-    if (P->smem_stage[P->factored]) {
-        size_t sm = P->smem_stage[P->factored];
-        auto go = [&](auto kern, const auto* lu) {
-            fvm_launch_pdl(c, kern, P->nb, P->apply_threads, sm, s, P->bstart.p, P->lu_ptr.p, P->lu_col.p, P->meta.p,
-                       P->meta_off.p, P->blk_lvl.p, P->blk_ulvl.p, lu, P->lu_row.p, r, z, P->status.p, skip);
-        };
-        if (P->factored) {
-            if (P->lanes == 8) go(k_ilu_apply_smem<float, 8>, P->lu32.p);
-            else go(k_ilu_apply_smem<float, 4>, P->lu32.p);
-        } else {
-            if (P->lanes == 8) go(k_ilu_apply_smem<double, 8>, P->lu64.p);
-            else go(k_ilu_apply_smem<double, 4>, P->lu64.p);
-        }
-    } else if (P->factored) {
-        size_t sm = sizeof(float) * P->maxb;
-        fvm_launch_pdl(c, k_ilu_apply<float>, P->nb, 128, sm, s, P->bstart.p, P->lu_ptr.p, P->lu_diag.p, P->lu_col.p, P->lvl_ptr.p,
-                                                 P->lvl_rows.p, P->blk_lvl.p, P->ulvl_ptr.p, P->ulvl_rows.p,
-                                                 P->blk_ulvl.p, P->lu32.p, P->lu_row.p, r, z, skip);
-    } else {
-        size_t sm = sizeof(double) * P->maxb;
-        fvm_launch_pdl(c, k_ilu_apply<double>, P->nb, 128, sm, s, P->bstart.p, P->lu_ptr.p, P->lu_diag.p, P->lu_col.p, P->lvl_ptr.p,
-                                                  P->lvl_rows.p, P->blk_lvl.p, P->ulvl_ptr.p, P->ulvl_rows.p,
-                                                  P->blk_ulvl.p, P->lu64.p, P->lu_row.p, r, z, skip);
-    }
+    const size_t sm = P->smem_stage[P->factored];
+    auto go = [&](auto staged, auto plain, const auto* lu) {
+        if (sm)
+            fvm_launch_pdl(c, staged, P->nb, P->apply_threads, sm, s, P->bstart.p, P->blk.p, P->lu_col.p, P->meta.p, lu,
+                           P->lu_row.p, r, z, P->status.p, skip);
+        else
+            fvm_launch_pdl(c, plain, P->nb, 128, sizeof(*lu) * ((size_t)P->maxb + 1), s, P->bstart.p, P->blk.p,
+                           P->lu_col.p, P->meta.p, lu, P->lu_row.p, r, z, skip);
+    };
+    if (P->factored) go(k_ilu_apply_smem<float>, k_ilu_apply<float>, P->lu32.p);
+    else go(k_ilu_apply_smem<double>, k_ilu_apply<double>, P->lu64.p);
 }
 
 } // namespace fvmb
