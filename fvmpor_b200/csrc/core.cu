@@ -435,6 +435,176 @@ __global__ void k_edge_upwind(int E, int nfe, const int* __restrict__ edge_ptr,
     }
 }
 
+// ---- the same, chunk by chunk.  Written out for all faces and read back edge by
+// edge, the fluxes and the flags were scattered accesses of single words: 38 + 43
+// us on the 214k-node box (1.2 M tetrahedra), 177 + 185 us on the 1M-node one
+// (one B200).  Here a block forms the fluxes of kUpChunk consecutive elements in
+// shared memory (from the vertices, as the element pass does) and sums every
+// edge's own there, in ascending face order.  An edge that no other chunk
+// touches is decided at once; of the others only the chunk's sum leaves, and
+// k_upwind_shared adds those in ascending chunk order and leaves its decision at
+// each of their places.  k_upwind_flags then writes the element-local flags, eight
+// bytes per element.  35 + 12 + 10 us and 150 + 43 + 37 us.
+// The reference divides each flux by the sum of the edge's face areas
+// (fvmpor.h:765), which is positive and does not change the sign asked for.
+struct UpArgs {
+    int T, N, kiso, estride, nnmax, edmax;   // edmax: most edges of a chunk
+    const int* node_ptr;
+    const int* node;
+    const ushort4* loc;
+    const int2* edge;
+    const unsigned short* start;
+    const unsigned short* slot;
+    const double* coef;
+    const double* xyz;
+    const double* eK;
+    const int* ezone;
+    const double* h;
+    const double* krw;
+    const unsigned char* flip;
+    double* part;
+    unsigned char* front;
+};
+constexpr int kUpThreads = 256;
+constexpr int kUpChunk = 512;
+// below this many chunks the blocks leave the chip idle, and the two
+// kernels above, an element and an edge per thread, are as fast (151k elements:
+// about 7 + 7 us)
+constexpr int kUpMinChunks = 296;
+
+constexpr int kUpPer = kUpChunk / kUpThreads;   // elements per thread
+
+static size_t up_smem_bytes(int nfe, int nnmax, int edmax, bool rc, bool mz) {
+    return 8 * ((size_t)nfe * kUpChunk + (size_t)nnmax * (1 + (mz ? 0 : 1) + (rc ? 3 : 0))) + 2 * (size_t)nfe * kUpChunk +
+           2 * ((size_t)edmax + 1);
+}
+
+// What a block reads besides its nodes (the elements' records, the edges' lists)
+// does not depend on the step and is on its way before the wait for the previous
+// kernel and while the nodes arrive: with the lists read where they are used, the
+// block's chain of dependent loads made it 46 us on the 214k-node box.
+template <int NPE, int NFE, bool RC, bool MZ>
+__global__ void __launch_bounds__(kUpThreads, 4) k_upwind_chunk(UpArgs a) {
+    extern __shared__ __align__(16) double up_smem[];
+    double* q = up_smem;                       // [NFE][kUpChunk] fluxes, front to back
+    unsigned short* slot = reinterpret_cast<unsigned short*>(q + NFE * kUpChunk);   // the edges' faces
+    double* sh = reinterpret_cast<double*>(slot + NFE * kUpChunk);   // the chunk's nodes: h, krw (one zone), coordinates
+    double* sk = sh + a.nnmax;
+    double* sx = sk + (MZ ? 0 : a.nnmax);
+    unsigned short* start = reinterpret_cast<unsigned short*>(sx + (RC ? 3 * a.nnmax : 0));
+    const int e0 = blockIdx.x * kUpChunk, ne = min(kUpChunk, a.T - e0);
+    const int2 ed = a.edge[blockIdx.x];
+    const int nedge = a.edge[blockIdx.x + 1].x - ed.x;
+    const int n0 = a.node_ptr[blockIdx.x], nn = a.node_ptr[blockIdx.x + 1] - n0;
+    ushort4 lq[kUpPer];
+    unsigned fl[kUpPer];
+    double K[kUpPer];
+#pragma unroll
+    for (int j = 0; j < kUpPer; ++j) {
+        const int e = e0 + min((int)threadIdx.x + j * kUpThreads, ne - 1);
+        lq[j] = a.loc[e];
+        fl[j] = a.flip[e];
+        K[j] = RC ? a.eK[e] : 0.0;
+    }
+    // (the list is padded to whole chunks)
+    constexpr int kVec = NFE * kUpChunk / 8;
+    const uint4* gs = reinterpret_cast<const uint4*>(a.slot + (size_t)NFE * e0);
+    for (int k = threadIdx.x; k < kVec; k += kUpThreads) reinterpret_cast<uint4*>(slot)[k] = gs[k];
+    for (int k = threadIdx.x; k <= nedge; k += kUpThreads) start[k] = a.start[ed.x + blockIdx.x + k];
+    pdl_wait_and_trigger();
+    for (int k = threadIdx.x; k < nn; k += kUpThreads) {
+        const int g = a.node[n0 + k];
+        sh[k] = a.h[g];
+        if (!MZ) sk[k] = a.krw[g];
+        if (RC) {
+            sx[k] = a.xyz[g];
+            sx[a.nnmax + k] = a.xyz[(size_t)a.N + g];
+            sx[2 * a.nnmax + k] = a.xyz[(size_t)2 * a.N + g];
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < kUpPer; ++j) {
+        const int el = threadIdx.x + j * kUpThreads, e = e0 + el;
+        if (el >= ne) break;
+        const int li[4] = {lq[j].x, lq[j].y, lq[j].z, lq[j].w};
+        double hv[NPE], kr[NPE], f6[NFE];
+        const size_t zo = MZ ? (size_t)a.ezone[e] * a.N : 0;
+#pragma unroll
+        for (int k = 0; k < NPE; ++k) {
+            hv[k] = sh[li[k]];
+            kr[k] = MZ ? a.krw[zo + a.node[n0 + li[k]]] : sk[li[k]];
+        }
+        if constexpr (RC) {
+            double X[4][3], Ky = K[j], Kz = K[j];
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+#pragma unroll
+                for (int d = 0; d < 3; ++d) X[k][d] = sx[d * a.nnmax + li[k]];
+            if (!a.kiso) {
+                Ky = a.eK[(size_t)a.estride + e];
+                Kz = a.eK[(size_t)2 * a.estride + e];
+            }
+            tet_face_fluxes(X[0], X[1], X[2], X[3], K[j], Ky, Kz, hv[0], hv[1], hv[2], hv[3], f6);
+        } else {
+#pragma unroll
+            for (int f = 0; f < NFE; ++f) {
+                const double* cf = a.coef + (size_t)(f * (NPE + 1)) * a.T + e;
+                double s = cf[0] * hv[0];
+#pragma unroll
+                for (int k = 1; k < NPE; ++k) s += cf[(size_t)k * a.T] * hv[k];
+                f6[f] = s + cf[(size_t)NPE * a.T];
+            }
+        }
+#pragma unroll
+        for (int f = 0; f < NFE; ++f) {
+            const int fa = NPE == 4 ? tet_edge_a(f) : tri_edge_a(f);
+            const int fb = NPE == 4 ? tet_edge_b(f) : tri_edge_b(f);
+            const double qn = f6[f] * (kr[fa] * 0.5 + kr[fb] * 0.5);
+            q[f * kUpChunk + el] = ((fl[j] >> f) & 1u) ? qn : -qn;
+        }
+    }
+    __syncthreads();
+    for (int k = threadIdx.x; k < nedge; k += kUpThreads) {
+        const int p1 = start[k + 1];
+        double s = 0.0;
+        for (int p = start[k]; p < p1; ++p) s += q[slot[p]];
+        if (k < ed.y) a.front[ed.x + k] = s < 0.0;
+        else a.part[ed.x + k] = s;
+    }
+}
+
+__global__ void k_upwind_shared(int n, const int* __restrict__ sptr, const int* __restrict__ place,
+                                const double* __restrict__ part, unsigned char* __restrict__ front) {
+    pdl_wait_and_trigger();
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= n) return;
+    const int p0 = sptr[t], p1 = sptr[t + 1];
+    double s = 0.0;
+    for (int p = p0; p < p1; ++p) s += part[place[p]];
+    for (int p = p0; p < p1; ++p) front[place[p]] = s < 0.0;
+}
+
+// upstream node of each face in element-local terms: node b where it is the
+// edge's upstream one
+template <int NFE>
+__global__ void k_upwind_flags(int T, const int2* __restrict__ edge, const unsigned short* __restrict__ of,
+                               const unsigned char* __restrict__ front, const unsigned char* __restrict__ flip,
+                               unsigned char* __restrict__ upw) {
+    pdl_wait_and_trigger();
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= T) return;
+    const unsigned char* fr = front + edge[e / kUpChunk].x;
+    const unsigned fl = flip[e];
+    unsigned w[2] = {0x02020202u, 0x02020202u};
+#pragma unroll
+    for (int f = 0; f < NFE; ++f) {
+        const unsigned b = (fr[of[(size_t)f * T + e]] ^ (fl >> f) ^ 1u) & 1u;
+        w[f >> 2] = (w[f >> 2] & ~(0xffu << (8 * (f & 3)))) | b << (8 * (f & 3));
+    }
+    *reinterpret_cast<uint2*>(upw + (size_t)8 * e) = make_uint2(w[0], w[1]);
+}
+
 // ------------------------------------------------------------------ drivers
 static NodeCopies node_copies(fvm_ctx* c) {
     NodeCopies cp;
@@ -644,6 +814,32 @@ void launch_begin_step(fvm_ctx* c, const double* y, const double* yp) {
     fvm_launch(c, k_node, grid_for(c->N, kBlock), kBlock, 0, s, c->N, y, yp, none, c->zones.p, c->nz, c->nz_ptr.p,
                                                       c->nz_zone.p, c->nz_w.p, c->rho0, c->krw.p,
                                                       c->hstar.p, c->stor.p, node_copies(c));
+    if (c->up_chunks) {
+        UpArgs a;
+        a.T = c->T; a.N = c->N; a.kiso = c->kiso ? 1 : 0; a.estride = c->estride; a.nnmax = c->up_nnmax;
+        a.edmax = c->up_edmax;
+        a.node_ptr = c->up_node_ptr.p; a.node = c->up_node.p; a.loc = c->up_loc.p;
+        a.edge = c->up_edge.p; a.start = c->up_start.p; a.slot = c->up_slot.p;
+        a.coef = c->coef.p; a.xyz = c->xyz.p; a.eK = c->eK.p; a.ezone = c->ezone.p;
+        a.h = y; a.krw = c->krw.p; a.flip = c->flip.p; a.part = c->up_part.p; a.front = c->up_front.p;
+        const bool mz = c->nz > 1, rc = c->dim == 3 && c->recompute;
+        auto go = [&](auto kern) {
+            const size_t sm = up_smem_bytes(c->nfe, c->up_nnmax, c->up_edmax, rc, mz);
+            if (sm > 48 * 1024) raise_smem_limit(kern, sm);
+            fvm_launch_pdl(c, kern, c->up_chunks, kUpThreads, sm, s, a);
+        };
+        if (c->dim == 2) mz ? go(k_upwind_chunk<3, 3, false, true>) : go(k_upwind_chunk<3, 3, false, false>);
+        else if (rc) mz ? go(k_upwind_chunk<4, 6, true, true>) : go(k_upwind_chunk<4, 6, true, false>);
+        else mz ? go(k_upwind_chunk<4, 6, false, true>) : go(k_upwind_chunk<4, 6, false, false>);
+        const int ns = (int)c->up_sptr.n - 1;
+        if (ns > 0)
+            fvm_launch_pdl(c, k_upwind_shared, grid_for(ns, kBlock), kBlock, 0, s, ns, c->up_sptr.p, c->up_splace.p,
+                           c->up_part.p, c->up_front.p);
+        auto flags = c->dim == 2 ? k_upwind_flags<3> : k_upwind_flags<6>;
+        fvm_launch_pdl(c, flags, grid_for(c->T, kBlock), kBlock, 0, s, c->T, c->up_edge.p, c->up_of.p, c->up_front.p,
+                       c->flip.p, c->upw.p);
+        return;
+    }
     int gb = grid_for(c->T, kBlock);
     if (c->dim == 3 && c->recompute) {
         if (c->nz > 1)
@@ -746,6 +942,110 @@ static void autotune(fvm_ctx* c, fvm_tune_result* out) {
     }
 }
 
+// Tables of k_upwind_chunk from every face's edge (eid) and every edge's number
+// of faces: per chunk its nodes and corner ids, its edges (those that no other
+// chunk touches first, each part ascending) with their faces' slots, each
+// face's edge, and the places of the edges of several chunks.
+static void build_upwind_chunks(fvm_ctx* c, const std::vector<int>& eid, const std::vector<int>& edge_ptr) {
+    const int T = c->T, npe = c->npe, nfe = c->nfe;
+    const int nch = (T + kUpChunk - 1) / kUpChunk;
+    struct Chunk {
+        std::vector<int> nodes, edges;
+        int own = 0;
+    };
+    std::vector<Chunk> chunk(nch);
+    std::vector<ushort4> loc(T);
+    std::vector<unsigned short> of((size_t)T * nfe), slot((size_t)nch * kUpChunk * nfe, 0);
+    std::vector<std::vector<unsigned short>> start(nch);
+    parallel_for(nch, 16, [&](long first, long last) {
+        std::vector<int> all, cnt, pos;
+        for (long ch = first; ch < last; ++ch) {
+            const int e0 = (int)ch * kUpChunk, e1 = std::min(T, e0 + kUpChunk);
+            Chunk& k = chunk[ch];
+            k.nodes.assign(&c->h_elem_nodes[(size_t)e0 * npe], &c->h_elem_nodes[0] + (size_t)e1 * npe);
+            std::sort(k.nodes.begin(), k.nodes.end());
+            k.nodes.erase(std::unique(k.nodes.begin(), k.nodes.end()), k.nodes.end());
+            for (int e = e0; e < e1; ++e) {
+                unsigned short l[4] = {0, 0, 0, 0};
+                for (int j = 0; j < npe; ++j)
+                    l[j] = (unsigned short)(std::lower_bound(k.nodes.begin(), k.nodes.end(),
+                                                             c->h_elem_nodes[(size_t)e * npe + j]) - k.nodes.begin());
+                loc[e] = make_ushort4(l[0], l[1], l[2], l[3]);
+            }
+            all.assign(&eid[(size_t)e0 * nfe], &eid[0] + (size_t)e1 * nfe);
+            std::sort(all.begin(), all.end());
+            // (whole edges first)
+            std::vector<int> shared;
+            for (size_t p = 0, q; p < all.size(); p = q) {
+                for (q = p; q < all.size() && all[q] == all[p]; ++q) {}
+                const bool whole = (int)(q - p) == edge_ptr[all[p] + 1] - edge_ptr[all[p]];
+                (whole ? k.edges : shared).push_back(all[p]);
+            }
+            k.own = (int)k.edges.size();
+            k.edges.insert(k.edges.end(), shared.begin(), shared.end());
+            const auto mid = k.edges.begin() + k.own;
+            cnt.assign(k.edges.size() + 1, 0);
+            for (int e = e0; e < e1; ++e)
+                for (int f = 0; f < nfe; ++f) {
+                    const int g = eid[(size_t)e * nfe + f];
+                    auto it = std::lower_bound(k.edges.begin(), mid, g);
+                    if (it == mid || *it != g) it = std::lower_bound(mid, k.edges.end(), g);
+                    const int i = (int)(it - k.edges.begin());
+                    of[(size_t)f * T + e] = (unsigned short)i;
+                    cnt[i + 1]++;
+                }
+            for (size_t i = 1; i < cnt.size(); ++i) cnt[i] += cnt[i - 1];
+            start[ch].assign(cnt.begin(), cnt.end());
+            pos.assign(cnt.begin(), cnt.end() - 1);
+            for (int e = e0; e < e1; ++e)
+                for (int f = 0; f < nfe; ++f)
+                    slot[(size_t)e0 * nfe + pos[of[(size_t)f * T + e]]++] = (unsigned short)(f * kUpChunk + (e - e0));
+        }
+    });
+    std::vector<int> node_ptr(1, 0), node, sptr(1, 0);
+    std::vector<int2> edge;
+    std::vector<unsigned short> all_start;
+    std::vector<int> copies(edge_ptr.size() - 1, 0);
+    int ne = 0;
+    for (int ch = 0; ch < nch; ++ch) {
+        const Chunk& k = chunk[ch];
+        node.insert(node.end(), k.nodes.begin(), k.nodes.end());
+        node_ptr.push_back((int)node.size());
+        c->up_nnmax = std::max(c->up_nnmax, (int)k.nodes.size());
+        edge.push_back(make_int2(ne, k.own));
+        c->up_edmax = std::max(c->up_edmax, (int)k.edges.size());
+        ne += (int)k.edges.size();
+        all_start.insert(all_start.end(), start[ch].begin(), start[ch].end());
+        for (size_t i = k.own; i < k.edges.size(); ++i) copies[k.edges[i]]++;
+    }
+    edge.push_back(make_int2(ne, 0));
+    // places of the edges of several chunks, ascending edge, then chunk
+    std::vector<int> at(copies.size(), -1);
+    for (size_t g = 0; g < copies.size(); ++g)
+        if (copies[g]) {
+            at[g] = sptr.back();
+            sptr.push_back(sptr.back() + copies[g]);
+        }
+    std::vector<int> place(sptr.back());
+    for (int ch = 0; ch < nch; ++ch)
+        for (size_t i = chunk[ch].own; i < chunk[ch].edges.size(); ++i)
+            place[at[chunk[ch].edges[i]]++] = edge[ch].x + (int)i;
+    cudaStream_t s = c->stream;
+    c->up_node_ptr.upload(node_ptr, s);
+    c->up_node.upload(node, s);
+    c->up_loc.upload(loc, s);
+    c->up_edge.upload(edge, s);
+    c->up_start.upload(all_start, s);
+    c->up_slot.upload(slot, s);
+    c->up_of.upload(of, s);
+    c->up_sptr.upload(sptr, s);
+    c->up_splace.upload(place, s);
+    c->up_part.alloc(ne);
+    c->up_front.alloc(ne);
+    c->up_chunks = nch;
+    FVM_CUDA(cudaStreamSynchronize(s));   // the copies read these vectors
+}
+
 // ------------------------------------------------------------------ set-up
 static void build(fvm_ctx* c, const fvm_mesh* m, const fvm_physics* ph, int flags) {
     if (!m || !ph) throw Error("fvm_create: null argument");
@@ -778,39 +1078,42 @@ static void build(fvm_ctx* c, const fvm_mesh* m, const fvm_physics* ph, int flag
     std::vector<int4> en(T);
     std::vector<double> coef((size_t)nfe * (npe + 1) * T), area((size_t)nfe * T), vol(T);
     std::vector<double> eK3((size_t)3 * T);
-    for (int e = 0; e < T; ++e) {
-        const int* v = m->elem_nodes + (size_t)e * npe;
-        for (int k = 0; k < npe; ++k)
-            if (v[k] < 0 || v[k] >= N) throw Error("fvm_create: element node id out of range");
-        int z = m->elem_zone[e];
-        if (z < 0 || z >= ph->n_zones) throw Error("fvm_create: element zone out of range");
-        const fvm_zone& Z = ph->zones[z];
-        double Kx = Z.Kxx, Ky = Z.Kyy, Kz = Z.Kzz;
-        if (m->elem_K) Kx = Ky = Kz = m->elem_K[e];
-        eK3[e] = Kx; eK3[(size_t)T + e] = Ky; eK3[(size_t)2 * T + e] = Kz;
-        en[e] = make_int4(v[0], v[1], v[2], dim == 3 ? v[3] : -1);
-        if (dim == 3) {
-            double C[6][4], G[6], A[6];
-            if (!tet_coefficients(m->coords + 3 * (size_t)v[0], m->coords + 3 * (size_t)v[1], m->coords + 3 * (size_t)v[2],
-                                  m->coords + 3 * (size_t)v[3], Kx, Ky, Kz, C, G, A, &vol[e]))
-                throw Error("fvm_create: degenerate tetrahedron " + std::to_string(e));
-            for (int f = 0; f < 6; ++f) {
-                for (int k = 0; k < 4; ++k) coef[(size_t)(f * 5 + k) * T + e] = C[f][k];
-                coef[(size_t)(f * 5 + 4) * T + e] = G[f];
-                area[(size_t)6 * e + f] = A[f];
-            }
-        } else {
-            double C[3][3], G[3], A[3];
-            if (!tri_coefficients(m->coords + 3 * (size_t)v[0], m->coords + 3 * (size_t)v[1], m->coords + 3 * (size_t)v[2],
-                                  Kx, Ky, C, G, A, &vol[e]))
-                throw Error("fvm_create: degenerate triangle " + std::to_string(e));
-            for (int f = 0; f < 3; ++f) {
-                for (int k = 0; k < 3; ++k) coef[(size_t)(f * 4 + k) * T + e] = C[f][k];
-                coef[(size_t)(f * 4 + 3) * T + e] = G[f];
-                area[(size_t)3 * e + f] = A[f];
+    parallel_for(T, 16384, [&](long first, long last) {
+        for (long el = first; el < last; ++el) {
+            const int e = (int)el;
+            const int* v = m->elem_nodes + (size_t)e * npe;
+            for (int k = 0; k < npe; ++k)
+                if (v[k] < 0 || v[k] >= N) throw Error("fvm_create: element node id out of range");
+            int z = m->elem_zone[e];
+            if (z < 0 || z >= ph->n_zones) throw Error("fvm_create: element zone out of range");
+            const fvm_zone& Z = ph->zones[z];
+            double Kx = Z.Kxx, Ky = Z.Kyy, Kz = Z.Kzz;
+            if (m->elem_K) Kx = Ky = Kz = m->elem_K[e];
+            eK3[e] = Kx; eK3[(size_t)T + e] = Ky; eK3[(size_t)2 * T + e] = Kz;
+            en[e] = make_int4(v[0], v[1], v[2], dim == 3 ? v[3] : -1);
+            if (dim == 3) {
+                double C[6][4], G[6], A[6];
+                if (!tet_coefficients(m->coords + 3 * (size_t)v[0], m->coords + 3 * (size_t)v[1], m->coords + 3 * (size_t)v[2],
+                                      m->coords + 3 * (size_t)v[3], Kx, Ky, Kz, C, G, A, &vol[e]))
+                    throw Error("fvm_create: degenerate tetrahedron " + std::to_string(e));
+                for (int f = 0; f < 6; ++f) {
+                    for (int k = 0; k < 4; ++k) coef[(size_t)(f * 5 + k) * T + e] = C[f][k];
+                    coef[(size_t)(f * 5 + 4) * T + e] = G[f];
+                    area[(size_t)6 * e + f] = A[f];
+                }
+            } else {
+                double C[3][3], G[3], A[3];
+                if (!tri_coefficients(m->coords + 3 * (size_t)v[0], m->coords + 3 * (size_t)v[1], m->coords + 3 * (size_t)v[2],
+                                      Kx, Ky, C, G, A, &vol[e]))
+                    throw Error("fvm_create: degenerate triangle " + std::to_string(e));
+                for (int f = 0; f < 3; ++f) {
+                    for (int k = 0; k < 3; ++k) coef[(size_t)(f * 4 + k) * T + e] = C[f][k];
+                    coef[(size_t)(f * 4 + 3) * T + e] = G[f];
+                    area[(size_t)3 * e + f] = A[f];
+                }
             }
         }
-    }
+    });
 
     // ---- control volumes and zone weights (fvmpor.h:471-498)
     std::vector<double> V(N, 0.0);
@@ -882,16 +1185,18 @@ static void build(fvm_ctx* c, const fvm_mesh* m, const fvm_physics* ph, int flag
                 const uint64_t key = ((uint64_t)(uint32_t)std::min(a, b) << 32) | (uint32_t)std::max(a, b);
                 keys[fill[std::min(a, b)]++] = {key, e * nfe + f};
             }
-        for (int i = 0; i < N; ++i)
-            for (size_t r = bptr[i] + 1; r < bptr[i + 1]; ++r) {
-                const auto kv = keys[r];
-                size_t q = r;
-                while (q > bptr[i] && keys[q - 1].first > kv.first) {
-                    keys[q] = keys[q - 1];
-                    --q;
+        parallel_for(N, 8192, [&](long first, long last) {
+            for (long i = first; i < last; ++i)
+                for (size_t r = bptr[i] + 1; r < bptr[i + 1]; ++r) {
+                    const auto kv = keys[r];
+                    size_t q = r;
+                    while (q > bptr[i] && keys[q - 1].first > kv.first) {
+                        keys[q] = keys[q - 1];
+                        --q;
+                    }
+                    keys[q] = kv;
                 }
-                keys[q] = kv;
-            }
+        });
     }
     std::vector<int> edge_ptr(1, 0), edge_face;
     std::vector<double> edge_w;
@@ -917,6 +1222,15 @@ static void build(fvm_ctx* c, const fvm_mesh* m, const fvm_physics* ph, int flag
         p = q;
     }
     c->E = (int)edge_w.size();
+    const bool by_chunk = (T + kUpChunk - 1) / kUpChunk >= kUpMinChunks;
+    std::vector<int> eid;   // each face's edge
+    if (by_chunk) {
+        eid.resize((size_t)T * nfe);
+        parallel_for(c->E, 4096, [&](long first, long last) {
+            for (long g = first; g < last; ++g)
+                for (int p = edge_ptr[g]; p < edge_ptr[g + 1]; ++p) eid[edge_face[p]] = (int)g;
+        });
+    }
 
     // ---- boundary-flux term and Dirichlet rows (process_fluxes :721-758,
     // residual_evaluation :113-114, initialise_vectors :405-451)
@@ -1023,17 +1337,21 @@ static void build(fvm_ctx* c, const fvm_mesh* m, const fvm_physics* ph, int flag
         zd[z] = ZoneDev{Z.phi, Z.alphaVG, Z.nVG, 1.0 - 1.0 / Z.nVG, Z.S_r};
     }
     c->zones.upload(zd, s);
-    c->edge_ptr.upload(edge_ptr, s);
-    c->edge_face.upload(edge_face, s);
-    c->edge_w.upload(edge_w, s);
     c->flip.upload(flip, s);
+    if (by_chunk) {
+        build_upwind_chunks(c, eid, edge_ptr);
+    } else {
+        c->edge_ptr.upload(edge_ptr, s);
+        c->edge_face.upload(edge_face, s);
+        c->edge_w.upload(edge_w, s);
+        c->faceq.alloc((size_t)T * nfe);
+    }
     // averaged weights until the first begin_step (fvmpor.h:594-595)
     c->upw.upload(std::vector<unsigned char>((size_t)8 * c->estride, 2), s);
     c->krw.alloc((size_t)c->nz * N);
     c->krw.zero(s);
     c->hstar.alloc(N);
     c->stor.alloc(N);
-    c->faceq.alloc((size_t)T * nfe);
     for (auto& b : c->tmpN) b.alloc(N);
     c->elem_err.alloc(1);
     c->elem_err.zero(s);

@@ -209,6 +209,18 @@ struct fvm_ctx {
     fvmb::DevBuf<int> edge_ptr, edge_face;  // edge -> e*nfe + f, ascending e
     fvmb::DevBuf<double> edge_w;            // 1 / sum of the edge's face areas
 
+    // the same by chunks of elements, for meshes of many chunks (k_upwind_chunk)
+    int up_chunks = 0, up_nnmax = 0, up_edmax = 0;   // chunks, most nodes and edges of one
+    fvmb::DevBuf<int> up_node_ptr, up_node;      // each chunk's distinct nodes
+    fvmb::DevBuf<ushort4> up_loc;                // [T] chunk-local corner ids
+    fvmb::DevBuf<int2> up_edge;                  // [chunks + 1] first edge, edges that no other chunk touches
+    fvmb::DevBuf<unsigned short> up_start;       // [edges + chunks] first slot of each of a chunk's edges, and its end
+    fvmb::DevBuf<unsigned short> up_slot;        // [T * nfe] a chunk's faces, edge by edge
+    fvmb::DevBuf<unsigned short> up_of;          // [nfe][T] chunk-local edge of each face
+    fvmb::DevBuf<int> up_sptr, up_splace;        // edges of several chunks: their places, ascending chunk
+    fvmb::DevBuf<double> up_part;                // [edges] chunk sums
+    fvmb::DevBuf<unsigned char> up_front;        // [edges] 1: the front node is upstream
+
     // workspace
     fvmb::DevBuf<double> krw;        // [nz][N]
     fvmb::DevBuf<double> hstar;      // perturbed head
