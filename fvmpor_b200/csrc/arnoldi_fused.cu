@@ -631,71 +631,86 @@ bool fused_prepare(fvm_ctx* c, int m) {
         P->fused_ok = false;
         const int nb = P->nb;
         if (!P->smem_stage[1]) return false;
-        std::vector<int> slptr(1, 0), blksl(1, 0), opcol, opsrc;
+        // a block's slices: entries' local columns and sources, slice starts; its
+        // node list (its rows in factor order, then the other operator
+        // columns, sorted) and the blocks owning those nodes.  A slice's rows
+        // have one colour and are consecutive in factor order, and so are,
+        // mostly, their neighbours of another colour: a warp's reads of the
+        // direction hit few banks twice (in node order, eight lanes to a bank)
+        struct Block {
+            std::vector<int> start, src, nodes, nbr;
+            std::vector<unsigned short> lcol;
+        };
+        std::vector<Block> block(nb);
+        parallel_for(nb, 1, [&](long first, long last) {
+            for (long b = first; b < last; ++b) {
+                const int r0 = P->h_bstart[b], r1 = P->h_bstart[b + 1];
+                Block& B = block[b];
+                std::vector<int> col, halo;
+                B.start.assign(1, 0);
+                for (int q0 = r0; q0 < r1; q0 += 32) {
+                    const int n = std::min(32, r1 - q0);
+                    int width = 0;
+                    for (int l = 0; l < n; ++l) {
+                        const int row = P->h_lu_row[q0 + l];
+                        width = std::max(width, P->h_rowptr[row + 1] - P->h_rowptr[row]);
+                    }
+                    width = (width + 3) & ~3;
+                    const size_t base = col.size();
+                    col.resize(base + 32 * (size_t)width);
+                    B.src.resize(base + 32 * (size_t)width);
+                    for (int l = 0; l < 32; ++l) {
+                        const int row = l < n ? P->h_lu_row[q0 + l] : P->h_lu_row[q0];
+                        const int p0 = P->h_rowptr[row], len = l < n ? P->h_rowptr[row + 1] - p0 : 0;
+                        for (int k = 0; k < width; ++k) {
+                            const size_t e = base + (size_t)kOpGroup * (k / 4) + 4 * l + k % 4;
+                            col[e] = k < len ? P->h_col[p0 + k] : row;
+                            B.src[e] = k < len ? p0 + k : -1;
+                            if (col[e] < r0 || col[e] >= r1) halo.push_back(col[e]);
+                        }
+                    }
+                    B.start.push_back((int)col.size());
+                }
+                std::sort(halo.begin(), halo.end());
+                halo.erase(std::unique(halo.begin(), halo.end()), halo.end());
+                B.nodes.assign(P->h_lu_row.begin() + r0, P->h_lu_row.begin() + r1);
+                std::vector<int> place(r1 - r0);   // of the block's own nodes
+                for (int q = r0; q < r1; ++q) place[P->h_lu_row[q] - r0] = q - r0;
+                B.nodes.insert(B.nodes.end(), halo.begin(), halo.end());
+                B.lcol.resize(col.size());
+                for (size_t e = 0; e < col.size(); ++e)
+                    B.lcol[e] = (unsigned short)(col[e] >= r0 && col[e] < r1
+                                                     ? place[col[e] - r0]
+                                                     : r1 - r0 + (std::lower_bound(halo.begin(), halo.end(), col[e]) -
+                                                                  halo.begin()));
+                if (b > 0) B.nbr.push_back((int)b - 1);
+                if (b + 1 < nb) B.nbr.push_back((int)b + 1);
+                for (int v : halo)
+                    B.nbr.push_back((int)(std::upper_bound(P->h_bstart.begin(), P->h_bstart.end(), v) -
+                                          P->h_bstart.begin()) - 1);
+                std::sort(B.nbr.begin(), B.nbr.end());
+                B.nbr.erase(std::unique(B.nbr.begin(), B.nbr.end()), B.nbr.end());
+            }
+        });
+        std::vector<int> slptr(1, 0), blksl(1, 0), opsrc;
         std::vector<int> halo_ptr(1, 0), halo_node, nbr_ptr(1, 0), nbr;
         std::vector<unsigned short> lcol;
-        std::vector<int> where(c->N, -1);
         int nr_max = 0, nh_max = 0, halo_max = 0;
         for (int b = 0; b < nb; ++b) {
-            const int r0 = P->h_bstart[b], r1 = P->h_bstart[b + 1];
-            nr_max = std::max(nr_max, r1 - r0);
-            const size_t ebase = opcol.size();
-            for (int q0 = r0; q0 < r1; q0 += 32) {
-                const int n = std::min(32, r1 - q0);
-                int width = 0;
-                for (int l = 0; l < n; ++l) {
-                    const int row = P->h_lu_row[q0 + l];
-                    width = std::max(width, P->h_rowptr[row + 1] - P->h_rowptr[row]);
-                }
-                width = (width + 3) & ~3;
-                const size_t base = opcol.size();
-                opcol.resize(base + 32 * (size_t)width);
-                opsrc.resize(base + 32 * (size_t)width);
-                for (int l = 0; l < 32; ++l) {
-                    const int row = l < n ? P->h_lu_row[q0 + l] : P->h_lu_row[q0];
-                    const int p0 = P->h_rowptr[row], len = l < n ? P->h_rowptr[row + 1] - p0 : 0;
-                    for (int k = 0; k < width; ++k) {
-                        const size_t e = base + (size_t)kOpGroup * (k / 4) + 4 * l + k % 4;
-                        opcol[e] = k < len ? P->h_col[p0 + k] : row;
-                        opsrc[e] = k < len ? p0 + k : -1;
-                    }
-                }
-                if (opcol.size() >= (size_t)INT32_MAX) return false;
-                slptr.push_back((int)opcol.size());
-            }
+            const Block& B = block[b];
+            const int nr = P->h_bstart[b + 1] - P->h_bstart[b];
+            if (B.nodes.size() >= 65535 || opsrc.size() + B.src.size() >= (size_t)INT32_MAX) return false;
+            nr_max = std::max(nr_max, nr);
+            nh_max = std::max(nh_max, (int)B.nodes.size());
+            halo_max = std::max(halo_max, (int)B.nodes.size() - nr);
+            for (size_t k = 1; k < B.start.size(); ++k) slptr.push_back((int)opsrc.size() + B.start[k]);
             blksl.push_back((int)slptr.size() - 1);
-            // the block's node list (its rows in factor order, then the other
-            // operator columns, sorted), local column indices, and the blocks
-            // owning those nodes.  A slice's rows have one colour and are
-            // consecutive in factor order, and so are, mostly, their
-            // neighbours of another colour: a warp's reads of the direction
-            // hit few banks twice (in node order, eight lanes to a bank)
-            std::vector<int> halo;
-            for (size_t e = ebase; e < opcol.size(); ++e)
-                if (opcol[e] < r0 || opcol[e] >= r1) halo.push_back(opcol[e]);
-            std::sort(halo.begin(), halo.end());
-            halo.erase(std::unique(halo.begin(), halo.end()), halo.end());
-            std::vector<int> nodes(P->h_lu_row.begin() + r0, P->h_lu_row.begin() + r1);
-            nodes.insert(nodes.end(), halo.begin(), halo.end());
-            if (nodes.size() >= 65535) return false;
-            nh_max = std::max(nh_max, (int)nodes.size());
-            halo_max = std::max(halo_max, (int)halo.size());
-            for (size_t k = 0; k < nodes.size(); ++k) where[nodes[k]] = (int)k;
-            for (size_t e = ebase; e < opcol.size(); ++e) lcol.push_back((unsigned short)where[opcol[e]]);
-            std::vector<int> nbs;
-            if (b > 0) nbs.push_back(b - 1);
-            if (b + 1 < nb) nbs.push_back(b + 1);
-            for (int v : halo) {
-                const int ob = (int)(std::upper_bound(P->h_bstart.begin(), P->h_bstart.end(), v) - P->h_bstart.begin()) - 1;
-                if (ob != b) nbs.push_back(ob);
-            }
-            std::sort(nbs.begin(), nbs.end());
-            nbs.erase(std::unique(nbs.begin(), nbs.end()), nbs.end());
-            nbr.insert(nbr.end(), nbs.begin(), nbs.end());
+            opsrc.insert(opsrc.end(), B.src.begin(), B.src.end());
+            lcol.insert(lcol.end(), B.lcol.begin(), B.lcol.end());
+            nbr.insert(nbr.end(), B.nbr.begin(), B.nbr.end());
             nbr_ptr.push_back((int)nbr.size());
-            halo_node.insert(halo_node.end(), nodes.begin(), nodes.end());
+            halo_node.insert(halo_node.end(), B.nodes.begin(), B.nodes.end());
             halo_ptr.push_back((int)halo_node.size());
-            for (int v : nodes) where[v] = -1;
         }
         P->op_slptr.upload(slptr, s);
         P->op_blksl.upload(blksl, s);
@@ -714,7 +729,7 @@ bool fused_prepare(fvm_ctx* c, int m) {
         P->nbr.upload(nbr, s);
         // the blocks' flags, then the barrier counter on its own 128-byte line
         P->flags.alloc(fused_sync_slot(nb) + 32);
-        P->op_val.alloc(opcol.size());
+        P->op_val.alloc(opsrc.size());
         P->op_val.zero(s);   // the padding entries stay zero
         P->op_dg.alloc(c->N);
         P->fused_nrmax = nr_max;

@@ -33,8 +33,9 @@ struct IluBlk {
 
 struct BlockILU {
     bool built = false;
-    int nnz = 0, ncol = 0;
-    std::vector<int> h_rowptr, h_col, h_colour;
+    int nnz = 0;
+    int ncol = 0;             // colours of the reference's set-up, 0 until asked for
+    std::vector<int> h_rowptr, h_col;
     DevBuf<int> col;
     DevBuf<double> J;
     // element-wise finite-difference Jacobian: chunks of consecutive elements

@@ -887,25 +887,94 @@ struct FdTables {
     int nnmax = 0, list_max = 0, grp_max = 0;
 };
 
+// greedy distance-2 colouring in node order (preconditioner_dss.cpp:61-94): the
+// number of residuals the reference's set-up takes.  The element-wise quotients
+// do not use it, so it is formed when asked for (fvm_precond_info).
+static int count_colours(const std::vector<int>& rp, const std::vector<int>& cl) {
+    const int N = (int)rp.size() - 1;
+    std::vector<int> colour(N, -1), cmark(N + 1, -1);
+    int maxc = 0;
+    for (int i = 0; i < N; ++i) {
+        for (int p = rp[i]; p < rp[i + 1]; ++p) {
+            const int nb = cl[p];
+            for (int q = rp[nb]; q < rp[nb + 1]; ++q) {
+                const int cc = colour[cl[q]];
+                if (cc >= 0) cmark[cc] = i;
+            }
+        }
+        int cc = 0;
+        while (cc < maxc && cmark[cc] == i) ++cc;
+        if (cc == maxc) ++maxc;
+        colour[i] = cc;
+    }
+    return maxc;
+}
+
 static void build_fd_tables(const fvm_ctx* c, const BlockILU* P, const std::vector<int>& rowof,
                             const std::vector<int>& lu_dst, FdTables& fd) {
-    const int N = c->N, T = c->T, npe = c->npe, npe2 = npe * npe;
+    const int T = c->T, npe = c->npe, npe2 = npe * npe;
     const std::vector<int>&rp = P->h_rowptr, &cl = P->h_col;
     const int nch = (T + kFdChunk - 1) / kFdChunk;
-    // chunks touching each non-zero, then the places of the shared ones'
-    // partials (non-zero-major, ascending chunk)
-    std::vector<int> fq((size_t)T * npe2), seen(P->nnz, -1), nchunk(P->nnz, 0);
-    for (int e = 0; e < T; ++e) {
-        const int* v = &c->h_elem_nodes[(size_t)e * npe];
-        for (int m = 0; m < npe; ++m)
-            for (int k = 0; k < npe; ++k) {
-                const int i = v[k], j = v[m];
-                const int q = (int)(std::lower_bound(&cl[rp[i]], &cl[0] + rp[i + 1], j) - &cl[0]);
-                fq[(size_t)e * npe2 + m * npe + k] = q;
-                if (seen[q] != e / kFdChunk) { seen[q] = e / kFdChunk; nchunk[q]++; }
+    // every chunk by itself: its nodes, its non-zeros (qs) and the slots of each
+    // (cnt many from pos on, ascending element)
+    struct Chunk {
+        std::vector<int> nodes, qs, cnt, pos;
+        std::vector<unsigned short> slots;
+        // then, once it is known which other chunks touch them
+        std::vector<int4> done;
+        std::vector<int> shared;
+        std::vector<unsigned short> list;
+        int ng = 0;
+    };
+    std::vector<Chunk> chunk(nch);
+    fd.cloc.assign(T, make_ushort4(0, 0, 0, 0));
+    parallel_for(nch, 32, [&](long first, long last) {
+        std::vector<int> fq((size_t)kFdChunk * npe2), at;
+        for (long ch = first; ch < last; ++ch) {
+            const int e0 = (int)ch * kFdChunk, e1 = std::min(T, e0 + kFdChunk);
+            Chunk& k = chunk[ch];
+            const int* v = &c->h_elem_nodes[(size_t)e0 * npe];
+            k.nodes.assign(v, v + (size_t)(e1 - e0) * npe);
+            std::sort(k.nodes.begin(), k.nodes.end());
+            k.nodes.erase(std::unique(k.nodes.begin(), k.nodes.end()), k.nodes.end());
+            // the chunk's part of each node's row, in a dense table: local
+            // number of the non-zero, -1 while not met
+            at.assign(1, 0);
+            for (int i : k.nodes) at.push_back(at.back() + rp[i + 1] - rp[i]);
+            std::vector<int> number(at.back(), -1);
+            for (int e = e0; e < e1; ++e, v += npe) {
+                int l[4] = {0, 0, 0, 0};
+                for (int j = 0; j < npe; ++j)
+                    l[j] = (int)(std::lower_bound(k.nodes.begin(), k.nodes.end(), v[j]) - k.nodes.begin());
+                fd.cloc[e] = make_ushort4((unsigned short)l[0], (unsigned short)l[1], (unsigned short)l[2],
+                                          (unsigned short)l[3]);
+                for (int m = 0; m < npe; ++m)
+                    for (int r = 0; r < npe; ++r) {
+                        const int i = v[r], q = (int)(std::lower_bound(&cl[rp[i]], &cl[0] + rp[i + 1], v[m]) - &cl[0]);
+                        int& n = number[at[l[r]] + q - rp[i]];
+                        if (n < 0) {
+                            n = (int)k.qs.size();
+                            k.qs.push_back(q);
+                            k.cnt.push_back(0);
+                        }
+                        k.cnt[n]++;
+                        fq[(size_t)(e - e0) * npe2 + m * npe + r] = n;
+                    }
             }
-    }
-    std::vector<int> place(P->nnz, -1);
+            k.pos.assign(k.qs.size() + 1, 0);
+            for (size_t p = 0; p < k.qs.size(); ++p) k.pos[p + 1] = k.pos[p] + k.cnt[p];
+            std::vector<int> next(k.pos.begin(), k.pos.end() - 1);
+            k.slots.resize((size_t)(e1 - e0) * npe2);
+            for (int e = 0; e < e1 - e0; ++e)
+                for (int t = 0; t < npe2; ++t)
+                    k.slots[next[fq[(size_t)e * npe2 + t]]++] = (unsigned short)(t * kFdChunk + e);
+        }
+    });
+    // chunks touching each non-zero, and the places of the shared ones'
+    // partials (non-zero-major, ascending chunk)
+    std::vector<int> nchunk(P->nnz, 0), place(P->nnz, -1);
+    for (const Chunk& k : chunk)
+        for (int q : k.qs) nchunk[q]++;
     fd.sptr.assign(1, 0);
     for (int q = 0; q < P->nnz; ++q)
         if (nchunk[q] > 1) {
@@ -913,89 +982,72 @@ static void build_fd_tables(const fvm_ctx* c, const BlockILU* P, const std::vect
             fd.shared.push_back(make_int4(q, lu_dst[q], 0, 2 * rowof[q] + (cl[q] == rowof[q] ? 1 : 0)));
             fd.sptr.push_back(fd.sptr.back() + nchunk[q]);
         }
+    parallel_for(nch, 32, [&](long first, long last) {
+        std::vector<int> asc, rank, order, hist;
+        for (long ch = first; ch < last; ++ch) {
+            Chunk& k = chunk[ch];
+            // the sums' places: finished non-zeros, then shared ones, ascending
+            const int np = (int)k.qs.size();
+            asc.resize(np);
+            for (int p = 0; p < np; ++p) asc[p] = p;
+            std::sort(asc.begin(), asc.end(), [&](int x, int y) {
+                const bool sx = nchunk[k.qs[x]] > 1, sy = nchunk[k.qs[y]] > 1;
+                return sx != sy ? sy : k.qs[x] < k.qs[y];
+            });
+            rank.resize(np);
+            for (int r = 0; r < np; ++r) {
+                const int q = k.qs[asc[r]], i = rowof[q];
+                rank[asc[r]] = r;
+                if (nchunk[q] > 1) {
+                    k.shared.push_back(q);
+                } else {
+                    const int li = (int)(std::lower_bound(k.nodes.begin(), k.nodes.end(), i) - k.nodes.begin());
+                    k.done.push_back(make_int4(q, lu_dst[q], 0, 2 * li + (cl[q] == i ? 1 : 0)));
+                }
+            }
+            // the non-zeros by falling number of slots (a counting sort)
+            const int most = *std::max_element(k.cnt.begin(), k.cnt.end());
+            hist.assign(most + 2, 0);
+            for (int p = 0; p < np; ++p) hist[most - k.cnt[p] + 1]++;
+            for (int n = 0; n <= most; ++n) hist[n + 1] += hist[n];
+            order.resize(np);
+            for (int p = 0; p < np; ++p) order[hist[most - k.cnt[p]]++] = p;
+            std::vector<unsigned short>& list = k.list;
+            const int ng = k.ng = (np + 31) / 32;
+            list.resize(fd_list_offs(ng), 0);
+            for (int g = 0; g < ng; ++g) list[g + 1] = (unsigned short)(list[g] + k.cnt[order[32 * g]]);
+            // lanes past the last non-zero leave their zero past the sums
+            for (int r = 0; r < 32 * ng; ++r) list.push_back((unsigned short)(r < np ? rank[order[r]] : r));
+            for (int g = 0; g < ng; ++g) {
+                const size_t base = list.size();
+                list.resize(base + 32 * (size_t)k.cnt[order[32 * g]], (unsigned short)(npe2 * kFdChunk));
+                for (int l = 0; l < 32 && 32 * g + l < np; ++l) {
+                    const int p = order[32 * g + l];
+                    for (int t = 0; t < k.cnt[p]; ++t) list[base + 32 * (size_t)t + l] = k.slots[k.pos[p] + t];
+                }
+            }
+        }
+    });
     fd.cnode_ptr.assign(1, 0);
     fd.done_ptr.assign(1, 0);
     fd.share_ptr.assign(1, 0);
-    fd.cloc.assign(T, make_ushort4(0, 0, 0, 0));
-    std::fill(seen.begin(), seen.end(), -1);
-    std::vector<int> stamp(N, -1), lid(N, 0), local(P->nnz, 0), nodes, qs, cnt, pos, order, hist, asc, rank;
-    std::vector<unsigned short> sl;
-    for (int ch = 0; ch < nch; ++ch) {
-        const int e0 = ch * kFdChunk, e1 = std::min(T, e0 + kFdChunk);
-        nodes.clear();
-        qs.clear();
-        cnt.clear();
-        for (int e = e0; e < e1; ++e) {
-            for (int k = 0; k < npe; ++k) {
-                const int g = c->h_elem_nodes[(size_t)e * npe + k];
-                if (stamp[g] != ch) { stamp[g] = ch; nodes.push_back(g); }
-            }
-            for (int t = 0; t < npe2; ++t) {
-                const int q = fq[(size_t)e * npe2 + t];
-                if (seen[q] != ch) { seen[q] = ch; local[q] = (int)qs.size(); qs.push_back(q); cnt.push_back(0); }
-                cnt[local[q]]++;
-            }
-        }
-        std::sort(nodes.begin(), nodes.end());
-        for (size_t k = 0; k < nodes.size(); ++k) lid[nodes[k]] = (int)k;
-        for (int e = e0; e < e1; ++e) {
-            unsigned short l[4] = {0, 0, 0, 0};
-            for (int k = 0; k < npe; ++k) l[k] = (unsigned short)lid[c->h_elem_nodes[(size_t)e * npe + k]];
-            fd.cloc[e] = make_ushort4(l[0], l[1], l[2], l[3]);
-        }
-        fd.nnmax = std::max(fd.nnmax, (int)nodes.size());
-        fd.cnode.insert(fd.cnode.end(), nodes.begin(), nodes.end());
+    size_t words = 0;
+    for (const Chunk& k : chunk) words += k.list.size();
+    if (words / 8 >= (size_t)INT32_MAX) throw Error("difference quotients: mesh too large");
+    fd.list.reserve(words);
+    for (const Chunk& k : chunk) {
+        fd.nnmax = std::max(fd.nnmax, (int)k.nodes.size());
+        fd.cnode.insert(fd.cnode.end(), k.nodes.begin(), k.nodes.end());
         fd.cnode_ptr.push_back((int)fd.cnode.size());
-        // the sums' places: finished non-zeros, then shared ones, ascending
-        const int np = (int)qs.size();
-        asc.resize(np);
-        for (int p = 0; p < np; ++p) asc[p] = p;
-        std::sort(asc.begin(), asc.end(), [&](int x, int y) {
-            const bool sx = place[qs[x]] >= 0, sy = place[qs[y]] >= 0;
-            return sx != sy ? sy : qs[x] < qs[y];
-        });
-        rank.resize(np);
-        for (int r = 0; r < np; ++r) {
-            const int q = qs[asc[r]];
-            rank[asc[r]] = r;
-            if (place[q] >= 0) fd.share.push_back(place[q]++);
-            else fd.done.push_back(make_int4(q, lu_dst[q], 0, 2 * lid[rowof[q]] + (cl[q] == rowof[q] ? 1 : 0)));
-        }
+        fd.done.insert(fd.done.end(), k.done.begin(), k.done.end());
         fd.done_ptr.push_back((int)fd.done.size());
+        for (int q : k.shared) fd.share.push_back(place[q]++);
         fd.share_ptr.push_back((int)fd.share.size());
-        // the non-zeros by falling number of slots (a counting sort)
-        const int most = *std::max_element(cnt.begin(), cnt.end());
-        hist.assign(most + 2, 0);
-        for (int p = 0; p < np; ++p) hist[most - cnt[p] + 1]++;
-        for (int k = 0; k <= most; ++k) hist[k + 1] += hist[k];
-        order.resize(np);
-        for (int p = 0; p < np; ++p) order[hist[most - cnt[p]]++] = p;
-        pos.assign(np + 1, 0);
-        for (int p = 0; p < np; ++p) pos[p + 1] = pos[p] + cnt[p];
-        sl.resize((size_t)(e1 - e0) * npe2);
-        for (int e = e0; e < e1; ++e)
-            for (int t = 0; t < npe2; ++t)
-                sl[pos[local[fq[(size_t)e * npe2 + t]]]++] = (unsigned short)(t * kFdChunk + (e - e0));
-        // pos[p] is now the end of non-zero p's slots
-        const int ng = (np + 31) / 32;
-        const size_t l0 = fd.list.size();
-        fd.list_at.push_back(make_int2((int)(l0 / 8), ng));
-        fd.list.resize(l0 + fd_list_offs(ng), 0);
-        for (int g = 0; g < ng; ++g) fd.list[l0 + g + 1] = (unsigned short)(fd.list[l0 + g] + cnt[order[32 * g]]);
-        // lanes past the last non-zero leave their zero past the sums
-        for (int r = 0; r < 32 * ng; ++r) fd.list.push_back((unsigned short)(r < np ? rank[order[r]] : r));
-        for (int g = 0; g < ng; ++g) {
-            const size_t base = fd.list.size();
-            fd.list.resize(base + 32 * (size_t)cnt[order[32 * g]], (unsigned short)(npe2 * kFdChunk));
-            for (int l = 0; l < 32 && 32 * g + l < np; ++l) {
-                const int p = order[32 * g + l];
-                for (int k = 0; k < cnt[p]; ++k) fd.list[base + 32 * (size_t)k + l] = sl[pos[p] - cnt[p] + k];
-            }
-        }
-        fd.list_max = std::max(fd.list_max, (int)(fd.list.size() - l0));
-        fd.grp_max = std::max(fd.grp_max, ng);
+        fd.list_at.push_back(make_int2((int)(fd.list.size() / 8), k.ng));
+        fd.list.insert(fd.list.end(), k.list.begin(), k.list.end());
+        fd.list_max = std::max(fd.list_max, (int)k.list.size());
+        fd.grp_max = std::max(fd.grp_max, k.ng);
     }
-    if (fd.list.size() / 8 >= (size_t)INT32_MAX) throw Error("difference quotients: mesh too large");
     fd.list_at.push_back(make_int2((int)(fd.list.size() / 8), 0));
 }
 
@@ -1012,42 +1064,33 @@ static void build_pattern(fvm_ctx* c, BlockILU* P) {
     }
     // pattern: node i couples to every node of every element containing i
     P->h_rowptr.assign(N + 1, 0);
-    P->h_col.clear();
-    std::vector<int> mark(N, -1), row;
-    for (int i = 0; i < N; ++i) {
+    auto row_of = [&](int i, std::vector<int>& row) {
         row.clear();
-        for (int p = inc_ptr[i]; p < inc_ptr[i + 1]; ++p) {
-            int e = inc[p];
-            for (int k = 0; k < npe; ++k) {
-                int j = c->h_elem_nodes[(size_t)e * npe + k];
-                if (mark[j] != i) { mark[j] = i; row.push_back(j); }
-            }
-        }
+        for (int p = inc_ptr[i]; p < inc_ptr[i + 1]; ++p)
+            for (int k = 0; k < npe; ++k) row.push_back(c->h_elem_nodes[(size_t)inc[p] * npe + k]);
         std::sort(row.begin(), row.end());
-        P->h_col.insert(P->h_col.end(), row.begin(), row.end());
-        P->h_rowptr[i + 1] = (int)P->h_col.size();
-    }
-    P->nnz = (int)P->h_col.size();
+        row.erase(std::unique(row.begin(), row.end()), row.end());
+    };
+    // (counted and formed in two passes: the rows' places follow from the counts)
+    parallel_for(N, 4096, [&](long first, long last) {
+        std::vector<int> row;
+        for (long i = first; i < last; ++i) {
+            row_of((int)i, row);
+            P->h_rowptr[i + 1] = (int)row.size();
+        }
+    });
+    for (int i = 0; i < N; ++i) P->h_rowptr[i + 1] += P->h_rowptr[i];
+    P->nnz = P->h_rowptr[N];
+    P->h_col.resize(P->nnz);
+    parallel_for(N, 4096, [&](long first, long last) {
+        std::vector<int> row;
+        for (long i = first; i < last; ++i) {
+            row_of((int)i, row);
+            std::copy(row.begin(), row.end(), P->h_col.begin() + P->h_rowptr[i]);
+        }
+    });
     const std::vector<int>& rp = P->h_rowptr;
     const std::vector<int>& cl = P->h_col;
-    // greedy distance-2 colouring in node order (preconditioner_dss.cpp:61-94)
-    P->h_colour.assign(N, -1);
-    std::vector<int> cmark(N + 1, -1);
-    int maxc = 0;
-    for (int i = 0; i < N; ++i) {
-        for (int p = rp[i]; p < rp[i + 1]; ++p) {
-            int nb = cl[p];
-            for (int q = rp[nb]; q < rp[nb + 1]; ++q) {
-                int cc = P->h_colour[cl[q]];
-                if (cc >= 0) cmark[cc] = i;
-            }
-        }
-        int cc = 0;
-        while (cc < maxc && cmark[cc] == i) ++cc;
-        if (cc == maxc) ++maxc;
-        P->h_colour[i] = cc;
-    }
-    P->ncol = maxc;
     std::vector<int> rowof(P->nnz);
     for (int i = 0; i < N; ++i)
         for (int p = rp[i]; p < rp[i + 1]; ++p) rowof[p] = i;
@@ -1082,77 +1125,109 @@ static void build_pattern(fvm_ctx* c, BlockILU* P) {
     std::vector<int> lu_ptr(N + 1, 0), lu_src, lu_diag(N), lu_row(N);
     std::vector<unsigned short> lu_col;
     std::vector<int> lvl(N), ulvl(N);
-    std::vector<int> lvl_ptr(1, 0), lvl_rows, blk_lvl(1, 0), ulvl_ptr(1, 0), ulvl_rows, blk_ulvl(1, 0);
+    // rows by level, a block's in [r0, r1); a block's levels end at its runs of
+    // lvl_ptr (from blk_lvl on)
+    std::vector<int> lvl_ptr(1, 0), lvl_rows(N), blk_lvl(1, 0), ulvl_ptr(1, 0), ulvl_rows(N), blk_ulvl(1, 0);
     int nlmax = 0;
     // Schur coupling: interface rows last, levels split by group, and the
     // off-block entries of each factor position
     P->schur_iters = c->schur_iters;
     const bool schur = P->schur_iters >= 0;
     std::vector<int> sch_lv(2 * (size_t)nb, 0), sch_nin(nb, 0), o_ptr(N + 1, 0), o_col, o_src;
-    for (int b = 0; b < nb; ++b) {
-        int r0 = bstart[b], r1 = bstart[b + 1];
-        int nin = r1 - r0;
-        const std::vector<int> ord = block_colour_order(rp, cl, r0, r1, schur, &nin);
-        sch_nin[b] = nin;
-        std::vector<int> linv(r1 - r0);
-        for (int ii = 0; ii < r1 - r0; ++ii) linv[ord[ii]] = ii;
-        std::vector<std::pair<int, int>> ent;
-        for (int ii = 0; ii < r1 - r0; ++ii) {
-            const int i = r0 + ord[ii], q = r0 + ii;
-            lu_row[q] = i;
-            ent.clear();
-            for (int p = rp[i]; p < rp[i + 1]; ++p) {
-                int j = cl[p];
-                if (j < r0 || j >= r1) {
-                    if (schur) { o_col.push_back(j); o_src.push_back(p); }
-                    continue;
+    std::vector<std::vector<int>> ends(nb), uends(nb);
+    parallel_for(nb, 1, [&](long first, long last) {
+        for (long b = first; b < last; ++b) {
+            const int r0 = bstart[b], r1 = bstart[b + 1];
+            int nin = r1 - r0;
+            const std::vector<int> ord = block_colour_order(rp, cl, r0, r1, schur, &nin);
+            sch_nin[b] = nin;
+            for (int ii = 0; ii < r1 - r0; ++ii) {
+                const int i = r0 + ord[ii];
+                lu_row[r0 + ii] = i;
+                int inside = 0;
+                for (int p = rp[i]; p < rp[i + 1]; ++p) inside += cl[p] >= r0 && cl[p] < r1;
+                lu_ptr[r0 + ii + 1] = inside;
+                if (schur) o_ptr[r0 + ii + 1] = rp[i + 1] - rp[i] - inside;
+            }
+        }
+    });
+    for (int q = 0; q < N; ++q) {
+        lu_ptr[q + 1] += lu_ptr[q];
+        o_ptr[q + 1] += o_ptr[q];
+    }
+    lu_src.resize(lu_ptr[N]);
+    lu_col.resize(lu_ptr[N]);
+    o_col.resize(o_ptr[N]);
+    o_src.resize(o_ptr[N]);
+    parallel_for(nb, 1, [&](long first, long last) {
+        for (long b = first; b < last; ++b) {
+            const int r0 = bstart[b], r1 = bstart[b + 1], nin = sch_nin[b];
+            std::vector<int> linv(r1 - r0);
+            for (int q = r0; q < r1; ++q) linv[lu_row[q] - r0] = q - r0;
+            std::vector<std::pair<int, int>> ent;
+            for (int q = r0; q < r1; ++q) {
+                const int i = lu_row[q];
+                ent.clear();
+                int o = o_ptr[q];
+                for (int p = rp[i]; p < rp[i + 1]; ++p) {
+                    const int j = cl[p];
+                    if (j >= r0 && j < r1) {
+                        ent.emplace_back(linv[j - r0], p);
+                    } else if (schur) {
+                        o_col[o] = j;
+                        o_src[o++] = p;
+                    }
                 }
-                ent.emplace_back(linv[j - r0], p);
+                std::sort(ent.begin(), ent.end());
+                lu_diag[q] = -1;
+                int at = lu_ptr[q];
+                for (auto& e : ent) {
+                    if (e.first == q - r0) lu_diag[q] = at;
+                    lu_src[at] = e.second;
+                    lu_col[at++] = (unsigned short)e.first;
+                }
+                if (lu_diag[q] < 0) throw Error("block-ILU: missing diagonal");
             }
-            o_ptr[q + 1] = (int)o_col.size();
-            std::sort(ent.begin(), ent.end());
-            lu_diag[q] = -1;
-            for (auto& e : ent) {
-                if (e.first == ii) lu_diag[q] = (int)lu_src.size();
-                lu_src.push_back(e.second);
-                lu_col.push_back((unsigned short)e.first);
+            // with the Schur coupling no level mixes interior and interface
+            // rows: forward, every interface row comes after the last interior
+            // level; backward, every interior row after the last interface level
+            int nl = 0, lvB = 0;
+            for (int i = r0; i < r1; ++i) {
+                int l = 0;
+                for (int p = lu_ptr[i]; p < lu_diag[i]; ++p) l = std::max(l, lvl[r0 + lu_col[p]] + 1);
+                if (schur && i - r0 >= nin) l = std::max(l, lvB);
+                lvl[i] = l;
+                nl = std::max(nl, l + 1);
+                if (i - r0 < nin) lvB = nl;
             }
-            lu_ptr[q + 1] = (int)lu_src.size();
-            if (lu_diag[q] < 0) throw Error("block-ILU: missing diagonal");
+            int nu = 0, uvS = 0;
+            for (int i = r1 - 1; i >= r0; --i) {
+                int l = 0;
+                for (int p = lu_diag[i] + 1; p < lu_ptr[i + 1]; ++p) l = std::max(l, ulvl[r0 + lu_col[p]] + 1);
+                if (schur && i - r0 < nin) l = std::max(l, uvS);
+                ulvl[i] = l;
+                nu = std::max(nu, l + 1);
+                if (i - r0 >= nin) uvS = nu;
+            }
+            sch_lv[2 * (size_t)b] = lvB;
+            sch_lv[2 * (size_t)b + 1] = uvS;
+            // rows by level, ascending in each
+            auto by_level = [&](const std::vector<int>& level, int n, std::vector<int>& rows, std::vector<int>& end) {
+                end.assign(n + 1, 0);
+                for (int i = r0; i < r1; ++i) end[level[i] + 1]++;
+                for (int l = 0; l < n; ++l) end[l + 1] += end[l];
+                std::vector<int> next(end.begin(), end.end() - 1);
+                for (int i = r0; i < r1; ++i) rows[r0 + next[level[i]]++] = i;
+            };
+            by_level(lvl, nl, lvl_rows, ends[b]);
+            by_level(ulvl, nu, ulvl_rows, uends[b]);
         }
-        // with the Schur coupling no level mixes interior and interface
-        // rows: forward, every interface row comes after the last interior
-        // level; backward, every interior row after the last interface level
-        int nl = 0, lvB = 0;
-        for (int i = r0; i < r1; ++i) {
-            int l = 0;
-            for (int p = lu_ptr[i]; p < lu_diag[i]; ++p) l = std::max(l, lvl[r0 + lu_col[p]] + 1);
-            if (schur && i - r0 >= nin) l = std::max(l, lvB);
-            lvl[i] = l;
-            nl = std::max(nl, l + 1);
-            if (i - r0 < nin) lvB = nl;
-        }
-        int nu = 0, uvS = 0;
-        for (int i = r1 - 1; i >= r0; --i) {
-            int l = 0;
-            for (int p = lu_diag[i] + 1; p < lu_ptr[i + 1]; ++p) l = std::max(l, ulvl[r0 + lu_col[p]] + 1);
-            if (schur && i - r0 < nin) l = std::max(l, uvS);
-            ulvl[i] = l;
-            nu = std::max(nu, l + 1);
-            if (i - r0 >= nin) uvS = nu;
-        }
-        sch_lv[2 * (size_t)b] = lvB;
-        sch_lv[2 * (size_t)b + 1] = uvS;
-        nlmax = std::max(nlmax, std::max(nl, nu));
-        for (int l = 0; l < nl; ++l) {
-            for (int i = r0; i < r1; ++i) if (lvl[i] == l) lvl_rows.push_back(i);
-            lvl_ptr.push_back((int)lvl_rows.size());
-        }
+    });
+    for (int b = 0; b < nb; ++b) {
+        nlmax = std::max(nlmax, (int)std::max(ends[b].size(), uends[b].size()) - 1);
+        for (size_t l = 1; l < ends[b].size(); ++l) lvl_ptr.push_back(bstart[b] + ends[b][l]);
+        for (size_t l = 1; l < uends[b].size(); ++l) ulvl_ptr.push_back(bstart[b] + uends[b][l]);
         blk_lvl.push_back((int)lvl_ptr.size() - 1);
-        for (int l = 0; l < nu; ++l) {
-            for (int i = r0; i < r1; ++i) if (ulvl[i] == l) ulvl_rows.push_back(i);
-            ulvl_ptr.push_back((int)ulvl_rows.size());
-        }
         blk_ulvl.push_back((int)ulvl_ptr.size() - 1);
     }
     P->nb = nb;
@@ -1161,98 +1236,117 @@ static void build_pattern(fvm_ctx* c, BlockILU* P) {
     // the sliced layout of every block (IluBlk) and its record: a level's rows
     // longest first, stable
     std::vector<IluBlk> blk(nb);
-    std::vector<unsigned short> meta, scol;
+    std::vector<std::vector<unsigned short>> bmeta(nb), bcol(nb);
     std::vector<int> spos(lu_src.size()), up(N);
+    parallel_for(nb, 1, [&](long b0, long b1) {
+        for (long b = b0; b < b1; ++b) {
+            const int r0 = bstart[b], r1 = bstart[b + 1], nr = r1 - r0;
+            IluBlk& B = blk[b];
+            B = IluBlk{};
+            B.nl = blk_lvl[b + 1] - blk_lvl[b];
+            B.nu = blk_ulvl[b + 1] - blk_ulvl[b];
+            B.seg = blk_lvl[b];
+            std::vector<int> first[2], start(1, 0), rows[2];
+            for (int upper = 0; upper < 2; ++upper) {
+                const std::vector<int>& ptr = upper ? ulvl_ptr : lvl_ptr;
+                std::vector<int>& ord = upper ? ulvl_rows : lvl_rows;
+                auto begin = [&](int i) { return upper ? lu_diag[i] + 1 : lu_ptr[i]; };
+                auto length = [&](int i) {
+                    return upper ? lu_ptr[i + 1] - lu_diag[i] - 1 : lu_diag[i] - lu_ptr[i];
+                };
+                first[upper].push_back(0);
+                const int g0 = upper ? blk_ulvl[b] : blk_lvl[b], g1 = upper ? blk_ulvl[b + 1] : blk_lvl[b + 1];
+                for (int g = g0; g < g1; ++g) {
+                    std::stable_sort(ord.begin() + ptr[g], ord.begin() + ptr[g + 1],
+                                     [&](int x, int y) { return length(x) > length(y); });
+                    for (int q = ptr[g]; q < ptr[g + 1]; q += 32) {
+                        const int w = length(ord[q]), at = 32 * start.back();
+                        for (int l = 0; l < 32; ++l) {
+                            const int i = q + l < ptr[g + 1] ? ord[q + l] : -1;
+                            if (i >= 0 && upper) up[i] = (int)rows[1].size();
+                            rows[upper].push_back(i < 0 ? (int)kIluNoRow : i - r0);
+                            for (int k = 0; i >= 0 && k < length(i); ++k) spos[begin(i) + k] = at + 32 * k + l;
+                        }
+                        start.push_back(start.back() + w);
+                    }
+                    first[upper].push_back((int)rows[upper].size() / 32);
+                }
+            }
+            B.dp = start.back();
+            if (B.dp > 65535) throw Error("block-ILU: block too large");
+            B.nsl = (int)rows[0].size() / 32;
+            B.nsu = (int)rows[1].size() / 32;
+            bcol[b].assign(32 * (size_t)B.dp, (unsigned short)nr);
+            for (int i = r0; i < r1; ++i) {
+                for (int p = lu_ptr[i]; p < lu_ptr[i + 1]; ++p)
+                    if (p != lu_diag[i]) bcol[b][spos[p]] = lu_col[p];
+                spos[lu_diag[i]] = 32 * B.dp + i - r0;
+            }
+            bcol[b].resize(ilu_columns(B.dp), 0);
+            for (const std::vector<int>* v : {&first[0], &first[1], &start, &rows[0], &rows[1]})
+                bmeta[b].insert(bmeta[b].end(), v->begin(), v->end());
+            bmeta[b].resize(ilu_meta_words(B.nl, B.nu, B.nsl, B.nsu), 0);
+            B.mw = (int)bmeta[b].size();
+        }
+    });
+    std::vector<unsigned short> meta, scol;
     size_t nlu = 0;
     for (int b = 0; b < nb; ++b) {
-        const int r0 = bstart[b], r1 = bstart[b + 1], nr = r1 - r0;
-        IluBlk& B = blk[b];
-        B = IluBlk{};
-        B.nl = blk_lvl[b + 1] - blk_lvl[b];
-        B.nu = blk_ulvl[b + 1] - blk_ulvl[b];
-        B.seg = blk_lvl[b];
-        std::vector<int> first[2], start(1, 0), rows[2];
-        for (int upper = 0; upper < 2; ++upper) {
-            const std::vector<int>& ptr = upper ? ulvl_ptr : lvl_ptr;
-            std::vector<int>& ord = upper ? ulvl_rows : lvl_rows;
-            auto begin = [&](int i) { return upper ? lu_diag[i] + 1 : lu_ptr[i]; };
-            auto length = [&](int i) { return upper ? lu_ptr[i + 1] - lu_diag[i] - 1 : lu_diag[i] - lu_ptr[i]; };
-            first[upper].push_back(0);
-            for (int g = upper ? blk_ulvl[b] : blk_lvl[b]; g < (upper ? blk_ulvl[b + 1] : blk_lvl[b + 1]); ++g) {
-                std::stable_sort(ord.begin() + ptr[g], ord.begin() + ptr[g + 1],
-                                 [&](int x, int y) { return length(x) > length(y); });
-                for (int q = ptr[g]; q < ptr[g + 1]; q += 32) {
-                    const int w = length(ord[q]), at = 32 * start.back();
-                    for (int l = 0; l < 32; ++l) {
-                        const int i = q + l < ptr[g + 1] ? ord[q + l] : -1;
-                        if (i >= 0 && upper) up[i] = (int)rows[1].size();
-                        rows[upper].push_back(i < 0 ? (int)kIluNoRow : i - r0);
-                        for (int k = 0; i >= 0 && k < length(i); ++k)
-                            spos[begin(i) + k] = (int)nlu + at + 32 * k + l;
-                    }
-                    start.push_back(start.back() + w);
-                }
-                first[upper].push_back((int)rows[upper].size() / 32);
-            }
-        }
-        B.v0 = (int)nlu;
-        B.dp = start.back();
-        B.nsl = (int)rows[0].size() / 32;
-        B.nsu = (int)rows[1].size() / 32;
-        for (int i = r0; i < r1; ++i) spos[lu_diag[i]] = (int)nlu + 32 * B.dp + i - r0;
-        nlu += ilu_window(nr, B.dp);
-        if (nlu >= (size_t)INT32_MAX || B.dp > 65535) throw Error("block-ILU: block too large");
-        B.c0 = (int)scol.size();
-        scol.resize(scol.size() + 32 * (size_t)B.dp, (unsigned short)nr);
-        for (int i = r0; i < r1; ++i)
-            for (int p = lu_ptr[i]; p < lu_ptr[i + 1]; ++p)
-                if (p != lu_diag[i]) scol[B.c0 + spos[p] - B.v0] = lu_col[p];
-        scol.resize(scol.size() + kIluSlack, 0);
-        if (scol.size() >= (size_t)INT32_MAX) throw Error("block-ILU: block too large");
-        B.mo = (int)meta.size();
-        B.mw = (int)ilu_meta_words(B.nl, B.nu, B.nsl, B.nsu);
-        for (const std::vector<int>* v : {&first[0], &first[1], &start, &rows[0], &rows[1]})
-            meta.insert(meta.end(), v->begin(), v->end());
-        meta.resize((size_t)B.mo + B.mw, 0);
-        if (meta.size() >= (size_t)INT32_MAX) throw Error("block-ILU: records too large");
+        blk[b].v0 = (int)nlu;
+        blk[b].c0 = (int)scol.size();
+        blk[b].mo = (int)meta.size();
+        nlu += ilu_window(bstart[b + 1] - bstart[b], blk[b].dp);
+        scol.insert(scol.end(), bcol[b].begin(), bcol[b].end());
+        meta.insert(meta.end(), bmeta[b].begin(), bmeta[b].end());
+        if (nlu >= (size_t)INT32_MAX || scol.size() >= (size_t)INT32_MAX || meta.size() >= (size_t)INT32_MAX)
+            throw Error("block-ILU: block too large");
     }
     P->nlu = nlu;
     // elimination schedule in level order (window positions relative to each
     // block's first entry, as the factorisation indexes); the same update set
     // and order as merging row i with U(k) for each L entry
     std::vector<int> seg_ptr(lvl_ptr.size(), 0);
-    std::vector<unsigned> upd;
-    size_t seg_max = 0;
-    for (int b = 0; b < nb; ++b) {
-        const int r0 = bstart[b], base = blk[b].v0;
-        for (int g = blk_lvl[b]; g < blk_lvl[b + 1]; ++g) {
-            seg_ptr[g] = (int)upd.size();
-            const int q0 = lvl_ptr[g], q1 = lvl_ptr[g + 1];
-            const size_t head = upd.size();
-            upd.resize(head + (q1 - q0 + 31) / 32 * 32, 0u);
-            for (int q = q0; q < q1; ++q) {
-                const int i = lvl_rows[q];
-                upd[head + (q - q0)] = (unsigned)(upd.size() - head);
-                for (int p = lu_ptr[i]; p < lu_diag[i]; ++p) {
-                    const size_t cw = upd.size();
-                    upd.push_back(0u);
-                    const int k = r0 + lu_col[p];
-                    int kpos = lu_diag[k] + 1;
-                    const int kend = lu_ptr[k + 1];
-                    for (int jj = p + 1; jj < lu_ptr[i + 1] && kpos < kend; ++jj) {
-                        const int j = lu_col[jj];
-                        while (kpos < kend && lu_col[kpos] < j) ++kpos;
-                        if (kpos < kend && lu_col[kpos] == j)
-                            upd.push_back((unsigned)(spos[jj] - base) | ((unsigned)(spos[kpos] - base) << 16));
+    std::vector<std::vector<unsigned>> bupd(nb);
+    parallel_for(nb, 1, [&](long b0, long b1) {
+        for (long b = b0; b < b1; ++b) {
+            const int r0 = bstart[b];
+            std::vector<unsigned>& u = bupd[b];
+            for (int g = blk_lvl[b]; g < blk_lvl[b + 1]; ++g) {
+                const int q0 = lvl_ptr[g], q1 = lvl_ptr[g + 1];
+                const size_t head = u.size();
+                u.resize(head + (q1 - q0 + 31) / 32 * 32, 0u);
+                for (int q = q0; q < q1; ++q) {
+                    const int i = lvl_rows[q];
+                    u[head + (q - q0)] = (unsigned)(u.size() - head);
+                    for (int p = lu_ptr[i]; p < lu_diag[i]; ++p) {
+                        const size_t cw = u.size();
+                        u.push_back(0u);
+                        const int k = r0 + lu_col[p];
+                        int kpos = lu_diag[k] + 1;
+                        const int kend = lu_ptr[k + 1];
+                        for (int jj = p + 1; jj < lu_ptr[i + 1] && kpos < kend; ++jj) {
+                            const int j = lu_col[jj];
+                            while (kpos < kend && lu_col[kpos] < j) ++kpos;
+                            if (kpos < kend && lu_col[kpos] == j)
+                                u.push_back((unsigned)spos[jj] | ((unsigned)spos[kpos] << 16));
+                        }
+                        u[cw] = (unsigned)(u.size() - cw - 1);
                     }
-                    upd[cw] = (unsigned)(upd.size() - cw - 1);
                 }
+                seg_ptr[g + 1] = (int)(u.size() - head);
             }
-            seg_max = std::max(seg_max, upd.size() - head);
         }
-        seg_ptr[blk_lvl[b + 1]] = (int)upd.size();
+    });
+    std::vector<unsigned> upd;
+    size_t seg_max = 0, nupd = 0;
+    for (const auto& u : bupd) nupd += u.size();
+    if (nupd >= (size_t)INT32_MAX) throw Error("block-ILU: elimination schedule too large");
+    upd.reserve(nupd);
+    for (const auto& u : bupd) upd.insert(upd.end(), u.begin(), u.end());
+    for (size_t g = 0; g + 1 < seg_ptr.size(); ++g) {
+        seg_max = std::max(seg_max, (size_t)seg_ptr[g + 1]);
+        seg_ptr[g + 1] += seg_ptr[g];
     }
-    if (upd.size() >= (size_t)INT32_MAX) throw Error("block-ILU: elimination schedule too large");
     {
         size_t need64 = 0, need32 = 0;
         bool fits16 = true;
@@ -1367,7 +1461,8 @@ static void build_pattern(fvm_ctx* c, BlockILU* P) {
     {
         // where the quotient kernels put each Jacobian entry for the factorisation
         std::vector<int> lu_dst(P->nnz, -1);
-        for (size_t p = 0; p < lu_src.size(); ++p) lu_dst[lu_src[p]] = spos[p];
+        for (int b = 0; b < nb; ++b)
+            for (int p = lu_ptr[bstart[b]]; p < lu_ptr[bstart[b + 1]]; ++p) lu_dst[lu_src[p]] = blk[b].v0 + spos[p];
         FdTables fd;
         build_fd_tables(c, P, rowof, lu_dst, fd);
         P->fd_cnode_ptr.upload(fd.cnode_ptr, s);
@@ -1674,7 +1769,10 @@ extern "C" int fvm_precond_info(fvm_ctx* c, int* nnz, int* ncolours, int* nblock
     try {
         if (!c || !c->ilu || !c->ilu->built) throw Error("fvm_precond_info: no preconditioner");
         if (nnz) *nnz = c->ilu->nnz;
-        if (ncolours) *ncolours = c->ilu->ncol;
+        if (ncolours) {
+            if (!c->ilu->ncol) c->ilu->ncol = count_colours(c->ilu->h_rowptr, c->ilu->h_col);
+            *ncolours = c->ilu->ncol;
+        }
         if (nblocks) *nblocks = c->ilu->nb;
         if (max_levels) *max_levels = c->ilu->nlevels_max;
         return 0;
