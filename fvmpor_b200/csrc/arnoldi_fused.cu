@@ -22,8 +22,8 @@
 //     through per-block partials);
 //   - every block computes the Hessenberg column, the rotations and the
 //     stopping test from the same reduced numbers, so all take the same
-//     decision without another barrier; block 0 writes them out for the
-//     host's back substitution.
+//     decision without another barrier; block 0 keeps them and at the end
+//     does the back substitution.
 // One bounded grid barrier per step with delayed reorthogonalisation, two
 // with CGS2 (after each dot pass).  The next
 // direction is published block by block: a block raises its flag once its
@@ -46,6 +46,8 @@ struct FusedArgs {
     int nqp;                   // quads per block row array in shared memory (quad-transposed, quad_pos)
     size_t stage_max;          // shared bytes of the largest block's staged factor
     ArnState* st;
+    double tol, sqrtN;         // stop when |g_j| / sqrt(N) <= tol
+    double* coef;              // the solution's coefficients (times the scales), for k_combine_dev
     float* U;
     size_t ld;
     double* scale;
@@ -58,8 +60,9 @@ struct FusedArgs {
     const int* halo_node;
     const int* nbr_ptr;        // [nb + 1] blocks whose flags a block waits for
     const int* nbr;
-    unsigned* flags;           // [nb] last step whose direction rows a block wrote
-    unsigned* sync;            // arrival counter of the cycle's grid barriers (cleared with the flags)
+    unsigned* flags;           // [nb] base + last step whose direction rows a block wrote
+    unsigned* sync;            // arrival counter of the grid barriers
+    unsigned base;             // above every flag of earlier launches
     const float* op_val;
     const float* op_dg;        // [N], factor order: ahh(h + d) on free rows, else 0
     float dcj;                 // cj - cj of the set-up
@@ -73,9 +76,6 @@ struct FusedArgs {
     double* partial;
     int* err;
     double* H;
-    double* cs;
-    double* sn;
-    double* g;
 };
 
 __device__ __forceinline__ unsigned ld_acquire_gpu(const unsigned* p) {
@@ -92,8 +92,8 @@ __device__ __forceinline__ unsigned atom_add_release_gpu(unsigned* p, unsigned v
     return old;
 }
 
-// Grid barrier of the cycle on a counter that only grows within a launch
-// (cleared with the flags before it): a block adds 1 with release semantics
+// Grid barrier of the cycle on a counter that only grows (a launch leaves it at a
+// multiple of the grid size, fused_cycle): a block adds 1 with release semantics
 // and waits (acquire, bounded) until the counter reaches the next multiple
 // of the grid size.  Its own arrival number says which multiple, so there is
 // no generation word, no reset and no further step for the last block to
@@ -198,6 +198,32 @@ __device__ __forceinline__ void op_apply(const FusedArgs& a, const OpSlice& R, f
     if (q < rows.z) x[q] = fmaf(-a.dcj * R.dg, tl[q], acc);
 }
 
+// Back substitution H y = g of the cycle's k columns (block 0), the coefficients
+// times the basis vectors' scales to a.coef: the solution is formed without the
+// host.  H comes back from global memory (this block wrote it) into the block's
+// shared memory, whose other contents are no longer needed, packed by columns.
+__host__ __device__ __forceinline__ int tri_words(int c) { return c * (c + 1) / 2; }
+__device__ __forceinline__ void back_substitute(const FusedArgs& a, int k, const double* sc, const double* gs) {
+    double* R = reinterpret_cast<double*>(ilu_smem());
+    for (int e = threadIdx.x; e < k * k; e += blockDim.x) {
+        const int i = e / k, c = e - i * k;
+        if (i <= c) R[tri_words(c) + i] = __ldcg(a.H + (size_t)i * a.m + c);
+    }
+    __syncthreads();
+    if (threadIdx.x >= 32) return;
+    const int lane = threadIdx.x;
+    // lane l holds rows l and l + 32
+    double r0 = lane < k ? gs[lane] : 0.0, r1 = lane + 32 < k ? gs[lane + 32] : 0.0;
+    for (int c = k - 1; c >= 0; --c) {
+        const double* col = R + tri_words(c);
+        const double d = col[c], top = __shfl_sync(0xffffffffu, c < 32 ? r0 : r1, c & 31);
+        const double y = d != 0.0 ? top / d : 0.0;
+        if (lane < c) r0 -= col[lane] * y;
+        if (lane + 32 < c) r1 -= col[lane + 32] * y;
+        if (lane == 0) a.coef[c] = y * sc[c];
+    }
+}
+
 // at most 384 threads (one per row quad of a 1,536-row block; larger blocks
 // loop), so a thread may hold up to 170 registers
 constexpr int kFusedThreads = 384;
@@ -256,18 +282,39 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_arnoldi_fused(FusedArgs a)
         s_rows = make_int3(a.blksl[b + 1] - a.blksl[b], r0, nr);
     }
     for (int q = threadIdx.x; q < nr; q += blockDim.x) inv[a.lu_row[r0 + q] - r0] = (unsigned short)q;
+    const int sl0 = a.blksl[b], nsl = a.blksl[b + 1] - sl0;
+    const int h0 = a.halo_ptr[b], nh = a.halo_ptr[b + 1] - h0;
+    for (int k = threadIdx.x; k <= nsl; k += blockDim.x) Sl[k] = a.slptr[sl0 + k];
+    // the padding rows of the edge quads stay zero
+    for (int k = threadIdx.x; k < 4 * nqp; k += blockDim.x) {
+        Ws[k] = 0.0;
+        if constexpr (DEL) {
+            Vs[k] = 0.0;
+            const int e = k / nqp, row = (r0 & ~3) + 4 * (k - e * nqp) + e;   // inverse of quad_pos
+            Es[k] = row >= r0 && row < r1 ? a.ewt[row] : 1.0;
+        }
+    }
+    if constexpr (DEL)
+        for (int k = nr + threadIdx.x; k < nh; k += blockDim.x) Hn[k - nr] = a.halo_node[h0 + k];
+    // All so far was there before the kernel ahead of this one, which wrote U_0
+    // and its norm, could start: its launch need not have ended
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     const int m = a.m;
-    const double tol = a.st->tol, sqrtN = a.st->sqrtN;
+    const double tol = a.tol, sqrtN = a.sqrtN;
     // the cycle's initial residual norm (||D P^-1 r||, left by the host's
     // launches in a.beta2) decides whether any step is needed
     const double beta = sqrt(*a.beta2);
     const double rn0 = beta / sqrtN;
     for (int i = threadIdx.x; i <= m; i += blockDim.x) gs[i] = i == 0 ? beta : 0.0;
-    // the scale of U_0 (1 / beta), also for the host's back substitution
+    // the scale of U_0 (1 / beta)
     const double s0 = beta > 0.0 ? 1.0 / beta : 0.0;
     if (threadIdx.x == 0) {
         sc[0] = s0;
-        if (b == 0) a.scale[0] = s0;
+        if (b == 0) {
+            a.scale[0] = s0;
+            a.st->done = 0;   // until the cycle ends
+            a.st->j = 0;
+        }
     }
     if (!isfinite(beta) || rn0 <= tol) {
         if (b == 0 && threadIdx.x == 0) {
@@ -282,7 +329,6 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_arnoldi_fused(FusedArgs a)
     if (!ok) ok = tc05::mbar_wait(mbar, 0);   // copies in flight get a second bounded chance
     if (!__syncthreads_and(ok ? 1 : 0) && threadIdx.x == 0) fused_fail(a.sync, a.err, 2);   // all blocks stop at the next barrier
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    const int sl0 = a.blksl[b], nsl = a.blksl[b + 1] - sl0;
     // vector-major partials: pa[v * nblk + b]
     double* pa = a.partial;
     double* pb = a.partial + (size_t)nblk * 64;
@@ -291,24 +337,12 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_arnoldi_fused(FusedArgs a)
     // out and belong to blocks it waits for), so the read-only path is safe
     const BasisRows<float, false> UR{a.U, a.ld};
     const int q0 = r0 & ~3;
-    const int h0 = a.halo_ptr[b], nh = a.halo_ptr[b + 1] - h0;
     const int nb0 = a.nbr_ptr[b], nb1 = a.nbr_ptr[b + 1];
-    for (int k = threadIdx.x; k <= nsl; k += blockDim.x) Sl[k] = a.slptr[sl0 + k];
     // step 0's direction s_0 U_0 / ewt at the block's own and halo nodes
     // (U_0 was written before the launch)
     for (int k = threadIdx.x; k < nh; k += blockDim.x) {
         const int node = a.halo_node[h0 + k];
-        if (DEL && k >= nr) Hn[k - nr] = node;
         tl[k] = (float)(s0 * (double)__ldcg(a.U + node) / a.ewt[node]);
-    }
-    // the padding rows of the edge quads stay zero
-    for (int k = threadIdx.x; k < 4 * nqp; k += blockDim.x) {
-        Ws[k] = 0.0;
-        if constexpr (DEL) {
-            Vs[k] = 0.0;
-            const int e = k / nqp, row = (r0 & ~3) + 4 * (k - e * nqp) + e;   // inverse of quad_pos
-            Es[k] = row >= r0 && row < r1 ? a.ewt[row] : 1.0;
-        }
     }
     __syncthreads();
     for (int j = 0;; ++j) {
@@ -512,7 +546,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_arnoldi_fused(FusedArgs a)
         }
         // publish this block's rows of the next direction
         __syncthreads();
-        if (threadIdx.x == 0) st_release_gpu(a.flags + b, (unsigned)nv);   // release: the block's writes before the barrier
+        if (threadIdx.x == 0) st_release_gpu(a.flags + b, a.base + (unsigned)nv);   // release: the block's writes before the barrier
         __syncthreads();
         // rotations and stopping test for the finalised column, the same in
         // every block (the same reduced numbers, the same operations), on
@@ -523,7 +557,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_arnoldi_fused(FusedArgs a)
                 for (int kk = nb0 + lane; kk < nb1; kk += 32) {
                     const unsigned* f = a.flags + a.nbr[kk];
                     long it = 0;
-                    while (ld_acquire_gpu(f) < (unsigned)nv) {
+                    while (ld_acquire_gpu(f) < a.base + (unsigned)nv) {
                         if (++it > (1l << 26)) { fused_fail(a.sync, a.err, 3); break; }
                     }
                 }
@@ -565,10 +599,6 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_arnoldi_fused(FusedArgs a)
                     else if (hcol + 1 == m) done = 2;
                     if (b == 0) {
                         for (int i = 0; i <= hcol; ++i) a.H[(size_t)i * m + hcol] = hc[i];
-                        a.cs[hcol] = cj_;
-                        a.sn[hcol] = sj_;
-                        a.g[hcol] = gs[hcol];
-                        a.g[hcol + 1] = gs[hcol + 1];
                         a.scale[hcol + 1] = newscale;
                         a.st->rnorm = rn;
                         a.st->j = hcol + 1;
@@ -579,7 +609,10 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_arnoldi_fused(FusedArgs a)
             s_done = done;
         }
         __syncthreads();
-        if (s_done) return;
+        if (s_done) {
+            if (b == 0 && s_done != 3) back_substitute(a, hcol + 1, sc, gs);
+            return;
+        }
     }
 }
 
@@ -597,7 +630,8 @@ static int fused_variant(const fvm_ctx* c) { return c->krylov_variant ? 1 : 0; }
 
 // dynamic shared bytes of a cycle of up to m steps
 static size_t fused_bytes(const BlockILU* P, int variant, int m) {
-    return variant ? P->fused_smem_d + 8 * (size_t)hess_words(m) : P->fused_smem;
+    const size_t cycle = variant ? P->fused_smem_d + 8 * (size_t)hess_words(m) : P->fused_smem;
+    return std::max(cycle, 8 * (size_t)tri_words(m));   // (back_substitute)
 }
 
 // values of the operator's slices from the set-up's Jacobian (FP64 CSR) and
@@ -614,6 +648,14 @@ __global__ void k_op_refresh(long ne, const int* __restrict__ src, const double*
         const int row = lu_row[t];
         dgq[t] = ntype[row] ? 0.f : (float)ahhp[row];
     }
+}
+
+// flags and barrier counter back to zero: first, after a failed launch (whose
+// blocks left at different barriers), and before either could overflow
+void fused_reset(fvm_ctx* c) {
+    if (!c->ilu || !c->ilu->flags.n) return;
+    c->ilu->flags.zero(c->stream);
+    c->ilu->fused_launches = 0;
 }
 
 // Host side: the slice layout (once per pattern), the launch checks, and the
@@ -729,6 +771,7 @@ bool fused_prepare(fvm_ctx* c, int m) {
         P->nbr.upload(nbr, s);
         // the blocks' flags, then the barrier counter on its own 128-byte line
         P->flags.alloc(fused_sync_slot(nb) + 32);
+        fused_reset(c);
         P->op_val.alloc(opsrc.size());
         P->op_val.zero(s);   // the padding entries stay zero
         P->op_dg.alloc(c->N);
@@ -790,10 +833,9 @@ bool fused_prepare(fvm_ctx* c, int m) {
     return true;
 }
 
-// one cycle: the Arnoldi state (j = 0), g[0] and U_0 with its scale are in
-// place; runs until convergence, a full basis or a breakdown
-void fused_cycle(fvm_ctx* c, Krylov* K, double cj, const double* ewt, double* H_d, double* cs_d, double* sn_d,
-                 double* g_d) {
+// one cycle from U_0 and its squared norm (K->res[0]); runs until convergence, a
+// full basis or a breakdown, and leaves the state and the coefficients
+void fused_cycle(fvm_ctx* c, Krylov* K, double cj, double tol, const double* ewt, double* H_d, double* coef) {
     BlockILU* P = c->ilu;
     cudaStream_t s = c->stream;
     float* U = reinterpret_cast<float*>(K->U);
@@ -807,6 +849,9 @@ void fused_cycle(fvm_ctx* c, Krylov* K, double cj, const double* ewt, double* H_
     a.halo_max = P->fused_hmax;
     a.stage_max = P->fused_stage;
     a.st = K->st.p;
+    a.tol = tol;
+    a.sqrtN = std::sqrt((double)c->N);
+    a.coef = coef;
     a.U = U;
     a.ld = K->ld;
     a.scale = K->scale.p;
@@ -834,21 +879,22 @@ void fused_cycle(fvm_ctx* c, Krylov* K, double cj, const double* ewt, double* H_
     a.partial = K->partial.p;
     a.err = K->err.p;
     a.H = H_d;
-    a.cs = cs_d;
-    a.sn = sn_d;
-    a.g = g_d;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(P->nb);
     cfg.blockDim = dim3(P->fused_threads);
     const int var = fused_variant(c);
     cfg.dynamicSmemBytes = fused_bytes(P, var, K->m);
     cfg.stream = s;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeCooperative;
     attr[0].val.cooperative = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    P->flags.zero(s);
+    cfg.numAttrs = 2;
+    // a launch takes at most 64 flag values and 64 barriers
+    if (P->fused_launches >= (1u << 29) / (64u * (unsigned)P->nb)) fused_reset(c);
+    a.base = 64u * P->fused_launches++;
     c->tm.begin(TM_CGS, s);
     if (var) FVM_CUDA(cudaLaunchKernelEx(&cfg, k_arnoldi_fused<true>, a));
     else FVM_CUDA(cudaLaunchKernelEx(&cfg, k_arnoldi_fused<false>, a));

@@ -31,24 +31,45 @@ struct Coef7 {
 
 __global__ void k_ewt(int N, const double* __restrict__ y, double rtol, double atol,
                       double* __restrict__ ewt) {
+    pdl_wait_and_trigger();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < N) ewt[i] = 1.0 / (rtol * fabs(y[i]) + atol);
 }
 
-// y = sum_{j<=k} phi_j ; yp = sum_{1<=j<=k} gamma_j phi_j ; e = 0
+// node i's phi_j0..phi_j1, all loads in flight together: taken one by one in a loop
+// that also stores, each waits for the last (7.6 us for a step's phi update on
+// the 214k-node box, an L2 latency per order)
+__device__ __forceinline__ void load_phi(const PhiPtrs& ph, int i, int j0, int j1, double (&v)[kNPhi]) {
+#pragma unroll
+    for (int j = 0; j < kNPhi; ++j) v[j] = j >= j0 && j <= j1 ? ph.p[j][i] : 0.0;
+}
+
+// y = sum_{j<=k} phi_j ; yp = sum_{1<=j<=k} gamma_j phi_j ; e = 0; out = the
+// weighted squared sum of y (the predictor's norm)
 __global__ void k_predict(int N, int k, PhiPtrs ph, Coef7 gamma, double* __restrict__ y,
-                          double* __restrict__ yp, double* __restrict__ e) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= N) return;
-    double s = ph.p[0][i], sp = 0.0;
-    for (int j = 1; j <= k; ++j) {
-        double v = ph.p[j][i];
-        s += v;
-        sp += gamma.v[j] * v;
+                          double* __restrict__ yp, double* __restrict__ e, const double* __restrict__ ewt,
+                          double* partial, unsigned* counter, double* out) {
+    pdl_wait_and_trigger();
+    double sum = 0.0;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) {
+        double v[kNPhi];
+        load_phi(ph, i, 0, k, v);
+        double s = v[0], sp = 0.0;
+#pragma unroll
+        for (int j = 1; j < kNPhi; ++j)
+            if (j <= k) {
+                s += v[j];
+                sp += gamma.v[j] * v[j];
+            }
+        y[i] = s;
+        yp[i] = sp;
+        e[i] = 0.0;
+        const double w = s * ewt[i];
+        sum += w * w;
     }
-    y[i] = s;
-    yp[i] = sp;
-    e[i] = 0.0;
+    const double t = block_sum(sum);
+    if (threadIdx.x == 0) partial[blockIdx.x] = t;
+    last_block_reduce(partial, 1, counter, out);
 }
 
 // dense output: y = sum_{j<=k} c_j phi_j ; yp = sum_{1<=j<=k} d_j phi_j
@@ -68,77 +89,88 @@ __global__ void k_interp(int N, int k, PhiPtrs ph, Coef7 c, Coef7 d, double* __r
 }
 
 __global__ void k_phi_scale(int N, int j0, int j1, PhiPtrs ph, Coef7 f) {
+    pdl_wait_and_trigger();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= N) return;
-    for (int j = j0; j <= j1; ++j) ph.p[j][i] *= f.v[j];
+    double v[kNPhi];
+    load_phi(ph, i, j0, j1, v);
+#pragma unroll
+    for (int j = 0; j < kNPhi; ++j)
+        if (j >= j0 && j <= j1) ph.p[j][i] = v[j] * f.v[j];
 }
 
 // y -= x, y' -= cj x, e -= x ; out = sum (x ewt)^2
+// weighted squared sums of the error estimates at orders k, k + 1, k - 1 ... of a
+// step with correction e (the controller's err_norms)
+struct ErrSums {
+    double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
+    __device__ __forceinline__ void add(int k, const PhiPtrs& ph, int i, double ei, double w) {
+        const double a = ei * w;
+        s0 += a * a;
+        const double d1 = ph.p[k][i] + ei;
+        const double b = d1 * w;
+        s1 += b * b;
+        if (k >= 2) {
+            const double d2 = ph.p[k - 1][i] + d1;
+            const double c2 = d2 * w;
+            s2 += c2 * c2;
+        }
+        if (k + 1 < kNPhi) {
+            const double d3 = ei - ph.p[k + 1][i];
+            const double c3 = d3 * w;
+            s3 += c3 * c3;
+        }
+    }
+    // the block's four sums, by thread 0
+    __device__ __forceinline__ void store(double* out) {
+        const double t0 = block_sum(s0), t1 = block_sum(s1), t2 = block_sum(s2), t3 = block_sum(s3);
+        if (threadIdx.x == 0) {
+            out[0] = t0;
+            out[1] = t1;
+            out[2] = t2;
+            out[3] = t3;
+        }
+    }
+};
+// Newton update and, of the e it leaves, the error norms of the step's test (the
+// sums of k_err_norms as out[1..4]): what the host waits for is one pass over the
+// vectors and one reduction, 12.0 us on the 214k-node box where the two kernels
+// took 10.2 + 11.1 us
 __global__ void k_newton_update(int N, const double* __restrict__ x, double cj,
                                 const double* __restrict__ ewt, double* __restrict__ y,
-                                double* __restrict__ yp, double* __restrict__ e, double* partial,
-                                unsigned* counter, double* out) {
+                                double* __restrict__ yp, double* __restrict__ e, int k, PhiPtrs ph, double* partial,
+                                unsigned* counter, double* out, const int* go, const int* status, double mark) {
+    pdl_wait_and_trigger();
+    // queued behind a solve (go): nothing unless it converged, with a factor
+    // without zero pivots; out[6] = mark tells the host that it was done
+    if (go && (*go != 1 || *status != 0)) return;
+    if (blockIdx.x == 0 && threadIdx.x == 0) out[6] = mark;
     double s = 0.0;
+    ErrSums q;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) {
-        double d = x[i];
+        const double d = x[i], w = ewt[i], ei = e[i] - d;
+        q.add(k, ph, i, ei, w);
         y[i] -= d;
         yp[i] -= cj * d;
-        e[i] -= d;
-        double w = d * ewt[i];
-        s += w * w;
+        e[i] = ei;
+        const double dw = d * w;
+        s += dw * dw;
     }
-    double t = block_sum(s);
-    if (threadIdx.x == 0) partial[blockIdx.x] = t;
-    last_block_reduce(partial, 1, counter, out);
+    const double t = block_sum(s);
+    if (threadIdx.x == 0) partial[5 * blockIdx.x] = t;
+    q.store(partial + 5 * blockIdx.x + 1);
+    last_block_reduce(partial, 5, counter, out);
 }
-
-// out = sum (y ewt)^2: the predictor's squared WRMS norm times N
-__global__ void k_pred_sumsq(int N, const double* __restrict__ y, const double* __restrict__ ewt, double* partial,
-                             unsigned* counter, double* out) {
-    double s = 0.0;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) {
-        const double w = y[i] * ewt[i];
-        s += w * w;
-    }
-    double t = block_sum(s);
-    if (threadIdx.x == 0) partial[blockIdx.x] = t;
-    last_block_reduce(partial, 1, counter, out);
-}
-
 // squared error-test norms times N:
 //  0: e  1: phi_k + e  2: phi_{k-1} + phi_k + e  3: e - phi_{k+1}
 __global__ void k_err_norms(int N, int k, PhiPtrs ph, const double* __restrict__ e,
                             const double* __restrict__ ewt, double* partial, unsigned* counter,
                             double* out) {
-    double s0 = 0, s1 = 0, s2 = 0, s3 = 0;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) {
-        double w = ewt[i], ei = e[i];
-        double a = ei * w;
-        s0 += a * a;
-        double d1 = ph.p[k][i] + ei;
-        double b = d1 * w;
-        s1 += b * b;
-        if (k >= 2) {
-            double d2 = ph.p[k - 1][i] + d1;
-            double c2 = d2 * w;
-            s2 += c2 * c2;
-        }
-        if (k + 1 < kNPhi) {
-            double d3 = ei - ph.p[k + 1][i];
-            double c3 = d3 * w;
-            s3 += c3 * c3;
-        }
-    }
-    double t0 = block_sum(s0);
-    double t1 = block_sum(s1);
-    double t2 = block_sum(s2);
-    double t3 = block_sum(s3);
-    if (threadIdx.x == 0) {
-        partial[4 * blockIdx.x + 0] = t0;
-        partial[4 * blockIdx.x + 1] = t1;
-        partial[4 * blockIdx.x + 2] = t2;
-        partial[4 * blockIdx.x + 3] = t3;
-    }
+    pdl_wait_and_trigger();
+    ErrSums q;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x)
+        q.add(k, ph, i, e[i], ewt[i]);
+    q.store(partial + 4 * blockIdx.x);
     last_block_reduce(partial, 4, counter, out);
 }
 
@@ -165,35 +197,9 @@ __global__ void k_newton_update_seg(const int* __restrict__ mp, const double* __
 __global__ void k_err_norms_seg(const int* __restrict__ mp, int k, PhiPtrs ph, const double* __restrict__ e,
                                 const double* __restrict__ ewt, double* out) {
     const int m = blockIdx.x;
-    double s0 = 0, s1 = 0, s2 = 0, s3 = 0;
-    for (int i = mp[m] + threadIdx.x; i < mp[m + 1]; i += blockDim.x) {
-        double w = ewt[i], ei = e[i];
-        double a = ei * w;
-        s0 += a * a;
-        double d1 = ph.p[k][i] + ei;
-        double b = d1 * w;
-        s1 += b * b;
-        if (k >= 2) {
-            double d2 = ph.p[k - 1][i] + d1;
-            double c2 = d2 * w;
-            s2 += c2 * c2;
-        }
-        if (k + 1 < kNPhi) {
-            double d3 = ei - ph.p[k + 1][i];
-            double c3 = d3 * w;
-            s3 += c3 * c3;
-        }
-    }
-    double t0 = block_sum(s0);
-    double t1 = block_sum(s1);
-    double t2 = block_sum(s2);
-    double t3 = block_sum(s3);
-    if (threadIdx.x == 0) {
-        out[4 * m + 0] = t0;
-        out[4 * m + 1] = t1;
-        out[4 * m + 2] = t2;
-        out[4 * m + 3] = t3;
-    }
+    ErrSums q;
+    for (int i = mp[m] + threadIdx.x; i < mp[m + 1]; i += blockDim.x) q.add(k, ph, i, e[i], ewt[i]);
+    q.store(out + 4 * m);
 }
 
 __global__ void k_sumsq_seg(const int* __restrict__ mp, const double* __restrict__ x,
@@ -210,16 +216,18 @@ __global__ void k_sumsq_seg(const int* __restrict__ mp, const double* __restrict
 
 // phi_{k+1} = e (set_kp2), phi_k += e, phi_j += phi_{j+1} for j = k-1..0
 __global__ void k_phi_update(int N, int k, int set_kp2, PhiPtrs ph, const double* __restrict__ e) {
+    pdl_wait_and_trigger();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= N) return;
-    double ei = e[i];
-    if (set_kp2) ph.p[k + 1][i] = ei;
-    double v = ph.p[k][i] + ei;
-    ph.p[k][i] = v;
-    for (int j = k - 1; j >= 0; --j) {
-        v = ph.p[j][i] + v;
-        ph.p[j][i] = v;
-    }
+    double p[kNPhi], v = e[i];
+    load_phi(ph, i, 0, k, p);
+    if (set_kp2) ph.p[k + 1][i] = v;
+#pragma unroll
+    for (int j = kNPhi - 1; j >= 0; --j)
+        if (j <= k) {
+            v = p[j] + v;
+            ph.p[j][i] = v;
+        }
 }
 
 // y'0 = F / ahh on free rows with ahh != 0, else 0
@@ -272,11 +280,12 @@ static IntegWork& integ_work(fvm_ctx* c) {
     const int N = c->N;
     for (int j = 0; j < kNPhi; ++j) w.phi[j].alloc(N);
     w.y.alloc(N); w.yp.alloc(N); w.e.alloc(N); w.ewt.alloc(N); w.F.alloc(N); w.x.alloc(N); w.tmp.alloc(N);
-    w.partial.alloc((size_t)kRedBlocks * 4);
+    w.partial.alloc((size_t)kRedBlocks * 5);
     // reduction results: Newton norms [0, nm), error norms [nm, 5 nm), the
     // predictor's norm at 5 nm (fetched together, one host wait)
     const size_t nh = (size_t)(5 * std::max(1, c->n_members) + 8);
     w.res.alloc(nh);
+    w.res.zero(c->stream);   // (no Newton update's mark)
     w.counter.alloc(1);
     if (w.host_n < nh) {
         if (w.host) FVM_CUDA(cudaFreeHost(w.host));
@@ -367,20 +376,19 @@ struct DeviceOps {
     // ---- controller interface
     void set_time(double t) { tcur = t; }
     void ewt_from_phi0(double rtol, double atol) {
-        fvm_launch(c, k_ewt, g(), 256, 0, c->stream, N, phi[0].p, rtol, atol, ewt.p);
+        fvm_launch_pdl(c, k_ewt, g(), 256, 0, c->stream, N, phi[0].p, rtol, atol, ewt.p);
     }
     void begin_step() { launch_begin_step(c, phi[0].p, yp.p); }
     void phi_scale(int j0, int j1, const double* f) {
         Coef7 cf;
         for (int j = 0; j < kNPhi; ++j) cf.v[j] = f[j];
-        fvm_launch(c, k_phi_scale, g(), 256, 0, c->stream, N, j0, j1, ptrs(), cf);
+        fvm_launch_pdl(c, k_phi_scale, g(), 256, 0, c->stream, N, j0, j1, ptrs(), cf);
     }
     void predict(int k, const double* gamma, double h) {
         Coef7 gm;
         for (int j = 0; j < kNPhi; ++j) gm.v[j] = gamma[j];
-        fvm_launch(c, k_predict, g(), 256, 0, c->stream, N, k, ptrs(), gm, y.p, yp.p, e.p);
-        fvm_launch(c, k_pred_sumsq, kRedBlocks, kRedThreads, 0, c->stream, N, y.p, ewt.p, partial.p, counter.p,
-                   res.p + pn_slot());
+        fvm_launch_pdl(c, k_predict, kRedBlocks, kRedThreads, 0, c->stream, N, k, ptrs(), gm, y.p, yp.p, e.p, ewt.p,
+                       partial.p, counter.p, res.p + pn_slot());
         err_ready = false;
         f_fresh = false;
         hcur = h;
@@ -391,6 +399,8 @@ struct DeviceOps {
             predictor_features(c, phi[0].p, hprev.p, ypred.p, h, feat.p);
         }
     }
+    double newton_mark = 0.0;   // numbers the Newton updates queued behind solves
+    bool newton_done = false;   // the one behind the last solve was done and fetched
     // the predictor's WRMS norm, as fetched by the attempt's first
     // newton_update (the only place the controller reads it)
     double pred_norm() const { return pn; }
@@ -452,13 +462,26 @@ struct DeviceOps {
     }
     int gmres(double cj, double tol, int* its, double* rn, long* nps, long* njv) {
         GmresCounters gc;
-        // the Newton update reads x next on the same stream: no wait here
+        // the Newton update is queued behind the solve's first cycle, so that
+        // one wait brings the solve's state and the update's norms
+        GmresTail tail;
+        newton_mark += 1.0;
+        tail.queue = [&](const int* done) {
+            launch_newton(cj, done, ilu_status_dev(c));
+            FVM_CUDA(cudaMemcpyAsync(host, res.p, sizeof(double) * (pn_slot() + 2), cudaMemcpyDeviceToHost, c->stream));
+        };
+        host[6] = 0.0;
         int r = gmres_dev(c, cj, y.p, yp.p, F.p, ewt.p, F.p, x.p, o.krylov_dim, o.max_restarts,
-                          o.precision, tol * tol_scale, its, rn, &gc, o.krylov_operator, false);
+                          o.precision, tol * tol_scale, its, rn, &gc, o.krylov_operator, false, nm > 1 ? nullptr : &tail);
+        newton_done = nm == 1 && r == 0 && host[6] == newton_mark;
         *nps = gc.nps;
         *njv = gc.njv;
         if (ilu_status_seen(c)) return 3;   // zero pivot in the factor this solve used
         return r;
+    }
+    void launch_newton(double cj, const int* go, const int* status) {
+        fvm_launch_pdl(c, k_newton_update, kRedBlocks, kRedThreads, 0, c->stream, N, x.p, cj, ewt.p, y.p, yp.p, e.p,
+                       korder, ptrs(), partial.p, counter.p, res.p, go, status, newton_mark);
     }
     double newton_update(double cj) {
         const size_t ps = pn_slot();
@@ -473,11 +496,12 @@ struct DeviceOps {
             pn = std::sqrt(host[ps] / N);
             return member_max(1, 0);
         }
-        fvm_launch(c, k_newton_update, kRedBlocks, kRedThreads, 0, c->stream, N, x.p, cj, ewt.p, y.p, yp.p, e.p,
-                                                                   partial.p, counter.p, res.p);
-        fvm_launch(c, k_err_norms, kRedBlocks, kRedThreads, 0, c->stream, N, korder, ptrs(), e.p, ewt.p, partial.p,
-                                                               counter.p, res.p + 1);
-        const double d = fetch((int)ps + 1);
+        if (!newton_done) {
+            launch_newton(cj, nullptr, nullptr);
+            fetch((int)ps + 1);
+        }
+        newton_done = false;
+        const double d = host[0];
         for (int q = 0; q < 4; ++q) err_cache[q] = std::sqrt(host[1 + q] / N);
         err_ready = true;
         pn = std::sqrt(host[ps] / N);
@@ -494,7 +518,7 @@ struct DeviceOps {
             for (int q = 0; q < 4; ++q) out[q] = member_max(4, q);
             return;
         }
-        fvm_launch(c, k_err_norms, kRedBlocks, kRedThreads, 0, c->stream, N, k, ptrs(), e.p, ewt.p, partial.p,
+        fvm_launch_pdl(c, k_err_norms, kRedBlocks, kRedThreads, 0, c->stream, N, k, ptrs(), e.p, ewt.p, partial.p,
                                                                counter.p, res.p);
         fetch(4);
         for (int q = 0; q < 4; ++q) out[q] = std::sqrt(host[q] / N);
@@ -513,7 +537,7 @@ struct DeviceOps {
             if (rec) recorder_push(c, rec, feat.p, y.p, ypred.p, phi[0].p, o.rtol, o.atol);
             FVM_CUDA(cudaMemcpyAsync(hprev.p, phi[0].p, sizeof(double) * N, cudaMemcpyDeviceToDevice, c->stream));
         }
-        fvm_launch(c, k_phi_update, g(), 256, 0, c->stream, N, k, set_kp2, ptrs(), e.p);
+        fvm_launch_pdl(c, k_phi_update, g(), 256, 0, c->stream, N, k, set_kp2, ptrs(), e.p);
     }
     // The learned iterate costs a network evaluation and one or two residual
     // evaluations per attempt.  After a run of attempts that the residual
@@ -551,7 +575,7 @@ struct DeviceOps {
         fvm_launch(c, k_fill, g(), 256, 0, s, N, 1.0, tmp.p);
         launch_residual(c, y.p, tmp.p, none, nullptr, x.p);   // leaves ahh * 1 in c->stor
         fvm_launch(c, k_initial_yp, g(), 256, 0, s, N, F.p, c->stor.p, c->ntype.p, yp.p);
-        fvm_launch(c, k_ewt, g(), 256, 0, s, N, y.p, o.rtol, o.atol, ewt.p);
+        fvm_launch_pdl(c, k_ewt, g(), 256, 0, s, N, y.p, o.rtol, o.atol, ewt.p);
         double ypn;
         if (nm > 1) {
             fvm_launch(c, k_sumsq_seg, nm, 256, 0, s, c->member_ptr.p, yp.p, ewt.p, res.p);

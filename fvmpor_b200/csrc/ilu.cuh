@@ -69,7 +69,8 @@ struct BlockILU {
     DevBuf<unsigned short> op_lcol;   // 16-bit columns into each block's node list
     DevBuf<int> halo_ptr, halo_node;           // each block's node list: its rows in factor order, its halo
     DevBuf<int> nbr_ptr, nbr;                  // blocks whose rows a block's operator reads
-    DevBuf<unsigned> flags;                    // per block: last step published
+    DevBuf<unsigned> flags;                    // per block: last step published; the barrier counter
+    unsigned fused_launches = 0;               // since the flags were zero
     DevBuf<float> op_val, op_dg;
     size_t fused_smem = 0, fused_smem_d = 0, fused_stage = 0;   // _d without the Hessenberg matrix
     size_t fused_room[2] = {0, 0};           // dynamic shared bytes each variant may have

@@ -3,6 +3,8 @@
 // integrator.
 #pragma once
 
+#include <functional>
+
 #include "ctx.cuh"
 
 namespace fvmb {
@@ -38,7 +40,6 @@ struct Krylov {
     DevBuf<float> tdir;       // FP32 direction of the fused cycle (arnoldi_fused.cu)
     DevBuf<double> ls;        // H [(m+1) x m], cs [m], sn [m], g [m+1]
     double* host = nullptr;   // pinned
-    double* host_ls = nullptr;   // pinned: H and g of a fused cycle
     // CUDA graph of one full batch (8 steps) of the device-driven Arnoldi
     // loop (fvm_opts.graph): captured for one key (operator, precision,
     // vectors, preconditioner state), replayed for every full batch; cj and
@@ -63,18 +64,29 @@ void fvmb_destroy_krylov_impl(Krylov* K);
 double reduce_sumsq(fvm_ctx* c, const double* x, const double* w);
 double reduce_dot(fvm_ctx* c, const double* x, const double* y);
 
+// What a caller does with a solution x when the solve converges, queued behind the
+// first fused cycle so that the host waits once for both: queue(done) launches
+// kernels that do nothing unless *done == 1 (a converged cycle)
+struct GmresTail {
+    std::function<void(const int* done)> queue;
+};
+
 // op 0: J v by the residual's difference quotient; 1: by the assembled
 // Jacobian of the last set-up (jacobian_apply).  sync_end false: a converged
 // solve returns with the update of x still queued on the context's stream
 int gmres_dev(fvm_ctx* c, double cj, const double* y, const double* yp, const double* F0,
               const double* ewt, const double* b, double* x, int m, int max_restarts,
               int precision, double tol, int* iters, double* res_norm, GmresCounters* cnt, int op = 0,
-              bool sync_end = true);
+              bool sync_end = true, const GmresTail* tail = nullptr);
 
 // preconditioner (precond.cu)
 void psetup_dev(fvm_ctx* c, double cj, double h, const double* y, const double* yp,
                 const double* F0, const double* ewt, int precision);
 void psolve_dev(fvm_ctx* c, const double* r, double* z, const int* skip = nullptr);
+// z = P^-1 of the residual rows gathered from the element pass's partials, where
+// psolve_gathers()
+bool psolve_gathers(fvm_ctx* c);
+void psolve_gather_dev(fvm_ctx* c, const GatherSrc& g, double* z, const int* skip);
 // y = J(cj) x with the assembled difference-quotient Jacobian of the last
 // set-up (the Krylov operator of fvm_opts.krylov_operator = 1)
 void jacobian_apply(fvm_ctx* c, double cj, const double* x, double* y, const int* skip = nullptr,
@@ -89,9 +101,10 @@ bool schur_active(fvm_ctx* c);          // the Schur-coupled apply is on
 // cycle can run (FP32 factor staged in shared memory, every block resident);
 // fused_cycle runs one cycle from the state gmres has put in place
 bool fused_prepare(fvm_ctx* c, int m);
-void fused_cycle(fvm_ctx* c, Krylov* K, double cj, const double* ewt, double* H_d, double* cs_d, double* sn_d,
-                 double* g_d);
+void fused_reset(fvm_ctx* c);   // after a failed cycle
+void fused_cycle(fvm_ctx* c, Krylov* K, double cj, double tol, const double* ewt, double* H_d, double* coef);
 bool ilu_ready(fvm_ctx* c);
+const int* ilu_status_dev(fvm_ctx* c);   // the status word on the device
 int ilu_status(fvm_ctx* c);   // 0 ok, 1 zero pivot in the last factorisation
 // the same status as the last host wait saw it (no wait of its own: valid
 // once any ctx_sync has followed the set-up)

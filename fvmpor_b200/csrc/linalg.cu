@@ -324,10 +324,31 @@ __global__ void k_combine(int N, int nv, const B* __restrict__ U, size_t ld,
 }
 
 // r~ = ewt * (b - Jx) (Jx may be null -> b); U_0 = r~; out = ||r~||^2
+// the same with what a fused cycle left: its number of columns (none after a
+// failure or breakdown) and their coefficients; set instead of added to first
+template <class B>
+__global__ void k_combine_dev(int N, const ArnState* __restrict__ st, const B* __restrict__ U, size_t ld,
+                              const double* __restrict__ ys, const double* __restrict__ ewt, double* __restrict__ x,
+                              int first) {
+    pdl_wait_and_trigger();
+    __shared__ double coef[64];
+    const int done = st->done, nv = done == 1 || done == 2 ? st->j : 0;
+    for (int i = threadIdx.x; i < nv; i += blockDim.x) coef[i] = ys[i];
+    __syncthreads();
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= N) return;
+    double acc = 0.0;
+#pragma unroll 8
+    for (int i = 0; i < nv; ++i) acc += coef[i] * ldb(U + ld * i, k);
+    acc /= ewt[k];
+    x[k] = first ? acc : x[k] + acc;
+}
+
 template <class B>
 __global__ void k_init_residual(int N, const double* __restrict__ b, const double* __restrict__ Jx,
                                 const double* __restrict__ ewt, B* __restrict__ U0, double* partial,
                                 unsigned* counter, double* out) {
+    pdl_wait_and_trigger();
     double s = 0.0;
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < N; k += gridDim.x * blockDim.x) {
         double r = Jx ? b[k] - Jx[k] : b[k];
@@ -413,7 +434,6 @@ Krylov* krylov_get(fvm_ctx* c, int m, int precision) {
     // results of the three passes, the m+1 basis scales, a status word and
     // the device-driven Arnoldi state
     FVM_CUDA(cudaMallocHost(&K->host, sizeof(double) * (4 * (m + 2) + 8) + sizeof(ArnState)));
-    FVM_CUDA(cudaMallocHost(&K->host_ls, sizeof(double) * ((size_t)(m + 1) * m + m + 1)));
     c->kry[precision] = K;
     return c->kry_last = K;
 }
@@ -424,7 +444,6 @@ void fvmb_destroy_krylov_impl(Krylov* K) {
     if (K->graph) cudaGraphDestroy(K->graph);
     if (K->U) cudaFree(K->U);
     if (K->host) cudaFreeHost(K->host);
-    if (K->host_ls) cudaFreeHost(K->host_ls);
     delete K;
 }
 
@@ -471,14 +490,20 @@ template <class B>
 static int gmres_impl(fvm_ctx* c, Krylov* K, double cj, const double* y, const double* yp,
                       const double* F0, const double* ewt, const double* b, double* x, int m,
                       int max_restarts, double tol, int* iters, double* res_norm,
-                      GmresCounters* cnt, int op, bool sync_end) {
+                      GmresCounters* cnt, int op, bool sync_end, const GmresTail* tail) {
     cudaStream_t s = c->stream;
     const int N = c->N;
     B* U = reinterpret_cast<B*>(K->U);
     const size_t ld = K->ld;
     const double sqrtN = std::sqrt((double)N);
     std::vector<double> H((size_t)(m + 1) * m), cs(m), sn(m), g(m + 1), hcol(m + 2);
-    FVM_CUDA(cudaMemsetAsync(x, 0, sizeof(double) * N, s));
+    // the assembled operator with the FP32 factor and basis: the whole cycle in
+    // one persistent launch (arnoldi_fused.cu), which also takes the initial
+    // norm from K->res, sets the first scale and direction, decides there
+    // whether any step is needed and forms the solution's coefficients, so the
+    // host waits once per cycle, for the state alone
+    const bool fused = op && sizeof(B) == sizeof(float) && K->coop_grid > 0 && fused_prepare(c, m);
+    if (!fused) FVM_CUDA(cudaMemsetAsync(x, 0, sizeof(double) * N, s));
     int total = 0;
     double rnorm = 0.0;
     bool have_x = false;
@@ -494,14 +519,8 @@ static int gmres_impl(fvm_ctx* c, Krylov* K, double cj, const double* y, const d
             psolve_dev(c, b, K->z.p);
         }
         if (cnt) cnt->nps++;
-        fvm_launch(c, k_init_residual<B>, kRedBlocks, kRedThreads, 0, s, N, K->z.p, nullptr, ewt, U,
+        fvm_launch_pdl(c, k_init_residual<B>, kRedBlocks, kRedThreads, 0, s, N, K->z.p, nullptr, ewt, U,
                                                               K->partial.p, K->counter.p, K->res.p);
-        // the assembled operator with the FP32 factor and basis: the whole
-        // cycle in one persistent launch (arnoldi_fused.cu), which also takes
-        // the initial norm from K->res, sets the first scale and direction
-        // and decides there whether any step is needed, so the host waits
-        // once per cycle
-        const bool fused = op && sizeof(B) == sizeof(float) && K->coop_grid > 0 && fused_prepare(c, m);
         if (!fused) fvm_launch(c, k_set_scale, 1, 1, 0, s, K->res.p, K->scale.p, 0);
         std::fill(g.begin(), g.end(), 0.0);
         if (!fused) {
@@ -517,41 +536,32 @@ static int gmres_impl(fvm_ctx* c, Krylov* K, double cj, const double* y, const d
         bool conv = false;
         if (fused) {
             ArnState* hst = reinterpret_cast<ArnState*>(K->host + 4 * (m + 2) + 8);
-            *hst = ArnState{0, 0, m, 0, tol, sqrtN, 0.0};
-            FVM_CUDA(cudaMemcpyAsync(K->st.p, hst, sizeof(ArnState), cudaMemcpyHostToDevice, s));
-            double* H_d = K->ls.p;
-            double* cs_d = H_d + (size_t)(m + 1) * m;
-            double* sn_d = cs_d + m;
-            double* g_d = sn_d + m;
-            fused_cycle(c, K, cj, ewt, H_d, cs_d, sn_d, g_d);
-            // state, status, least-squares data and scales in one wait
-            int* herr = reinterpret_cast<int*>(K->host + 4 * (m + 2) + 7);
-            double* hls = K->host_ls;
+            double* coef = K->res.p + 1;   // (m + 2) values follow the squared norm
+            fused_cycle(c, K, cj, tol, ewt, K->ls.p, coef);
+            fvm_launch_pdl(c, k_combine_dev<B>, grid_for(N, 256), 256, 0, s, N, K->st.p, U, ld, coef, ewt, x,
+                           have_x ? 0 : 1);
+            have_x = true;
+            if (tail && cycle == 0) tail->queue(&K->st.p->done);
             FVM_CUDA(cudaMemcpyAsync(hst, K->st.p, sizeof(ArnState), cudaMemcpyDeviceToHost, s));
-            FVM_CUDA(cudaMemcpyAsync(herr, K->err.p, sizeof(int), cudaMemcpyDeviceToHost, s));
-            FVM_CUDA(cudaMemcpyAsync(hls, H_d, sizeof(double) * ((size_t)(m + 1) * m), cudaMemcpyDeviceToHost, s));
-            FVM_CUDA(cudaMemcpyAsync(hls + (size_t)(m + 1) * m, g_d, sizeof(double) * (m + 1), cudaMemcpyDeviceToHost,
-                                     s));
-            FVM_CUDA(cudaMemcpyAsync(K->host + 3 * (m + 2), K->scale.p, sizeof(double) * (m + 1),
-                                     cudaMemcpyDeviceToHost, s));
             ctx_sync(c);
-            if (*herr != 0) {
+            j = hst->j;
+            total += j;
+            rnorm = hst->rnorm;
+            if (hst->done == 0) {
                 // a grid barrier, a flag wait or the factor copy gave up
                 K->err.zero(s);
                 K->bar.zero(s);
-                *iters = total + hst->j;
-                *res_norm = hst->rnorm;
-                return 2;
+                fused_reset(c);
+            } else if (cnt) {
+                cnt->njv += j;
+                cnt->nps += j;
             }
-            j = hst->j;
-            total += j;
-            if (cnt) { cnt->njv += j; cnt->nps += j; }
-            rnorm = hst->rnorm;
-            if (hst->done == 3) { *iters = total; *res_norm = rnorm; return 2; }
-            if (j == 0) { *iters = total; *res_norm = rnorm; return 0; }   // already within tol
-            conv = hst->done == 1;
-            std::copy(hls, hls + (size_t)(m + 1) * m, H.begin());
-            std::copy(hls + (size_t)(m + 1) * m, hls + (size_t)(m + 1) * m + m + 1, g.begin());
+            if (hst->done != 2) {   // converged (x is complete), failed or broken down
+                *iters = total;
+                *res_norm = rnorm;
+                return hst->done == 1 ? 0 : 2;
+            }
+            continue;
         } else if (K->coop_grid > 0) {
             // Device-driven Arnoldi: each step is J*v, the preconditioner,
             // the fused CGS2 and the Givens update, all reading the step
@@ -597,8 +607,12 @@ static int gmres_impl(fvm_ctx* c, Krylov* K, double cj, const double* y, const d
                     pt.sigma_dev = K->sigma.p;
                     pt.skip = skip;
                     if (op) jacobian_apply(c, cj, K->t.p, K->Jv.p, skip, dev_cj ? K->cjd.p + 1 : nullptr);
-                    else launch_residual(c, y, yp, pt, F0, K->Jv.p);
-                    psolve_dev(c, K->Jv.p, K->z.p, skip);
+                    if (!op && psolve_gathers(c)) {
+                        psolve_gather_dev(c, launch_residual_partials(c, y, yp, pt, F0), K->z.p, skip);
+                    } else {
+                        if (!op) launch_residual(c, y, yp, pt, F0, K->Jv.p);
+                        psolve_dev(c, K->Jv.p, K->z.p, skip);
+                    }
                     c->tm.begin(TM_CGS, s);
                     int Ni = N;
                     ArnState* stp = K->st.p;
@@ -799,14 +813,15 @@ static int gmres_impl(fvm_ctx* c, Krylov* K, double cj, const double* y, const d
 
 int gmres_dev(fvm_ctx* c, double cj, const double* y, const double* yp, const double* F0,
               const double* ewt, const double* b, double* x, int m, int max_restarts,
-              int precision, double tol, int* iters, double* res_norm, GmresCounters* cnt, int op, bool sync_end) {
+              int precision, double tol, int* iters, double* res_norm, GmresCounters* cnt, int op, bool sync_end,
+              const GmresTail* tail) {
     if (m < 1 || m > 60) throw Error("gmres: krylov dimension must be in [1, 60]");
     Krylov* K = krylov_get(c, m, precision);
     const int r = precision
                       ? gmres_impl<float>(c, K, cj, y, yp, F0, ewt, b, x, m, max_restarts, tol, iters, res_norm, cnt, op,
-                                          sync_end)
+                                          sync_end, tail)
                       : gmres_impl<double>(c, K, cj, y, yp, F0, ewt, b, x, m, max_restarts, tol, iters, res_norm, cnt, op,
-                                           sync_end);
+                                           sync_end, tail);
     // a timed-out barrier of the Schur-coupled apply voids the solve
     if (schur_status(c)) return 2;
     return r;

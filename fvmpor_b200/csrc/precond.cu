@@ -74,6 +74,7 @@ __global__ void k_fd_node(int N, const double* __restrict__ y, const double* __r
                           const ZoneDev* __restrict__ zones, int nz, const int* __restrict__ nz_ptr,
                           const int* __restrict__ nz_zone, const double* __restrict__ nz_w, double rho0,
                           const unsigned char* __restrict__ ntype, const double* __restrict__ hD, FdNode o) {
+    pdl_wait_and_trigger();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= N) return;
     const double h = y[i], ypi = yp[i];
@@ -224,6 +225,7 @@ __global__ void __launch_bounds__(kFdThreads, 4) k_fd_chunk(FdArgs a) {
     double* sums = sh;
     double2* srow = reinterpret_cast<double2*>(smem_raw + L.rows);
     uint64_t* bar = reinterpret_cast<uint64_t*>(smem_raw + L.bar);
+    pdl_wait_and_trigger();
     const int2 la = a.list_at[blockIdx.x];
     const int ng = la.y;
     const unsigned short* goff = reinterpret_cast<const unsigned short*>(smem_raw + L.list);
@@ -399,6 +401,7 @@ __global__ void __launch_bounds__(kFdThreads, 4) k_fd_chunk(FdArgs a) {
 template <class S>
 __global__ void k_fd_shared(int n, const int4* __restrict__ at, const int* __restrict__ sptr,
                             const double* __restrict__ part, FdOut out) {
+    pdl_wait_and_trigger();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= n) return;
     const int4 w = at[t];
@@ -491,14 +494,22 @@ __global__ void __launch_bounds__(128) k_ilu_apply(const int* __restrict__ bstar
     for (int i = threadIdx.x; i < nr; i += blockDim.x) z[lu_row[r0 + i]] = (double)x[i];
 }
 
-template <class T>
+// the right-hand side of an apply: a vector, or the rows of a residual whose
+// partials the element pass has left (gather_row)
+struct RhsVector {
+    const double* r;
+};
+__device__ __forceinline__ double rhs_row(const RhsVector& v, int i) { return v.r[i]; }
+__device__ __forceinline__ double rhs_row(const GatherSrc& g, int i) { return gather_row(g, i); }
+
+template <class T, class Rhs>
 __global__ void __launch_bounds__(kIluThreads, 1) k_ilu_apply_smem(const int* __restrict__ bstart,
                                                         const IluBlk* __restrict__ blk,
                                                         const unsigned short* __restrict__ lu_col,
                                                         const unsigned short* __restrict__ meta,
                                                         const T* __restrict__ lu,
                                                         const int* __restrict__ lu_row,
-                                                        const double* __restrict__ r,
+                                                        const Rhs rhs,
                                                         double* __restrict__ z, int* __restrict__ err,
                                                         const int* __restrict__ skip) {
     unsigned char* const smem_raw = ilu_smem();
@@ -523,7 +534,8 @@ __global__ void __launch_bounds__(kIluThreads, 1) k_ilu_apply_smem(const int* __
         tc05::mbar_wait(S.bar, 0);
         return;
     }
-    for (int i = threadIdx.x; i < nr; i += blockDim.x) x[i] = (T)r[lu_row[r0 + i]];
+#pragma unroll 2
+    for (int i = threadIdx.x; i < nr; i += blockDim.x) x[i] = (T)rhs_row(rhs, lu_row[r0 + i]);
     if (threadIdx.x == 0) x[nr] = (T)0;
     bool ok = tc05::mbar_wait(S.bar, 0);
     if (!ok) ok = tc05::mbar_wait(S.bar, 0);   // copies in flight get a second bounded chance
@@ -731,6 +743,7 @@ __global__ void __launch_bounds__(kIluFactorThreads, 1) k_ilu_factor_smem(const 
         asm volatile("fence.mbarrier_init.release.cluster;");
     }
     __syncthreads();
+    pdl_wait_and_trigger();
     ilu_stage_bulk(S, B, nr, Jw, lu_col, meta);
     const int la = B.seg, nl = B.nl;
     // Each level's schedule segment is in shared memory when its rows run
@@ -1386,11 +1399,13 @@ static void build_pattern(fvm_ctx* c, BlockILU* P) {
             raise_smem_limit(k_ilu_apply<float>, sizeof(float) * ((size_t)maxb + 1));
         }
         if (P->smem_stage[0]) {
-            raise_smem_limit(k_ilu_apply_smem<double>, (size_t)P->smem_stage[0]);
+            raise_smem_limit(k_ilu_apply_smem<double, RhsVector>, P->smem_stage[0]);
+            raise_smem_limit(k_ilu_apply_smem<double, GatherSrc>, P->smem_stage[0]);
             raise_smem_limit(k_ilu_factor_smem<double>, (size_t)(round16(P->smem_stage[0]) + 8 * (size_t)P->scr_words[0]));
         }
         if (P->smem_stage[1]) {
-            raise_smem_limit(k_ilu_apply_smem<float>, (size_t)P->smem_stage[1]);
+            raise_smem_limit(k_ilu_apply_smem<float, RhsVector>, P->smem_stage[1]);
+            raise_smem_limit(k_ilu_apply_smem<float, GatherSrc>, P->smem_stage[1]);
             raise_smem_limit(k_ilu_factor_smem<float>, (size_t)(round16(P->smem_stage[1]) + 8 * (size_t)P->scr_words[1]));
         }
     }
@@ -1520,10 +1535,11 @@ void psetup_dev(fvm_ctx* c, double cj, double h, const double* y, const double* 
     cudaStream_t s = c->stream;
     const int N = c->N;
     c->tm.begin(TM_FD_JAC, s);
+    FVM_CUDA(cudaMemsetAsync(P->status.p, 0, sizeof(int), s));
     (void)F0;   // the element-wise quotients difference each element's own partials
     // the fused cycle's operator values too, once its layout exists
     const bool op = P->op_built && P->fused_ok;
-    fvm_launch(c, k_fd_node, grid_for(N, 256), 256, 0, s, N, y, yp, ewt, h, std::sqrt(DBL_EPSILON), cj, c->zones.p,
+    fvm_launch_pdl(c, k_fd_node, grid_for(N, 256), 256, 0, s, N, y, yp, ewt, h, std::sqrt(DBL_EPSILON), cj, c->zones.p,
                c->nz, c->nz_ptr.p, c->nz_zone.p, c->nz_w.p, c->rho0, c->ntype.p, c->hD.p,
                FdNode{P->fd_g.p, P->fd_dg.p, P->fd_gq.p, P->fd_diag.p, P->ahhp.p, op ? P->op_dg.p : nullptr,
                       P->lu_pos.p});
@@ -1553,7 +1569,7 @@ void psetup_dev(fvm_ctx* c, double cj, double h, const double* y, const double* 
             using S = decltype(one);
             auto go = [&](auto kern, size_t sm) {
                 if (sm > 48 * 1024) raise_smem_limit(kern, sm);
-                fvm_launch(c, kern, (c->T + kFdChunk - 1) / kFdChunk, kFdThreads, sm, s, a);
+                fvm_launch_pdl(c, kern, (c->T + kFdChunk - 1) / kFdChunk, kFdThreads, sm, s, a);
             };
 #define FVM_FD(NPE, NFE, RC, MZ) \
     go(k_fd_chunk<NPE, NFE, RC, MZ, S>, FdSmem(NPE, RC, MZ, sizeof(S), a.nnmax, a.list_max, a.grp_max).bytes)
@@ -1564,14 +1580,13 @@ void psetup_dev(fvm_ctx* c, double cj, double h, const double* y, const double* 
 #undef FVM_FD
             const int ns = (int)P->fd_shared.n;
             if (ns)
-                fvm_launch(c, k_fd_shared<S>, grid_for(ns, 256), 256, 0, s, ns, P->fd_shared.p, P->fd_sptr.p,
+                fvm_launch_pdl(c, k_fd_shared<S>, grid_for(ns, 256), 256, 0, s, ns, P->fd_shared.p, P->fd_sptr.p,
                            P->fd_part.p, a.out);
         };
         if (precision) run(0.f);
         else run(0.0);
     }
     c->tm.end(TM_FD_JAC, s);
-    FVM_CUDA(cudaMemsetAsync(P->status.p, 0, sizeof(int), s));
     c->tm.begin(TM_ILU_FACTOR, s);
     auto factor = [&](auto& lu, auto* Jw) {
         using T = std::remove_pointer_t<decltype(Jw)>;
@@ -1579,7 +1594,7 @@ void psetup_dev(fvm_ctx* c, double cj, double h, const double* y, const double* 
         if (P->smem_stage[precision]) {
             const int so = (int)round16(P->smem_stage[precision]);
             const int sw = P->scr_words[precision];
-            fvm_launch(c, k_ilu_factor_smem<T>, P->nb, kIluFactorThreads, (size_t)so + 8 * (size_t)sw, s, P->bstart.p,
+            fvm_launch_pdl(c, k_ilu_factor_smem<T>, P->nb, kIluFactorThreads, (size_t)so + 8 * (size_t)sw, s, P->bstart.p,
                        P->blk.p, P->meta.p, (const T*)Jw, P->lu_col.p, P->seg_ptr.p, P->upd.p, so, sw, lu.p,
                        P->status.p);
         } else {
@@ -1612,6 +1627,8 @@ int ilu_status(fvm_ctx* c) {
 }
 
 int ilu_status_seen(fvm_ctx* c) { return c->ilu && c->ilu->h_status ? *c->ilu->h_status : 0; }
+
+const int* ilu_status_dev(fvm_ctx* c) { return c->ilu ? c->ilu->status.p : nullptr; }
 
 bool ilu_ready(fvm_ctx* c) { return c->ilu && c->ilu->factored >= 0; }
 
@@ -1646,13 +1663,35 @@ void psolve_dev(fvm_ctx* c, const double* r, double* z, const int* skip) {
     auto go = [&](auto staged, auto plain, const auto* lu) {
         if (sm)
             fvm_launch_pdl(c, staged, P->nb, P->apply_threads, sm, s, P->bstart.p, P->blk.p, P->lu_col.p, P->meta.p, lu,
-                           P->lu_row.p, r, z, P->status.p, skip);
+                           P->lu_row.p, RhsVector{r}, z, P->status.p, skip);
         else
             fvm_launch_pdl(c, plain, P->nb, 128, sizeof(*lu) * ((size_t)P->maxb + 1), s, P->bstart.p, P->blk.p,
                            P->lu_col.p, P->meta.p, lu, P->lu_row.p, r, z, skip);
     };
-    if (P->factored) go(k_ilu_apply_smem<float>, k_ilu_apply<float>, P->lu32.p);
-    else go(k_ilu_apply_smem<double>, k_ilu_apply<double>, P->lu64.p);
+    if (P->factored) go(k_ilu_apply_smem<float, RhsVector>, k_ilu_apply<float>, P->lu32.p);
+    else go(k_ilu_apply_smem<double, RhsVector>, k_ilu_apply<double>, P->lu64.p);
+}
+
+// The apply takes the residual's rows straight from the element pass's partials
+// where a block's threads have few rows each: z = P^-1 (gather), one launch and
+// one pass less per Jacobian-free Arnoldi step.  A block of many rows would wait
+// longer for its chains of dependent loads than the gather's own launch takes
+// with an eighth of a warp's rows per SM.
+constexpr int kGatherRows = 512;
+bool psolve_gathers(fvm_ctx* c) {
+    BlockILU* P = c->ilu;
+    return P && P->factored >= 0 && P->schur_iters < 0 && P->smem_stage[P->factored] && P->maxb <= kGatherRows;
+}
+void psolve_gather_dev(fvm_ctx* c, const GatherSrc& g, double* z, const int* skip) {
+    BlockILU* P = c->ilu;
+    c->tm.begin(TM_ILU_APPLY, c->stream);
+    auto go = [&](auto kern, const auto* lu) {
+        fvm_launch_pdl(c, kern, P->nb, P->apply_threads, P->smem_stage[P->factored], c->stream, P->bstart.p, P->blk.p,
+                       P->lu_col.p, P->meta.p, lu, P->lu_row.p, g, z, P->status.p, skip);
+    };
+    if (P->factored) go(k_ilu_apply_smem<float, GatherSrc>, P->lu32.p);
+    else go(k_ilu_apply_smem<double, GatherSrc>, P->lu64.p);
+    c->tm.end(TM_ILU_APPLY, c->stream);
 }
 
 } // namespace fvmb
