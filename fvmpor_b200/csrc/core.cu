@@ -180,9 +180,11 @@ struct StageLayout {
     }
 };
 
+// chunk c's copies: what the mesh and the step's start left, and what the node pass
+// left (its heads and krw), counted together on the stage's barrier
 template <int NPE, bool VAR1, bool MZ>
-__device__ __forceinline__ void elem_issue(const ElemArgs& a, const StageLayout& L, unsigned char* st,
-                                           int4* meta, uint64_t* bar, int c) {
+__device__ __forceinline__ void elem_issue_mesh(const ElemArgs& a, const StageLayout& L, unsigned char* st,
+                                                int4* meta, uint64_t* bar, int c) {
     const int2 sg = a.ch_seg[c];
     const int e0 = c * a.CE;
     const int ne = min(a.CE, a.T - e0);
@@ -192,8 +194,6 @@ __device__ __forceinline__ void elem_issue(const ElemArgs& a, const StageLayout&
                      (VAR1 ? (uint32_t)nep * 8 * (a.kiso ? 1 : 3) : 0) + (uint32_t)nep * NPE * 2 + (uint32_t)nnp * 2;
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(tc05::smem_u32(bar)), "r"(bytes)
                  : "memory");
-    if (MZ) tc05::bulk_g2s(st + L.h, a.ch_h + sg.x, nnp * 8, bar);
-    else tc05::bulk_g2s(st + L.h, a.ch_hk + 2 * (size_t)sg.x, nnp * 16, bar);
     if (VAR1)
         for (int d = 0; d < 3; ++d) tc05::bulk_g2s(st + L.xyz + (size_t)d * a.nnmax * 8, a.ch_xyz + d * a.P + sg.x, nnp * 8, bar);
     tc05::bulk_g2s(st + L.eloc, a.elocal + e0, nep * 8, bar);
@@ -206,6 +206,13 @@ __device__ __forceinline__ void elem_issue(const ElemArgs& a, const StageLayout&
     tc05::bulk_g2s(st + L.lc, a.ch_lc + (size_t)e0 * NPE, nep * NPE * 2, bar);
     tc05::bulk_g2s(st + L.lp, a.ch_lptr + sg.x, nnp * 2, bar);
 }
+template <bool MZ>
+__device__ __forceinline__ void elem_issue_nodes(const ElemArgs& a, const StageLayout& L, unsigned char* st,
+                                                 const int4& meta, uint64_t* bar) {
+    const int nnp = pad8(meta.y + 1);
+    if (MZ) tc05::bulk_g2s(st + L.h, a.ch_h + meta.x, nnp * 8, bar);
+    else tc05::bulk_g2s(st + L.h, a.ch_hk + 2 * (size_t)meta.x, nnp * 16, bar);
+}
 
 template <int NPE, int NFE, int VAR, bool MZ, int EPT>
 __global__ void __launch_bounds__(kElemThreads) k_elem_chunk(ElemArgs a) {
@@ -214,16 +221,23 @@ __global__ void __launch_bounds__(kElemThreads) k_elem_chunk(ElemArgs a) {
     double* cc = reinterpret_cast<double*>(smem_e + 2 * L.bytes);               // [NPE][CE]
     int4* meta = reinterpret_cast<int4*>(cc + (size_t)NPE * a.CE);                // [2]
     uint64_t* full = reinterpret_cast<uint64_t*>(meta + 2);                      // [2]
-    pdl_wait_and_trigger();
     if ((int)blockIdx.x >= a.nch) return;
-    if (a.skip && *a.skip) return;
+    // the first chunk's mesh data is on its way while the node pass still runs
+    // (the step's upwind flags were complete before that could start)
     if (threadIdx.x == 0) {
         tc05::mbar_init(&full[0], 1);
         tc05::mbar_init(&full[1], 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        elem_issue<NPE, VAR == 1, MZ>(a, L, smem_e, &meta[0], &full[0], blockIdx.x);
+        elem_issue_mesh<NPE, VAR == 1, MZ>(a, L, smem_e, &meta[0], &full[0], blockIdx.x);
     }
+    pdl_wait_and_trigger();
+    if (threadIdx.x == 0) elem_issue_nodes<MZ>(a, L, smem_e, meta[0], &full[0]);
     __syncthreads();
+    if (a.skip && *a.skip) {
+        // a step queued after the stop: let the copies land (bounded), leave
+        tc05::mbar_wait(&full[0], 0);
+        return;
+    }
     int i = 0;
     for (int c = blockIdx.x; c < a.nch; c += gridDim.x, ++i) {
         const int s = i & 1;
@@ -232,7 +246,8 @@ __global__ void __launch_bounds__(kElemThreads) k_elem_chunk(ElemArgs a) {
             // the other stage was released by the barrier that ended the
             // previous chunk; order those generic reads before the copies
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            elem_issue<NPE, VAR == 1, MZ>(a, L, smem_e + (s ^ 1) * L.bytes, &meta[s ^ 1], &full[s ^ 1], cn);
+            elem_issue_mesh<NPE, VAR == 1, MZ>(a, L, smem_e + (s ^ 1) * L.bytes, &meta[s ^ 1], &full[s ^ 1], cn);
+            elem_issue_nodes<MZ>(a, L, smem_e + (s ^ 1) * L.bytes, meta[s ^ 1], &full[s ^ 1]);
         }
         const bool ok = tc05::mbar_wait(&full[s], (uint32_t)((i >> 1) & 1));
         if (!__syncthreads_and(ok ? 1 : 0)) {
@@ -335,11 +350,22 @@ __global__ void __launch_bounds__(kElemThreads) k_elem_chunk(ElemArgs a) {
 // part_ptr[i+1]) in ascending chunk order; sum them in that order.
 // F0 != nullptr turns the result into (F - F0) * inv_sigma.
 __global__ void k_gather(int N, GatherSrc g, double* __restrict__ out, const int* __restrict__ skip) {
+    // the row's places, which the element pass does not write, before the wait
+    // for it: the rest is one load per chunk and the row's terms side by side
+    constexpr int kPre = 4;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x, r = min(i, N - 1);
+    const int p0 = g.part_ptr[r], p1 = g.part_ptr[r + 1];
+    int at[kPre];
+#pragma unroll
+    for (int k = 0; k < kPre; ++k) at[k] = p0 + k < p1 ? g.cpos[p0 + k] : 0;
     pdl_wait_and_trigger();
-    if (skip && *skip) return;
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= N) return;
-    out[i] = gather_row(g, i);
+    if (i >= N || (skip && *skip)) return;
+    double s = 0.0;
+#pragma unroll
+    for (int k = 0; k < kPre; ++k)
+        if (p0 + k < p1) s += g.part[at[k]];
+    for (int p = p0 + kPre; p < p1; ++p) s += g.part[g.cpos[p]];
+    out[i] = gather_finish(g, i, s);
 }
 
 // begin-step element pass: averaged-weight face fluxes in the global edge

@@ -139,20 +139,26 @@ struct GatherSrc {
 };
 
 #ifdef __CUDACC__
-__device__ __forceinline__ double gather_row(const GatherSrc& g, int i) {
+// row i from the sum s of its partials in ascending chunk order
+__device__ __forceinline__ double gather_finish(const GatherSrc& g, int i, double s) {
     double r;
     if (g.ntype[i]) {
         r = g.hD[i] - g.h[i];
     } else {
-        double s = 0.0;
-        const int p1 = g.part_ptr[i + 1];
-        for (int p = g.part_ptr[i]; p < p1; ++p) s += g.part[g.cpos[p]];
         r = s * g.invV[i];
         r = r + g.bterm[i];
         r = r - g.stor[i];
     }
     if (g.F0) r = (r - g.F0[i]) * (g.sigma_dev ? 1.0 / *g.sigma_dev : g.inv_sigma);
     return r;
+}
+__device__ __forceinline__ double gather_row(const GatherSrc& g, int i) {
+    double s = 0.0;
+    if (!g.ntype[i]) {
+        const int p1 = g.part_ptr[i + 1];
+        for (int p = g.part_ptr[i]; p < p1; ++p) s += g.part[g.cpos[p]];
+    }
+    return gather_finish(g, i, s);
 }
 #endif
 
