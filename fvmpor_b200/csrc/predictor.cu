@@ -44,6 +44,10 @@ constexpr int kW2s = kW1s + kMlpH * kMlpK0;   // 64 x 64
 constexpr int kW3s = kW2s + kMlpH * kMlpH;    // 64 x 64
 constexpr int kWsz = kW3s + kMlpH * kMlpH;    // 9216 halves = 18432 B
 
+// floats of a CTA's partial gradient: the parameters and the loss, 16-byte rows
+constexpr int kPartial = (kNTrain + 1 + 3) & ~3;
+static_assert(kOffW2 % 4 == 0 && kOffW3 % 4 == 0, "vector stores of the weights' gradients");
+
 constexpr uint32_t kIdescFwd = idesc_bf16_f32(128, 64, false, false);
 constexpr uint32_t kIdescBwd = idesc_bf16_f32(128, 64, false, true);
 
@@ -51,7 +55,7 @@ struct Predictor {
     DevBuf<float> p;          // [kNParam] FP32 master parameters
     DevBuf<float> m, v;       // Adam moments
     DevBuf<unsigned short> wl;
-    DevBuf<float> partial;    // per-CTA gradients [nblk][kNTrain + 1]
+    DevBuf<float> partial;    // per-CTA gradients [nblk][kPartial]
     DevBuf<float> gsum;       // [kNTrain + 1] (last = loss sum)
     DevBuf<float> X, out;     // features / network output for all nodes
     DevBuf<double> yg, ypg, Fg;
@@ -418,9 +422,11 @@ __global__ void __launch_bounds__(kTrainThreads, 1) k_mlp_train(const float* __r
         mbar_init(s.bar, 1);
         asm volatile("fence.mbarrier_init.release.cluster;");
     }
-    pdl_wait_and_trigger();
+    // the samples do not come from the kernel ahead (the last batch's step), the
+    // parameters do
     const long first = (long)blockIdx.x * tiles_per_cta;
     float4 f = load_features(X, begin + first * kTile, end);
+    pdl_wait_and_trigger();
     load_params(s, P, wl);
     fence_before_sync();
     __syncthreads();
@@ -529,20 +535,22 @@ __global__ void __launch_bounds__(kTrainThreads, 1) k_mlp_train(const float* __r
     }
     // the CTA's gradient: weights from TMEM (rows at lanes 0..63), bias sums
     // over the four row groups
-    float* g = partial + (size_t)blockIdx.x * (kNTrain + 1);
+    float* g = partial + (size_t)blockIdx.x * kPartial;
+    auto store = [&](float* dst, const float* v, int n) {
+#pragma unroll
+        for (int j = 0; j < n; j += 4)
+            *reinterpret_cast<float4*>(dst + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+    };
     const int q = (threadIdx.x >> 5) & 3, lane = threadIdx.x & 31;
     if (q < 2) {
         float v[NC];
         tmem_ld<NC>(lane_addr(W3, c0), v);
-#pragma unroll
-        for (int j = 0; j < NC; ++j) g[kOffW3 + r * 64 + c0 + j] = v[j];
+        store(g + kOffW3 + r * 64 + c0, v, NC);
         tmem_ld<NC>(lane_addr(W2, c0), v);
-#pragma unroll
-        for (int j = 0; j < NC; ++j) g[kOffW2 + r * 64 + c0 + j] = v[j];
+        store(g + kOffW2 + r * 64 + c0, v, NC);
         if (cg == 0) {
             tmem_ld<NC>(lane_addr(W1, 0), v);
-#pragma unroll
-            for (int j = 0; j < kMlpIn; ++j) g[kOffW1 + r * kMlpIn + j] = v[j];
+            store(g + kOffW1 + r * kMlpIn, v, kMlpIn);
         }
     }
     float* red = s.red + q * kRedN;
@@ -595,7 +603,7 @@ __global__ void __launch_bounds__(32 * kSumGroups) k_grad_step(const float* __re
     float s = 0.0f;
     if (j <= kNTrain) {
 #pragma unroll 8
-        for (int b = grp * per; b < b1; ++b) s += partial[(size_t)b * (kNTrain + 1) + j];
+        for (int b = grp * per; b < b1; ++b) s += partial[(size_t)b * kPartial + j];
     }
     part[grp][lane] = s;
     __syncthreads();
@@ -814,7 +822,7 @@ static void train_pass(fvm_ctx* c, Predictor* p, const float* X, const float* Y,
     int nblk = (int)std::min<long>(ntiles, 148);
     long per = (ntiles + nblk - 1) / nblk;
     nblk = (int)((ntiles + per - 1) / per);
-    if ((long)p->partial.n < (long)nblk * (kNTrain + 1)) p->partial.alloc((size_t)nblk * (kNTrain + 1));
+    if ((long)p->partial.n < (long)nblk * kPartial) p->partial.alloc((size_t)nblk * kPartial);
     fvm_launch_pdl(c, k_mlp_train, nblk, kTrainThreads, mlp_smem_bytes(true), c->stream, X, Y, begin, end, per, p->p.p,
                    p->wl.p, p->partial.p, p->err.p);
     fvm_launch_pdl(c, k_grad_step, (kNTrain + 32) / 32, 32 * kSumGroups, 0, c->stream, p->partial.p, nblk, p->gsum.p,
