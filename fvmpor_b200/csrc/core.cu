@@ -897,6 +897,31 @@ static std::vector<double> initial_head_host(const fvm_ctx* c, double water_tabl
     return h;
 }
 
+// The stored face coefficients of a 3D context, for the element pass variant (and
+// the kernels beside it) that streams them: formed when first asked for.  The
+// default rebuilds them from the vertices and never does; forming and copying
+// them made up a quarter of the 214k-node box's context set-up.
+static void ensure_coef(fvm_ctx* c) {
+    if (c->coef.n) return;
+    const int N = c->N, T = c->T;
+    std::vector<double> coef((size_t)30 * T);
+    parallel_for(T, 16384, [&](long first, long last) {
+        for (long e = first; e < last; ++e) {
+            double X[4][3], C[6][4], G[6], A[6], K[3], vol;
+            for (int k = 0; k < 4; ++k)
+                for (int d = 0; d < 3; ++d) X[k][d] = c->h_xyz[(size_t)d * N + c->h_elem_nodes[4 * (size_t)e + k]];
+            for (int d = 0; d < 3; ++d) K[d] = c->h_eK[(c->kiso ? 0 : (size_t)d * c->estride) + e];
+            tet_coefficients(X[0], X[1], X[2], X[3], K[0], K[1], K[2], C, G, A, &vol);
+            for (int f = 0; f < 6; ++f) {
+                for (int k = 0; k < 4; ++k) coef[(size_t)(f * 5 + k) * T + e] = C[f][k];
+                coef[(size_t)(f * 5 + 4) * T + e] = G[f];
+            }
+        }
+    });
+    c->coef.upload(coef, c->stream);
+    FVM_CUDA(cudaStreamSynchronize(c->stream));
+}
+
 // ------------------------------------------------------------------ autotuner
 // Times the element pass for every (variant, chunk size) candidate on the
 // context's own mesh and keeps the fastest.  Each candidate runs on the
@@ -907,6 +932,7 @@ static std::vector<double> initial_head_host(const fvm_ctx* c, double water_tabl
 static void autotune(fvm_ctx* c, fvm_tune_result* out) {
     const int chunks[] = {256, 512, 1024, 2048};
     const int nvar = c->dim == 3 ? 2 : 1;
+    if (c->dim == 3) ensure_coef(c);
     cudaStream_t s = c->stream;
     std::vector<double> y0 = initial_head_host(c, 0.0);
     DevBuf<double> y, yp, flush;
@@ -1102,7 +1128,9 @@ static void build(fvm_ctx* c, const fvm_mesh* m, const fvm_physics* ph, int flag
     // ---- element geometry
     c->h_elem_nodes.assign(m->elem_nodes, m->elem_nodes + (size_t)T * npe);
     std::vector<int4> en(T);
-    std::vector<double> coef((size_t)nfe * (npe + 1) * T), area((size_t)nfe * T), vol(T);
+    // (3D: the stored coefficients, 240 bytes per element, only where the element
+    // pass may stream them, ensure_coef)
+    std::vector<double> coef(dim == 2 ? (size_t)nfe * (npe + 1) * T : 0), area((size_t)nfe * T), vol(T);
     std::vector<double> eK3((size_t)3 * T);
     parallel_for(T, 16384, [&](long first, long last) {
         for (long el = first; el < last; ++el) {
@@ -1122,11 +1150,7 @@ static void build(fvm_ctx* c, const fvm_mesh* m, const fvm_physics* ph, int flag
                 if (!tet_coefficients(m->coords + 3 * (size_t)v[0], m->coords + 3 * (size_t)v[1], m->coords + 3 * (size_t)v[2],
                                       m->coords + 3 * (size_t)v[3], Kx, Ky, Kz, C, G, A, &vol[e]))
                     throw Error("fvm_create: degenerate tetrahedron " + std::to_string(e));
-                for (int f = 0; f < 6; ++f) {
-                    for (int k = 0; k < 4; ++k) coef[(size_t)(f * 5 + k) * T + e] = C[f][k];
-                    coef[(size_t)(f * 5 + 4) * T + e] = G[f];
-                    area[(size_t)6 * e + f] = A[f];
-                }
+                for (int f = 0; f < 6; ++f) area[(size_t)6 * e + f] = A[f];
             } else {
                 double C[3][3], G[3], A[3];
                 if (!tri_coefficients(m->coords + 3 * (size_t)v[0], m->coords + 3 * (size_t)v[1], m->coords + 3 * (size_t)v[2],
@@ -1346,8 +1370,10 @@ static void build(fvm_ctx* c, const fvm_mesh* m, const fvm_physics* ph, int flag
         for (int d = 0; d < (c->kiso ? 1 : 3); ++d)
             for (int e = 0; e < T; ++e) ek[(size_t)d * ES + e] = eK3[(size_t)d * T + e];
         c->eK.upload(ek, s);
+        c->h_eK = ek;
     }
-    c->coef.upload(coef, s);
+    if (dim == 2) c->coef.upload(coef, s);
+    else if (!c->recompute) ensure_coef(c);
     if (c->nz > 1) c->ezone.upload(std::vector<int>(m->elem_zone, m->elem_zone + T), s);
     c->invV.upload(invV, s);
     c->bterm.upload(bterm, s);
@@ -1524,6 +1550,7 @@ extern "C" int fvm_set_element_pass(fvm_ctx* c, int variant, int chunk) {
     if (variant == 1 && c->dim != 3) throw Error("fvm_set_element_pass: rebuilt geometry is a 3D variant");
     const bool old_rc = c->recompute;
     const int old_ce = c->chunk_e;
+    if (c->dim == 3 && variant == 0) ensure_coef(c);
     c->recompute = variant == 1;
     try {
         build_chunks(c, chunk);

@@ -191,10 +191,11 @@ struct fvm_ctx {
     std::vector<double> h_vert;      // elevation of each node
     std::vector<double> h_hD;        // Dirichlet head (valid where type 1)
     std::vector<double> h_xyz;       // [3][N] coordinates (3D)
+    std::vector<double> h_eK;        // conductivities as in eK (3D)
 
     // element data
     fvmb::DevBuf<int4> enodes;        // [T] node ids (4th = -1 for triangles)
-    fvmb::DevBuf<double> coef;        // [(f*(npe+1)+k)*T + e]
+    fvmb::DevBuf<double> coef;        // [(f*(npe+1)+k)*T + e]; 3D: only where streamed (ensure_coef)
     fvmb::DevBuf<int> ezone;          // [T], only when nz > 1
     fvmb::DevBuf<double> eK;          // [T] (kiso) or [3][T] conductivities (3D)
     fvmb::DevBuf<double> xyz;         // [3][N] coordinates (3D)
