@@ -526,7 +526,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_arnoldi_fused(FusedArgs a)
             const double vcoef = k == 0 ? 0.0 : ck * rb;
             for (int r = q0 + 4 * threadIdx.x; r < r1; r += 4 * blockDim.x) {
                 double acc1[4], acc2[4];
-                quad_combine2(UR, c1, c2, nbv, r, acc1, acc2);
+                quad_combine2(a.U, a.ld, c1, c2, nbv, r, acc1, acc2);
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
                     const int q = r + e;

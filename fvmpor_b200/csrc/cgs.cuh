@@ -428,26 +428,29 @@ __device__ __forceinline__ void block_dots2_by_quad(const float* __restrict__ U,
     __syncthreads();
 }
 
-// acc1[e] = sum_i c1[i] U_i[r + e], acc2[e] = sum_i c2[i] U_i[r + e] (e < 4)
-// from one load of each basis row quad
-template <class B, bool CG>
-__device__ __forceinline__ void quad_combine2(const BasisRows<B, CG>& U, const double* c1, const double* c2, int nv,
-                                              int r, double acc1[4], double acc2[4]) {
+// acc1[e] = sum_i c1[i] U_i[r + e], acc2[e] = sum_i c2[i] U_i[r + e] (e < 4) of an
+// FP32 basis from one load of each row quad, a group's loads all in flight: the
+// last group loads its last vector again in place of the missing ones, and adds
+// nothing for them
+__device__ __forceinline__ void quad_combine2(const float* __restrict__ U, size_t ld, const double* c1,
+                                              const double* c2, int nv, int r, double acc1[4], double acc2[4]) {
 #pragma unroll
     for (int e = 0; e < 4; ++e) acc1[e] = acc2[e] = 0.0;
+#pragma unroll 1
     for (int i0 = 0; i0 < nv; i0 += kCgsGroup) {
+        float4 q[kCgsGroup];
 #pragma unroll
-        for (int q = 0; q < kCgsGroup; ++q) {
-            const int i = i0 + q;
-            if (i < nv) {
-                double u[4];
-                U.quad(i, r, u);
-                const double a = c1[i], b = c2[i];
+        for (int g = 0; g < kCgsGroup; ++g)
+            q[g] = __ldg(reinterpret_cast<const float4*>(U + ld * min(i0 + g, nv - 1) + r));
 #pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    acc1[e] += a * u[e];
-                    acc2[e] += b * u[e];
-                }
+        for (int g = 0; g < kCgsGroup; ++g) {
+            if (i0 + g >= nv) break;
+            const double u[4] = {q[g].x, q[g].y, q[g].z, q[g].w};
+            const double a = c1[i0 + g], b = c2[i0 + g];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                acc1[e] += a * u[e];
+                acc2[e] += b * u[e];
             }
         }
     }

@@ -493,10 +493,11 @@ struct UpArgs {
 };
 constexpr int kUpThreads = 256;
 constexpr int kUpChunk = 512;
-// below this many chunks the blocks leave the chip idle, and the two
-// kernels above, an element and an edge per thread, are as fast (151k elements:
-// about 7 + 7 us)
-constexpr int kUpMinChunks = 296;
+// The line between this and the two kernels above, an element and an edge per
+// thread: both sides take the same at 30,000 elements (a begin-step call 26.6 us
+// against 27.0 on a plane, 26.8 against 27.8 on a box; 30.5 against 35.2 at 155,520
+// and 31.8 against 44.2 at 300,000); below, the third launch costs more
+constexpr int kUpMinChunks = 59;
 
 constexpr int kUpPer = kUpChunk / kUpThreads;   // elements per thread
 

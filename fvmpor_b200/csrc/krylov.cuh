@@ -83,10 +83,6 @@ int gmres_dev(fvm_ctx* c, double cj, const double* y, const double* yp, const do
 void psetup_dev(fvm_ctx* c, double cj, double h, const double* y, const double* yp,
                 const double* F0, const double* ewt, int precision);
 void psolve_dev(fvm_ctx* c, const double* r, double* z, const int* skip = nullptr);
-// z = P^-1 of the residual rows gathered from the element pass's partials, where
-// psolve_gathers()
-bool psolve_gathers(fvm_ctx* c);
-void psolve_gather_dev(fvm_ctx* c, const GatherSrc& g, double* z, const int* skip);
 // y = J(cj) x with the assembled difference-quotient Jacobian of the last
 // set-up (the Krylov operator of fvm_opts.krylov_operator = 1)
 void jacobian_apply(fvm_ctx* c, double cj, const double* x, double* y, const int* skip = nullptr,

@@ -607,12 +607,8 @@ static int gmres_impl(fvm_ctx* c, Krylov* K, double cj, const double* y, const d
                     pt.sigma_dev = K->sigma.p;
                     pt.skip = skip;
                     if (op) jacobian_apply(c, cj, K->t.p, K->Jv.p, skip, dev_cj ? K->cjd.p + 1 : nullptr);
-                    if (!op && psolve_gathers(c)) {
-                        psolve_gather_dev(c, launch_residual_partials(c, y, yp, pt, F0), K->z.p, skip);
-                    } else {
-                        if (!op) launch_residual(c, y, yp, pt, F0, K->Jv.p);
-                        psolve_dev(c, K->Jv.p, K->z.p, skip);
-                    }
+                    else launch_residual(c, y, yp, pt, F0, K->Jv.p);
+                    psolve_dev(c, K->Jv.p, K->z.p, skip);
                     c->tm.begin(TM_CGS, s);
                     int Ni = N;
                     ArnState* stp = K->st.p;

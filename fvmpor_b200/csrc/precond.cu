@@ -494,22 +494,14 @@ __global__ void __launch_bounds__(128) k_ilu_apply(const int* __restrict__ bstar
     for (int i = threadIdx.x; i < nr; i += blockDim.x) z[lu_row[r0 + i]] = (double)x[i];
 }
 
-// the right-hand side of an apply: a vector, or the rows of a residual whose
-// partials the element pass has left (gather_row)
-struct RhsVector {
-    const double* r;
-};
-__device__ __forceinline__ double rhs_row(const RhsVector& v, int i) { return v.r[i]; }
-__device__ __forceinline__ double rhs_row(const GatherSrc& g, int i) { return gather_row(g, i); }
-
-template <class T, class Rhs>
+template <class T>
 __global__ void __launch_bounds__(kIluThreads, 1) k_ilu_apply_smem(const int* __restrict__ bstart,
                                                         const IluBlk* __restrict__ blk,
                                                         const unsigned short* __restrict__ lu_col,
                                                         const unsigned short* __restrict__ meta,
                                                         const T* __restrict__ lu,
                                                         const int* __restrict__ lu_row,
-                                                        const Rhs rhs,
+                                                        const double* __restrict__ r,
                                                         double* __restrict__ z, int* __restrict__ err,
                                                         const int* __restrict__ skip) {
     unsigned char* const smem_raw = ilu_smem();
@@ -531,7 +523,7 @@ __global__ void __launch_bounds__(kIluThreads, 1) k_ilu_apply_smem(const int* __
     // the nodes of the thread's rows, for the way in and the way out: set-up data
     // too, and with them at hand the right-hand side is one round of loads
     // (17.0 us per apply on the 214k-node box with both read row by row)
-    constexpr int kRows = std::is_same_v<Rhs, RhsVector> ? 8 : 4;
+    constexpr int kRows = 8;
     int node[kRows];
 #pragma unroll
     for (int k = 0; k < kRows; ++k) node[k] = lu_row[r0 + min((int)(threadIdx.x + k * blockDim.x), nr - 1)];
@@ -544,12 +536,12 @@ __global__ void __launch_bounds__(kIluThreads, 1) k_ilu_apply_smem(const int* __
     {
         double v[kRows];
 #pragma unroll
-        for (int k = 0; k < kRows; ++k) v[k] = threadIdx.x + k * blockDim.x < nr ? rhs_row(rhs, node[k]) : 0.0;
+        for (int k = 0; k < kRows; ++k) v[k] = threadIdx.x + k * blockDim.x < nr ? r[node[k]] : 0.0;
 #pragma unroll
         for (int k = 0; k < kRows; ++k)
             if (threadIdx.x + k * blockDim.x < nr) x[threadIdx.x + k * blockDim.x] = (T)v[k];
     }
-    for (int i = threadIdx.x + kRows * blockDim.x; i < nr; i += blockDim.x) x[i] = (T)rhs_row(rhs, lu_row[r0 + i]);
+    for (int i = threadIdx.x + kRows * blockDim.x; i < nr; i += blockDim.x) x[i] = (T)r[lu_row[r0 + i]];
     if (threadIdx.x == 0) x[nr] = (T)0;
     bool ok = tc05::mbar_wait(S.bar, 0);
     if (!ok) ok = tc05::mbar_wait(S.bar, 0);   // copies in flight get a second bounded chance
@@ -1417,13 +1409,11 @@ static void build_pattern(fvm_ctx* c, BlockILU* P) {
             raise_smem_limit(k_ilu_apply<float>, sizeof(float) * ((size_t)maxb + 1));
         }
         if (P->smem_stage[0]) {
-            raise_smem_limit(k_ilu_apply_smem<double, RhsVector>, P->smem_stage[0]);
-            raise_smem_limit(k_ilu_apply_smem<double, GatherSrc>, P->smem_stage[0]);
+            raise_smem_limit(k_ilu_apply_smem<double>, P->smem_stage[0]);
             raise_smem_limit(k_ilu_factor_smem<double>, (size_t)(round16(P->smem_stage[0]) + 8 * (size_t)P->scr_words[0]));
         }
         if (P->smem_stage[1]) {
-            raise_smem_limit(k_ilu_apply_smem<float, RhsVector>, P->smem_stage[1]);
-            raise_smem_limit(k_ilu_apply_smem<float, GatherSrc>, P->smem_stage[1]);
+            raise_smem_limit(k_ilu_apply_smem<float>, P->smem_stage[1]);
             raise_smem_limit(k_ilu_factor_smem<float>, (size_t)(round16(P->smem_stage[1]) + 8 * (size_t)P->scr_words[1]));
         }
     }
@@ -1681,35 +1671,13 @@ void psolve_dev(fvm_ctx* c, const double* r, double* z, const int* skip) {
     auto go = [&](auto staged, auto plain, const auto* lu) {
         if (sm)
             fvm_launch_pdl(c, staged, P->nb, P->apply_threads, sm, s, P->bstart.p, P->blk.p, P->lu_col.p, P->meta.p, lu,
-                           P->lu_row.p, RhsVector{r}, z, P->status.p, skip);
+                           P->lu_row.p, r, z, P->status.p, skip);
         else
             fvm_launch_pdl(c, plain, P->nb, 128, sizeof(*lu) * ((size_t)P->maxb + 1), s, P->bstart.p, P->blk.p,
                            P->lu_col.p, P->meta.p, lu, P->lu_row.p, r, z, skip);
     };
-    if (P->factored) go(k_ilu_apply_smem<float, RhsVector>, k_ilu_apply<float>, P->lu32.p);
-    else go(k_ilu_apply_smem<double, RhsVector>, k_ilu_apply<double>, P->lu64.p);
-}
-
-// The apply takes the residual's rows straight from the element pass's partials
-// where a block's threads have few rows each: z = P^-1 (gather), one launch and
-// one pass less per Jacobian-free Arnoldi step.  A block of many rows would wait
-// longer for its chains of dependent loads than the gather's own launch takes
-// with an eighth of a warp's rows per SM.
-constexpr int kGatherRows = 512;
-bool psolve_gathers(fvm_ctx* c) {
-    BlockILU* P = c->ilu;
-    return P && P->factored >= 0 && P->schur_iters < 0 && P->smem_stage[P->factored] && P->maxb <= kGatherRows;
-}
-void psolve_gather_dev(fvm_ctx* c, const GatherSrc& g, double* z, const int* skip) {
-    BlockILU* P = c->ilu;
-    c->tm.begin(TM_ILU_APPLY, c->stream);
-    auto go = [&](auto kern, const auto* lu) {
-        fvm_launch_pdl(c, kern, P->nb, P->apply_threads, P->smem_stage[P->factored], c->stream, P->bstart.p, P->blk.p,
-                       P->lu_col.p, P->meta.p, lu, P->lu_row.p, g, z, P->status.p, skip);
-    };
-    if (P->factored) go(k_ilu_apply_smem<float, GatherSrc>, P->lu32.p);
-    else go(k_ilu_apply_smem<double, GatherSrc>, P->lu64.p);
-    c->tm.end(TM_ILU_APPLY, c->stream);
+    if (P->factored) go(k_ilu_apply_smem<float>, k_ilu_apply<float>, P->lu32.p);
+    else go(k_ilu_apply_smem<double>, k_ilu_apply<double>, P->lu64.p);
 }
 
 } // namespace fvmb

@@ -1,5 +1,5 @@
-"""The step's upwind directions formed chunk by chunk (meshes of some hundred
-chunks of 512 elements; smaller ones go edge by edge) against the CPU oracle:
+"""The step's upwind directions formed chunk by chunk (meshes of 59 chunks of 512
+elements or more; smaller ones go edge by edge) against the CPU oracle:
 the residual with the frozen directions.
 
 Tolerance as in test_gpu_parity.py for residuals: 1e-10 of the largest entry.
@@ -14,10 +14,10 @@ from oracle.pyoracle import Oracle
 
 pytestmark = pytest.mark.gpu
 
-# 296 chunks (the least that go chunk by chunk) to 311, a full last chunk, one
-# and two zones, rebuilt and stored geometry
-CASES = [("richards2d", dict(nx=294, ny=259), 0), ("richards2d", dict(nx=401, ny=200), 0),
-         ("richards3d", dict(nx=31, ny=33, nz=25), 0), ("richards3d", dict(nx=31, ny=33, nz=25), fb.FLAG_STORED_GEOMETRY),
+# 59 chunks (the least that go chunk by chunk) to 311, a full last chunk, one and
+# two zones, rebuilt and stored geometry
+CASES = [("richards2d", dict(nx=123, ny=123), 0), ("richards2d", dict(nx=401, ny=200), 0),
+         ("richards3d", dict(nx=31, ny=33, nz=25), 0), ("richards3d", dict(nx=17, ny=16, nz=19), fb.FLAG_STORED_GEOMETRY),
          ("richards3d", dict(nx=32, ny=33, nz=24), 0)]
 
 
