@@ -22,6 +22,8 @@
 // 0-1 1-2 2-0 0-3 1-3 2-3.
 #pragma once
 
+#include <cmath>
+
 #ifdef __CUDACC__
 #define FVM_HD __host__ __device__ __forceinline__
 #else

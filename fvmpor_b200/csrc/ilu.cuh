@@ -4,32 +4,13 @@
 #pragma once
 
 #include "ctx.cuh"
+#include "ilu_layout.hpp"
 #include "tc05.cuh"
 
 #include <cstdint>
 #include <vector>
 
 namespace fvmb {
-
-// One block's factor: rows in colour order, the off-diagonal entries sliced by
-// level for the sweeps.  The rows of a level are taken longest first, 32 to a
-// slice (a lane each), and a slice's entries are stored entry-major: entry k
-// of lane l at 32 (start + k) + l, padded to the slice's longest row with
-// zeros whose column is nr, a slot of the vector that stays zero.  The lower
-// sweep's slices come first, then the upper sweep's, then the (inverted)
-// pivots in row order.  A warp so reads 32 consecutive values and columns.
-// Stored row by row instead, with a row per lane, every read hit about four
-// lanes' worth of bank conflicts, and the sweeps were bound by those.
-struct IluBlk {
-    int v0;    // first entry in the value arrays (a multiple of 32)
-    int c0;    // and in the column array
-    int dp;    // slices' length / 32: the pivots start at 32 dp
-    int mo;    // the record's first word (a multiple of 8)
-    int mw;    // its words
-    int nl, nu;      // levels of the lower and the upper sweep
-    int nsl, nsu;    // their slices
-    int seg;     // first level in the elimination schedule
-};
 
 struct BlockILU {
     bool built = false;
@@ -121,7 +102,7 @@ struct BlockILU {
     DevBuf<int> serr;                // 3: a grid barrier of the coupled apply timed out
     int* h_serr = nullptr;           // pinned
     size_t schur_smem[2] = {0, 0};   // dynamic shared bytes of the coupled apply, 0 = not possible
-    int schur_nrmax = 0;
+    bool schur_staged[2] = {false, false};   // its factor in shared memory, or read in place
 };
 
 // largest dynamic shared-memory carve-out a CTA may request on sm_100
@@ -137,32 +118,9 @@ constexpr int kIluThreads = 256;   // largest CTA of the staged apply
 // contiguous 16-byte aligned range, moved by 1D TMA bulk copies
 // (cp.async.bulk, completion counted on an mbarrier, bounded wait), while the
 // threads fill the right-hand side alongside.
-// Shared layout: x[T nr + 1, 16-B padded] | val[T wn] | col[u16 32 dp + slack] |
+// Shared layout: x[T nr + 1, 16-B padded] | val[T wn] | col[u16 ds + slack] |
 // record | mbarrier (a sweep's reads past the values stay inside)
-__host__ __device__ __forceinline__ size_t round16(size_t b) { return (b + 15) & ~(size_t)15; }
-
-// entries of a block's window: its slices and its pivots
-__host__ __device__ __forceinline__ size_t ilu_window(size_t nr, size_t dp) { return 32 * dp + ((nr + 31) & ~(size_t)31); }
-
-// u16 words of a block's record: first slice of each level of the lower
-// (nl + 1) and of the upper sweep (nu + 1), the slices' starts / 32 (lower,
-// upper, end), then the rows of the lower and of the upper slices' lanes
-// (kIluNoRow past a level's last), padded to 16 bytes
-constexpr unsigned short kIluNoRow = 0xffff;
-__host__ __device__ __forceinline__ size_t ilu_meta_words(size_t nl, size_t nu, size_t nsl, size_t nsu) {
-    return (nl + nu + 3 + 33 * (nsl + nsu) + 7) & ~(size_t)7;
-}
-
-// entries that a sweep may read past the last slice: values of any kind, columns
-// of zero (a place of the vector); part of each block's columns and window
-constexpr int kIluSlack = 256;
-__host__ __device__ __forceinline__ size_t ilu_columns(size_t dp) { return 32 * dp + kIluSlack; }
-
-// shared bytes of the staged kernels for one block (host and device agree)
-__host__ __device__ __forceinline__ size_t ilu_stage_bytes(size_t nr, size_t dp, size_t mw, size_t sz) {
-    return round16((nr + 1) * sz) + ilu_window(nr, dp) * sz + ilu_columns(dp) * 2 + 2 * mw + 16 + kIluSlack * sz;
-}
-
+// (sizes in ilu_layout.hpp)
 // The dynamic shared memory of the sweeps' kernels; the block's vector is at
 // its start.  The staged factor is addressed by offsets from it, so that every
 // access is known to be one to shared memory.
@@ -173,9 +131,12 @@ __device__ __forceinline__ unsigned char* ilu_smem() {
 // a block's factor and record for the sweeps, staged in shared memory ...
 template <class T> struct IluShared {
     unsigned ov, oc, om;   // offsets of the values, the columns and the record
-    int nl, nu, nsl, nsu, dp;
+    int nl, nu, ngl, ngu, nwide, ds;
     __device__ __forceinline__ unsigned meta(int i) const {
         return *reinterpret_cast<const unsigned short*>(ilu_smem() + om + 2 * i);
+    }
+    __device__ __forceinline__ unsigned meta2(int i) const {   // a double word, i even
+        return *reinterpret_cast<const unsigned*>(ilu_smem() + om + 2 * i);
     }
     __device__ __forceinline__ T val(int i) const { return reinterpret_cast<const T*>(ilu_smem() + ov)[i]; }
     __device__ __forceinline__ unsigned col(int i) const {
@@ -186,23 +147,52 @@ template <class T> struct IluShared {
 template <class T> struct IluGlobal {
     const T* v;
     const unsigned short *c, *m;
-    int nl, nu, nsl, nsu, dp;
+    int nl, nu, ngl, ngu, nwide, ds;
     __device__ __forceinline__ unsigned meta(int i) const { return m[i]; }
+    __device__ __forceinline__ unsigned meta2(int i) const { return *reinterpret_cast<const unsigned*>(m + i); }
     __device__ __forceinline__ T val(int i) const { return v[i]; }
     __device__ __forceinline__ unsigned col(int i) const { return c[i]; }
 };
 template <class V, class A, class C, class M> __device__ __forceinline__ V ilu_view(const IluBlk& B, A v, C c, M m) {
-    return V{v, c, m, B.nl, B.nu, B.nsl, B.nsu, B.dp};
+    return V{v, c, m, B.nl, B.nu, B.ngl, B.ngu, B.nwide, B.ds};
 }
-// the record's parts (ilu_meta_words)
+// the record's parts (ilu_meta_words); g counts a sweep's groups from 0
 template <class V> __device__ __forceinline__ int ilu_level(const V& f, bool upper, int l) {
     return (int)f.meta((upper ? f.nl + 1 : 0) + l);
 }
-template <class V> __device__ __forceinline__ int ilu_start(const V& f, bool upper, int s) {
-    return (int)f.meta(f.nl + f.nu + 2 + (upper ? f.nsl : 0) + s);
+template <class V> __device__ __forceinline__ int ilu_groups_at(const V& f) { return (f.nl + f.nu + 3) & ~1; }
+template <class V> __device__ __forceinline__ unsigned ilu_group(const V& f, bool upper, int g) {
+    return f.meta2(ilu_groups_at(f) + 2 * ((upper ? f.ngl : 0) + g));
 }
-template <class V> __device__ __forceinline__ int ilu_row(const V& f, bool upper, int q) {
-    return (int)f.meta(f.nl + f.nu + 3 + f.nsl + f.nsu + (upper ? 32 * f.nsl : 0) + q);
+template <class V> __device__ __forceinline__ int ilu_row(const V& f, bool upper, int g, int j) {
+    return (int)f.meta(ilu_groups_at(f) + 2 * (f.ngl + f.ngu) + kIluGroup * ((upper ? f.ngl : 0) + g) + j);
+}
+// a wide row's first entry past kIluWide and its entries
+template <class V> __device__ __forceinline__ int2 ilu_wide(const V& f, bool upper, int g) {
+    const int at = ilu_groups_at(f) + (2 + kIluGroup) * (f.ngl + f.ngu), key = (upper ? f.ngl : 0) + g;
+    int lo = 0;
+    for (int n = f.nwide; n > 1;) {   // ascending groups
+        const int h = n >> 1;
+        if ((int)f.meta2(at + 6 * (lo + h)) <= key) lo += h;
+        n -= h;
+    }
+    return make_int2((int)f.meta2(at + 6 * lo + 2), (int)f.meta2(at + 6 * lo + 4));
+}
+// where the entries of lane j's row of a group are: the general form, for the
+// factorisations
+struct IluSpan {
+    int at, tail, w;
+    __device__ __forceinline__ int entry(int k) const { return k < kIluWide ? at + 32 * k : tail + k - kIluWide; }
+};
+template <class V> __device__ __forceinline__ IluSpan ilu_span(const V& f, bool upper, int g, int j) {
+    const unsigned word = ilu_group(f, upper, g);
+    IluSpan s{(int)(word >> kIluWidthBits) + j, 0, (int)(word & ((1u << kIluWidthBits) - 1u))};
+    if (s.w > kIluWide) {
+        const int2 t = ilu_wide(f, upper, g);
+        s.tail = t.x;
+        s.w = t.y;
+    }
+    return s;
 }
 
 // a staged block: where its parts sit in shared memory
@@ -216,8 +206,8 @@ template <class T> struct IluStage {
     __device__ __forceinline__ IluStage(const IluBlk& B, int nr) {
         unsigned char* smem = ilu_smem();
         ov = (unsigned)round16(sizeof(T) * (nr + 1));
-        oc = ov + (unsigned)(sizeof(T) * ilu_window(nr, B.dp));
-        om = oc + 2u * (unsigned)ilu_columns(B.dp);
+        oc = ov + (unsigned)(sizeof(T) * ilu_window(nr, B.ds));
+        om = oc + 2u * (unsigned)ilu_columns(B.ds);
         x = reinterpret_cast<T*>(smem);
         val = reinterpret_cast<T*>(smem + ov);
         col = reinterpret_cast<unsigned short*>(smem + oc);
@@ -236,7 +226,7 @@ __device__ __forceinline__ void ilu_stage_bulk(const IluStage<T>& S, const IluBl
                                                const unsigned short* lu_col, const unsigned short* meta) {
     if (threadIdx.x == 0) {
         const uint32_t b = tc05::smem_u32(S.bar);
-        const uint32_t vb = (uint32_t)(ilu_window(nr, B.dp) * sizeof(T)), cb = 2u * (uint32_t)ilu_columns(B.dp), mb = 2u * (uint32_t)B.mw;
+        const uint32_t vb = (uint32_t)(ilu_window(nr, B.ds) * sizeof(T)), cb = 2u * (uint32_t)ilu_columns(B.ds), mb = 2u * (uint32_t)B.mw;
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(b), "r"(vb + cb + mb) : "memory");
         tc05::bulk_g2s(S.val, lu + B.v0, vb, S.bar);
         tc05::bulk_g2s(S.col, lu_col + B.c0, cb, S.bar);
@@ -255,16 +245,16 @@ __device__ __forceinline__ int tid_here() {
 }
 
 // One triangular sweep over the levels [l0, l1): rows of a level are
-// independent, a warp takes a slice of 32.  UPPER: x_i = (x_i - sum over the
-// upper entries) * inverse pivot; else x_i = x_i - sum over the lower ones
-// (unit lower triangle).  A warp's slice of level l+1 -- its rows and the first
-// kIluPre columns, which do not depend on x -- is fetched while level l is
+// independent, a warp takes a slice of kIluSlice groups.  UPPER: x_i = (x_i - sum
+// over the upper entries) * inverse pivot; else x_i = x_i - sum over the lower
+// ones (unit lower triangle).  A warp's slice of level l+1 -- its rows and the
+// first kIluPre columns, which do not depend on x -- is fetched while level l is
 // computed, so after each barrier only the x loads (independent of each other,
 // the values loaded beside them) and the accumulation remain on the critical
 // path; a warp without a slice goes straight to the barrier.  Entries in column
-// order.  All bounds are the same for a warp's lanes; loads are taken four
-// entries at a time, past a slice's last entry (kIluSlack entries after the
-// arrays), and what lies there is left unused.
+// order.  Loads are taken four entries at a time, past a group's last entry
+// (kIluSlack entries after the arrays), and what lies there is left unused, as
+// is what the lanes past a level's last group read (its entries again).
 // Most rows of a tetrahedral mesh have more than kIluPre entries (up to 14), but
 // a level is bound by the instructions that its warps issue: the two sweeps of
 // a 1,447-row block of the 214k-node box took 5.0 us with 4 columns fetched
@@ -276,19 +266,22 @@ struct IluLane {
     unsigned c[kIluPre];
 };
 
+// lane's row of group g, a group of the level that ends at g1 (past it: no row)
 template <bool UPPER, class V>
-__device__ __forceinline__ void ilu_fetch(IluLane& R, const V& f, int lane, int s) {
-    const int p = ilu_start(f, UPPER, s);
-    R.w = ilu_start(f, UPPER, s + 1) - p;
-    R.at = 32 * p + lane;
-    R.row = ilu_row(f, UPPER, 32 * s + lane);
+__device__ __forceinline__ void ilu_fetch(IluLane& R, const V& f, int lane, int g, int g1) {
+    const int gi = min(g, g1 - 1), j = lane & (kIluGroup - 1);
+    const unsigned word = ilu_group(f, UPPER, gi);
+    R.w = (int)(word & ((1u << kIluWidthBits) - 1u));
+    R.at = (int)(word >> kIluWidthBits) + j;
+    R.row = g < g1 ? ilu_row(f, UPPER, gi, j) : kIluNoRow;
 #pragma unroll
     for (int k = 0; k < kIluPre; ++k) R.c[k] = f.col(R.at + 32 * k);
 }
 
-// acc += entries [k, w) of a row
+// acc += entries [k, w) of a row, the first kIluWide of a wide one
 template <class T, class V>
 __device__ __forceinline__ void ilu_rest(T& acc, const T* x, const V& f, int at, int w, int k) {
+    w = min(w, kIluWide);
 #pragma unroll 1
     for (; k < w; k += 4) {
         T v[4], xv[4];
@@ -302,11 +295,18 @@ __device__ __forceinline__ void ilu_rest(T& acc, const T* x, const V& f, int at,
             if (k + t < w) acc += v[t] * xv[t];
     }
 }
+// ... and the others
+template <class T, class V> __device__ __forceinline__ T ilu_wide_rest(T acc, const T* x, const V& f, bool upper, int g) {
+    const int2 t = ilu_wide(f, upper, g);
+    for (int k = 0; k < t.y - kIluWide; ++k) acc += f.val(t.x + k) * x[f.col(t.x + k)];
+    return acc;
+}
 
 template <class T, bool UPPER, class V>
 __device__ __forceinline__ void ilu_sweep(const V& f, int l0, int l1) {
     T* const x = reinterpret_cast<T*>(ilu_smem());
-    const int tid = tid_here(), warp = tid >> 5, lane = tid & 31, nw = blockDim.x >> 5;
+    const int tid = tid_here(), lane = tid & 31, stride = (blockDim.x >> 5) * kIluSlice;
+    const int first = (tid >> 5) * kIluSlice, mine = tid / kIluGroup;   // the warp's and the lane's group of a level
     // set before the conditional fetches: registers that a loop writes only
     // under a condition count as live all the way round it
     IluLane cur, nxt;
@@ -317,12 +317,12 @@ __device__ __forceinline__ void ilu_sweep(const V& f, int l0, int l1) {
     nxt = cur;
     if (l0 >= l1) return;
     int s0 = ilu_level(f, UPPER, l0), s1 = ilu_level(f, UPPER, l0 + 1);
-    if (s0 + warp < s1) ilu_fetch<UPPER>(cur, f, lane, s0 + warp);
+    if (s0 + first < s1) ilu_fetch<UPPER>(cur, f, lane, s0 + mine, s1);
 #pragma unroll 1
     for (int l = l0; l < l1; ++l) {
         const int s2 = l + 1 < l1 ? ilu_level(f, UPPER, l + 2) : s1;
-        const bool more = s1 + warp < s2;
-        if (s0 + warp < s1) {
+        const bool more = s1 + first < s2;
+        if (s0 + first < s1) {
             // this level's x and value loads first, then the next level's
             // slice while they are in flight, then the accumulation
             T xv[kIluPre], v[kIluPre];
@@ -333,25 +333,31 @@ __device__ __forceinline__ void ilu_sweep(const V& f, int l0, int l1) {
             }
             const bool act = cur.row != kIluNoRow;
             const int row = act ? cur.row : 0;
-            const T xi = x[row], piv = UPPER ? f.val(32 * f.dp + row) : (T)1;
-            if (more) ilu_fetch<UPPER>(nxt, f, lane, s1 + warp);
+            const T xi = x[row], piv = UPPER ? f.val(f.ds + row) : (T)1;
+            if (more) ilu_fetch<UPPER>(nxt, f, lane, s1 + mine, s2);
             T acc = (T)0;
 #pragma unroll
             for (int k = 0; k < kIluPre; ++k)
                 if (k < cur.w) acc += v[k] * xv[k];
             ilu_rest(acc, x, f, cur.at, cur.w, kIluPre);
+            if (cur.w > kIluWide && act) acc = ilu_wide_rest(acc, x, f, UPPER, s0 + mine);
             if (act) x[row] = UPPER ? (xi - acc) * piv : xi - acc;
             // slices of a level with more of them than the CTA has warps
 #pragma unroll 1
-            for (int s = s0 + warp + nw; s < s1; s += nw) {
-                const int p = ilu_start(f, UPPER, s), w = ilu_start(f, UPPER, s + 1) - p;
-                const int i = ilu_row(f, UPPER, 32 * s + lane);
+            for (int s = s0 + stride; s + first < s1; s += stride) {
+                const int g = s + mine, gi = min(g, s1 - 1), j = lane & (kIluGroup - 1);
+                const unsigned word = ilu_group(f, UPPER, gi);
+                const int w = (int)(word & ((1u << kIluWidthBits) - 1u));
+                const int i = g < s1 ? ilu_row(f, UPPER, gi, j) : kIluNoRow;
                 T a = (T)0;
-                ilu_rest(a, x, f, 32 * p + lane, w, 0);
-                if (i != kIluNoRow) x[i] = UPPER ? (x[i] - a) * f.val(32 * f.dp + i) : x[i] - a;
+                ilu_rest(a, x, f, (int)(word >> kIluWidthBits) + j, w, 0);
+                if (i != kIluNoRow) {
+                    if (w > kIluWide) a = ilu_wide_rest(a, x, f, UPPER, g);
+                    x[i] = UPPER ? (x[i] - a) * f.val(f.ds + i) : x[i] - a;
+                }
             }
         } else if (more) {
-            ilu_fetch<UPPER>(nxt, f, lane, s1 + warp);
+            ilu_fetch<UPPER>(nxt, f, lane, s1 + mine, s2);
         }
         __syncthreads();
         cur = nxt;

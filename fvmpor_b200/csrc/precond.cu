@@ -422,43 +422,43 @@ __global__ void __launch_bounds__(128) k_ilu_factor(const int* __restrict__ bsta
                                                     const unsigned short* __restrict__ lu_col, T* lu, int* status) {
     const IluBlk B = blk[blockIdx.x];
     const int r0 = bstart[blockIdx.x], nr = bstart[blockIdx.x + 1] - r0;
-    const long wn = (long)ilu_window(nr, B.dp);
+    const long wn = (long)ilu_window(nr, B.ds);
     T* val = lu + B.v0;
     for (long p = threadIdx.x; p < wn; p += blockDim.x) val[p] = Jw[B.v0 + p];
     __syncthreads();
     const auto V = ilu_view<IluGlobal<T>>(B, val, lu_col + B.c0, meta + B.mo);
-    const int D = 32 * B.dp;
+    const int D = B.ds;
     for (int l = 0; l < B.nl; ++l) {
-        for (int q = 32 * ilu_level(V, false, l) + threadIdx.x; q < 32 * ilu_level(V, false, l + 1); q += blockDim.x) {
-            const int i = ilu_row(V, false, q);
+        const int q1 = kIluGroup * ilu_level(V, false, l + 1);
+        for (int q = kIluGroup * ilu_level(V, false, l) + threadIdx.x; q < q1; q += blockDim.x) {
+            const int i = ilu_row(V, false, q / kIluGroup, q % kIluGroup);
             if (i == kIluNoRow) continue;
-            const int w = ilu_start(V, false, (q >> 5) + 1) - ilu_start(V, false, q >> 5);
-            const int lo = 32 * ilu_start(V, false, q >> 5) + (q & 31);
-            const int ui = up[r0 + i], ai = ilu_start(V, true, ui >> 5);
-            const int uwi = ilu_start(V, true, (ui >> 5) + 1) - ai, hi = 32 * ai + (ui & 31);
-            for (int kk = 0; kk < w; ++kk) {
-                const int k = (int)V.col(lo + 32 * kk);
+            const IluSpan lo = ilu_span(V, false, q / kIluGroup, q % kIluGroup);
+            const int ui = up[r0 + i];
+            const IluSpan hi = ilu_span(V, true, ui / kIluGroup, ui % kIluGroup);
+            for (int kk = 0; kk < lo.w; ++kk) {
+                const int p = lo.entry(kk), k = (int)V.col(p);
                 if (k == nr) break;
-                const T lik = val[lo + 32 * kk] * val[D + k];
-                val[lo + 32 * kk] = lik;
+                const T lik = val[p] * val[D + k];
+                val[p] = lik;
                 // U(k) against the rest of row i
-                const int uk = up[r0 + k], ak = ilu_start(V, true, uk >> 5);
-                const int uwk = ilu_start(V, true, (uk >> 5) + 1) - ak, hk = 32 * ak + (uk & 31);
+                const int uk = up[r0 + k];
+                const IluSpan ku = ilu_span(V, true, uk / kIluGroup, uk % kIluGroup);
                 int a = kk + 1, c = 0;
-                for (int u = 0; u < uwk; ++u) {
-                    const int j = (int)V.col(hk + 32 * u);
+                for (int u = 0; u < ku.w; ++u) {
+                    const int j = (int)V.col(ku.entry(u));
                     if (j == nr) break;
                     int at = -1;
                     if (j < i) {
-                        while (a < w && (int)V.col(lo + 32 * a) < j) ++a;
-                        if (a < w && (int)V.col(lo + 32 * a) == j) at = lo + 32 * a;
+                        while (a < lo.w && (int)V.col(lo.entry(a)) < j) ++a;
+                        if (a < lo.w && (int)V.col(lo.entry(a)) == j) at = lo.entry(a);
                     } else if (j == i) {
                         at = D + i;
                     } else {
-                        while (c < uwi && (int)V.col(hi + 32 * c) < j) ++c;
-                        if (c < uwi && (int)V.col(hi + 32 * c) == j) at = hi + 32 * c;
+                        while (c < hi.w && (int)V.col(hi.entry(c)) < j) ++c;
+                        if (c < hi.w && (int)V.col(hi.entry(c)) == j) at = hi.entry(c);
                     }
-                    if (at >= 0) val[at] = val[at] - lik * val[hk + 32 * u];
+                    if (at >= 0) val[at] = val[at] - lik * val[ku.entry(u)];
                 }
             }
             T d = val[D + i];
@@ -494,8 +494,10 @@ __global__ void __launch_bounds__(128) k_ilu_apply(const int* __restrict__ bstar
     for (int i = threadIdx.x; i < nr; i += blockDim.x) z[lu_row[r0 + i]] = (double)x[i];
 }
 
+// (three CTAs of 256 threads per SM: 80 registers, no spills; unbounded, the build
+// takes 98 and leaves small blocks a CTA less per SM)
 template <class T>
-__global__ void __launch_bounds__(kIluThreads, 1) k_ilu_apply_smem(const int* __restrict__ bstart,
+__global__ void __launch_bounds__(kIluThreads, 3) k_ilu_apply_smem(const int* __restrict__ bstart,
                                                         const IluBlk* __restrict__ blk,
                                                         const unsigned short* __restrict__ lu_col,
                                                         const unsigned short* __restrict__ meta,
@@ -570,7 +572,8 @@ __global__ void __launch_bounds__(kIluThreads, 1) k_ilu_apply_smem(const int* __
 // C - F B^-1 E on C's pattern; the interface system of the whole matrix is
 // S = L_S U_S + C_o, C_o the couplings to the other blocks' interface rows.
 // One cooperative launch, one CTA per block, the factor staged in shared
-// memory once for the whole apply:
+// memory once for the whole apply, or read in place where its padding keeps
+// that from fitting (STAGED false, schur_layout):
 //   z = L^-1 r (the forward sweep; x_L = M_B f and g - F x_L of the
 //     reference), kept in shared memory;
 //   x_S = U_S^-1 z_S, then `iters` times: publish x_S, grid barrier,
@@ -606,8 +609,10 @@ template <class T> struct SchurArgs {
     const int* skip;
 };
 
-template <class T>
-__global__ void __launch_bounds__(kIluThreads, 1) k_ilu_apply_schur(SchurArgs<T> a) {
+// (registers for as many CTAs of 256 threads per SM as blocks may have to be
+// resident: four in FP32, three in FP64)
+template <class T, bool STAGED>
+__global__ void __launch_bounds__(kIluThreads, sizeof(T) == 4 ? 4 : 3) k_ilu_apply_schur(SchurArgs<T> a) {
     unsigned char* const smem_raw = ilu_smem();
     const int b = blockIdx.x;
     const IluBlk B = a.blk[b];
@@ -616,26 +621,31 @@ __global__ void __launch_bounds__(kIluThreads, 1) k_ilu_apply_schur(SchurArgs<T>
     T* x = S.x;
     uint64_t* mbar = S.bar;
     T* zs = reinterpret_cast<T*>(smem_raw + a.stage_max);
-    if (threadIdx.x == 0) {
-        tc05::mbar_init(mbar, 1);
-        asm volatile("fence.mbarrier_init.release.cluster;");
+    if constexpr (STAGED) {
+        if (threadIdx.x == 0) {
+            tc05::mbar_init(mbar, 1);
+            asm volatile("fence.mbarrier_init.release.cluster;");
+        }
+        __syncthreads();
+        ilu_stage_bulk(S, B, nr, a.lu, a.lu_col, a.meta);
     }
-    __syncthreads();
-    ilu_stage_bulk(S, B, nr, a.lu, a.lu_col, a.meta);
     pdl_wait_and_trigger();
     if (a.skip && *a.skip) {
         // a step queued after the stop: every block leaves before any barrier
-        tc05::mbar_wait(mbar, 0);
+        if constexpr (STAGED) tc05::mbar_wait(mbar, 0);
         return;
     }
     for (int i = threadIdx.x; i < nr; i += blockDim.x) x[i] = (T)a.r[a.lu_row[r0 + i]];
     if (threadIdx.x == 0) x[nr] = (T)0;
-    bool ok = tc05::mbar_wait(mbar, 0);
-    if (!ok) ok = tc05::mbar_wait(mbar, 0);
+    bool ok = true;
+    if constexpr (STAGED) ok = tc05::mbar_wait(mbar, 0) || tc05::mbar_wait(mbar, 0);
     const bool good = __syncthreads_and(ok ? 1 : 0) != 0;
     if (!good && threadIdx.x == 0) atomicExch(a.err, 2);
     const int lvB = a.sch_lv[2 * b], uvS = a.sch_lv[2 * b + 1], nin = a.sch_nin[b];
-    const IluShared<T> V = S.view(B);
+    const auto V = [&] {
+        if constexpr (STAGED) return S.view(B);
+        else return ilu_view<IluGlobal<T>>(B, a.lu + B.v0, a.lu_col + B.c0, a.meta + B.mo);
+    }();
     if (good) {
         ilu_sweep<T, false>(V, 1, V.nl);
         for (int i = threadIdx.x; i < nr; i += blockDim.x) zs[i] = x[i];
@@ -674,8 +684,38 @@ __global__ void __launch_bounds__(kIluThreads, 1) k_ilu_apply_schur(SchurArgs<T>
     for (int i = threadIdx.x; i < nr; i += blockDim.x) a.z[a.lu_row[r0 + i]] = (double)x[i];
 }
 
-static const void* schur_kernel(int precision) {
-    return precision ? (const void*)k_ilu_apply_schur<float> : (const void*)k_ilu_apply_schur<double>;
+static const void* schur_kernel(int precision, bool staged) {
+    if (precision) return staged ? (const void*)k_ilu_apply_schur<float, true> : (const void*)k_ilu_apply_schur<float, false>;
+    return staged ? (const void*)k_ilu_apply_schur<double, true> : (const void*)k_ilu_apply_schur<double, false>;
+}
+
+// Whether the coupled apply runs on these blocks, and how.  It keeps each block's
+// forward result in shared memory through its grid barriers, and all blocks
+// must be resident at once.  It is offered where the factor's own entries (rows
+// end to end, with row pointers and level lists: `exact` bytes for the largest
+// block) fit beside that.  The window that the sweeps read is padded, by up to 7 %
+// on small blocks in this order; where only the padding is too much, the sweeps
+// read the factor in place.
+static void schur_layout(const fvm_ctx* c, BlockILU* P, int pr, size_t exact) {
+    int nsm = 148, coop = 0;
+    FVM_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device));
+    FVM_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, c->device));
+    P->schur_smem[pr] = 0;
+    if (!coop) return;
+    const size_t sz = pr ? sizeof(float) : sizeof(double), fwd = round16(sz * (size_t)P->maxb);
+    auto resident = [&](bool staged, size_t bytes) {
+        if (bytes > kMaxDynSmem) return false;
+        const void* kfn = schur_kernel(pr, staged);
+        raise_smem_limit(kfn, bytes);
+        int per_sm = 0;
+        FVM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kfn, P->apply_threads, bytes));
+        return (long)per_sm * nsm >= P->nb;
+    };
+    if (!exact || !resident(true, round16(exact) + fwd)) return;
+    const size_t staged = round16(P->smem_stage[pr]) + fwd, plain = round16(sz * ((size_t)P->maxb + 1)) + fwd;
+    P->schur_staged[pr] = P->smem_stage[pr] && resident(true, staged);
+    if (P->schur_staged[pr]) P->schur_smem[pr] = staged;
+    else if (resident(false, plain)) P->schur_smem[pr] = plain;
 }
 
 template <class T>
@@ -683,7 +723,8 @@ static void launch_schur_apply(fvm_ctx* c, BlockILU* P, const T* lu, const doubl
     SchurArgs<T> a;
     a.N = c->N;
     a.iters = P->schur_iters;
-    a.stage_max = round16(P->smem_stage[P->factored]);
+    const bool staged = P->schur_staged[P->factored];
+    a.stage_max = staged ? round16(P->smem_stage[P->factored]) : round16(sizeof(T) * ((size_t)P->maxb + 1));
     a.bstart = P->bstart.p;
     a.blk = P->blk.p;
     a.lu_col = P->lu_col.p;
@@ -715,7 +756,8 @@ static void launch_schur_apply(fvm_ctx* c, BlockILU* P, const T* lu, const doubl
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 2;
-    FVM_CUDA(cudaLaunchKernelEx(&cfg, k_ilu_apply_schur<T>, a));
+    if (staged) FVM_CUDA(cudaLaunchKernelEx(&cfg, k_ilu_apply_schur<T, true>, a));
+    else FVM_CUDA(cudaLaunchKernelEx(&cfg, k_ilu_apply_schur<T, false>, a));
     c->launches++;
 }
 
@@ -776,8 +818,8 @@ __global__ void __launch_bounds__(kIluFactorThreads, 1) k_ilu_factor_smem(const 
         return;
     }
     const IluShared<T> V = S.view(B);
-    const int D = 32 * B.dp;
-    constexpr int G = kIluFactorLanes, R = 32 / G;   // lanes per row, rows per warp
+    const int D = B.ds;
+    constexpr int G = kIluFactorLanes, R = 32 / (G * kIluGroup);   // lanes per row, groups per warp
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
     for (int l = 0; l < nl; ++l) {
         int sgn = 0, lenn = 0;
@@ -796,20 +838,22 @@ __global__ void __launch_bounds__(kIluFactorThreads, 1) k_ilu_factor_smem(const 
             }
         }
         const unsigned* L = cur_smem ? ((l & 1) ? buf1 : buf0) : upd + sgc;
-        const int s0 = ilu_level(V, false, l), s1 = ilu_level(V, false, l + 1);
-        // a warp takes R consecutive lanes' rows of a slice
-        for (int it = warp; it < (s1 - s0) * G; it += nw) {
-            const int s = s0 + it / G, q = (it % G) * R + lane / G, g = lane % G;
-            const int ps = ilu_start(V, false, s), w = ilu_start(V, false, s + 1) - ps, p0 = 32 * ps + q;
-            const int i = ilu_row(V, false, 32 * s + q);
+        const int g0 = ilu_level(V, false, l), g1 = ilu_level(V, false, l + 1);
+        // a warp takes R consecutive groups; the first has the longest rows
+        for (int gw = g0 + R * warp; gw < g1; gw += R * nw) {
+            const int gr = gw + lane / (G * kIluGroup), q = lane / G % kIluGroup, g = lane % G;
+            const int i = gr < g1 ? ilu_row(V, false, gr, q) : kIluNoRow;
+            const IluSpan S = ilu_span(V, false, min(gr, g1 - 1), q);
+            const int w = __shfl_sync(0xffffffffu, S.w, 0);
             const bool row = i != kIluNoRow;
             // IKJ with the precomputed schedule: the updates of each L entry,
             // in the order a merge of the row with U(k) would find them
-            int t = row ? (int)L[32 * (s - s0) + q] : 0;
+            int t = row ? (int)L[kIluGroup * (gr - g0) + q] : 0;
             for (int kk = 0; kk < w; ++kk) {
-                const int p = p0 + 32 * kk;
-                const int k = (int)V.col(p);
-                const bool act = row && k != nr;
+                const bool in = row && kk < S.w;
+                const int p = S.entry(in ? kk : 0);
+                const int k = in ? (int)V.col(p) : nr;
+                const bool act = k != nr;
                 T lik = (T)0;
                 if (act) {
                     const int cnt = (int)L[t];
@@ -847,7 +891,7 @@ __global__ void __launch_bounds__(kIluFactorThreads, 1) k_ilu_factor_smem(const 
         lenc = lenn;
         cur_smem = nxt_smem;
     }
-    const int wn = (int)ilu_window(nr, B.dp);
+    const int wn = (int)ilu_window(nr, B.ds);
     for (int p = threadIdx.x; p < wn; p += blockDim.x) lu[B.v0 + p] = val[p];
 }
 
@@ -1256,69 +1300,29 @@ static void build_pattern(fvm_ctx* c, BlockILU* P) {
     P->nb = nb;
     P->maxb = maxb;
     P->nlevels_max = nlmax;
-    // the sliced layout of every block (IluBlk) and its record: a level's rows
-    // longest first, stable
+    // the layout of every block's factor and its record
     std::vector<IluBlk> blk(nb);
     std::vector<std::vector<unsigned short>> bmeta(nb), bcol(nb);
-    std::vector<int> spos(lu_src.size()), up(N);
+    IluPlaces at;
+    at.entry.resize(lu_src.size());
+    at.upper.resize(N);
+    at.lower.resize(N);
     parallel_for(nb, grain, [&](long b0, long b1) {
         for (long b = b0; b < b1; ++b) {
-            const int r0 = bstart[b], r1 = bstart[b + 1], nr = r1 - r0;
-            IluBlk& B = blk[b];
-            B = IluBlk{};
-            B.nl = blk_lvl[b + 1] - blk_lvl[b];
-            B.nu = blk_ulvl[b + 1] - blk_ulvl[b];
-            B.seg = blk_lvl[b];
-            std::vector<int> first[2], start(1, 0), rows[2];
-            for (int upper = 0; upper < 2; ++upper) {
-                const std::vector<int>& ptr = upper ? ulvl_ptr : lvl_ptr;
-                std::vector<int>& ord = upper ? ulvl_rows : lvl_rows;
-                auto begin = [&](int i) { return upper ? lu_diag[i] + 1 : lu_ptr[i]; };
-                auto length = [&](int i) {
-                    return upper ? lu_ptr[i + 1] - lu_diag[i] - 1 : lu_diag[i] - lu_ptr[i];
-                };
-                first[upper].push_back(0);
-                const int g0 = upper ? blk_ulvl[b] : blk_lvl[b], g1 = upper ? blk_ulvl[b + 1] : blk_lvl[b + 1];
-                for (int g = g0; g < g1; ++g) {
-                    std::stable_sort(ord.begin() + ptr[g], ord.begin() + ptr[g + 1],
-                                     [&](int x, int y) { return length(x) > length(y); });
-                    for (int q = ptr[g]; q < ptr[g + 1]; q += 32) {
-                        const int w = length(ord[q]), at = 32 * start.back();
-                        for (int l = 0; l < 32; ++l) {
-                            const int i = q + l < ptr[g + 1] ? ord[q + l] : -1;
-                            if (i >= 0 && upper) up[i] = (int)rows[1].size();
-                            rows[upper].push_back(i < 0 ? (int)kIluNoRow : i - r0);
-                            for (int k = 0; i >= 0 && k < length(i); ++k) spos[begin(i) + k] = at + 32 * k + l;
-                        }
-                        start.push_back(start.back() + w);
-                    }
-                    first[upper].push_back((int)rows[upper].size() / 32);
-                }
-            }
-            B.dp = start.back();
-            if (B.dp > 65535) throw Error("block-ILU: block too large");
-            B.nsl = (int)rows[0].size() / 32;
-            B.nsu = (int)rows[1].size() / 32;
-            bcol[b].assign(32 * (size_t)B.dp, (unsigned short)nr);
-            for (int i = r0; i < r1; ++i) {
-                for (int p = lu_ptr[i]; p < lu_ptr[i + 1]; ++p)
-                    if (p != lu_diag[i]) bcol[b][spos[p]] = lu_col[p];
-                spos[lu_diag[i]] = 32 * B.dp + i - r0;
-            }
-            bcol[b].resize(ilu_columns(B.dp), 0);
-            for (const std::vector<int>* v : {&first[0], &first[1], &start, &rows[0], &rows[1]})
-                bmeta[b].insert(bmeta[b].end(), v->begin(), v->end());
-            bmeta[b].resize(ilu_meta_words(B.nl, B.nu, B.nsl, B.nsu), 0);
-            B.mw = (int)bmeta[b].size();
+            blk[b] = ilu_layout(bstart[b], bstart[b + 1], lu_ptr, lu_diag, lu_col,
+                                {lvl_ptr, lvl_rows, blk_lvl[b], blk_lvl[b + 1]},
+                                {ulvl_ptr, ulvl_rows, blk_ulvl[b], blk_ulvl[b + 1]}, at, bmeta[b], bcol[b]);
+            blk[b].seg = blk_lvl[b];
         }
     });
+    const std::vector<int>& spos = at.entry;
     std::vector<unsigned short> meta, scol;
     size_t nlu = 0;
     for (int b = 0; b < nb; ++b) {
         blk[b].v0 = (int)nlu;
         blk[b].c0 = (int)scol.size();
         blk[b].mo = (int)meta.size();
-        nlu += ilu_window(bstart[b + 1] - bstart[b], blk[b].dp);
+        nlu += ilu_window(bstart[b + 1] - bstart[b], blk[b].ds);
         scol.insert(scol.end(), bcol[b].begin(), bcol[b].end());
         meta.insert(meta.end(), bmeta[b].begin(), bmeta[b].end());
         if (nlu >= (size_t)INT32_MAX || scol.size() >= (size_t)INT32_MAX || meta.size() >= (size_t)INT32_MAX)
@@ -1337,10 +1341,10 @@ static void build_pattern(fvm_ctx* c, BlockILU* P) {
             for (int g = blk_lvl[b]; g < blk_lvl[b + 1]; ++g) {
                 const int q0 = lvl_ptr[g], q1 = lvl_ptr[g + 1];
                 const size_t head = u.size();
-                u.resize(head + (q1 - q0 + 31) / 32 * 32, 0u);
+                u.resize(head + at.lower[lvl_rows[q1 - 1]] / kIluGroup * kIluGroup + kIluGroup, 0u);
                 for (int q = q0; q < q1; ++q) {
                     const int i = lvl_rows[q];
-                    u[head + (q - q0)] = (unsigned)(u.size() - head);
+                    u[head + at.lower[i]] = (unsigned)(u.size() - head);
                     for (int p = lu_ptr[i]; p < lu_diag[i]; ++p) {
                         const size_t cw = u.size();
                         u.push_back(0u);
@@ -1371,16 +1375,24 @@ static void build_pattern(fvm_ctx* c, BlockILU* P) {
         seg_ptr[g + 1] += seg_ptr[g];
     }
     {
-        size_t need64 = 0, need32 = 0;
-        bool fits16 = true;
+        size_t need64 = 0, need32 = 0, exact64 = 0, exact32 = 0;
+        bool fits16 = true, exact16 = true;
         for (int b = 0; b < nb; ++b) {
-            const size_t nr = bstart[b + 1] - bstart[b], dp = blk[b].dp;
+            const size_t nr = bstart[b + 1] - bstart[b], ds = blk[b].ds;
             // the schedule's window positions and the columns are 16-bit words
-            if (ilu_window(nr, dp) >= 65536 || nr + 1 >= 65535) fits16 = false;
+            if (ilu_window(nr, ds) >= 65536 || nr + 1 >= 65535) fits16 = false;
             for (size_t sz : {(size_t)8, (size_t)4}) {
-                const size_t need = ilu_stage_bytes(nr, dp, blk[b].mw, sz);
+                const size_t need = ilu_stage_bytes(nr, ds, blk[b].mw, sz);
                 if (sz == 8) need64 = std::max(need64, need);
                 else need32 = std::max(need32, need);
+                // rows end to end: vector, values, 16-bit columns; row pointers, pivots'
+                // places, rows of the two sweeps and their levels' ends; mbarrier
+                const size_t nnz = (size_t)(lu_ptr[bstart[b + 1]] - lu_ptr[bstart[b]]);
+                const size_t words = 4 * nr + (size_t)blk[b].nl + blk[b].nu + 3;
+                const size_t e = round16(round16(nr * sz) + nnz * (sz + 2) + round16(2 * words)) + 16;
+                if (nnz >= 65535 || nr + 1 >= 65535) exact16 = false;
+                if (sz == 8) exact64 = std::max(exact64, e);
+                else exact32 = std::max(exact32, e);
             }
         }
         P->smem_stage[0] = (fits16 && need64 <= kMaxDynSmem) ? need64 : 0;
@@ -1416,27 +1428,10 @@ static void build_pattern(fvm_ctx* c, BlockILU* P) {
             raise_smem_limit(k_ilu_apply_smem<float>, P->smem_stage[1]);
             raise_smem_limit(k_ilu_factor_smem<float>, (size_t)(round16(P->smem_stage[1]) + 8 * (size_t)P->scr_words[1]));
         }
-    }
-    if (schur) {
-        // the coupled apply keeps each block's staged factor plus the
-        // forward result in shared memory through its grid barriers, so it
-        // needs both to fit and every block resident at once
-        int nsm2 = 148, coop = 0;
-        FVM_CUDA(cudaDeviceGetAttribute(&nsm2, cudaDevAttrMultiProcessorCount, c->device));
-        FVM_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, c->device));
-        for (int pr = 0; pr < 2; ++pr) {
-            P->schur_smem[pr] = 0;
-            if (!P->smem_stage[pr] || !coop) continue;
-            const size_t sz = pr ? sizeof(float) : sizeof(double);
-            const size_t need = round16(P->smem_stage[pr]) + round16(sz * (size_t)maxb);
-            if (need > kMaxDynSmem) continue;
-            const void* kfn = schur_kernel(pr);
-            raise_smem_limit(kfn, need);
-            int per_sm = 0;
-            FVM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kfn, P->apply_threads, need));
-            if ((long)per_sm * nsm2 >= nb) P->schur_smem[pr] = need;
+        if (schur) {
+            schur_layout(c, P, 0, exact16 && exact64 <= kMaxDynSmem ? exact64 : 0);
+            schur_layout(c, P, 1, exact16 && exact32 <= kMaxDynSmem ? exact32 : 0);
         }
-        P->schur_nrmax = maxb;
     }
     cudaStream_t s = c->stream;
     if (schur) {
@@ -1507,7 +1502,7 @@ static void build_pattern(fvm_ctx* c, BlockILU* P) {
         FVM_CUDA(cudaStreamSynchronize(s));
     }
     P->blk.upload(blk, s);
-    if (!P->smem_stage[0] || !P->smem_stage[1]) P->lu_up.upload(up, s);
+    if (!P->smem_stage[0] || !P->smem_stage[1]) P->lu_up.upload(at.upper, s);
     P->lu_row.upload(lu_row, s);
     P->lu_col.upload(scol, s);
     if (upd.empty()) upd.push_back(0u);
@@ -1661,7 +1656,7 @@ void psolve_dev(fvm_ctx* c, const double* r, double* z, const int* skip) {
     } end_timer{c};
     if (P->schur_iters >= 0) {
         if (!P->schur_smem[P->factored])
-            throw Error("psolve: the Schur coupling needs every block's staged factor and forward result in shared "
+            throw Error("psolve: the Schur coupling needs every block's factor and forward result in shared "
                         "memory with all blocks resident at once (use the FP32 factor on large blocks)");
         if (P->factored) launch_schur_apply(c, P, P->lu32.p, r, z, skip);
         else launch_schur_apply(c, P, P->lu64.p, r, z, skip);
