@@ -833,16 +833,18 @@ bool fused_prepare(fvm_ctx* c, int m) {
     return true;
 }
 
-// one cycle from U_0 and its squared norm (K->res[0]); runs until convergence, a
-// full basis or a breakdown, and leaves the state and the coefficients
-void fused_cycle(fvm_ctx* c, Krylov* K, double cj, double tol, const double* ewt, double* H_d, double* coef) {
+// one cycle of at most m steps (the dimension that fused_prepare was asked for; the
+// workspace K may be a larger one's) from U_0 and its squared norm (K->res[0]);
+// runs until convergence, a full basis or a breakdown, and leaves the state and
+// the coefficients
+void fused_cycle(fvm_ctx* c, Krylov* K, int m, double cj, double tol, const double* ewt, double* H_d, double* coef) {
     BlockILU* P = c->ilu;
     cudaStream_t s = c->stream;
     float* U = reinterpret_cast<float*>(K->U);
     if (K->tdir.n < (size_t)c->N) K->tdir.alloc(c->N);
     FusedArgs a;
     a.N = c->N;
-    a.m = K->m;
+    a.m = m;
     a.nr_max = P->fused_nrmax;
     a.nqp = P->fused_nqp;
     a.nh_max = P->fused_nhmax;
@@ -883,7 +885,7 @@ void fused_cycle(fvm_ctx* c, Krylov* K, double cj, double tol, const double* ewt
     cfg.gridDim = dim3(P->nb);
     cfg.blockDim = dim3(P->fused_threads);
     const int var = fused_variant(c);
-    cfg.dynamicSmemBytes = fused_bytes(P, var, K->m);
+    cfg.dynamicSmemBytes = fused_bytes(P, var, m);
     cfg.stream = s;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeCooperative;

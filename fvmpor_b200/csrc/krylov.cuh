@@ -98,7 +98,7 @@ bool schur_active(fvm_ctx* c);          // the Schur-coupled apply is on
 // fused_cycle runs one cycle from the state gmres has put in place
 bool fused_prepare(fvm_ctx* c, int m);
 void fused_reset(fvm_ctx* c);   // after a failed cycle
-void fused_cycle(fvm_ctx* c, Krylov* K, double cj, double tol, const double* ewt, double* H_d, double* coef);
+void fused_cycle(fvm_ctx* c, Krylov* K, int m, double cj, double tol, const double* ewt, double* H_d, double* coef);
 bool ilu_ready(fvm_ctx* c);
 const int* ilu_status_dev(fvm_ctx* c);   // the status word on the device
 int ilu_status(fvm_ctx* c);   // 0 ok, 1 zero pivot in the last factorisation

@@ -537,7 +537,7 @@ static int gmres_impl(fvm_ctx* c, Krylov* K, double cj, const double* y, const d
         if (fused) {
             ArnState* hst = reinterpret_cast<ArnState*>(K->host + 4 * (m + 2) + 8);
             double* coef = K->res.p + 1;   // (m + 2) values follow the squared norm
-            fused_cycle(c, K, cj, tol, ewt, K->ls.p, coef);
+            fused_cycle(c, K, m, cj, tol, ewt, K->ls.p, coef);
             fvm_launch_pdl(c, k_combine_dev<B>, grid_for(N, 256), 256, 0, s, N, K->st.p, U, ld, coef, ewt, x,
                            have_x ? 0 : 1);
             have_x = true;
