@@ -98,8 +98,8 @@ __device__ __forceinline__ unsigned atom_add_release_gpu(unsigned* p, unsigned v
 // of the grid size.  Its own arrival number says which multiple, so there is
 // no generation word, no reset and no further step for the last block to
 // arrive.  A block that gives up, or meets an error elsewhere, sets
-// kSyncFail (far above any count of one launch): every block sees it at its
-// next barrier and leaves, and err carries the reason to the host.
+// kSyncFail (above any count, fused_cycle): every block sees it at its next
+// barrier and leaves, and err carries the reason to k_combine_dev.
 constexpr unsigned kSyncFail = 1u << 30;
 __device__ __forceinline__ void fused_fail(unsigned* sync, int* err, int code) {
     atomicExch(err, code);
@@ -894,8 +894,10 @@ void fused_cycle(fvm_ctx* c, Krylov* K, int m, double cj, double tol, const doub
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 2;
-    // a launch takes at most 64 flag values and 64 barriers
-    if (P->fused_launches >= (1u << 29) / (64u * (unsigned)P->nb)) fused_reset(c);
+    // a launch takes at most 64 flag values (the last one published is m + 1) and
+    // 128 barriers (CGS2: two per step); the counter has to stay below kSyncFail
+    static_assert(kFusedMaxDim + 1 < 64, "flag values and barriers of a launch");
+    if (P->fused_launches >= kSyncFail / (128u * (unsigned)P->nb)) fused_reset(c);
     a.base = 64u * P->fused_launches++;
     c->tm.begin(TM_CGS, s);
     if (var) FVM_CUDA(cudaLaunchKernelEx(&cfg, k_arnoldi_fused<true>, a));

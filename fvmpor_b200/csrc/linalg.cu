@@ -323,16 +323,21 @@ __global__ void k_combine(int N, int nv, const B* __restrict__ U, size_t ld,
     x[k] += acc / ewt[k];
 }
 
-// r~ = ewt * (b - Jx) (Jx may be null -> b); U_0 = r~; out = ||r~||^2
 // the same with what a fused cycle left: its number of columns (none after a
-// failure or breakdown) and their coefficients; set instead of added to first
+// failure or breakdown) and their coefficients; set instead of added to first.
+// The cycle failed if any of its blocks gave up a wait, also in the last step
+// after block 0 had found it converged: done is 0 then, for what is queued
+// behind and for the host.
 template <class B>
-__global__ void k_combine_dev(int N, const ArnState* __restrict__ st, const B* __restrict__ U, size_t ld,
+__global__ void k_combine_dev(int N, ArnState* st, const int* __restrict__ err, const B* __restrict__ U, size_t ld,
                               const double* __restrict__ ys, const double* __restrict__ ewt, double* __restrict__ x,
                               int first) {
     pdl_wait_and_trigger();
     __shared__ double coef[64];
-    const int done = st->done, nv = done == 1 || done == 2 ? st->j : 0;
+    const bool failed = *err != 0;
+    if (failed && blockIdx.x == 0 && threadIdx.x == 0) st->done = 0;
+    // (the other blocks may read done before or after that)
+    const int done = failed ? 0 : st->done, nv = done == 1 || done == 2 ? st->j : 0;
     for (int i = threadIdx.x; i < nv; i += blockDim.x) coef[i] = ys[i];
     __syncthreads();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
@@ -344,6 +349,7 @@ __global__ void k_combine_dev(int N, const ArnState* __restrict__ st, const B* _
     x[k] = first ? acc : x[k] + acc;
 }
 
+// r~ = ewt * (b - Jx) (Jx may be null -> b); U_0 = r~; out = ||r~||^2
 template <class B>
 __global__ void k_init_residual(int N, const double* __restrict__ b, const double* __restrict__ Jx,
                                 const double* __restrict__ ewt, B* __restrict__ U0, double* partial,
@@ -538,7 +544,7 @@ static int gmres_impl(fvm_ctx* c, Krylov* K, double cj, const double* y, const d
             ArnState* hst = reinterpret_cast<ArnState*>(K->host + 4 * (m + 2) + 8);
             double* coef = K->res.p + 1;   // (m + 2) values follow the squared norm
             fused_cycle(c, K, m, cj, tol, ewt, K->ls.p, coef);
-            fvm_launch_pdl(c, k_combine_dev<B>, grid_for(N, 256), 256, 0, s, N, K->st.p, U, ld, coef, ewt, x,
+            fvm_launch_pdl(c, k_combine_dev<B>, grid_for(N, 256), 256, 0, s, N, K->st.p, K->err.p, U, ld, coef, ewt, x,
                            have_x ? 0 : 1);
             have_x = true;
             if (tail && cycle == 0) tail->queue(&K->st.p->done);

@@ -1,7 +1,12 @@
 """The fused GMRES cycle (assembled FP32 operator, blocks resident in shared
 memory) over the calls of one context: the dimension is the call's own, whatever
 workspace an earlier call has left, also where only the smaller one's cycle fits
-the shared memory."""
+the shared memory; and a cycle in which a wait ran out after it had converged
+fails by itself and leaves nothing to the next one."""
+import os
+import shutil
+import subprocess
+
 import numpy as np
 import pytest
 import torch
@@ -9,6 +14,8 @@ import torch
 import fvmpor_b200 as fb
 
 pytestmark = pytest.mark.gpu
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
 def box(nx, ny, nz):
@@ -48,3 +55,13 @@ def test_dimension_is_the_call_s_own(nx, ny, nz, per_sm, first, then, variant, c
         ph.close()
     assert out[0][1]["nli"] == out[1][1]["nli"]
     assert np.array_equal(out[0][0], out[1][0])
+
+
+def test_late_failure_is_seen_when_it_happens(cuda, tmp_path):
+    exe, lib = tmp_path / "late_failure_check", os.path.join(ROOT, "fvmpor_b200")
+    nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+    subprocess.run([nvcc, "-gencode", "arch=compute_100a,code=sm_100a", "-std=c++17", "--expt-relaxed-constexpr",
+                    "-I", os.path.join(lib, "csrc"), os.path.join(ROOT, "tests", "late_failure_check.cu"), "-o", str(exe),
+                    "-L", lib, "-lfvmpor_b200", "-Xlinker", "-rpath=" + lib], check=True)
+    r = subprocess.run([str(exe)], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, r.stdout + r.stderr
