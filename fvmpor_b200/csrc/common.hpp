@@ -11,7 +11,6 @@
 #include <mutex>
 #include <stdexcept>
 #include <string>
-#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -54,10 +53,12 @@ template <class F> void parallel_for(long n, long grain, F&& body) {
         }
     };
     std::vector<std::thread> pool;
+    pool.reserve(threads - 1);
     try {
         for (long t = 1; t < threads; ++t) pool.emplace_back(work);
-    } catch (const std::system_error&) {
-        // fewer threads than asked for: those there are do the work
+    } catch (...) {
+        // no thread or no memory for one: those there are do the work (leaving
+        // here with threads still running would end the process)
     }
     work();
     for (std::thread& t : pool) t.join();
