@@ -290,12 +290,25 @@ inline void fvm_launch(fvm_ctx* c, void (*k)(KArgs...), dim3 grid, dim3 block, s
     c->launches++;
 }
 
-// Programmatic dependent launch for the short kernels of the Krylov step
-// (node pass, element pass, gather, preconditioner apply): the launch may
+// Programmatic dependent launch for the short kernels of a step: the launch may
 // be processed, and the kernel's blocks made resident, while the previous
-// kernel on the stream finishes.  Every kernel launched this way calls
-// pdl_wait_and_trigger() first, so it reads nothing before its predecessor
-// has completed and its writes are visible.
+// kernel on the stream finishes.  The rule for every kernel launched this way:
+//   - it waits (griddepcontrol.wait: its predecessor has completed and its writes
+//     are visible) before it lets the next one start, and before it writes
+//     anything in global memory;
+//   - before that wait it reads only set-up data and what was complete before its
+//     predecessor could start: data written at least one waiting kernel, or
+//     one copy, earlier.  Never what the kernel directly ahead writes, also if
+//     that one is the caller's.
+// What is read early, and what must lie between it and its writer:
+//   k_elem_chunk: the step's upwind flags; the node pass
+//   k_ilu_apply_smem, k_ilu_apply_schur: the factor; the copy of the status word
+//     (psetup_dev)
+//   k_arnoldi_fused: the factor and the error weights; the apply and
+//     k_init_residual
+//   k_mlp_train: the samples; the batch before (an epoch's first batch is an
+//     ordinary launch)
+//   k_gather, k_upwind_chunk: set-up data only.
 template <typename... KArgs, typename... Args>
 inline void fvm_launch_pdl(fvm_ctx* c, void (*k)(KArgs...), dim3 grid, dim3 block, size_t smem,
                            cudaStream_t s, Args&&... args) {
@@ -313,15 +326,15 @@ inline void fvm_launch_pdl(fvm_ctx* c, void (*k)(KArgs...), dim3 grid, dim3 bloc
     c->launches++;
 }
 
-// first statement of a kernel launched by fvm_launch_pdl: wait for the
-// previous kernel's completion (a no-op after an ordinary launch), then let
-// the next programmatic launch begin
 // the host waits for the context's stream (counted: fvm_stats.nsync)
 inline void ctx_sync(fvm_ctx* c) {
     c->n_syncs++;
     FVM_CUDA(cudaStreamSynchronize(c->stream));
 }
 
+// in a kernel launched by fvm_launch_pdl: wait for the previous kernel's
+// completion (a no-op after an ordinary launch), then let the next
+// programmatic launch begin
 __device__ __forceinline__ void pdl_wait_and_trigger() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

@@ -520,7 +520,8 @@ __global__ void __launch_bounds__(kIluThreads, 3) k_ilu_apply_smem(const int* __
     // right-hand side by the threads meanwhile.  The copies read only set-up
     // data, so they are issued before the wait for the previous kernel (the
     // factorisation has completed before any kernel that lets this launch
-    // start early); the right-hand side and the skip flag are read after it.
+    // start early: the copy of the status word lies between, psetup_dev); the
+    // right-hand side and the skip flag are read after it.
     ilu_stage_bulk(S, B, nr, lu, lu_col, meta);
     // the nodes of the thread's rows, for the way in and the way out: set-up data
     // too, and with them at hand the right-hand side is one round of loads
@@ -1608,6 +1609,8 @@ void psetup_dev(fvm_ctx* c, double cj, double h, const double* y, const double* 
     if (precision) factor(P->lu32, P->Jw32.p);
     else factor(P->lu64, P->Jw.p);
     c->tm.end(TM_ILU_FACTOR, s);
+    // (also what keeps an apply's early reads of the factor behind the kernel above,
+    // which lets its successor start before it factors: fvm_launch_pdl)
     FVM_CUDA(cudaMemcpyAsync(P->h_status, P->status.p, sizeof(int), cudaMemcpyDeviceToHost, s));
     P->factored = precision;
 }

@@ -422,8 +422,8 @@ __global__ void __launch_bounds__(kTrainThreads, 1) k_mlp_train(const float* __r
         mbar_init(s.bar, 1);
         asm volatile("fence.mbarrier_init.release.cluster;");
     }
-    // the samples do not come from the kernel ahead (the last batch's step), the
-    // parameters do
+    // the samples do not come from the kernel ahead (the last batch's step; an
+    // epoch's first batch has none, train_pass), the parameters do
     const long first = (long)blockIdx.x * tiles_per_cta;
     float4 f = load_features(X, begin + first * kTile, end);
     pdl_wait_and_trigger();
@@ -816,15 +816,21 @@ void recorder_push(fvm_ctx* c, Recorder* r, const float* Xall, const double* y_n
     r->step++;
 }
 
-// gradient of the rows [begin, end) and, where the step names the parameters, one Adam step
-static void train_pass(fvm_ctx* c, Predictor* p, const float* X, const float* Y, long begin, long end, AdamArgs step) {
+// gradient of the rows [begin, end) and, where the step names the parameters, one Adam
+// step; chained: the kernel ahead on the stream is another batch's step (else
+// it may be the one that writes X, which the training kernel reads early)
+static void train_pass(fvm_ctx* c, Predictor* p, const float* X, const float* Y, long begin, long end, AdamArgs step,
+                       bool chained) {
     long ntiles = (end - begin + kTile - 1) / kTile;
     int nblk = (int)std::min<long>(ntiles, 148);
     long per = (ntiles + nblk - 1) / nblk;
     nblk = (int)((ntiles + per - 1) / per);
     if ((long)p->partial.n < (long)nblk * kPartial) p->partial.alloc((size_t)nblk * kPartial);
-    fvm_launch_pdl(c, k_mlp_train, nblk, kTrainThreads, mlp_smem_bytes(true), c->stream, X, Y, begin, end, per, p->p.p,
-                   p->wl.p, p->partial.p, p->err.p);
+    auto launch = [&](auto&&... args) {
+        if (chained) fvm_launch_pdl(c, k_mlp_train, nblk, kTrainThreads, mlp_smem_bytes(true), c->stream, args...);
+        else fvm_launch(c, k_mlp_train, nblk, kTrainThreads, mlp_smem_bytes(true), c->stream, args...);
+    };
+    launch(X, Y, begin, end, per, p->p.p, p->wl.p, p->partial.p, p->err.p);
     fvm_launch_pdl(c, k_grad_step, (kNTrain + 32) / 32, 32 * kSumGroups, 0, c->stream, p->partial.p, nblk, p->gsum.p,
                    step);
 }
@@ -892,7 +898,7 @@ extern "C" int fvm_mlp_grad(fvm_ctx* c, const float* X, const float* Y, int n, f
                             float* loss) {
     API_TRY
     if (!c || !X || !Y || !c->pred) throw Error("fvm_mlp_grad: no predictor or null argument");
-    train_pass(c, c->pred, X, Y, 0, n, AdamArgs{});
+    train_pass(c, c->pred, X, Y, 0, n, AdamArgs{}, false);
     std::vector<float> g(kNTrain + 1);
     FVM_CUDA(cudaMemcpyAsync(g.data(), c->pred->gsum.p, sizeof(float) * (kNTrain + 1), cudaMemcpyDeviceToHost,
                              c->stream));
@@ -918,7 +924,8 @@ extern "C" int fvm_mlp_train(fvm_ctx* c, const float* X, const float* Y, int n, 
             p->adam_t++;
             const float bc1 = 1.0f - std::pow(b1, (float)p->adam_t), bc2 = 1.0f - std::pow(b2, (float)p->adam_t);
             train_pass(c, p, X, Y, b0, std::min<long>(n, b0 + batch),
-                       AdamArgs{lr, b1, b2, eps, bc1, bc2, p->p.p, p->m.p, p->v.p, p->wl.p, p->losses.p + b0 / batch});
+                       AdamArgs{lr, b1, b2, eps, bc1, bc2, p->p.p, p->m.p, p->v.p, p->wl.p, p->losses.p + b0 / batch},
+                       b0 > 0);
         }
         FVM_CUDA(cudaMemcpyAsync(loss.data(), p->losses.p, sizeof(float) * nbatch, cudaMemcpyDeviceToHost, c->stream));
         FVM_CUDA(cudaStreamSynchronize(c->stream));
