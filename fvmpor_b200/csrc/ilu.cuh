@@ -105,8 +105,6 @@ struct BlockILU {
     bool schur_staged[2] = {false, false};   // its factor in shared memory, or read in place
 };
 
-// largest dynamic shared-memory carve-out a CTA may request on sm_100
-constexpr size_t kMaxDynSmem = 227 * 1024;
 // threads of a staged triangular-solve CTA: levels hold a few dozen rows,
 // so a small CTA keeps the per-level barrier cheap
 constexpr int kIluThreads = 256;   // largest CTA of the staged apply
@@ -142,19 +140,26 @@ template <class T> struct IluShared {
     __device__ __forceinline__ unsigned col(int i) const {
         return reinterpret_cast<const unsigned short*>(ilu_smem() + oc)[i];
     }
+    // the vector's value for a column; the padding's column is nr, a slot of its own
+    static __device__ __forceinline__ T x(unsigned c) { return reinterpret_cast<const T*>(ilu_smem())[c]; }
 };
-// ... or read in place
+// ... or read in place, where the vector may fill the shared memory to the last
+// value and has no such slot
 template <class T> struct IluGlobal {
     const T* v;
     const unsigned short *c, *m;
     int nl, nu, ngl, ngu, nwide, ds;
+    unsigned nr;
+    __device__ __forceinline__ T x(unsigned c) const { return c < nr ? reinterpret_cast<const T*>(ilu_smem())[c] : (T)0; }
     __device__ __forceinline__ unsigned meta(int i) const { return m[i]; }
     __device__ __forceinline__ unsigned meta2(int i) const { return *reinterpret_cast<const unsigned*>(m + i); }
     __device__ __forceinline__ T val(int i) const { return v[i]; }
     __device__ __forceinline__ unsigned col(int i) const { return c[i]; }
 };
-template <class V, class A, class C, class M> __device__ __forceinline__ V ilu_view(const IluBlk& B, A v, C c, M m) {
-    return V{v, c, m, B.nl, B.nu, B.ngl, B.ngu, B.nwide, B.ds};
+template <class T>
+__device__ __forceinline__ IluGlobal<T> ilu_in_place(const IluBlk& B, int nr, const T* v, const unsigned short* c,
+                                                     const unsigned short* m) {
+    return IluGlobal<T>{v + B.v0, c + B.c0, m + B.mo, B.nl, B.nu, B.ngl, B.ngu, B.nwide, B.ds, (unsigned)nr};
 }
 // the record's parts (ilu_meta_words); g counts a sweep's groups from 0
 template <class V> __device__ __forceinline__ int ilu_level(const V& f, bool upper, int l) {
@@ -215,7 +220,7 @@ template <class T> struct IluStage {
         bar = reinterpret_cast<uint64_t*>(smem + om + 2u * B.mw);
     }
     __device__ __forceinline__ IluShared<T> view(const IluBlk& B) const {
-        return ilu_view<IluShared<T>>(B, ov, oc, om);
+        return IluShared<T>{ov, oc, om, B.nl, B.nu, B.ngl, B.ngu, B.nwide, B.ds};
     }
 };
 
@@ -280,14 +285,14 @@ __device__ __forceinline__ void ilu_fetch(IluLane& R, const V& f, int lane, int 
 
 // acc += entries [k, w) of a row, the first kIluWide of a wide one
 template <class T, class V>
-__device__ __forceinline__ void ilu_rest(T& acc, const T* x, const V& f, int at, int w, int k) {
+__device__ __forceinline__ void ilu_rest(T& acc, const V& f, int at, int w, int k) {
     w = min(w, kIluWide);
 #pragma unroll 1
     for (; k < w; k += 4) {
         T v[4], xv[4];
 #pragma unroll
         for (int t = 0; t < 4; ++t) {
-            xv[t] = x[f.col(at + 32 * (k + t))];
+            xv[t] = f.x(f.col(at + 32 * (k + t)));
             v[t] = f.val(at + 32 * (k + t));
         }
 #pragma unroll
@@ -296,9 +301,9 @@ __device__ __forceinline__ void ilu_rest(T& acc, const T* x, const V& f, int at,
     }
 }
 // ... and the others
-template <class T, class V> __device__ __forceinline__ T ilu_wide_rest(T acc, const T* x, const V& f, bool upper, int g) {
+template <class T, class V> __device__ __forceinline__ T ilu_wide_rest(T acc, const V& f, bool upper, int g) {
     const int2 t = ilu_wide(f, upper, g);
-    for (int k = 0; k < t.y - kIluWide; ++k) acc += f.val(t.x + k) * x[f.col(t.x + k)];
+    for (int k = 0; k < t.y - kIluWide; ++k) acc += f.val(t.x + k) * f.x(f.col(t.x + k));
     return acc;
 }
 
@@ -328,7 +333,7 @@ __device__ __forceinline__ void ilu_sweep(const V& f, int l0, int l1) {
             T xv[kIluPre], v[kIluPre];
 #pragma unroll
             for (int k = 0; k < kIluPre; ++k) {
-                xv[k] = x[cur.c[k]];
+                xv[k] = f.x(cur.c[k]);
                 v[k] = f.val(cur.at + 32 * k);
             }
             const bool act = cur.row != kIluNoRow;
@@ -339,8 +344,8 @@ __device__ __forceinline__ void ilu_sweep(const V& f, int l0, int l1) {
 #pragma unroll
             for (int k = 0; k < kIluPre; ++k)
                 if (k < cur.w) acc += v[k] * xv[k];
-            ilu_rest(acc, x, f, cur.at, cur.w, kIluPre);
-            if (cur.w > kIluWide && act) acc = ilu_wide_rest(acc, x, f, UPPER, s0 + mine);
+            ilu_rest(acc, f, cur.at, cur.w, kIluPre);
+            if (cur.w > kIluWide && act) acc = ilu_wide_rest(acc, f, UPPER, s0 + mine);
             if (act) x[row] = UPPER ? (xi - acc) * piv : xi - acc;
             // slices of a level with more of them than the CTA has warps
 #pragma unroll 1
@@ -350,9 +355,9 @@ __device__ __forceinline__ void ilu_sweep(const V& f, int l0, int l1) {
                 const int w = (int)(word & ((1u << kIluWidthBits) - 1u));
                 const int i = g < s1 ? ilu_row(f, UPPER, gi, j) : kIluNoRow;
                 T a = (T)0;
-                ilu_rest(a, x, f, (int)(word >> kIluWidthBits) + j, w, 0);
+                ilu_rest(a, f, (int)(word >> kIluWidthBits) + j, w, 0);
                 if (i != kIluNoRow) {
-                    if (w > kIluWide) a = ilu_wide_rest(a, x, f, UPPER, g);
+                    if (w > kIluWide) a = ilu_wide_rest(a, f, UPPER, g);
                     x[i] = UPPER ? (x[i] - a) * f.val(f.ds + i) : x[i] - a;
                 }
             }

@@ -77,6 +77,13 @@ FVM_HD size_t ilu_stage_bytes(size_t nr, size_t ds, size_t mw, size_t sz) {
     return need > reach ? need : round16(reach);
 }
 
+// shared bytes of a block's vector where the factor is read in place: no slot for
+// the padding's column (IluGlobal::x)
+FVM_HD size_t ilu_plain_bytes(size_t nr, size_t sz) { return nr * sz; }
+
+// largest dynamic shared-memory carve-out a CTA may request on sm_100
+constexpr size_t kMaxDynSmem = 227 * 1024;
+
 // the levels of one sweep: block's are [first, last), level g's rows
 // rows[ptr[g]] .. rows[ptr[g + 1] - 1]
 struct IluLevels {

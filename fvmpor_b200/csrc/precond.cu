@@ -426,7 +426,7 @@ __global__ void __launch_bounds__(128) k_ilu_factor(const int* __restrict__ bsta
     T* val = lu + B.v0;
     for (long p = threadIdx.x; p < wn; p += blockDim.x) val[p] = Jw[B.v0 + p];
     __syncthreads();
-    const auto V = ilu_view<IluGlobal<T>>(B, val, lu_col + B.c0, meta + B.mo);
+    const auto V = ilu_in_place<T>(B, nr, lu, lu_col, meta);
     const int D = B.ds;
     for (int l = 0; l < B.nl; ++l) {
         const int q1 = kIluGroup * ilu_level(V, false, l + 1);
@@ -485,9 +485,8 @@ __global__ void __launch_bounds__(128) k_ilu_apply(const int* __restrict__ bstar
     const IluBlk B = blk[blockIdx.x];
     const int r0 = bstart[blockIdx.x], nr = bstart[blockIdx.x + 1] - r0;
     for (int i = threadIdx.x; i < nr; i += blockDim.x) x[i] = (T)r[lu_row[r0 + i]];
-    if (threadIdx.x == 0) x[nr] = (T)0;
     __syncthreads();
-    const auto V = ilu_view<IluGlobal<T>>(B, lu + B.v0, lu_col + B.c0, meta + B.mo);
+    const auto V = ilu_in_place(B, nr, lu, lu_col, meta);
     // level 0 of the lower sweep has no off-diagonal entries
     ilu_sweep<T, false>(V, 1, V.nl);
     ilu_sweep<T, true>(V, 0, V.nu);
@@ -637,7 +636,7 @@ __global__ void __launch_bounds__(kIluThreads, sizeof(T) == 4 ? 4 : 3) k_ilu_app
         return;
     }
     for (int i = threadIdx.x; i < nr; i += blockDim.x) x[i] = (T)a.r[a.lu_row[r0 + i]];
-    if (threadIdx.x == 0) x[nr] = (T)0;
+    if (STAGED && threadIdx.x == 0) x[nr] = (T)0;
     bool ok = true;
     if constexpr (STAGED) ok = tc05::mbar_wait(mbar, 0) || tc05::mbar_wait(mbar, 0);
     const bool good = __syncthreads_and(ok ? 1 : 0) != 0;
@@ -645,7 +644,7 @@ __global__ void __launch_bounds__(kIluThreads, sizeof(T) == 4 ? 4 : 3) k_ilu_app
     const int lvB = a.sch_lv[2 * b], uvS = a.sch_lv[2 * b + 1], nin = a.sch_nin[b];
     const auto V = [&] {
         if constexpr (STAGED) return S.view(B);
-        else return ilu_view<IluGlobal<T>>(B, a.lu + B.v0, a.lu_col + B.c0, a.meta + B.mo);
+        else return ilu_in_place(B, nr, a.lu, a.lu_col, a.meta);
     }();
     if (good) {
         ilu_sweep<T, false>(V, 1, V.nl);
@@ -713,7 +712,7 @@ static void schur_layout(const fvm_ctx* c, BlockILU* P, int pr, size_t exact) {
         return (long)per_sm * nsm >= P->nb;
     };
     if (!exact || !resident(true, round16(exact) + fwd)) return;
-    const size_t staged = round16(P->smem_stage[pr]) + fwd, plain = round16(sz * ((size_t)P->maxb + 1)) + fwd;
+    const size_t staged = round16(P->smem_stage[pr]) + fwd, plain = round16(ilu_plain_bytes(P->maxb, sz)) + fwd;
     P->schur_staged[pr] = P->smem_stage[pr] && resident(true, staged);
     if (P->schur_staged[pr]) P->schur_smem[pr] = staged;
     else if (resident(false, plain)) P->schur_smem[pr] = plain;
@@ -725,7 +724,7 @@ static void launch_schur_apply(fvm_ctx* c, BlockILU* P, const T* lu, const doubl
     a.N = c->N;
     a.iters = P->schur_iters;
     const bool staged = P->schur_staged[P->factored];
-    a.stage_max = staged ? round16(P->smem_stage[P->factored]) : round16(sizeof(T) * ((size_t)P->maxb + 1));
+    a.stage_max = staged ? round16(P->smem_stage[P->factored]) : round16(ilu_plain_bytes(P->maxb, sizeof(T)));
     a.bstart = P->bstart.p;
     a.blk = P->blk.p;
     a.lu_col = P->lu_col.p;
@@ -1412,14 +1411,14 @@ static void build_pattern(fvm_ctx* c, BlockILU* P) {
         P->apply_threads = widest > 128 ? 256 : 128;
         // the global-memory apply keeps the block's vector in shared memory
         if (!P->smem_stage[0]) {
-            if (sizeof(double) * ((size_t)maxb + 1) > kMaxDynSmem)
+            if (ilu_plain_bytes(maxb, sizeof(double)) > kMaxDynSmem)
                 throw Error("block-ILU: blocks too large for the FP64 apply (set more blocks per SM)");
-            raise_smem_limit(k_ilu_apply<double>, sizeof(double) * ((size_t)maxb + 1));
+            raise_smem_limit(k_ilu_apply<double>, ilu_plain_bytes(maxb, sizeof(double)));
         }
         if (!P->smem_stage[1]) {
-            if (sizeof(float) * ((size_t)maxb + 1) > kMaxDynSmem)
+            if (ilu_plain_bytes(maxb, sizeof(float)) > kMaxDynSmem)
                 throw Error("block-ILU: blocks too large for the FP32 apply (set more blocks per SM)");
-            raise_smem_limit(k_ilu_apply<float>, sizeof(float) * ((size_t)maxb + 1));
+            raise_smem_limit(k_ilu_apply<float>, ilu_plain_bytes(maxb, sizeof(float)));
         }
         if (P->smem_stage[0]) {
             raise_smem_limit(k_ilu_apply_smem<double>, P->smem_stage[0]);
@@ -1671,7 +1670,7 @@ void psolve_dev(fvm_ctx* c, const double* r, double* z, const int* skip) {
             fvm_launch_pdl(c, staged, P->nb, P->apply_threads, sm, s, P->bstart.p, P->blk.p, P->lu_col.p, P->meta.p, lu,
                            P->lu_row.p, r, z, P->status.p, skip);
         else
-            fvm_launch_pdl(c, plain, P->nb, 128, sizeof(*lu) * ((size_t)P->maxb + 1), s, P->bstart.p, P->blk.p,
+            fvm_launch_pdl(c, plain, P->nb, 128, ilu_plain_bytes(P->maxb, sizeof(*lu)), s, P->bstart.p, P->blk.p,
                            P->lu_col.p, P->meta.p, lu, P->lu_row.p, r, z, skip);
     };
     if (P->factored) go(k_ilu_apply_smem<float>, k_ilu_apply<float>, P->lu32.p);

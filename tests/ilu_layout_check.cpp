@@ -23,6 +23,8 @@ int main(int argc, char** argv) {
     const int nr = std::atoi(argv[1]), per_row = std::atoi(argv[2]), hubs = std::atoi(argv[3]);
     const int hub_len = std::atoi(argv[4]), r0 = 3;   // (a block need not start at row 0)
     std::mt19937 rng(std::atoi(argv[5]));
+    // a block read in place may fill a CTA's shared memory to the last value
+    CHECK(ilu_plain_bytes(29056, 8) <= kMaxDynSmem && ilu_plain_bytes(58112, 4) <= kMaxDynSmem);
     std::vector<std::set<int>> adj(nr);
     auto couple = [&](int a, int b) { adj[a].insert(b); adj[b].insert(a); };
     for (int i = 0; i < nr; ++i) {
