@@ -1,7 +1,16 @@
-// A fused GMRES cycle whose blocks all finished, with the error word set: what a
-// block leaves that gave up a bounded wait after block 0 had found the cycle
-// converged.  The word is set from the host between two solves.  That solve must
-// report a failure, and the next one must be the first one again, bit by bit.
+// The fused GMRES cycle through the solver's own entry, on a box of 2,145 nodes
+// (two blocks).
+//
+// late: a cycle whose blocks all finished, with the error word set: what a block
+// leaves that gave up a bounded wait after block 0 had found the cycle converged.
+// The word is set from the host between two solves.  That solve must report a
+// failure, and the next one must be the first one again, bit by bit.
+//
+// restart: solves that converge in one cycle and solves that take several, both
+// orthogonalisations: the preconditioned residual of what they return, formed
+// with the separate kernels of operator and preconditioner, meets the tolerance
+// (half of it more for the FP32 basis: a cycle's own estimate is good to a few
+// 1e-6 of the residual it started from, at most 1e5 times the tolerance here).
 #include "ctx.cuh"
 #include "krylov.cuh"
 
@@ -17,45 +26,99 @@ using namespace fvmb;
         if (!(cond)) { std::printf("line %d: %s (%s)\n", __LINE__, #cond, fvm_last_error()); return 1; } \
     } while (0)
 
-int main() {
+struct Case {
     fvm_problem p;
-    CHECK(fvm_problem_richards3d(14, 12, 10, 14.0, 12.0, 10.0, 0.15, 1, 1.0, 10.0, 10.0, 2.0, 1e-5, &p) == 0);
-    fvm_ctx* c = fvm_create(&p.mesh, &p.phys, 0);
-    CHECK(c);
-    const int N = p.mesh.n_nodes, m = 30;
-    std::vector<double> hy(N), hw(N), first(N), again(N);
-    for (int i = 0; i < N; ++i) {
-        hy[i] = p.water_table - p.mesh.coords[3 * (size_t)i + 2] + 0.02 * std::sin(1.7 * i);
-        hw[i] = 1.0 / (1e-6 * std::fabs(hy[i]) + 1e-6);
+    fvm_ctx* c = nullptr;
+    int N = 0;
+    DevBuf<double> y, yp, w, F, x, t, z;
+    std::vector<double> hw;
+    int set_up() {
+        CHECK(fvm_problem_richards3d(14, 12, 10, 14.0, 12.0, 10.0, 0.15, 1, 1.0, 10.0, 10.0, 2.0, 1e-5, &p) == 0);
+        c = fvm_create(&p.mesh, &p.phys, 0);
+        CHECK(c);
+        N = p.mesh.n_nodes;
+        std::vector<double> hy(N);
+        hw.resize(N);
+        for (int i = 0; i < N; ++i) {
+            hy[i] = p.water_table - p.mesh.coords[3 * (size_t)i + 2] + 0.02 * std::sin(1.7 * i);
+            hw[i] = 1.0 / (1e-6 * std::fabs(hy[i]) + 1e-6);
+        }
+        y.upload(hy, c->stream);
+        w.upload(hw, c->stream);
+        for (DevBuf<double>* b : {&yp, &F, &x, &t, &z}) b->alloc(N);
+        yp.zero(c->stream);
+        CHECK(fvm_begin_step(c, 0.0, y.p, yp.p) == 0);
+        CHECK(fvm_residual(c, 0.0, y.p, yp.p, F.p) == 0);
+        CHECK(fvm_psetup(c, 0.0, 2e-3, 500.0, y.p, yp.p, F.p, w.p, 1) == 0);
+        return 0;
     }
-    DevBuf<double> y, yp, w, F, x;
-    y.upload(hy, c->stream);
-    w.upload(hw, c->stream);
-    yp.alloc(N);
-    F.alloc(N);
-    x.alloc(N);
-    yp.zero(c->stream);
-    CHECK(fvm_begin_step(c, 0.0, y.p, yp.p) == 0);
-    CHECK(fvm_residual(c, 0.0, y.p, yp.p, F.p) == 0);
-    CHECK(fvm_psetup(c, 0.0, 2e-3, 500.0, y.p, yp.p, F.p, w.p, 1) == 0);
-    auto solve = [&](std::vector<double>& out, int& its) {
+    int solve(int m, int restarts, double tol, int* its, GmresCounters* cnt) {
         double rn = 0.0;
-        GmresCounters cnt;
-        const int r = gmres_dev(c, 2e-3, y.p, yp.p, F.p, w.p, F.p, x.p, m, 5, 1, 1.0, &its, &rn, &cnt, 1);
-        cudaMemcpy(out.data(), x.p, sizeof(double) * N, cudaMemcpyDeviceToHost);
-        return r;
-    };
+        return gmres_dev(c, 2e-3, y.p, yp.p, F.p, w.p, F.p, x.p, m, restarts, 1, tol, its, &rn, cnt, 1);
+    }
+    std::vector<double> host(const DevBuf<double>& b) {
+        std::vector<double> v(N);
+        cudaMemcpy(v.data(), b.p, sizeof(double) * N, cudaMemcpyDeviceToHost);
+        return v;
+    }
+    // sqrt(mean((w P^-1 (F - J x))^2))
+    double residual() {
+        jacobian_apply(c, 2e-3, x.p, t.p);
+        ctx_sync(c);
+        std::vector<double> b = host(F), j = host(t);
+        for (int i = 0; i < N; ++i) b[i] -= j[i];
+        t.upload(b, c->stream);
+        psolve_dev(c, t.p, z.p);
+        ctx_sync(c);
+        const std::vector<double> r = host(z);
+        double s = 0.0;
+        for (int i = 0; i < N; ++i) s += r[i] * hw[i] * r[i] * hw[i];
+        return std::sqrt(s / N);
+    }
+};
+
+static int late() {
+    Case k;
+    if (k.set_up()) return 1;
     int its1 = 0, its2 = 0, its3 = 0;
-    const long before = c->launches;
-    CHECK(solve(first, its1) == 0 && its1 > 3);
-    CHECK(c->launches - before < its1 + 10);   // (one launch for all steps)
-    Krylov* K = c->kry[1];
-    const int late = 3;
-    CHECK(cudaMemcpy(K->err.p, &late, sizeof(int), cudaMemcpyHostToDevice) == cudaSuccess);
-    CHECK(solve(again, its2) == 2);
-    CHECK(solve(again, its3) == 0 && its3 == its1);
-    CHECK(!std::memcmp(first.data(), again.data(), sizeof(double) * N));
-    fvm_destroy(c);
-    std::printf("ok\n");
+    GmresCounters cnt;
+    const long before = k.c->launches;
+    CHECK(k.solve(30, 5, 1.0, &its1, &cnt) == 0 && its1 > 3);
+    CHECK(k.c->launches - before < its1 + 10);   // (one launch for all steps)
+    const std::vector<double> first = k.host(k.x);
+    const int word = 3;
+    CHECK(cudaMemcpy(k.c->kry[1]->err.p, &word, sizeof(int), cudaMemcpyHostToDevice) == cudaSuccess);
+    CHECK(k.solve(30, 5, 1.0, &its2, &cnt) == 2);
+    CHECK(k.solve(30, 5, 1.0, &its3, &cnt) == 0 && its3 == its1);
+    CHECK(!std::memcmp(first.data(), k.host(k.x).data(), sizeof(double) * k.N));
+    fvm_destroy(k.c);
     return 0;
+}
+
+static int restart() {
+    Case k;
+    if (k.set_up()) return 1;
+    k.x.zero(k.c->stream);
+    const double tol = k.residual() * 1e-5;
+    for (int variant : {0, 1})
+        for (int m : {60, 5, 3}) {
+            CHECK(fvm_set_krylov_variant(k.c, variant) == 0);
+            GmresCounters cnt;
+            int its = 0;
+            const long waits = k.c->n_syncs;
+            CHECK(k.solve(m, 400, tol, &its, &cnt) == 0);
+            const long cycles = k.c->n_syncs - waits;   // one wait per cycle: the fused form ran
+            CHECK(cnt.nps == its + cycles);
+            CHECK(m == 60 || cycles > 2);
+            CHECK(k.residual() <= 1.5 * tol);
+        }
+    fvm_destroy(k.c);
+    return 0;
+}
+
+int main(int argc, char** argv) {
+    if (argc != 2) return 2;
+    const int r = !std::strcmp(argv[1], "late") ? late() : restart();
+    if (!r) std::printf("ok\n");
+    return r;
 }
