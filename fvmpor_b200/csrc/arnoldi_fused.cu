@@ -684,7 +684,7 @@ bool fused_prepare(fvm_ctx* c, int m) {
             std::vector<unsigned short> lcol;
         };
         std::vector<Block> block(nb);
-        parallel_for(nb, std::max(1l, 8192l * nb / c->N), [&](long first, long last) {
+        parallel_for(nb, std::max(1l, 1024l * nb / c->N), [&](long first, long last) {
             for (long b = first; b < last; ++b) {
                 const int r0 = P->h_bstart[b], r1 = P->h_bstart[b + 1];
                 Block& B = block[b];

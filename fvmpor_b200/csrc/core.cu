@@ -1010,8 +1010,10 @@ static void build_upwind_chunks(fvm_ctx* c, const std::vector<int>& eid, const s
     std::vector<ushort4> loc(T);
     std::vector<unsigned short> of((size_t)T * nfe), slot((size_t)nch * kUpChunk * nfe, 0);
     std::vector<std::vector<unsigned short>> start(nch);
-    parallel_for(nch, 16, [&](long first, long last) {
-        std::vector<int> all, cnt, pos;
+    // (a chunk takes 0.15 ms, a thread's start about 0.05)
+    parallel_for(nch, 2, [&](long first, long last) {
+        std::vector<uint64_t> faces((size_t)kUpChunk * nfe);
+        std::vector<int> shared;   // first faces of the chunk's edges that others touch too
         for (long ch = first; ch < last; ++ch) {
             const int e0 = (int)ch * kUpChunk, e1 = std::min(T, e0 + kUpChunk);
             Chunk& k = chunk[ch];
@@ -1025,34 +1027,33 @@ static void build_upwind_chunks(fvm_ctx* c, const std::vector<int>& eid, const s
                                                              c->h_elem_nodes[(size_t)e * npe + j]) - k.nodes.begin());
                 loc[e] = make_ushort4(l[0], l[1], l[2], l[3]);
             }
-            all.assign(&eid[(size_t)e0 * nfe], &eid[0] + (size_t)e1 * nfe);
-            std::sort(all.begin(), all.end());
+            // the faces by edge, ascending in each
+            const int nf = (e1 - e0) * nfe;
+            for (int q = 0; q < nf; ++q) faces[q] = (uint64_t)(uint32_t)eid[(size_t)e0 * nfe + q] << 32 | (uint32_t)q;
+            std::sort(faces.begin(), faces.begin() + nf);
             // (whole edges first)
-            std::vector<int> shared;
-            for (size_t p = 0, q; p < all.size(); p = q) {
-                for (q = p; q < all.size() && all[q] == all[p]; ++q) {}
-                const bool whole = (int)(q - p) == edge_ptr[all[p] + 1] - edge_ptr[all[p]];
-                (whole ? k.edges : shared).push_back(all[p]);
+            shared.clear();
+            start[ch].assign(1, 0);
+            const size_t slot0 = (size_t)e0 * nfe;
+            int at = 0;
+            auto take = [&](int p) {
+                const int g = (int)(faces[p] >> 32), i = (int)k.edges.size();
+                k.edges.push_back(g);
+                for (; p < nf && (int)(faces[p] >> 32) == g; ++p) {
+                    const int q = (int)(uint32_t)faces[p], e = q / nfe, f = q - e * nfe;
+                    of[(size_t)f * T + e0 + e] = (unsigned short)i;
+                    slot[slot0 + at++] = (unsigned short)(f * kUpChunk + e);
+                }
+                start[ch].push_back((unsigned short)at);
+            };
+            for (int p = 0, q; p < nf; p = q) {
+                const int g = (int)(faces[p] >> 32);
+                for (q = p; q < nf && (int)(faces[q] >> 32) == g; ++q) {}
+                if (q - p == edge_ptr[g + 1] - edge_ptr[g]) take(p);
+                else shared.push_back(p);
             }
             k.own = (int)k.edges.size();
-            k.edges.insert(k.edges.end(), shared.begin(), shared.end());
-            const auto mid = k.edges.begin() + k.own;
-            cnt.assign(k.edges.size() + 1, 0);
-            for (int e = e0; e < e1; ++e)
-                for (int f = 0; f < nfe; ++f) {
-                    const int g = eid[(size_t)e * nfe + f];
-                    auto it = std::lower_bound(k.edges.begin(), mid, g);
-                    if (it == mid || *it != g) it = std::lower_bound(mid, k.edges.end(), g);
-                    const int i = (int)(it - k.edges.begin());
-                    of[(size_t)f * T + e] = (unsigned short)i;
-                    cnt[i + 1]++;
-                }
-            for (size_t i = 1; i < cnt.size(); ++i) cnt[i] += cnt[i - 1];
-            start[ch].assign(cnt.begin(), cnt.end());
-            pos.assign(cnt.begin(), cnt.end() - 1);
-            for (int e = e0; e < e1; ++e)
-                for (int f = 0; f < nfe; ++f)
-                    slot[(size_t)e0 * nfe + pos[of[(size_t)f * T + e]]++] = (unsigned short)(f * kUpChunk + (e - e0));
+            for (int p : shared) take(p);
         }
     });
     std::vector<int> node_ptr(1, 0), node, sptr(1, 0);

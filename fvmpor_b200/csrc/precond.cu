@@ -994,7 +994,7 @@ static void build_fd_tables(const fvm_ctx* c, const BlockILU* P, const std::vect
     };
     std::vector<Chunk> chunk(nch);
     fd.cloc.assign(T, make_ushort4(0, 0, 0, 0));
-    parallel_for(nch, 32, [&](long first, long last) {
+    parallel_for(nch, 4, [&](long first, long last) {
         std::vector<int> fq((size_t)kFdChunk * npe2), at;
         for (long ch = first; ch < last; ++ch) {
             const int e0 = (int)ch * kFdChunk, e1 = std::min(T, e0 + kFdChunk);
@@ -1048,7 +1048,7 @@ static void build_fd_tables(const fvm_ctx* c, const BlockILU* P, const std::vect
             fd.shared.push_back(make_int4(q, lu_dst[q], 0, 2 * rowof[q] + (cl[q] == rowof[q] ? 1 : 0)));
             fd.sptr.push_back(fd.sptr.back() + nchunk[q]);
         }
-    parallel_for(nch, 32, [&](long first, long last) {
+    parallel_for(nch, 4, [&](long first, long last) {
         std::vector<int> asc, rank, order, hist;
         for (long ch = first; ch < last; ++ch) {
             Chunk& k = chunk[ch];
@@ -1097,10 +1097,17 @@ static void build_fd_tables(const fvm_ctx* c, const BlockILU* P, const std::vect
     fd.cnode_ptr.assign(1, 0);
     fd.done_ptr.assign(1, 0);
     fd.share_ptr.assign(1, 0);
-    size_t words = 0;
-    for (const Chunk& k : chunk) words += k.list.size();
+    size_t words = 0, nodes = 0, done = 0;
+    for (const Chunk& k : chunk) {
+        words += k.list.size();
+        nodes += k.nodes.size();
+        done += k.done.size();
+    }
     if (words / 8 >= (size_t)INT32_MAX) throw Error("difference quotients: mesh too large");
     fd.list.reserve(words);
+    fd.cnode.reserve(nodes);
+    fd.done.reserve(done);
+    fd.share.reserve(fd.sptr.back());
     for (const Chunk& k : chunk) {
         fd.nnmax = std::max(fd.nnmax, (int)k.nodes.size());
         fd.cnode.insert(fd.cnode.end(), k.nodes.begin(), k.nodes.end());
@@ -1138,7 +1145,7 @@ static void build_pattern(fvm_ctx* c, BlockILU* P) {
         row.erase(std::unique(row.begin(), row.end()), row.end());
     };
     // (counted and formed in two passes: the rows' places follow from the counts)
-    parallel_for(N, 4096, [&](long first, long last) {
+    parallel_for(N, 512, [&](long first, long last) {
         std::vector<int> row;
         for (long i = first; i < last; ++i) {
             row_of((int)i, row);
@@ -1148,7 +1155,7 @@ static void build_pattern(fvm_ctx* c, BlockILU* P) {
     for (int i = 0; i < N; ++i) P->h_rowptr[i + 1] += P->h_rowptr[i];
     P->nnz = P->h_rowptr[N];
     P->h_col.resize(P->nnz);
-    parallel_for(N, 4096, [&](long first, long last) {
+    parallel_for(N, 512, [&](long first, long last) {
         std::vector<int> row;
         for (long i = first; i < last; ++i) {
             row_of((int)i, row);
@@ -1201,7 +1208,7 @@ static void build_pattern(fvm_ctx* c, BlockILU* P) {
     const bool schur = P->schur_iters >= 0;
     std::vector<int> sch_lv(2 * (size_t)nb, 0), sch_nin(nb, 0), o_ptr(N + 1, 0), o_col, o_src;
     std::vector<std::vector<int>> ends(nb), uends(nb);
-    const long grain = std::max(1l, 8192l * nb / N);   // blocks that are worth a thread
+    const long grain = std::max(1l, 1024l * nb / N);   // blocks that are worth a thread (0.1 ms each of its uses)
     parallel_for(nb, grain, [&](long first, long last) {
         for (long b = first; b < last; ++b) {
             const int r0 = bstart[b], r1 = bstart[b + 1];
