@@ -99,7 +99,6 @@ __global__ void k_phi_scale(int N, int j0, int j1, PhiPtrs ph, Coef7 f) {
         if (j >= j0 && j <= j1) ph.p[j][i] = v[j] * f.v[j];
 }
 
-// y -= x, y' -= cj x, e -= x ; out = sum (x ewt)^2
 // weighted squared sums of the error estimates at orders k, k + 1, k - 1 ... of a
 // step with correction e (the controller's err_norms)
 struct ErrSums {
@@ -132,7 +131,8 @@ struct ErrSums {
         }
     }
 };
-// Newton update and, of the e it leaves, the error norms of the step's test (the
+// Newton update (y -= x, y' -= cj x, e -= x, out[0] = sum (x ewt)^2) and, of the e
+// it leaves, the error norms of the step's test (the
 // sums of k_err_norms as out[1..4]): what the host waits for is one pass over the
 // vectors and one reduction, 12.0 us on the 214k-node box where the two kernels
 // took 10.2 + 11.1 us

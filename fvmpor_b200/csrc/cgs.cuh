@@ -282,69 +282,12 @@ __device__ __forceinline__ void block_dots_by_warp(const float* __restrict__ U, 
     __syncthreads();
 }
 
-// Two block-local dot-product sets in one pass over the basis (FP32, one
-// warp per basis vector): out[i] = <U_i, A>, out[nb + i] = <U_i, B> for
-// i < nb, then out[2 nb] = <A, A> and out[2 nb + 1] = <A, B>, with A and B
-// the block's rows in shared memory (quad-transposed, quad_pos).  Each
-// basis row quad is loaded once for both products.  out[] is valid in every
-// thread after the call.
-__device__ __forceinline__ void block_dots2_by_warp(const float* __restrict__ U, size_t ld,
-                                                    const double* __restrict__ A, const double* __restrict__ Bv,
-                                                    int nqp, int k0, int k1, int nb, double* out) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    const int a0 = k0 & ~3;
-    const int nq = (k1 - a0 + 3) >> 2;
-    for (int i = warp; i < nb + 1; i += nw) {
-        double sa = 0.0, sb = 0.0;
-        const float* Ui = U + ld * (i < nb ? i : 0);
-        for (int q0 = lane; q0 < nq; q0 += 32 * 8) {
-            float4 u[8];
-#pragma unroll
-            for (int t = 0; t < 8; ++t) {
-                const int q = q0 + 32 * t;
-                u[t] = (i < nb && q < nq) ? __ldg(reinterpret_cast<const float4*>(Ui + a0 + 4 * q))
-                                          : make_float4(0.f, 0.f, 0.f, 0.f);
-            }
-#pragma unroll
-            for (int t = 0; t < 8; ++t) {
-                const int q = q0 + 32 * t;
-                if (q >= nq) continue;
-                double va[4], vb[4];
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    va[e] = A[e * nqp + q];
-                    vb[e] = Bv[e * nqp + q];
-                }
-                if (i < nb) {
-                    sa += (double)u[t].x * va[0] + (double)u[t].y * va[1] + (double)u[t].z * va[2] +
-                          (double)u[t].w * va[3];
-                    sb += (double)u[t].x * vb[0] + (double)u[t].y * vb[1] + (double)u[t].z * vb[2] +
-                          (double)u[t].w * vb[3];
-                } else {
-                    sa += va[0] * va[0] + va[1] * va[1] + va[2] * va[2] + va[3] * va[3];
-                    sb += va[0] * vb[0] + va[1] * vb[1] + va[2] * vb[2] + va[3] * vb[3];
-                }
-            }
-        }
-        sa = warp_sum(sa);
-        sb = warp_sum(sb);
-        if (lane == 0) {
-            if (i < nb) {
-                out[i] = sa;
-                out[nb + i] = sb;
-            } else {
-                out[2 * nb] = sa;
-                out[2 * nb + 1] = sb;
-            }
-        }
-    }
-    __syncthreads();
-}
-
-// The same two dot-product sets (and the same out[] layout) with one thread
-// per row quad: a thread reads its rows of A and B from shared memory once
-// per kCgsGroup basis vectors and keeps that group's loads in flight
-// together.  The warp's 2 kCgsGroup partial sums are reduced by a
+// Two block-local dot-product sets in one pass over the basis (FP32): out[i] =
+// <U_i, A>, out[nb + i] = <U_i, B> for i < nb, then out[2 nb] = <A, A> and
+// out[2 nb + 1] = <A, B>, with A and B the block's rows in shared memory
+// (quad-transposed, quad_pos); valid in every thread after the call.  One thread
+// per row quad: it reads its rows of A and B from shared memory once per
+// kCgsGroup basis vectors and keeps that group's loads in flight together.  The warp's 2 kCgsGroup partial sums are reduced by a
 // transposing butterfly: each exchange hands the partner the half of the
 // values it keeps, so after offsets 16, 8, 4, 2 every lane holds one value
 // (index b1 + 2 b2 + 4 b3 + 8 b4 of its lane bits) summed over 16 lanes, and

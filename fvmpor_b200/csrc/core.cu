@@ -474,7 +474,7 @@ __global__ void k_edge_upwind(int E, int nfe, const int* __restrict__ edge_ptr,
 // The reference divides each flux by the sum of the edge's face areas
 // (fvmpor.h:765), which is positive and does not change the sign asked for.
 struct UpArgs {
-    int T, N, kiso, estride, nnmax, edmax;   // edmax: most edges of a chunk
+    int T, N, kiso, estride, nnmax;
     const int* node_ptr;
     const int* node;
     const ushort4* loc;
@@ -844,7 +844,6 @@ void launch_begin_step(fvm_ctx* c, const double* y, const double* yp) {
     if (c->up_chunks) {
         UpArgs a;
         a.T = c->T; a.N = c->N; a.kiso = c->kiso ? 1 : 0; a.estride = c->estride; a.nnmax = c->up_nnmax;
-        a.edmax = c->up_edmax;
         a.node_ptr = c->up_node_ptr.p; a.node = c->up_node.p; a.loc = c->up_loc.p;
         a.edge = c->up_edge.p; a.start = c->up_start.p; a.slot = c->up_slot.p;
         a.coef = c->coef.p; a.xyz = c->xyz.p; a.eK = c->eK.p; a.ezone = c->ezone.p;

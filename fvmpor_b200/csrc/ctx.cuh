@@ -152,14 +152,6 @@ __device__ __forceinline__ double gather_finish(const GatherSrc& g, int i, doubl
     if (g.F0) r = (r - g.F0[i]) * (g.sigma_dev ? 1.0 / *g.sigma_dev : g.inv_sigma);
     return r;
 }
-__device__ __forceinline__ double gather_row(const GatherSrc& g, int i) {
-    double s = 0.0;
-    if (!g.ntype[i]) {
-        const int p1 = g.part_ptr[i + 1];
-        for (int p = g.part_ptr[i]; p < p1; ++p) s += g.part[g.cpos[p]];
-    }
-    return gather_finish(g, i, s);
-}
 #endif
 
 struct BlockILU;   // precond.cu
