@@ -228,7 +228,7 @@ __device__ __forceinline__ void back_substitute(const FusedArgs& a, int k, const
 // loop), so a thread may hold up to 170 registers
 constexpr int kFusedThreads = 384;
 
-template <bool DEL>
+template <bool DEL, bool WIDE>
 __global__ void __launch_bounds__(kFusedThreads, 1) k_arnoldi_fused(FusedArgs a) {
     // ca holds up to 2 (m + 1) + 2 reduced numbers on the delayed variant
     __shared__ double ca[DEL ? 132 : 64], cb[64], coef[64], sc[64], rc[64], rs[64], gs[64];
@@ -366,8 +366,8 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_arnoldi_fused(FusedArgs a)
         // preconditioner: both triangular sweeps in shared memory
         {
             const IluShared<float> V = s_view;
-            ilu_sweep<float, false>(V, 1, V.nl);
-            ilu_sweep<float, true>(V, 0, V.nu);
+            ilu_sweep<float, false, WIDE>(V, 1, V.nl);
+            ilu_sweep<float, true, WIDE>(V, 0, V.nu);
         }
         for (int k = threadIdx.x; k < nr; k += blockDim.x) {
             const int qp = quad_pos(r0, nqp, r0 + k);
@@ -618,8 +618,10 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_arnoldi_fused(FusedArgs a)
 
 static int fused_sync_slot(int nb) { return ((nb + 31) & ~31) + 32; }
 
-static const void* fused_kernel(int variant) {
-    return variant ? (const void*)k_arnoldi_fused<true> : (const void*)k_arnoldi_fused<false>;
+using FusedKernel = void (*)(FusedArgs);
+static FusedKernel fused_kernel(int variant, bool wide) {
+    if (wide) return variant ? k_arnoldi_fused<true, true> : k_arnoldi_fused<false, true>;
+    return variant ? k_arnoldi_fused<true, false> : k_arnoldi_fused<false, false>;
 }
 
 constexpr int kFusedMaxDim = 62;   // the reduced numbers' arrays
@@ -799,7 +801,7 @@ bool fused_prepare(fvm_ctx* c, int m) {
         FVM_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
         FVM_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
         for (int v = 0; v < 2; ++v) {
-            const void* kfn = fused_kernel(v);
+            const void* kfn = (const void*)fused_kernel(v, P->wide);
             cudaFuncAttributes fa;
             FVM_CUDA(cudaFuncGetAttributes(&fa, kfn));
             P->fused_room[v] = kMaxDynSmem - fa.sharedSizeBytes;
@@ -900,8 +902,7 @@ void fused_cycle(fvm_ctx* c, Krylov* K, int m, double cj, double tol, const doub
     if (P->fused_launches >= kSyncFail / (128u * (unsigned)P->nb)) fused_reset(c);
     a.base = 64u * P->fused_launches++;
     c->tm.begin(TM_CGS, s);
-    if (var) FVM_CUDA(cudaLaunchKernelEx(&cfg, k_arnoldi_fused<true>, a));
-    else FVM_CUDA(cudaLaunchKernelEx(&cfg, k_arnoldi_fused<false>, a));
+    FVM_CUDA(cudaLaunchKernelEx(&cfg, fused_kernel(var, P->wide), a));
     c->tm.end(TM_CGS, s);
     c->launches++;
 }

@@ -61,6 +61,7 @@ struct BlockILU {
     DevBuf<int> bstart;
     DevBuf<IluBlk> blk;       // [nb] where each block's factor and records start
     size_t nlu = 0;           // factor entries of all blocks (padding included)
+    bool wide = false;        // a block has wide rows
     // the set-up's Jacobian in factor order, for an FP64 and an FP32 factor
     // (written by the quotient kernels; allocated at the first use of each)
     DevBuf<double> Jw;
@@ -166,21 +167,26 @@ template <class V> __device__ __forceinline__ int ilu_level(const V& f, bool upp
     return (int)f.meta((upper ? f.nl + 1 : 0) + l);
 }
 template <class V> __device__ __forceinline__ int ilu_groups_at(const V& f) { return (f.nl + f.nu + 3) & ~1; }
-template <class V> __device__ __forceinline__ unsigned ilu_group(const V& f, bool upper, int g) {
-    return f.meta2(ilu_groups_at(f) + 2 * ((upper ? f.ngl : 0) + g));
+template <class V> __device__ __forceinline__ int ilu_group_at(const V& f, bool upper, int g) {
+    return ilu_groups_at(f) + 2 * ((upper ? f.ngl : 0) + g);
+}
+template <class V> __device__ __forceinline__ int ilu_row_at(const V& f, bool upper, int g, int j) {
+    return ilu_groups_at(f) + 2 * (f.ngl + f.ngu + (int)kIluPad) + kIluGroup * ((upper ? f.ngl : 0) + g) + j;
 }
 template <class V> __device__ __forceinline__ int ilu_row(const V& f, bool upper, int g, int j) {
-    return (int)f.meta(ilu_groups_at(f) + 2 * (f.ngl + f.ngu) + kIluGroup * ((upper ? f.ngl : 0) + g) + j);
+    return (int)f.meta(ilu_row_at(f, upper, g, j));
 }
-// a wide row's first entry past kIluWide and its entries
+// a wide row's first entry past kIluWide and its entries, (0, 0) for a group that
+// is none; only where the block has any (nwide)
 template <class V> __device__ __forceinline__ int2 ilu_wide(const V& f, bool upper, int g) {
-    const int at = ilu_groups_at(f) + (2 + kIluGroup) * (f.ngl + f.ngu), key = (upper ? f.ngl : 0) + g;
+    const int at = ilu_groups_at(f) + (2 + kIluGroup) * (f.ngl + f.ngu + (int)kIluPad), key = (upper ? f.ngl : 0) + g;
     int lo = 0;
     for (int n = f.nwide; n > 1;) {   // ascending groups
         const int h = n >> 1;
         if ((int)f.meta2(at + 6 * (lo + h)) <= key) lo += h;
         n -= h;
     }
+    if ((int)f.meta2(at + 6 * lo) != key) return make_int2(0, 0);
     return make_int2((int)f.meta2(at + 6 * lo + 2), (int)f.meta2(at + 6 * lo + 4));
 }
 // where the entries of lane j's row of a group are: the general form, for the
@@ -190,12 +196,14 @@ struct IluSpan {
     __device__ __forceinline__ int entry(int k) const { return k < kIluWide ? at + 32 * k : tail + k - kIluWide; }
 };
 template <class V> __device__ __forceinline__ IluSpan ilu_span(const V& f, bool upper, int g, int j) {
-    const unsigned word = ilu_group(f, upper, g);
+    const unsigned word = f.meta2(ilu_group_at(f, upper, g));
     IluSpan s{(int)(word >> kIluWidthBits) + j, 0, (int)(word & ((1u << kIluWidthBits) - 1u))};
-    if (s.w > kIluWide) {
+    if (f.nwide) {
         const int2 t = ilu_wide(f, upper, g);
-        s.tail = t.x;
-        s.w = t.y;
+        if (t.y) {
+            s.tail = t.x;
+            s.w = t.y;
+        }
     }
     return s;
 }
@@ -259,9 +267,11 @@ __device__ __forceinline__ int tid_here() {
 // path; a warp without a slice goes straight to the barrier.  Entries in column
 // order.  Loads are taken four entries at a time, past a group's last entry
 // (kIluSlack entries after the arrays), and what lies there is left unused, as
-// is what the lanes past a level's last group read (its entries again).
+// is what the lanes past a level's last group read (the next groups' entries).
 // Most rows of a tetrahedral mesh have more than kIluPre entries (up to 14), but
-// a level is bound by the instructions that its warps issue: the two sweeps of
+// a level is bound by the instructions that its warps issue (so wide rows, WIDE,
+// have a form of their own: with their code in every level an apply on the
+// 214k-node box took 12.7 us instead of 12.2): the two sweeps of
 // a 1,447-row block of the 214k-node box took 5.0 us with 4 columns fetched
 // ahead, 5.1 with 8 and more with 12 and 16.  Stored row by row with a row per
 // lane they took 9.2 us.
@@ -271,28 +281,29 @@ struct IluLane {
     unsigned c[kIluPre];
 };
 
-// lane's row of group g, a group of the level that ends at g1 (past it: no row)
-template <bool UPPER, class V>
-__device__ __forceinline__ void ilu_fetch(IluLane& R, const V& f, int lane, int g, int g1) {
-    const int gi = min(g, g1 - 1), j = lane & (kIluGroup - 1);
-    const unsigned word = ilu_group(f, UPPER, gi);
-    R.w = (int)(word & ((1u << kIluWidthBits) - 1u));
+// the lane's row of a slice from group s on, in a level that ends at g1 (past it:
+// no row); gw, gr: places of its group's word and of its row there for s = 0
+template <class V>
+__device__ __forceinline__ void ilu_fetch(IluLane& R, const V& f, int gw, int gr, int j, bool in, int s) {
+    const unsigned word = f.meta2(gw + 2 * s);
+    const int row = (int)f.meta(gr + kIluGroup * s);
+    R.w = in ? (int)(word & ((1u << kIluWidthBits) - 1u)) : 0;
     R.at = (int)(word >> kIluWidthBits) + j;
-    R.row = g < g1 ? ilu_row(f, UPPER, gi, j) : kIluNoRow;
+    R.row = in ? row : kIluNoRow;
 #pragma unroll
     for (int k = 0; k < kIluPre; ++k) R.c[k] = f.col(R.at + 32 * k);
 }
 
-// acc += entries [k, w) of a row, the first kIluWide of a wide one
+// acc += entries [k, w) of a row in the strip
 template <class T, class V>
 __device__ __forceinline__ void ilu_rest(T& acc, const V& f, int at, int w, int k) {
-    w = min(w, kIluWide);
 #pragma unroll 1
     for (; k < w; k += 4) {
         T v[4], xv[4];
 #pragma unroll
         for (int t = 0; t < 4; ++t) {
-            xv[t] = f.x(f.col(at + 32 * (k + t)));
+            const unsigned c = f.col(at + 32 * (k + t));
+            xv[t] = f.x(c);
             v[t] = f.val(at + 32 * (k + t));
         }
 #pragma unroll
@@ -300,18 +311,20 @@ __device__ __forceinline__ void ilu_rest(T& acc, const V& f, int at, int w, int 
             if (k + t < w) acc += v[t] * xv[t];
     }
 }
-// ... and the others
+// ... and a wide row's others
 template <class T, class V> __device__ __forceinline__ T ilu_wide_rest(T acc, const V& f, bool upper, int g) {
     const int2 t = ilu_wide(f, upper, g);
+#pragma unroll 1
     for (int k = 0; k < t.y - kIluWide; ++k) acc += f.val(t.x + k) * f.x(f.col(t.x + k));
     return acc;
 }
 
-template <class T, bool UPPER, class V>
+template <class T, bool UPPER, bool WIDE, class V>
 __device__ __forceinline__ void ilu_sweep(const V& f, int l0, int l1) {
     T* const x = reinterpret_cast<T*>(ilu_smem());
-    const int tid = tid_here(), lane = tid & 31, stride = (blockDim.x >> 5) * kIluSlice;
+    const int tid = tid_here(), stride = (blockDim.x >> 5) * kIluSlice;
     const int first = (tid >> 5) * kIluSlice, mine = tid / kIluGroup;   // the warp's and the lane's group of a level
+    const int j = tid & (kIluGroup - 1), gw = ilu_group_at(f, UPPER, mine), gr = ilu_row_at(f, UPPER, mine, j);
     // set before the conditional fetches: registers that a loop writes only
     // under a condition count as live all the way round it
     IluLane cur, nxt;
@@ -322,7 +335,7 @@ __device__ __forceinline__ void ilu_sweep(const V& f, int l0, int l1) {
     nxt = cur;
     if (l0 >= l1) return;
     int s0 = ilu_level(f, UPPER, l0), s1 = ilu_level(f, UPPER, l0 + 1);
-    if (s0 + first < s1) ilu_fetch<UPPER>(cur, f, lane, s0 + mine, s1);
+    if (s0 + first < s1) ilu_fetch(cur, f, gw, gr, j, s0 + mine < s1, s0);
 #pragma unroll 1
     for (int l = l0; l < l1; ++l) {
         const int s2 = l + 1 < l1 ? ilu_level(f, UPPER, l + 2) : s1;
@@ -339,36 +352,40 @@ __device__ __forceinline__ void ilu_sweep(const V& f, int l0, int l1) {
             const bool act = cur.row != kIluNoRow;
             const int row = act ? cur.row : 0;
             const T xi = x[row], piv = UPPER ? f.val(f.ds + row) : (T)1;
-            if (more) ilu_fetch<UPPER>(nxt, f, lane, s1 + mine, s2);
+            if (more) ilu_fetch(nxt, f, gw, gr, j, s1 + mine < s2, s1);
             T acc = (T)0;
 #pragma unroll
             for (int k = 0; k < kIluPre; ++k)
                 if (k < cur.w) acc += v[k] * xv[k];
             ilu_rest(acc, f, cur.at, cur.w, kIluPre);
-            if (cur.w > kIluWide && act) acc = ilu_wide_rest(acc, f, UPPER, s0 + mine);
+            if (WIDE && act) acc = ilu_wide_rest(acc, f, UPPER, s0 + mine);
             if (act) x[row] = UPPER ? (xi - acc) * piv : xi - acc;
             // slices of a level with more of them than the CTA has warps
 #pragma unroll 1
             for (int s = s0 + stride; s + first < s1; s += stride) {
-                const int g = s + mine, gi = min(g, s1 - 1), j = lane & (kIluGroup - 1);
-                const unsigned word = ilu_group(f, UPPER, gi);
-                const int w = (int)(word & ((1u << kIluWidthBits) - 1u));
-                const int i = g < s1 ? ilu_row(f, UPPER, gi, j) : kIluNoRow;
+                const unsigned word = f.meta2(gw + 2 * s);
+                const int i = s + mine < s1 ? (int)f.meta(gr + kIluGroup * s) : kIluNoRow;
                 T a = (T)0;
-                ilu_rest(a, f, (int)(word >> kIluWidthBits) + j, w, 0);
                 if (i != kIluNoRow) {
-                    if (w > kIluWide) a = ilu_wide_rest(a, f, UPPER, g);
+                    ilu_rest(a, f, (int)(word >> kIluWidthBits) + j, (int)(word & ((1u << kIluWidthBits) - 1u)), 0);
+                    if (WIDE) a = ilu_wide_rest(a, f, UPPER, s + mine);
                     x[i] = UPPER ? (x[i] - a) * f.val(f.ds + i) : x[i] - a;
                 }
             }
         } else if (more) {
-            ilu_fetch<UPPER>(nxt, f, lane, s1 + mine, s2);
+            ilu_fetch(nxt, f, gw, gr, j, s1 + mine < s2, s1);
         }
         __syncthreads();
         cur = nxt;
         s0 = s1;
         s1 = s2;
     }
+}
+
+// for kernels that take both kinds of block
+template <class T, bool UPPER, class V> __device__ __forceinline__ void ilu_sweep_any(const V& f, int l0, int l1) {
+    if (f.nwide) ilu_sweep<T, UPPER, true>(f, l0, l1);
+    else ilu_sweep<T, UPPER, false>(f, l0, l1);
 }
 
 } // namespace fvmb

@@ -53,15 +53,16 @@ FVM_HD size_t ilu_window(size_t nr, size_t ds) { return ds + ((nr + 3) & ~(size_
 
 // u16 words of a block's record: first group of each level of the lower (nl + 1)
 // and of the upper sweep (nu + 1); from an even word on, two words for each
-// group, lower and upper (bits 7 and up: its at; below: its entries per row,
-// kIluWide + 1 for a wide row); the groups' rows (kIluNoRow for none); three
-// double words for each wide row: group, first entry past kIluWide, entries;
-// padded to 16 bytes
+// group, lower and upper (bits 7 and up: its at; below: its entries per row in
+// the strip); the groups' rows (kIluNoRow for none); three double words for each
+// wide row: group, first entry past kIluWide, entries; padded to 16 bytes.  A
+// warp may read kIluSlice - 1 groups past the last one, words and rows.
 constexpr unsigned short kIluNoRow = 0xffff;
 constexpr unsigned kIluWidthBits = 7;
-static_assert(kIluWide + 1 < 1 << kIluWidthBits, "the group's word");
+static_assert(kIluWide < 1 << kIluWidthBits, "the group's word");
+constexpr size_t kIluPad = kIluSlice - 1;   // groups' words and rows behind the last
 FVM_HD size_t ilu_meta_words(size_t nl, size_t nu, size_t ng, size_t nwide) {
-    return (((nl + nu + 3) & ~(size_t)1) + (2 + kIluGroup) * ng + 6 * nwide + 7) & ~(size_t)7;
+    return (((nl + nu + 3) & ~(size_t)1) + (2 + kIluGroup) * (ng + kIluPad) + 6 * nwide + 7) & ~(size_t)7;
 }
 
 // entries that a sweep may read past the last one of the strip or the wide rows:
@@ -201,9 +202,11 @@ inline IluBlk ilu_layout(int r0, int r1, const std::vector<int>& ptr, const std:
     };
     for (const std::vector<int>& v : first) meta.insert(meta.end(), v.begin(), v.end());
     if (meta.size() & 1) meta.push_back(0);
-    for (const Group& k : groups) put2((unsigned)k.at << kIluWidthBits | (unsigned)std::min(k.w, kIluWide + 1));
+    for (const Group& k : groups) put2((unsigned)k.at << kIluWidthBits | (unsigned)std::min(k.w, kIluWide));
+    meta.resize(meta.size() + 2 * kIluPad, 0);
     for (const Group& k : groups)
         for (int i : k.row) meta.push_back(i < 0 ? kIluNoRow : (unsigned short)(i - r0));
+    meta.resize(meta.size() + kIluGroup * kIluPad, kIluNoRow);
     for (int g = 0; g < (int)groups.size(); ++g)
         if (groups[g].w > kIluWide) {
             put2((unsigned)g);

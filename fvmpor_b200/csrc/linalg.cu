@@ -334,10 +334,10 @@ __global__ void k_combine_dev(int N, ArnState* st, const int* __restrict__ err, 
                               int first) {
     pdl_wait_and_trigger();
     __shared__ double coef[64];
-    const bool failed = *err != 0;
-    if (failed && blockIdx.x == 0 && threadIdx.x == 0) st->done = 0;
+    const int failed = *err, done = st->done, steps = st->j;   // (one round of loads)
+    const int nv = !failed && (done == 1 || done == 2) ? steps : 0;
     // (the other blocks may read done before or after that)
-    const int done = failed ? 0 : st->done, nv = done == 1 || done == 2 ? st->j : 0;
+    if (failed && blockIdx.x == 0 && threadIdx.x == 0) st->done = 0;
     for (int i = threadIdx.x; i < nv; i += blockDim.x) coef[i] = ys[i];
     __syncthreads();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;

@@ -416,7 +416,7 @@ __global__ void k_fd_shared(int n, const int4* __restrict__ at, const int* __res
 // memory, in place in global memory.  Row i's entries in column order: its
 // lower ones, the pivot, its upper ones (up[] gives an upper lane's place).
 template <class T>
-__global__ void __launch_bounds__(128) k_ilu_factor(const int* __restrict__ bstart, const IluBlk* __restrict__ blk,
+__global__ void __launch_bounds__(128, 1) k_ilu_factor(const int* __restrict__ bstart, const IluBlk* __restrict__ blk,
                                                     const unsigned short* __restrict__ meta, const int* __restrict__ up,
                                                     const T* __restrict__ Jw,
                                                     const unsigned short* __restrict__ lu_col, T* lu, int* status) {
@@ -488,15 +488,13 @@ __global__ void __launch_bounds__(128) k_ilu_apply(const int* __restrict__ bstar
     __syncthreads();
     const auto V = ilu_in_place(B, nr, lu, lu_col, meta);
     // level 0 of the lower sweep has no off-diagonal entries
-    ilu_sweep<T, false>(V, 1, V.nl);
-    ilu_sweep<T, true>(V, 0, V.nu);
+    ilu_sweep_any<T, false>(V, 1, V.nl);
+    ilu_sweep_any<T, true>(V, 0, V.nu);
     for (int i = threadIdx.x; i < nr; i += blockDim.x) z[lu_row[r0 + i]] = (double)x[i];
 }
 
-// (three CTAs of 256 threads per SM: 80 registers, no spills; unbounded, the build
-// takes 98 and leaves small blocks a CTA less per SM)
-template <class T>
-__global__ void __launch_bounds__(kIluThreads, 3) k_ilu_apply_smem(const int* __restrict__ bstart,
+template <class T, bool WIDE>
+__global__ void __launch_bounds__(kIluThreads, 1) k_ilu_apply_smem(const int* __restrict__ bstart,
                                                         const IluBlk* __restrict__ blk,
                                                         const unsigned short* __restrict__ lu_col,
                                                         const unsigned short* __restrict__ meta,
@@ -556,8 +554,8 @@ __global__ void __launch_bounds__(kIluThreads, 3) k_ilu_apply_smem(const int* __
     }
     const IluShared<T> V = S.view(B);
     // level 0 of the lower sweep has no off-diagonal entries
-    ilu_sweep<T, false>(V, 1, V.nl);
-    ilu_sweep<T, true>(V, 0, V.nu);
+    ilu_sweep<T, false, WIDE>(V, 1, V.nl);
+    ilu_sweep<T, true, WIDE>(V, 0, V.nu);
 #pragma unroll
     for (int k = 0; k < kRows; ++k)
         if (threadIdx.x + k * blockDim.x < nr) z[node[k]] = (double)x[threadIdx.x + k * blockDim.x];
@@ -647,10 +645,10 @@ __global__ void __launch_bounds__(kIluThreads, sizeof(T) == 4 ? 4 : 3) k_ilu_app
         else return ilu_in_place(B, nr, a.lu, a.lu_col, a.meta);
     }();
     if (good) {
-        ilu_sweep<T, false>(V, 1, V.nl);
+        ilu_sweep_any<T, false>(V, 1, V.nl);
         for (int i = threadIdx.x; i < nr; i += blockDim.x) zs[i] = x[i];
         __syncthreads();
-        ilu_sweep<T, true>(V, 0, uvS);
+        ilu_sweep_any<T, true>(V, 0, uvS);
     }
     for (int it = 0; it < a.iters; ++it) {
         double* xo = a.xg + (size_t)(it & 1) * a.N;
@@ -667,10 +665,10 @@ __global__ void __launch_bounds__(kIluThreads, sizeof(T) == 4 ? 4 : 3) k_ilu_app
             x[q] = acc;
         }
         __syncthreads();
-        ilu_sweep<T, false>(V, lvB, V.nl);
+        ilu_sweep_any<T, false>(V, lvB, V.nl);
         for (int q = nin + threadIdx.x; q < nr; q += blockDim.x) x[q] = zs[q] - x[q];
         __syncthreads();
-        ilu_sweep<T, true>(V, 0, uvS);
+        ilu_sweep_any<T, true>(V, 0, uvS);
     }
     if (!good) {
         for (int i = threadIdx.x; i < nr; i += blockDim.x) a.z[a.lu_row[r0 + i]] = (double)x[i];
@@ -680,7 +678,7 @@ __global__ void __launch_bounds__(kIluThreads, sizeof(T) == 4 ? 4 : 3) k_ilu_app
         for (int q = threadIdx.x; q < nin; q += blockDim.x) x[q] = zs[q];
         __syncthreads();
     }
-    ilu_sweep<T, true>(V, uvS, V.nu);
+    ilu_sweep_any<T, true>(V, uvS, V.nu);
     for (int i = threadIdx.x; i < nr; i += blockDim.x) a.z[a.lu_row[r0 + i]] = (double)x[i];
 }
 
@@ -1336,6 +1334,7 @@ static void build_pattern(fvm_ctx* c, BlockILU* P) {
             throw Error("block-ILU: block too large");
     }
     P->nlu = nlu;
+    for (int b = 0; b < nb; ++b) P->wide = P->wide || blk[b].nwide > 0;
     // elimination schedule in level order (window positions relative to each
     // block's first entry, as the factorisation indexes); the same update set
     // and order as merging row i with U(k) for each L entry
@@ -1428,11 +1427,11 @@ static void build_pattern(fvm_ctx* c, BlockILU* P) {
             raise_smem_limit(k_ilu_apply<float>, ilu_plain_bytes(maxb, sizeof(float)));
         }
         if (P->smem_stage[0]) {
-            raise_smem_limit(k_ilu_apply_smem<double>, P->smem_stage[0]);
+            raise_smem_limit(P->wide ? k_ilu_apply_smem<double, true> : k_ilu_apply_smem<double, false>, P->smem_stage[0]);
             raise_smem_limit(k_ilu_factor_smem<double>, (size_t)(round16(P->smem_stage[0]) + 8 * (size_t)P->scr_words[0]));
         }
         if (P->smem_stage[1]) {
-            raise_smem_limit(k_ilu_apply_smem<float>, P->smem_stage[1]);
+            raise_smem_limit(P->wide ? k_ilu_apply_smem<float, true> : k_ilu_apply_smem<float, false>, P->smem_stage[1]);
             raise_smem_limit(k_ilu_factor_smem<float>, (size_t)(round16(P->smem_stage[1]) + 8 * (size_t)P->scr_words[1]));
         }
         if (schur) {
@@ -1680,8 +1679,8 @@ void psolve_dev(fvm_ctx* c, const double* r, double* z, const int* skip) {
             fvm_launch_pdl(c, plain, P->nb, 128, ilu_plain_bytes(P->maxb, sizeof(*lu)), s, P->bstart.p, P->blk.p,
                            P->lu_col.p, P->meta.p, lu, P->lu_row.p, r, z, skip);
     };
-    if (P->factored) go(k_ilu_apply_smem<float>, k_ilu_apply<float>, P->lu32.p);
-    else go(k_ilu_apply_smem<double>, k_ilu_apply<double>, P->lu64.p);
+    if (P->factored) go(P->wide ? k_ilu_apply_smem<float, true> : k_ilu_apply_smem<float, false>, k_ilu_apply<float>, P->lu32.p);
+    else go(P->wide ? k_ilu_apply_smem<double, true> : k_ilu_apply_smem<double, false>, k_ilu_apply<double>, P->lu64.p);
 }
 
 } // namespace fvmb

@@ -89,7 +89,8 @@ int main(int argc, char** argv) {
     std::vector<double> x(nr + 1, 0.0), y(nr);
     for (int i = 0; i < nr; ++i) x[i] = y[i] = (double)(rng() % 2000) / 1000.0 - 1.0;
     auto meta2 = [&](int i) { return (unsigned)meta[i] | (unsigned)meta[i + 1] << 16; };
-    const int at0 = (B.nl + B.nu + 3) & ~1, ng = B.ngl + B.ngu, rows0 = at0 + 2 * ng, wide0 = rows0 + kIluGroup * ng;
+    const int at0 = (B.nl + B.nu + 3) & ~1, ng = B.ngl + B.ngu, rows0 = at0 + 2 * (ng + (int)kIluPad);
+    const int wide0 = rows0 + kIluGroup * (ng + (int)kIluPad);
     CHECK(wide0 + 6 * B.nwide <= (int)meta.size());
     const int reach = B.ds + kIluSlack;   // ilu_stage_bytes
     for (int up = 0; up < 2; ++up) {
@@ -100,33 +101,35 @@ int main(int argc, char** argv) {
             for (int s = g0; s < g1; s += kIluSlice) {
                 std::set<int> columns, pairs[2];
                 for (int lane = 0; lane < 32; ++lane) {
-                    const int g = s + lane / kIluGroup, gi = std::min(g, g1 - 1), j = lane % kIluGroup;
-                    const unsigned word = meta2(at0 + 2 * (gbase + gi));
-                    const int w = (int)(word & ((1u << kIluWidthBits) - 1u)), at = (int)(word >> kIluWidthBits) + j;
-                    const int row = g < g1 ? meta[rows0 + kIluGroup * (gbase + gi) + j] : kIluNoRow;
+                    const int g = s + lane / kIluGroup, j = lane % kIluGroup;
+                    const int word_at = at0 + 2 * (gbase + g), row_at = rows0 + kIluGroup * (gbase + g) + j;
+                    CHECK(word_at + 1 < rows0 && row_at < wide0);
+                    const unsigned word = meta2(word_at);
+                    const int at = (int)(word >> kIluWidthBits) + j;
+                    const int w = g < g1 ? (int)(word & ((1u << kIluWidthBits) - 1u)) : 0;
+                    const int row = g < g1 ? meta[row_at] : kIluNoRow;
+                    CHECK(w <= kIluWide);
                     if (g < g1 && j == 0 && w > 0) {
                         CHECK(columns.insert(at % 32 / kIluGroup).second);
                         CHECK(pairs[lane / 16].insert(at % 16 / kIluGroup).second);
                     }
                     double acc = 0.0;
-                    const int shown = std::min(w, kIluWide);
-                    for (int k = 0; k < std::max(4, (shown + 3) & ~3); ++k) {
+                    for (int k = 0; k < std::max(4, (w + 3) & ~3); ++k) {
                         CHECK(at + 32 * k < reach);
                         const double v = val[at + 32 * k], xv = x[cols[at + 32 * k]];
                         if (k < w) acc += v * xv;
                     }
                     if (row == kIluNoRow) continue;
-                    if (w > kIluWide) {
-                        CHECK(j == 0);
-                        int t = 0;
-                        while (t < B.nwide && (int)meta2(wide0 + 6 * t) != gbase + gi) ++t;
-                        CHECK(t < B.nwide);
+                    int t = 0;
+                    while (t < B.nwide && (int)meta2(wide0 + 6 * t) != gbase + g) ++t;
+                    if (t < B.nwide) {
+                        CHECK(j == 0 && w == kIluWide);
                         const int tail = (int)meta2(wide0 + 6 * t + 2), len = (int)meta2(wide0 + 6 * t + 4);
                         for (int k = 0; k < len - kIluWide; ++k) acc += val[tail + k] * x[cols[tail + k]];
                     }
                     // the places of the factorisation's lists
-                    if (up) CHECK(place.upper[r0 + row] == kIluGroup * gi + j);
-                    else CHECK(place.lower[r0 + row] == kIluGroup * (gi - g0) + j);
+                    if (up) CHECK(place.upper[r0 + row] == kIluGroup * g + j);
+                    else CHECK(place.lower[r0 + row] == kIluGroup * (g - g0) + j);
                     x[row] = up ? (x[row] - acc) * val[B.ds + row] : x[row] - acc;
                 }
             }

@@ -116,3 +116,7 @@ def test_late_failure_is_seen_when_it_happens(cuda, check):
 
 def test_restarted_solves_meet_their_tolerance(cuda, check):
     check("restart")
+
+
+def test_solves_with_a_node_of_many_neighbours(cuda, check):
+    check("wide")
