@@ -414,9 +414,12 @@ __global__ void k_fd_shared(int n, const int4* __restrict__ at, const int* __res
 
 // Factorisation and sweeps of a block whose window does not fit into shared
 // memory, in place in global memory.  Row i's entries in column order: its
-// lower ones, the pivot, its upper ones (up[] gives an upper lane's place).
+// lower ones, the pivot, its upper ones (up[] gives an upper lane's place).  A row
+// per thread, whose chain of dependent loads is what it waits for: levels of a few
+// hundred rows want as many threads.
+constexpr int kIluPlainFactorThreads = 512;
 template <class T>
-__global__ void __launch_bounds__(128, 1) k_ilu_factor(const int* __restrict__ bstart, const IluBlk* __restrict__ blk,
+__global__ void __launch_bounds__(kIluPlainFactorThreads, 1) k_ilu_factor(const int* __restrict__ bstart, const IluBlk* __restrict__ blk,
                                                     const unsigned short* __restrict__ meta, const int* __restrict__ up,
                                                     const T* __restrict__ Jw,
                                                     const unsigned short* __restrict__ lu_col, T* lu, int* status) {
@@ -473,7 +476,7 @@ __global__ void __launch_bounds__(128, 1) k_ilu_factor(const int* __restrict__ b
 }
 
 template <class T>
-__global__ void __launch_bounds__(128) k_ilu_apply(const int* __restrict__ bstart, const IluBlk* __restrict__ blk,
+__global__ void __launch_bounds__(kIluThreads) k_ilu_apply(const int* __restrict__ bstart, const IluBlk* __restrict__ blk,
                                                    const unsigned short* __restrict__ lu_col,
                                                    const unsigned short* __restrict__ meta, const T* __restrict__ lu,
                                                    const int* __restrict__ lu_row, const double* __restrict__ r,
@@ -1607,7 +1610,7 @@ void psetup_dev(fvm_ctx* c, double cj, double h, const double* y, const double* 
                        P->blk.p, P->meta.p, (const T*)Jw, P->lu_col.p, P->seg_ptr.p, P->upd.p, so, sw, lu.p,
                        P->status.p);
         } else {
-            fvm_launch(c, k_ilu_factor<T>, P->nb, 128, 0, s, P->bstart.p, P->blk.p, P->meta.p, P->lu_up.p,
+            fvm_launch(c, k_ilu_factor<T>, P->nb, kIluPlainFactorThreads, 0, s, P->bstart.p, P->blk.p, P->meta.p, P->lu_up.p,
                        (const T*)Jw, P->lu_col.p, lu.p, P->status.p);
         }
     };
@@ -1676,7 +1679,7 @@ void psolve_dev(fvm_ctx* c, const double* r, double* z, const int* skip) {
             fvm_launch_pdl(c, staged, P->nb, P->apply_threads, sm, s, P->bstart.p, P->blk.p, P->lu_col.p, P->meta.p, lu,
                            P->lu_row.p, r, z, P->status.p, skip);
         else
-            fvm_launch_pdl(c, plain, P->nb, 128, ilu_plain_bytes(P->maxb, sizeof(*lu)), s, P->bstart.p, P->blk.p,
+            fvm_launch_pdl(c, plain, P->nb, P->apply_threads, ilu_plain_bytes(P->maxb, sizeof(*lu)), s, P->bstart.p, P->blk.p,
                            P->lu_col.p, P->meta.p, lu, P->lu_row.p, r, z, skip);
     };
     if (P->factored) go(P->wide ? k_ilu_apply_smem<float, true> : k_ilu_apply_smem<float, false>, k_ilu_apply<float>, P->lu32.p);
