@@ -134,8 +134,8 @@ struct ErrSums {
 // Newton update (y -= x, y' -= cj x, e -= x, out[0] = sum (x ewt)^2) and, of the e
 // it leaves, the error norms of the step's test (the
 // sums of k_err_norms as out[1..4]): what the host waits for is one pass over the
-// vectors and one reduction, 12.0 us on the 214k-node box where the two kernels
-// took 10.2 + 11.1 us
+// vectors and one reduction, 15.2 us on the 214k-node box (ncu, cold caches) where
+// the two kernels took 10.2 + 11.1 us
 __global__ void k_newton_update(int N, const double* __restrict__ x, double cj,
                                 const double* __restrict__ ewt, double* __restrict__ y,
                                 double* __restrict__ yp, double* __restrict__ e, int k, PhiPtrs ph, double* partial,

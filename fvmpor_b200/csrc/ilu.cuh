@@ -66,12 +66,12 @@ struct BlockILU {
     // (written by the quotient kernels; allocated at the first use of each)
     DevBuf<double> Jw;
     DevBuf<float> Jw32;
-    DevBuf<int> lu_up;        // [N] lane of each row in the upper slices (blocks not staged)
+    DevBuf<int> lu_up;        // [N] IluPlaces::upper (blocks not staged)
     DevBuf<int> lu_row;       // global row of each factor position (colour order inside the blocks)
     // ILU(0) elimination schedule of the shared-memory factorisation, one
     // contiguous segment per level (upd[seg_ptr[g] .. seg_ptr[g+1]), g the
     // block's first level (IluBlk::seg) plus the level): the offset of the
-    // list of each lane of the level's slices, then per row and per L entry
+    // list of each lane of the level's groups, then per row and per L entry
     // in column order a count word followed by that many (target | source <<
     // 16) window positions
     DevBuf<int> seg_ptr;
@@ -273,8 +273,10 @@ __device__ __forceinline__ int tid_here() {
 // have a form of their own: with their code in every level an apply on the
 // 214k-node box took 12.7 us instead of 12.2): the two sweeps of
 // a 1,447-row block of the 214k-node box took 5.0 us with 4 columns fetched
-// ahead, 5.1 with 8 and more with 12 and 16.  Stored row by row with a row per
-// lane they took 9.2 us.
+// ahead, 5.1 with 8 and more with 12 and 16 (with slices of 32 rows).  Stored row
+// by row with a row per lane they took 9.2 us.  One common bound for a slice's lanes
+// in the loop over the rest, so that they do not part, was slower (30-day run of
+// that box: fused cycle 0.630 ms instead of 0.611).
 constexpr int kIluPre = 4;
 struct IluLane {
     int row, w, at;

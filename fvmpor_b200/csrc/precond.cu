@@ -203,10 +203,10 @@ __host__ __device__ inline int fd_list_offs(int ng) { return (ng + 8) & ~7; }
 // on the 214k-node box (19.4 M FP32 quotients, one B200).  Here they stay in
 // shared memory (column-major over the chunk's elements, so a warp writes
 // consecutive words) and about two chunk sums per non-zero leave the block:
-// 85 us, and 24 us for the sums over chunks.  A block's phases (its nodes, its
-// quotients, its sums, its entries) each wait on memory or on FP64 chains, so
-// what counts is how many blocks share an SM: 192 elements, one per thread,
-// four blocks per SM at 85 registers; 512 elements over 256 threads at two per
+// 88 us, and 33 us for the sums over chunks (ncu, cold caches).  A block's phases
+// (its nodes, its quotients, its sums, its entries) each wait on memory or on
+// FP64 chains, so what counts is how many blocks share an SM: 192 elements, one
+// per thread, four blocks per SM at 80 registers; 512 elements over 256 threads at two per
 // SM took 108 us, 256 over 256 at three 91 us, 128 over 128 at six 92 us.
 // Everything a block reads after its quotients (the list of slots, by a bulk
 // copy; the sums' places) is on its way while they are formed.  The sums are
@@ -1567,7 +1567,7 @@ void psetup_dev(fvm_ctx* c, double cj, double h, const double* y, const double* 
         a.list_max = P->fd_list_max; a.grp_max = P->fd_grp_max; a.part = P->fd_part.p;
         a.coef = c->coef.p; a.xyz = c->xyz.p; a.eK = c->eK.p; a.ezone = c->ezone.p;
         a.y = y; a.g = P->fd_g.p; a.dg = P->fd_dg.p; a.gq = P->fd_gq.p; a.upw = c->upw.p;
-        // one buffer per precision: the slices' padding stays zero in each
+        // one buffer per precision: the groups' padding stays zero in each
         auto window = [&](auto& w) -> void* {
             if (!w.n) {
                 w.alloc(P->nlu);

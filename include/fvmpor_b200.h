@@ -264,9 +264,10 @@ int fvm_set_precond_blocks(fvm_ctx* ctx, int per_sm);
  * so its ILU(0) holds the ILU(0) of its local Schur complement, and each
  * apply runs `iters` block-Jacobi sweeps of the global interface system
  * (local Schur factors plus the couplings between blocks) before the
- * interior back substitution.  Needs every block's staged factor in shared
- * memory (the FP32 factor on the 3D meshes); fvm_psolve reports an error
- * otherwise.  Drops the current factor; the next fvm_psetup rebuilds the
+ * interior back substitution.  Needs every block's factor and forward
+ * result to fit the shared memory, all blocks at once (the FP32 factor on
+ * large 3D blocks; fvm_precond_schur_info tells); fvm_psolve reports an
+ * error otherwise.  Drops the current factor; the next fvm_psetup rebuilds the
  * pattern.  The Krylov paths then use separate kernels per Arnoldi step
  * (no fused cycle). */
 int fvm_set_precond_schur(fvm_ctx* ctx, int iters);
