@@ -26,8 +26,8 @@ namespace fvmb {
 // With slices of 32 rows padded to their longest, and to 32 rows at the end of
 // each level, the window grew by 7 % on the 214k-node box in FP32 and doubled in
 // the Schur order of small blocks (many short levels); in groups of four it is
-// smaller than row by row there (120.3 KB against 124.3 and 131.0), and within
-// 7 % of it in Schur order.
+// smaller than row by row there (120.4 KB against 124.4 and 133.1), and within
+// 5 % of it in Schur order.
 // A row of more than kIluWide entries on one side of the diagonal has a group
 // to itself; its entries past kIluWide follow the strip, one after another.
 // Then come the (inverted) pivots in row order.

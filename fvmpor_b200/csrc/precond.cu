@@ -694,7 +694,7 @@ static const void* schur_kernel(int precision, bool staged) {
 // forward result in shared memory through its grid barriers, and all blocks
 // must be resident at once.  It is offered where the factor's own entries (rows
 // end to end, with row pointers and level lists: `exact` bytes for the largest
-// block) fit beside that.  The window that the sweeps read is padded, by up to 7 %
+// block) fit beside that.  The window that the sweeps read is padded, by up to 5 %
 // on small blocks in this order; where only the padding is too much, the sweeps
 // read the factor in place.
 static void schur_layout(const fvm_ctx* c, BlockILU* P, int pr, size_t exact) {
